@@ -5,12 +5,12 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
-#include <mutex>
 #include <string>
 #include <tuple>
 #include <vector>
 
 #include "glqb_kernels.cuh"
+#include "glqb_fused.cuh"
 #include "glqb_gemm.cuh"
 #include "glqb_launch.h"
 
@@ -65,7 +65,7 @@ struct GlqbPlan {
   int max_batch_gemm = 1;
   size_t ws_bytes = 0;
   int max_batch = 1;
-  int max_bs_in = 32, max_bs_out = 32;
+  bool out_plain_static = false; // every output item takes the plain transform when the output is aligned
   int max_elems_in = 32, max_elems_out = 32;    // floats of shared memory the transform CTAs need
   int sm_count = 0;
   int64_t code_bytes = 0, flops = 0;
@@ -316,39 +316,35 @@ static long long layer_code_bytes(const GlqbLinearDesc& d) {
   return (long long)d.n_stages * d.m_pad * (d.n_pad / 8) * 2;
 }
 
-// one thread per 32-value segment of the largest tile, between 64 and RHT_THREADS
-// ... except for decode-sized plans (at most 8 tokens), whose transforms use all 256 threads per array
-static int rht_threads(int max_elems, int max_batch = 1 << 30) {
-  if (max_batch <= FUSED_MAX_TOKENS) return RHT_THREADS;
-  return std::max(64, std::min(RHT_THREADS, (max_elems / 32 + 31) / 32 * 32));
+// Does rht_out_plain_kernel serve every output item of the plan (rht_out_is_plain, host side)?  The static part is
+// decided once; the alignment of this run's output is not known before.
+static bool out_plain(const GlqbPlan* P, const uint8_t* y_base) {
+  if (!P->out_plain_static) return false;
+  for (const DevLinear& L : P->dev) {
+    const int es = L.y_dtype == GLQB_DT_F32 ? 4 : 2;
+    if (((L.y_off | L.y_stride) & 3) || (reinterpret_cast<uintptr_t>(y_base) & (4 * es - 1))) return false;
+  }
+  return true;
 }
-static int rht_smem(int max_elems) { return (max_elems + max_elems / 32) * 4 + 64; }
 
-static cudaError_t raise_rht_smem_limits() {
-  const int lim = rht_smem(32768);
-  cudaError_t e = cudaFuncSetAttribute(rht_in_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(rht_in_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(rht_in_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(rht_out_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(rht_out_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  return e;
-}
+static int rht_smem(int max_elems) { return fht_words(max_elems) * 4 + 64; }
 
 // one item per (layer, block, tile of tokens); tracks the largest tile (floats) for the launch's smem.
-// Decode-sized layers (at most 8 tokens): a block of 4096 values or more is shared by S = bs / 1024 CTAs, each
-// producing one run of 1024 outputs for all tokens (RhtItem::sub).  `min_log`: only blocks of at least
-// 2^min_log values get items (the single-launch kernel transforms the shorter output blocks itself).
+// A block of more than 8192 values is shared by S = bs / 8192 CTAs per token, each producing one run of 8192 outputs
+// (RhtItem::sub).  `min_log`: only blocks of at least 2^min_log values get items (the single-launch kernel transforms
+// the shorter output blocks itself).
 static void add_rht_items(std::vector<RhtItem>& items, int layer, int nblocks, const int* logs, int batch,
-                          int& max_elems, bool latency, int min_log = 0) {
+                          int& max_elems, int min_log = 0) {
   for (int b = 0; b < nblocks; ++b) {
     if (logs[b] < min_log) continue;
     const int bs = 1 << logs[b];
-    if (latency && batch <= FUSED_MAX_TOKENS && logs[b] >= RHT_SPLIT_MIN_LOG) {
-      for (int k = 0; k < (bs >> RHT_SPLIT_LOG); ++k) items.push_back(RhtItem{layer, b, 0, batch, k});
-      max_elems = std::max(max_elems, 1 << RHT_SPLIT_LOG);
+    if (logs[b] > FHT_LOG) {
+      for (int t = 0; t < batch; ++t)
+        for (int k = 0; k < (bs >> FHT_LOG); ++k) items.push_back(RhtItem{layer, b, t, 1, k});
+      max_elems = std::max(max_elems, 1 << FHT_LOG);
       continue;
     }
-    const int tt = rht_tile_tokens(bs, batch);
+    const int tt = rht_tile_tokens(bs, batch, nblocks);
     for (int t0 = 0; t0 < batch; t0 += tt) {
       const int nt = std::min(tt, batch - t0);
       items.push_back(RhtItem{layer, b, t0, nt, -1});
@@ -425,12 +421,10 @@ static int build_plan(GlqbPlan* P) {
     int off = 0;
     for (int i = 0; i < d.n_blocks_n; ++i) {
       L.bn_off[i] = off; L.bn_log[i] = ilog2(d.blocks_n[i]); off += d.blocks_n[i];
-      P->max_bs_in = std::max(P->max_bs_in, d.blocks_n[i]);
     }
     off = 0;
     for (int i = 0; i < d.n_blocks_m; ++i) {
       L.bm_off[i] = off; L.bm_log[i] = ilog2(d.blocks_m[i]); off += d.blocks_m[i];
-      P->max_bs_out = std::max(P->max_bs_out, d.blocks_m[i]);
     }
     if (d.format == GLQB_FMT_TRELLIS_3INST) {
       L.groups_per_strip = d.n_pad / 32;
@@ -479,13 +473,14 @@ static int build_plan(GlqbPlan* P) {
       // the extra launch); so is a fused RMSNorm whose output block is too long for the in-kernel transform
       static const int in_max_n = [] { const char* e = getenv("GLQB_FUSED_IN_MAX_N"); return e ? atoi(e) : 4096; }();
       bool xr_global = d0.n_pad > in_max_n;
-      // Output blocks of at least 2^out_split_log rows are left to rht_out_kernel (S CTAs share one); shorter
+      for (int i = 0; i < d0.n_blocks_n; ++i) xr_global = xr_global || d0.blocks_n[i] > (1 << FUSED_IN_MAX_LOG);
+      // Output blocks of at least 2^out_split_log rows are left to rht_out_kernel; shorter
       // ones are transformed inside the decode kernel by the CTA that completes them.  Measured on B200 (decoder
       // chain, SmolLM3-3B shapes): an extra launch costs more than the 8192-row transform it takes out of the
       // kernel's tail (101 vs 90 us per layer), so only blocks beyond 8192 rows are split off.
       static const int out_split_log = [] {
         const char* e = getenv("GLQB_FUSED_OUT_SPLIT_LOG");
-        return std::max(RHT_SPLIT_MIN_LOG, std::min(e ? atoi(e) : FUSED_OUT_MAX_LOG + 1, FUSED_OUT_MAX_LOG + 1));
+        return std::max(12, std::min(e ? atoi(e) : FUSED_OUT_MAX_LOG + 1, FUSED_OUT_MAX_LOG + 1));
       }();
       static const int cta_factor = [] { const char* e = getenv("GLQB_FUSED_CTA_FACTOR"); return e ? std::max(1, atoi(e)) : 1; }();
       int scratch = 32;
@@ -706,8 +701,6 @@ static int build_plan(GlqbPlan* P) {
                   "layer %d: the fused norm / activation / residual steps are served by the single-launch decode form only "
                   "(at most %d tokens, all layers of the call reading one input)", P->order[pos], FUSED_MAX_TOKENS);
   }
-  // a call of a few layers is bound by the latency of one transform item, a sweep of many by their throughput
-  const bool latency = n <= FUSED_MAX_LAYERS;
   for (int pos = 0; pos < n; ++pos) {
     DevLinear& L = P->dev[pos];
     const GlqbLinearDesc& d = P->descs[P->order[pos]];
@@ -721,7 +714,7 @@ static int build_plan(GlqbPlan* P) {
         if (first == pos) {
           L.xr_off = (long long)ws;
           ws = align_up(ws + (size_t)L.batch * L.n * sizeof(__half) * XR_TRELLIS_EXPAND, 1024);
-          add_rht_items(P->items_in, pos, L.nbn, L.bn_log, L.batch, P->max_elems_in, latency);
+          add_rht_items(P->items_in, pos, L.nbn, L.bn_log, L.batch, P->max_elems_in);
         } else {
           L.xr_off = P->dev[first].xr_off;
         }
@@ -730,7 +723,7 @@ static int build_plan(GlqbPlan* P) {
       ws = align_up(ws + (size_t)L.slots * L.batch * L.m * sizeof(float), 256);
       L.rstd_off = (long long)ws;
       ws += 256;
-      add_rht_items(P->items_out, pos, L.nbm, L.bm_log, L.batch, P->max_elems_out, latency, L.stop_at_yrht ? 64 : L.out_split_log);
+      add_rht_items(P->items_out, pos, L.nbm, L.bm_log, L.batch, P->max_elems_out, L.stop_at_yrht ? 64 : L.out_split_log);
       continue;
     }
     int same = -1;
@@ -755,13 +748,13 @@ static int build_plan(GlqbPlan* P) {
       if (L.gemm_tn) {
         const size_t n_tiles = (L.batch + L.gemm_tn - 1) / L.gemm_tn, kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
         ws = align_up(ws + n_tiles * kchunks * L.gemm_tn * 128, 256);
-        add_rht_items(P->items_in_gemm, pos, L.nbn, L.bn_log, L.batch, P->max_elems_in, false);
+        add_rht_items(P->items_in_gemm, pos, L.nbn, L.bn_log, L.batch, P->max_elems_in);
       } else {
         // E8 with several tokens interleaves groups of 8 tokens: round the token count up
         const size_t xr_tokens = (L.format == GLQB_FMT_E8_SHELL && L.batch > 1) ? (size_t)((L.batch + 7) / 8 * 8) : (size_t)L.batch;
         ws = align_up(ws + xr_tokens * L.n * sizeof(__half) *
                                (L.format == GLQB_FMT_TRELLIS_3INST ? XR_TRELLIS_EXPAND : 1), 256);
-        add_rht_items(P->items_in, pos, L.nbn, L.bn_log, L.batch, P->max_elems_in, latency);
+        add_rht_items(P->items_in, pos, L.nbn, L.bn_log, L.batch, P->max_elems_in);
       }
     }
     L.part_off = (long long)ws;
@@ -771,9 +764,16 @@ static int build_plan(GlqbPlan* P) {
       L.atile_off = (long long)ws;
       ws += (size_t)((L.m + GM_TILE_M - 1) / GM_TILE_M) * ((L.n + GM_TILE_K - 1) / GM_TILE_K) * GM_A_BYTES;
     }
-    add_rht_items(P->items_out, pos, L.nbm, L.bm_log, L.batch, P->max_elems_out, latency);
+    add_rht_items(P->items_out, pos, L.nbm, L.bm_log, L.batch, P->max_elems_out);
   }
   P->ws_bytes = ws;
+  P->out_plain_static = true;
+  for (const RhtItem& it : P->items_out) {
+    const DevLinear& L = P->dev[it.layer];
+    const int off = L.bm_off[it.block], bs = 1 << L.bm_log[it.block];
+    P->out_plain_static = P->out_plain_static && !L.stop_at_yrht && ((L.m | off) & 3) == 0 && bs >= 4 && L.fixed_slots > 0 &&
+                          it.sub < 0 && !L.row_scale && !L.y_accumulate && !(L.in_norm_w && !L.xr_global) && off + bs <= L.out_f;
+  }
 
   // ---- upload
   CUDA_TRY(cudaMalloc(&P->d_layers, sizeof(DevLinear) * n));
@@ -792,11 +792,6 @@ static int build_plan(GlqbPlan* P) {
   CUDA_TRY(cudaMemset(P->d_tickets, 0, sizeof(int) * std::max(1, P->n_tickets)));
   CUDA_TRY(cudaMalloc(&P->d_items_out, sizeof(RhtItem) * std::max<size_t>(1, P->items_out.size())));
   CUDA_TRY(cudaMemcpy(P->d_items_out, P->items_out.data(), sizeof(RhtItem) * P->items_out.size(), cudaMemcpyHostToDevice));
-
-  // The shared-memory limit is a property of the kernel, not of a plan: every plan sets it to the largest
-  // value any plan can need (one 32768-value Hadamard block), so a later plan never lowers what an earlier
-  // one relies on.
-  CUDA_TRY(raise_rht_smem_limits());
   return GLQB_OK;
 }
 
@@ -872,11 +867,11 @@ int glqb_plan_run(GlqbPlan* P, const void* x_base, void* y_base, void* workspace
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
   if (!P->items_in.empty()) {
-    rht_in_kernel<false><<<(unsigned)P->items_in.size(), rht_threads(P->max_elems_in, P->max_batch), rht_smem(P->max_elems_in), stream>>>(
+    rht_in_kernel<false><<<(unsigned)P->items_in.size(), RHT_THREADS, rht_smem(P->max_elems_in), stream>>>(
         P->d_layers, P->d_items_in, reinterpret_cast<const uint8_t*>(x_base), ws);
   }
   if (!P->items_in_gemm.empty()) {
-    rht_in_gemm_kernel<<<(unsigned)P->items_in_gemm.size(), rht_threads(P->max_elems_in), rht_smem(P->max_elems_in), stream>>>(
+    rht_in_gemm_kernel<<<(unsigned)P->items_in_gemm.size(), RHT_THREADS, rht_smem(P->max_elems_in), stream>>>(
         P->d_layers, P->d_items_in_gemm, reinterpret_cast<const uint8_t*>(x_base), ws);
   }
   if (P->timing) {
@@ -914,7 +909,7 @@ int glqb_plan_run(GlqbPlan* P, const void* x_base, void* y_base, void* workspace
     // kernel's tail (it waits for it before reading anything)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)P->items_out.size());
-    cfg.blockDim = dim3(rht_threads(P->max_elems_out, P->max_batch));
+    cfg.blockDim = dim3(RHT_THREADS);
     cfg.dynamicSmemBytes = rht_smem(P->max_elems_out);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -927,7 +922,8 @@ int glqb_plan_run(GlqbPlan* P, const void* x_base, void* y_base, void* workspace
     const uint8_t* cws = ws;
     uint8_t* yb = reinterpret_cast<uint8_t*>(y_base);
     const float* none = nullptr;
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, rht_out_kernel<false>, dl, di, cws, yb, none));
+    if (out_plain(P, yb)) CUDA_TRY(cudaLaunchKernelEx(&cfg, rht_out_plain_kernel, dl, di, cws, yb));
+    else CUDA_TRY(cudaLaunchKernelEx(&cfg, rht_out_kernel<false>, dl, di, cws, yb, none));
   }
   CUDA_TRY(cudaGetLastError());
   return GLQB_OK;
@@ -1079,11 +1075,12 @@ static int run_rht_single(bool input, const void* src, int src_dtype, int64_t sr
     if (o < 0 || o + b > pad) return fail(GLQB_E_INVALID, "rht: block %d at column %d exceeds %d columns", b, o, pad);
     if (input) { L.bn_off[i] = o; L.bn_log[i] = ilog2(b); } else { L.bm_off[i] = o; L.bm_log[i] = ilog2(b); }
     off += b;
-    const int tt = rht_tile_tokens(b, batch);
+    const int tt = rht_tile_tokens(b, batch, n_blocks);
     S.first_cta[i] = ctas;
     S.tile_tokens[i] = tt;
-    ctas += (batch + tt - 1) / tt;
-    max_elems = std::max(max_elems, tt * b);
+    S.runs[i] = std::max(1, b >> FHT_LOG);
+    ctas += (batch + tt - 1) / tt * S.runs[i];
+    max_elems = std::max(max_elems, std::min(tt * b, 1 << FHT_LOG));
   }
   S.first_cta[n_blocks] = ctas;
   S.n_blocks = n_blocks;
@@ -1097,26 +1094,12 @@ static int run_rht_single(bool input, const void* src, int src_dtype, int64_t sr
     L.m = pad; L.out_f = feat; L.su = reinterpret_cast<const __half*>(signs);
     L.y_dtype = dst_dtype; L.y_stride = dst_stride; L.nbm = n_blocks; L.wscale = 1.f;
   }
-  int dev_id = 0;
-  CUDA_TRY(cudaGetDevice(&dev_id));
-  {
-    // once per device: the two kernels may need more than the default 48 KiB of dynamic shared memory
-    static std::mutex mu;
-    static bool done[64] = {false};
-    std::lock_guard<std::mutex> lock(mu);
-    if (dev_id >= 0 && dev_id < 64 && !done[dev_id]) {
-      const int lim = rht_smem(32768);
-      CUDA_TRY(cudaFuncSetAttribute(rht_in_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-      CUDA_TRY(cudaFuncSetAttribute(rht_out_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-      done[dev_id] = true;
-    }
-  }
   const int smem = rht_smem(max_elems);
   if (input)
-    rht_in_single_kernel<<<(unsigned)ctas, rht_threads(max_elems), smem, stream>>>(
+    rht_in_single_kernel<<<(unsigned)ctas, RHT_THREADS, smem, stream>>>(
         L, S, reinterpret_cast<const uint8_t*>(src), reinterpret_cast<uint8_t*>(dst));
   else
-    rht_out_single_kernel<<<(unsigned)ctas, rht_threads(max_elems), smem, stream>>>(
+    rht_out_single_kernel<<<(unsigned)ctas, RHT_THREADS, smem, stream>>>(
         L, S, reinterpret_cast<uint8_t*>(dst), reinterpret_cast<const float*>(src));
   CUDA_TRY(cudaGetLastError());
   return GLQB_OK;

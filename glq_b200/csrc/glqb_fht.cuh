@@ -50,392 +50,224 @@ __device__ __forceinline__ void fht_smem(float* buf, int logbs) {
   }
 }
 
-// Several rows at once: buf holds `rows` consecutive arrays of 2^logbs floats; each row is transformed
-// independently.  The (row, butterfly group) pairs are spread over all threads, so a CTA that owns a
-// tile of tokens of a small Hadamard block keeps every thread busy.
-template <int R>
-__device__ __forceinline__ void fht_pass_rows(float* buf, int logbs, int done, int rows) {
-  constexpr int N = 1 << R;
-  const int stride = 1 << done;
-  const int glog = logbs - R;                 // log2(groups per row)
-  const int total = rows << glog;
-  for (int o = threadIdx.x; o < total; o += blockDim.x) {
-    const int row = o >> glog;
-    const int oo = o & ((1 << glog) - 1);
-    const int low = oo & (stride - 1);
-    const int high = oo >> done;
-    float* p = buf + ((size_t)row << logbs) + ((high << (done + R)) | low);
-    float v[N];
-#pragma unroll
-    for (int k = 0; k < N; ++k) v[k] = p[k * stride];
-#pragma unroll
-    for (int s = 0; s < R; ++s) {
-#pragma unroll
-      for (int k = 0; k < N; ++k) {
-        if (!(k & (1 << s))) {
-          float a = v[k], b = v[k | (1 << s)];
-          v[k] = a + b;
-          v[k | (1 << s)] = a - b;
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < N; ++k) p[k * stride] = v[k];
-  }
-}
-
-__device__ __forceinline__ void fht_smem_rows(float* buf, int logbs, int rows) {
-  int done = 0;
-  __syncthreads();
-  while (done < logbs) {
-    const int r = min(3, logbs - done);
-    if (r == 3) fht_pass_rows<3>(buf, logbs, done, rows);
-    else if (r == 2) fht_pass_rows<2>(buf, logbs, done, rows);
-    else fht_pass_rows<1>(buf, logbs, done, rows);
-    __syncthreads();
-    done += r;
-  }
-}
-
 }  // namespace glqb
 
 // ---------------------------------------------------------------------------------------------------
-// Tiled transform with radix-32 register passes.
+// Tile transform of the transform kernels, the grouped-expert kernels and the single-launch decode kernels.
 //
-// A tile is `rows` independent arrays of 2^logbs values.  Pass 1 is fused with the load: a thread pulls
-// 32 consecutive values straight from global memory (the caller's `load32`), does butterfly stages 0-4 in
-// registers and parks them in shared memory; the last pass is fused with the store (`store1` receives
-// every finished value).  Arrays of up to 32 values never touch shared memory, up to 1024 values make one
-// round trip, up to 32768 two.  Shared memory is padded by one word per 32 (index i lives at i + i/32), which
-// makes the 32-consecutive accesses of pass 1 and the strided accesses of the later passes conflict-free.
-// Butterfly order is the reference's: ascending distance, lower index gets a+b.
+// A tile is up to 8192 values held by 256 threads, 32 per thread: `total` = rows << logbs values, value e being
+// element e & (bs - 1) of row e >> logbs, each row of bs = 2^logbs (1 .. 8192) values transformed by itself.
+// The 13 bits of e are taken in three register passes:
+//   1  e = k << 10 | warp << 7 | lane << 2 | j     bits 0, 1 and 10 .. 12, straight from the caller's loads
+//   2  e = warp << 10 | (lane >> 2) << 7 | r << 2 | (lane & 3)                    bits 2 .. 6
+//   3  e = warp << 10 | k << 7 | lane << 2 | j                                    bits 7 .. 9, handed to the stores
+// so every global access is four consecutive values per thread and 128 per warp (the earlier form loaded 32
+// consecutive values per thread: 32 half-used sectors per warp instruction), pass 2 -> 3 stays inside a warp and
+// one block barrier remains.  Shared memory is padded by four words per 128 values, which makes the 16-byte
+// accesses of passes 1 and 3 and the stride-4 accesses of pass 2 conflict-free.  Butterflies run on packed fp32
+// pairs (add / fma .f32x2, the same roundings as the scalar forms).  Bound by the latency of a tile (long-scoreboard
+// stalls; issue slots 33 % busy where the earlier form had 51 instructions per value and 50 %).  Measured, warm caches:
+// output transform 2048 x 11008 70 -> 43 us, 21504 columns x 700 tokens of input 57 -> 37 us, one token of 14336 outputs
+// 49 -> 14 us.
 // ---------------------------------------------------------------------------------------------------
 namespace glqb {
 
-__device__ __forceinline__ int fht_pad(int i) { return i + (i >> 5); }
-__host__ __device__ __forceinline__ int fht_tile_words(int logbs, int rows) {
-  const int bs = 1 << logbs;
-  return rows * (bs + (bs >> 5));
+typedef unsigned long long f2;                   // two packed fp32
+__device__ __forceinline__ f2 f2_pack(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+constexpr f2 F2_MINUS1 = 0xBF800000BF800000ull, F2_ONE = 0x3F8000003F800000ull;
+// (a, b) <- (a + b, a - b), both pairs at once; a - b as fma(b, -1, a): one rounding, the same value
+__device__ __forceinline__ void f2_butterfly(f2& a, f2& b) {
+  const f2 s = f2_add(a, b);
+  b = f2_fma(b, F2_MINUS1, a);
+  a = s;
+}
+// the butterfly inside one pair
+__device__ __forceinline__ void f2_cross(f2& v) {
+  float lo, hi;
+  f2_unpack(v, lo, hi);
+  v = f2_pack(lo + hi, lo - hi);
 }
 
-template <int R>
-__device__ __forceinline__ void fht_regs(float (&v)[1 << R]) {
+constexpr int FHT_LOG = 13;                      // largest array of a tile; longer blocks: RhtItem::sub
+constexpr int FHT_THREADS = 256;
+__host__ __device__ __forceinline__ int fht_pos(int e) { return e + ((e >> 7) << 2); }
+__host__ __device__ __forceinline__ int fht_words(int total) { return ((total + 127) >> 7) * 132; }
+
+__device__ __forceinline__ void fht_ld4(const float* p, f2 (&v)[2]) {
+  const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p);
+  v[0] = t.x; v[1] = t.y;
+}
+__device__ __forceinline__ void fht_st4(float* p, const f2 (&v)[2]) { *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v[0], v[1]); }
+
+// Element offset of a thread's k-th group of four from its first one, in a matrix of `stride` elements per row; `step`
+// is 1024 when loading and 128 when storing.  (The bits of k * step and of the first group's index are disjoint, so
+// row and column add up; the offsets are the same for all threads.)
+__device__ __forceinline__ int fht_row(int k, int step, int logbs) { return (k * step) >> logbs; }
+__device__ __forceinline__ int fht_col(int k, int step, int logbs) { return (k * step) & ((1 << logbs) - 1); }
+
+// load(e0, v): v[k] <- values e0 + 1024 k .. + 3 of the tile (zero past `total`); store(e1, v): takes the finished values
+// e1 + 128 k .. + 3 (those below `total`).  `sm`: fht_words(total) floats, 16-byte aligned.  All 256 threads call; a
+// caller that reuses `sm` puts a barrier in between.
+// LOG >= 0: logbs known at compile time (stages behind a runtime test cost a select per value and stage: 2 x the
+// instructions of the whole transform).
+template <int LOG, class Load, class Store>
+__device__ __forceinline__ void fht_block_t(float* sm, int logbs_, int total, Load load, Store store) {
+  const int logbs = LOG >= 0 ? LOG : logbs_;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  f2 v[8][2];
+  const int e0 = (warp << 7) | (lane << 2);
+  load(e0, v);
+  if (logbs > 0) {
 #pragma unroll
-  for (int s = 0; s < R; ++s) {
+    for (int k = 0; k < 8; ++k) { f2_cross(v[k][0]); f2_cross(v[k][1]); }
+  }
+  if (logbs > 1) {
 #pragma unroll
-    for (int k = 0; k < (1 << R); ++k) {
-      if (!(k & (1 << s))) {
-        const float a = v[k], b = v[k | (1 << s)];
-        v[k] = a + b;
-        v[k | (1 << s)] = a - b;
+    for (int k = 0; k < 8; ++k) f2_butterfly(v[k][0], v[k][1]);
+  }
+#pragma unroll
+  for (int s = 0; s < 3; ++s)
+    if (logbs > 10 + s) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (!(k & (1 << s))) { f2_butterfly(v[k][0], v[k | (1 << s)][0]); f2_butterfly(v[k][1], v[k | (1 << s)][1]); }
+    }
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (e0 + (k << 10) < total) fht_st4(sm + fht_pos(e0) + k * (1024 + 32), v[k]);
+  __syncthreads();
+  if ((warp << 10) >= total) return;
+  if (logbs > 2) {
+    float* p = sm + fht_pos((warp << 10) | ((lane >> 2) << 7)) + (lane & 3);
+    if (((warp << 10) | ((lane >> 2) << 7)) < total) {
+      f2 w[16];                                  // pair i = (r = 2 i, 2 i + 1)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) w[i] = f2_pack(p[8 * i], p[8 * i + 4]);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) f2_cross(w[i]);
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+        if (logbs > 3 + s) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (!(i & (1 << s))) f2_butterfly(w[i], w[i | (1 << s)]);
+        }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        float lo, hi;
+        f2_unpack(w[i], lo, hi);
+        p[8 * i] = lo;
+        p[8 * i + 4] = hi;
       }
     }
+    __syncwarp();
+  }
+  const int e1 = (warp << 10) | (lane << 2);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (e1 + (k << 7) < total) fht_ld4(sm + fht_pos(e1) + k * 132, v[k]);
+    else { v[k][0] = 0; v[k][1] = 0; }
+#pragma unroll
+  for (int s = 0; s < 3; ++s)
+    if (logbs > 7 + s) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (!(k & (1 << s))) { f2_butterfly(v[k][0], v[k | (1 << s)][0]); f2_butterfly(v[k][1], v[k | (1 << s)][1]); }
+    }
+  store(e1, v);
+}
+
+template <class Load, class Store>
+__device__ __forceinline__ void fht_block_all(float* sm, int logbs, int total, Load load, Store store) {
+  switch (logbs) {
+    case 13: fht_block_t<13>(sm, logbs, total, load, store); break;
+    case 12: fht_block_t<12>(sm, logbs, total, load, store); break;
+    case 11: fht_block_t<11>(sm, logbs, total, load, store); break;
+    case 10: fht_block_t<10>(sm, logbs, total, load, store); break;
+    case 9: fht_block_t<9>(sm, logbs, total, load, store); break;
+    case 8: fht_block_t<8>(sm, logbs, total, load, store); break;
+    default: fht_block_t<-1>(sm, logbs, total, load, store); break;
   }
 }
 
-// last pass: R remaining stages at distance 2^done; every finished value goes to store1(row, index, value)
-template <int R, class Store1>
-__device__ __forceinline__ void fht_last_pass(const float* smem, int logbs, int done, int rows, int row_words,
-                                              Store1& store1) {
-  const int S = 1 << done;                     // R == logbs - done: one group spans the whole array
-  const int total = rows << done;
-  for (int o = threadIdx.x; o < total; o += blockDim.x) {
-    const int row = o >> done, low = o & (S - 1);
-    const float* p = smem + row * row_words;
-    float v[1 << R];
+// the same with a store(e, q) per group of four and one body for all lengths
+template <class Load, class Store>
+__device__ __forceinline__ void fht_block(float* sm, int logbs, int total, Load load, Store store) {
+  fht_block_t<-1>(sm, logbs, total, load, [&](int e1, const f2 (&v)[8][2]) {
 #pragma unroll
-    for (int k = 0; k < (1 << R); ++k) v[k] = p[fht_pad(low + k * S)];
-    fht_regs<R>(v);
-#pragma unroll
-    for (int k = 0; k < (1 << R); ++k) store1(row, low + k * S, v[k]);
-  }
+    for (int k = 0; k < 8; ++k)
+      if (e1 + (k << 7) < total) store(e1 + (k << 7), v[k]);
+  });
 }
 
-template <class Load32, class Load1, class Store1>
-__device__ __forceinline__ void fht_tile(float* smem, int logbs, int rows, Load32 load32, Load1 load1, Store1 store1) {
-  const int bs = 1 << logbs;
-  if (logbs < 5) {
-    // tiny arrays (E8 layers whose width is not a multiple of 32): one thread per array, all in registers
-    for (int row = threadIdx.x; row < rows; row += blockDim.x) {
-      float v[16];
+// One warp, 1024 values, two register passes and no block barrier: v[k] holds values k << 7 | lane << 2 | j (bits 0, 1
+// and 7 .. 9), the second pass bits 2 .. 6; arrays of 2^logbs <= 1024 values side by side (logbs >= 5).  Blocks longer
+// than 1024 are 1024-value chunks whose remaining bits the consumer of the results combines.  Results: value e at
+// sm[fht_pos(e)] (FHT_CHUNK_WORDS floats), visible to the warp.
+constexpr int FHT_CHUNK_WORDS = 1056;
+template <int LOG>
+__device__ __forceinline__ void fht_warp_t(float* sm, f2 (&v)[8][2], int logbs_) {
+  const int logbs = LOG >= 0 ? LOG : logbs_;
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-      for (int k = 0; k < 16; ++k) v[k] = k < bs ? load1(row, k) : 0.f;
-      for (int h = 1; h < bs; h <<= 1)
+  for (int k = 0; k < 8; ++k) { f2_cross(v[k][0]); f2_cross(v[k][1]); f2_butterfly(v[k][0], v[k][1]); }
 #pragma unroll
-        for (int k = 0; k < 16; ++k)
-          if (!(k & h) && (k | h) < bs) { const float a = v[k], b = v[k | h]; v[k] = a + b; v[k | h] = a - b; }
+  for (int s = 0; s < 3; ++s)
+    if (logbs > 7 + s) {
 #pragma unroll
-      for (int k = 0; k < 16; ++k) if (k < bs) store1(row, k, v[k]);
+      for (int k = 0; k < 8; ++k)
+        if (!(k & (1 << s))) { f2_butterfly(v[k][0], v[k | (1 << s)][0]); f2_butterfly(v[k][1], v[k | (1 << s)][1]); }
     }
-    return;
-  }
-  const int row_words = bs + (bs >> 5);
-  const int slog = logbs - 5;                  // log2(32-value segments per array)
-  const int nseg = rows << slog;
-  for (int s = threadIdx.x; s < nseg; s += blockDim.x) {
-    const int row = s >> slog, i0 = (s & ((1 << slog) - 1)) << 5;
-    float v[32];
-    load32(row, i0, v);
-    fht_regs<5>(v);
-    if (logbs == 5) {
 #pragma unroll
-      for (int k = 0; k < 32; ++k) store1(row, k, v[k]);
-    } else {
-      float* p = smem + row * row_words + fht_pad(i0);
+  for (int k = 0; k < 8; ++k) fht_st4(sm + (lane << 2) + k * 132, v[k]);
+  __syncwarp();
+  float* p = sm + (lane >> 2) * 132 + (lane & 3);
+  f2 w[16];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) p[k] = v[k];
+  for (int i = 0; i < 16; ++i) w[i] = f2_pack(p[8 * i], p[8 * i + 4]);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) f2_cross(w[i]);
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+    if (s < 2 || logbs > 3 + s) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (!(i & (1 << s))) f2_butterfly(w[i], w[i | (1 << s)]);
     }
-  }
-  if (logbs == 5) return;
-  __syncthreads();
-  int done = 5;
-  if (logbs > 10) {
-    // middle pass: stages 5..9 (distance 32..512), in place
-    const int total = rows << slog;
-    for (int o = threadIdx.x; o < total; o += blockDim.x) {
-      const int row = o >> slog, oo = o & ((1 << slog) - 1);
-      const int low = oo & 31, high = oo >> 5;
-      float* p = smem + row * row_words;
-      const int base = (high << 10) | low;
-      float v[32];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) v[k] = p[fht_pad(base + (k << 5))];
-      fht_regs<5>(v);
-#pragma unroll
-      for (int k = 0; k < 32; ++k) p[fht_pad(base + (k << 5))] = v[k];
-    }
-    __syncthreads();
-    done = 10;
+  for (int i = 0; i < 16; ++i) {
+    float lo, hi;
+    f2_unpack(w[i], lo, hi);
+    p[8 * i] = lo;
+    p[8 * i + 4] = hi;
   }
-  switch (logbs - done) {
-    case 1: fht_last_pass<1>(smem, logbs, done, rows, row_words, store1); break;
-    case 2: fht_last_pass<2>(smem, logbs, done, rows, row_words, store1); break;
-    case 3: fht_last_pass<3>(smem, logbs, done, rows, row_words, store1); break;
-    case 4: fht_last_pass<4>(smem, logbs, done, rows, row_words, store1); break;
-    default: fht_last_pass<5>(smem, logbs, done, rows, row_words, store1); break;
-  }
+  __syncwarp();
 }
-
-// ---------------------------------------------------------------------------------------------------
-// Same transform with vector output: after the last butterfly pass the finished values go back to shared
-// memory and every thread hands 8 consecutive values of one array to `store8(row, i0, v, count)` (count < 8
-// only for arrays shorter than 8), so the caller can scale, convert and store them with one 16-byte access.
-// The stages after the first five are split evenly over one or two strided in-place passes
-// (2048 values: 5 + 3 + 3, 8192: 5 + 4 + 4), which keeps every pass at 8 or more values per thread.
-// ---------------------------------------------------------------------------------------------------
-template <int R>
-__device__ __forceinline__ void fht_strided_pass(float* smem, int logbs, int done, int rows, int row_words) {
-  const int S = 1 << done;
-  const int glog = logbs - R;
-  const int total = rows << glog;
-  for (int o = threadIdx.x; o < total; o += blockDim.x) {
-    const int row = o >> glog, oo = o & ((1 << glog) - 1);
-    const int low = oo & (S - 1), high = oo >> done;
-    float* p = smem + row * row_words + fht_pad(((high << (done + R)) | low));
-    const int step = S + (S >> 5);             // S is a multiple of 32: the padding grows linearly with k
-    float v[1 << R];
-#pragma unroll
-    for (int k = 0; k < (1 << R); ++k) v[k] = p[k * step];
-    fht_regs<R>(v);
-#pragma unroll
-    for (int k = 0; k < (1 << R); ++k) p[k * step] = v[k];
-  }
+__device__ __forceinline__ void fht_warp(float* sm, f2 (&v)[8][2], int logbs) {
+  if (logbs >= 10) fht_warp_t<10>(sm, v, logbs);
+  else if (logbs == 9) fht_warp_t<9>(sm, v, logbs);
+  else if (logbs == 8) fht_warp_t<8>(sm, v, logbs);
+  else fht_warp_t<-1>(sm, v, logbs);
 }
-
-__device__ __forceinline__ void fht_strided_dispatch(float* smem, int logbs, int done, int r, int rows, int row_words) {
-  switch (r) {
-    case 1: fht_strided_pass<1>(smem, logbs, done, rows, row_words); break;
-    case 2: fht_strided_pass<2>(smem, logbs, done, rows, row_words); break;
-    case 3: fht_strided_pass<3>(smem, logbs, done, rows, row_words); break;
-    case 4: fht_strided_pass<4>(smem, logbs, done, rows, row_words); break;
-    default: fht_strided_pass<5>(smem, logbs, done, rows, row_words); break;
-  }
-}
-
-// The passes alone, for arrays of 32 values or more: on return (after a __syncthreads) value i of array `row`
-// sits at smem[row * (bs + bs / 32) + fht_pad(i)].
-template <class Load32>
-__device__ __forceinline__ void fht_tile_core(float* smem, int logbs, int rows, Load32 load32) {
-  const int bs = 1 << logbs;
-  const int row_words = bs + (bs >> 5);
-  const int slog = logbs - 5;
-  const int nseg = rows << slog;
-  for (int s = threadIdx.x; s < nseg; s += blockDim.x) {
-    const int row = s >> slog, i0 = (s & ((1 << slog) - 1)) << 5;
-    float v[32];
-    load32(row, i0, v);
-    fht_regs<5>(v);
-    float* p = smem + row * row_words + fht_pad(i0);
-#pragma unroll
-    for (int k = 0; k < 32; ++k) p[k] = v[k];
-  }
-  __syncthreads();
-  const int rem = logbs - 5;
-  if (rem > 0) {
-    const int r1 = rem <= 5 ? rem : (rem + 1) >> 1;
-    fht_strided_dispatch(smem, logbs, 5, r1, rows, row_words);
-    __syncthreads();
-    if (rem > r1) {
-      fht_strided_dispatch(smem, logbs, 5 + r1, rem - r1, rows, row_words);
-      __syncthreads();
-    }
-  }
-}
-
-template <class Load32, class Load1, class Store8>
-__device__ __forceinline__ void fht_tile8(float* smem, int logbs, int rows, Load32 load32, Load1 load1, Store8 store8) {
-  const int bs = 1 << logbs;
-  if (logbs < 5) {
-    for (int row = threadIdx.x; row < rows; row += blockDim.x) {
-      float v[16];
-#pragma unroll
-      for (int k = 0; k < 16; ++k) v[k] = k < bs ? load1(row, k) : 0.f;
-      for (int h = 1; h < bs; h <<= 1)
-#pragma unroll
-        for (int k = 0; k < 16; ++k)
-          if (!(k & h) && (k | h) < bs) { const float a = v[k], b = v[k | h]; v[k] = a + b; v[k | h] = a - b; }
-      const float lo[8] = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]};
-      const float hi[8] = {v[8], v[9], v[10], v[11], v[12], v[13], v[14], v[15]};
-      store8(row, 0, lo, bs < 8 ? bs : 8);
-      if (bs > 8) store8(row, 8, hi, bs - 8);
-    }
-    return;
-  }
-  const int row_words = bs + (bs >> 5);
-  fht_tile_core(smem, logbs, rows, load32);
-  const int plog = logbs - 3;                  // log2(8-value pieces per array)
-  const int total = rows << plog;
-  for (int o = threadIdx.x; o < total; o += blockDim.x) {
-    const int row = o >> plog, i0 = (o & ((1 << plog) - 1)) << 3;
-    const float* p = smem + row * row_words + fht_pad(i0);
-    float v[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = p[k];
-    store8(row, i0, v, 8);
-  }
-}
-
-// ---------------------------------------------------------------------------------------------------
-// Low-latency transform of ONE array of 32 .. 8192 values by a 256-thread CTA, for the single-launch decode
-// kernel where the transform sits on the critical path of a few-microsecond kernel: one round of global
-// loads, one shared-memory exchange, one __syncthreads.
-//   thread t holds E = max(1, bs / 256) consecutive values (index t * E + j): stages 0 .. log2(E) - 1 run in
-//   registers, the next five across the lanes of a warp with shuffles, the last log2(W) (W = warps holding the
-//   array, at most 8) after an exchange through shared memory, where a thread gathers the W values that differ
-//   in the warp bits, finishes the butterflies and hands every finished value to `store(i, value)`; for a fixed
-//   call of `store` the lanes of a warp hold consecutive i.
-// Same butterflies in the same (ascending) order as fht_tile, so the results are bit-identical to it.
-// `smem` needs bs + bs / 32 floats.  All 256 threads must call; `load(i0, v)` fills v[0..E) with values
-// i0 .. i0 + E - 1.
-// ---------------------------------------------------------------------------------------------------
-template <int E, class Load, class Pre, class Store>
-__device__ __forceinline__ void fht_fast_e(float* smem, int logbs, Load& load, Pre& pre, Store& store) {
-  constexpr int LOGE = E == 1 ? 0 : E == 2 ? 1 : E == 4 ? 2 : E == 8 ? 3 : E == 16 ? 4 : 5;
-  constexpr int QMAX = E >= 8 ? E / 8 : 1;         // rounds of the final loop (values per warp / 256)
-  const int bs = 1 << logbs;
-  const int t = threadIdx.x, lane = t & 31;
-  const int nthreads = bs >> LOGE;                 // threads that hold values (32 .. 256)
-  const int W = nthreads >> 5;                     // warps that hold values (1 .. 8)
-  const bool active = t < nthreads;
-  const int span = 32 << LOGE;                     // values per warp = distance between the W partners
-  // What `store` needs besides the transformed value (a sign, the old output, ...) is requested first by
-  // `pre(i)`, for exactly the indices this thread will store, so that it arrives while the transform runs.
-  float aux[QMAX][8];
-  if (W == 1) {
-    if (active) {
-#pragma unroll
-      for (int j = 0; j < E; ++j) aux[0][j] = pre(t * E + j);        // E <= 1 here (32 values, one warp)
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < QMAX; ++q) {
-      const int r = t + 256 * q;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) aux[q][w] = (r < span && w < W) ? pre(w * span + r) : 0.f;
-    }
-  }
-  float v[E];
-  if (active) {
-    load(t * E, v);
-    fht_regs<LOGE>(v);
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      const bool upper = (lane >> k) & 1;
-#pragma unroll
-      for (int j = 0; j < E; ++j) {
-        const float p = __shfl_xor_sync(0xffffffffu, v[j], 1 << k);
-        v[j] = upper ? (p - v[j]) : (v[j] + p);    // lower index: a + b, upper index: a - b (a = lower element)
-      }
-    }
-  }
-  if (W == 1) {
-    if (active) {
-#pragma unroll
-      for (int j = 0; j < E; ++j) store(t * E + j, v[j], aux[0][j]);
-    }
-    return;
-  }
-  if (active) {
-#pragma unroll
-    for (int j = 0; j < E; ++j) smem[fht_pad(t * E + j)] = v[j];
-  }
-  __syncthreads();
-  const int logw = W == 2 ? 1 : W == 4 ? 2 : 3;
-#pragma unroll
-  for (int q = 0; q < QMAX; ++q) {
-    const int r = t + 256 * q;
-    if (r < span) {
-      float u[8];
-#pragma unroll
-      for (int w = 0; w < 8; ++w) u[w] = w < W ? smem[fht_pad(w * span + r)] : 0.f;
-      if (logw == 1) {
-        const float a = u[0], b = u[1];
-        u[0] = a + b; u[1] = a - b;
-      } else if (logw == 2) {
-        float h[4] = {u[0], u[1], u[2], u[3]};
-        fht_regs<2>(h);
-        u[0] = h[0]; u[1] = h[1]; u[2] = h[2]; u[3] = h[3];
-      } else {
-        fht_regs<3>(u);
-      }
-#pragma unroll
-      for (int w = 0; w < 8; ++w)
-        if (w < W) store(w * span + r, u[w], aux[q][w]);
-    }
-  }
-}
-
-// dispatch on the array length (2^logbs, 32 .. 8192)
-template <int MAXLOG = 13, class Load1, class Load4, class Pre, class Store>
-__device__ __forceinline__ void fht_fast(float* smem, int logbs, Load1 load1, Load4 load4, Pre pre, Store store) {
-  // load1(i) -> value i;  load4(i0, float (&q)[4]) -> values i0 .. i0 + 3 (i0 a multiple of 4);
-  // pre(i) -> float handed back to store(i, value, that float)
-  auto ld1 = [&](int i0, float (&v)[1]) { v[0] = load1(i0); };
-  auto ld2 = [&](int i0, float (&v)[2]) { v[0] = load1(i0); v[1] = load1(i0 + 1); };
-  auto ld4 = [&](int i0, float (&v)[4]) { load4(i0, v); };
-  auto ld8 = [&](int i0, float (&v)[8]) {
-    float q[4];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) { load4(i0 + 4 * k, q); v[4 * k] = q[0]; v[4 * k + 1] = q[1]; v[4 * k + 2] = q[2]; v[4 * k + 3] = q[3]; }
-  };
-  auto ld16 = [&](int i0, float (&v)[16]) {
-    float q[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) { load4(i0 + 4 * k, q); v[4 * k] = q[0]; v[4 * k + 1] = q[1]; v[4 * k + 2] = q[2]; v[4 * k + 3] = q[3]; }
-  };
-  auto ld32 = [&](int i0, float (&v)[32]) {
-    float q[4];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { load4(i0 + 4 * k, q); v[4 * k] = q[0]; v[4 * k + 1] = q[1]; v[4 * k + 2] = q[2]; v[4 * k + 3] = q[3]; }
-  };
-  // arrays longer than 2^MAXLOG never reach this instantiation (their cases are not compiled)
-  if (logbs == 9) { fht_fast_e<2>(smem, logbs, ld2, pre, store); return; }
-  if (logbs == 10) { fht_fast_e<4>(smem, logbs, ld4, pre, store); return; }
-  if constexpr (MAXLOG >= 11) if (logbs == 11) { fht_fast_e<8>(smem, logbs, ld8, pre, store); return; }
-  if constexpr (MAXLOG >= 12) if (logbs == 12) { fht_fast_e<16>(smem, logbs, ld16, pre, store); return; }
-  if constexpr (MAXLOG >= 13) if (logbs == 13) { fht_fast_e<32>(smem, logbs, ld32, pre, store); return; }
-  fht_fast_e<1>(smem, logbs, ld1, pre, store);                        // 32 .. 256 values
-}
-constexpr int FHT_FAST_MAX_LOG = 13;
 
 }  // namespace glqb

@@ -1,6 +1,6 @@
 // Instantiations and launches of the single-launch decode kernels (trellis_fused_kernel, e8_fused_kernel,
-// glqb_kernels.cuh).
-#include "glqb_kernels.cuh"
+// glqb_fused.cuh).
+#include "glqb_fused.cuh"
 #include <cstdlib>
 #include <cstring>
 

@@ -15,7 +15,7 @@
 // Stages hand over through mbarriers.  Every wait is bounded: on expiry the kernel records a status
 // word, stops issuing work, frees its TMEM columns and returns.
 #pragma once
-#include "glqb_kernels.cuh"
+#include "glqb_rht.cuh"
 
 namespace glqb {
 
@@ -140,28 +140,24 @@ __device__ __forceinline__ uint32_t sw128_offset(int r, int e) {
 // One CTA per (layer, Hadamard block, tile of tokens); tiles ordered [n_tile][k_chunk], each TN*128
 // bytes.  Columns past n (the last chunk of a layer whose n is not a multiple of 64) are written as
 // zeros by the CTAs of the last block.
-static __global__ void __launch_bounds__(RHT_THREADS, GLQB_RHT_MINB) rht_in_gemm_kernel(const DevLinear* __restrict__ layers,
+static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_gemm_kernel(const DevLinear* __restrict__ layers,
                                                                   const RhtItem* __restrict__ items,
                                                                   const uint8_t* __restrict__ x_base,
                                                                   uint8_t* __restrict__ ws) {
-  extern __shared__ float fbuf[];
+  extern __shared__ __align__(16) float fbuf[];
   const RhtItem it = items[blockIdx.x];
   const DevLinear& L = layers[it.layer];
-  const int tn = L.gemm_tn;
+  const int tn = L.gemm_tn, tn_log = tn == 128 ? 7 : 8;
   const int off = L.bn_off[it.block];
   const int logbs = L.bn_log[it.block];
   const int bs = 1 << logbs;
   const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
-  const bool vec_ok = (off & 3) == 0 && act_rows_aligned4(x_base, L.x_off, L.x_stride, L.x_dtype);
   const float rs = L.x_is_rotated ? 1.0f : rsqrtf((float)bs);
-  auto store1 = [&](int row, int i, float val) {
-    const int token = it.tok0 + row;
-    const int nt = token / tn, r = token - nt * tn;
-    const int col = off + i;
-    const int kc = col >> 6, e = col & 63;
-    *reinterpret_cast<__half*>(ws + L.xr_off + ((size_t)nt * kchunks + kc) * tn * 128 + sw128_offset(r, e)) =
-        __float2half_rn(val * rs);
+  uint8_t* xr = ws + L.xr_off;
+  auto place = [&](int token, int col) -> uint8_t* {
+    return xr + (((size_t)(token >> tn_log) * kchunks + (col >> 6)) << (tn_log + 7)) + sw128_offset(token & (tn - 1), col & 63);
   };
+  auto store1 = [&](int row, int i, float v) { *reinterpret_cast<__half*>(place(it.tok0 + row, off + i)) = __float2half_rn(v); };
   auto load1 = [&](int row, int i) -> float {
     const int col = off + i;
     if (col >= L.in_f) return 0.f;
@@ -169,39 +165,58 @@ static __global__ void __launch_bounds__(RHT_THREADS, GLQB_RHT_MINB) rht_in_gemm
     if (!L.x_is_rotated) v *= __half2float(L.sv[col]);
     return v;
   };
+  const int S = it.sub >= 0 ? bs >> FHT_LOG : 1, log_t = min(logbs, FHT_LOG), run0 = max(it.sub, 0) << FHT_LOG;
+  const int total = it.ntok << log_t;
   if (L.x_is_rotated) {
-    const int total = it.ntok << logbs;
-    for (int o = threadIdx.x; o < total; o += blockDim.x) store1(o >> logbs, o & (bs - 1), load1(o >> logbs, o & (bs - 1)));
+    for (int o = threadIdx.x; o < total; o += blockDim.x) {
+      const int row = o >> log_t, i = run0 + (o & ((1 << log_t) - 1));
+      store1(row, i, load1(row, i));
+    }
   } else {
-    auto load32 = [&](int row, int i0, float (&v)[32]) { rht_load_x32(L, x_base, it.tok0 + row, off + i0, vec_ok, v); };
-    uint8_t* xr = ws + L.xr_off;
-    const int tok0 = it.tok0;
-    // 8 consecutive columns are one 16-byte unit of a swizzled 128-byte row
-    auto store8 = [&](int row, int i0, const float (&v)[8], int count) {
-      const int col0 = off + i0;
-      if (count == 8 && (col0 & 7) == 0) {
-        const int token = tok0 + row;
-        const int nt = token / tn, r = token - nt * tn;
-        const __half2 a = __floats2half2_rn(v[0] * rs, v[1] * rs), b = __floats2half2_rn(v[2] * rs, v[3] * rs);
-        const __half2 c = __floats2half2_rn(v[4] * rs, v[5] * rs), d = __floats2half2_rn(v[6] * rs, v[7] * rs);
-        *reinterpret_cast<uint4*>(xr + ((size_t)nt * kchunks + (col0 >> 6)) * tn * 128 + sw128_offset(r, col0 & 63)) =
-            make_uint4(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b),
-                       *reinterpret_cast<const uint32_t*>(&c), *reinterpret_cast<const uint32_t*>(&d));
-      } else {
-        for (int k = 0; k < count; ++k) store1(row, i0 + k, v[k]);
-      }
-    };
-    fht_tile8(fbuf, logbs, it.ntok, load32, load1, store8);
+    const bool vec = (off & 3) == 0 && log_t >= 2 && act_rows_aligned4(x_base, L.x_off, L.x_stride, L.x_dtype);
+    if (vec && off + bs <= L.in_f && logbs >= 10) {
+      // whole blocks of 1024 columns and more: a warp's stores stay in one token, two 64-column chunks apart each
+      auto load_plain = [&](int e0, f2 (&v)[8][2]) { rht_load_x_plain(L, it, x_base, off, log_t, total, S, e0, v); };
+      auto store_plain = [&](int e1, const f2 (&v)[8][2]) {
+        const f2 rs2 = f2_pack(rs, rs);
+        uint8_t* p = place(it.tok0 + (e1 >> log_t), off + run0 + (e1 & ((1 << log_t) - 1)));
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (e1 + (k << 7) < total) {
+            float r[4];
+            f2_unpack(f2_mul(v[k][0], rs2), r[0], r[1]);
+            f2_unpack(f2_mul(v[k][1], rs2), r[2], r[3]);
+            const __half2 a = __floats2half2_rn(r[0], r[1]), b = __floats2half2_rn(r[2], r[3]);
+            *reinterpret_cast<uint2*>(p + ((size_t)k << (tn_log + 8))) =
+                make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+          }
+      };
+      fht_block_all(fbuf, log_t, total, load_plain, store_plain);
+    } else {
+      auto load = [&](int e0, f2 (&v)[8][2]) { rht_load_x(L, it, x_base, off, log_t, total, S, vec, load1, e0, v); };
+      const bool out_vec = (off & 3) == 0 && log_t >= 2;
+      auto store = [&](int e, const f2 (&q)[2]) {
+        float r[4];
+        f2_unpack(q[0], r[0], r[1]);
+        f2_unpack(q[1], r[2], r[3]);
+        if (out_vec) {         // four columns are 8 bytes of a swizzled 128-byte row, a warp writes 256 bytes
+          const __half2 a = __floats2half2_rn(r[0] * rs, r[1] * rs), b = __floats2half2_rn(r[2] * rs, r[3] * rs);
+          *reinterpret_cast<uint2*>(place(it.tok0 + (e >> log_t), off + run0 + (e & ((1 << log_t) - 1)))) =
+              make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        } else {
+  #pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (e + j < total) store1((e + j) >> log_t, run0 + ((e + j) & ((1 << log_t) - 1)), r[j] * rs);
+        }
+      };
+      fht_block(fbuf, log_t, total, load, store);
+    }
   }
-  if (it.block == L.nbn - 1) {
+  if (it.block == L.nbn - 1 && it.sub <= 0) {
     const int padc = kchunks * GM_TILE_K - L.n;
     for (int o = threadIdx.x; o < it.ntok * padc; o += blockDim.x) {
-      const int tk = o / padc, col = L.n + (o - tk * padc);
-      const int token = it.tok0 + tk;
-      const int nt = token / tn, r = token - nt * tn;
-      const int kc = col >> 6, e = col & 63;
-      *reinterpret_cast<__half*>(ws + L.xr_off + ((size_t)nt * kchunks + kc) * tn * 128 + sw128_offset(r, e)) =
-          __float2half_rn(0.f);
+      const int tk = o / padc;
+      *reinterpret_cast<__half*>(place(it.tok0 + tk, L.n + (o - tk * padc))) = __float2half_rn(0.f);
     }
   }
 }

@@ -58,20 +58,20 @@ struct RhtItem {
   int block;
   int tok0;    // first token of the tile this CTA transforms
   int ntok;    // tokens in the tile (the CTA's shared memory holds ntok * block floats)
-  int sub;     // -1: the whole block.  k >= 0 (decode-sized plans, blocks of 4096 values or more): the CTA produces
-               // the k-th run of 1024 outputs only, as H_1024( sum_k' H_S[k][k'] * input run k' ) — H_(S*1024) =
-               // H_S (x) H_1024 with the short factor applied first, so S CTAs share a long block without talking
+  int sub;     // -1: the whole block.  k >= 0 (blocks of more than 8192 values, one token): the CTA produces the k-th
+               // run of 8192 outputs, as H_8192( sum_k' H_S[k][k'] * input run k' ) — H_(S*8192) = H_S (x) H_8192 with
+               // the short factor applied while loading, so S CTAs share a long block without talking
 };
 
-#ifndef GLQB_RHT_TILE
-#define GLQB_RHT_TILE 8192
-#endif
-// tokens per CTA of the transform kernels: about GLQB_RHT_TILE floats of shared memory per CTA
-static inline int rht_tile_tokens(int block_size, int batch) {
-  int t = GLQB_RHT_TILE / block_size;
+// Tokens per CTA of the transform kernels: a tile of 8192 values (fht_block), less when that would leave SMs without
+// work (`ctas` is what the launch has besides, at one token per CTA and block).
+static inline int rht_tile_tokens(int block_size, int batch, int blocks) {
+  int t = 8192 / block_size;
   if (t < 1) t = 1;
   if (t > 64) t = 64;
-  return t < batch ? t : batch;
+  if (t > batch) t = batch;
+  while (t > 1 && (long long)blocks * ((batch + t - 1) / t) < 148) t = (t + 1) / 2;
+  return t;
 }
 
 // Stores the message glqb_last_error() returns for the calling thread (defined in glqb_api.cu).

@@ -75,8 +75,9 @@ constexpr int MOE_B_BYTES = MOE_TN * 128;      // one 64-column chunk of a token
 __device__ __forceinline__ float moe_act(float g, int act) {
   if (act == GLQB_ACT_SILU || act == 3) return g / (1.0f + __expf(-g));
   if (act == GLQB_ACT_GELU_TANH) {
+    // (1 + tanh(u)) / 2 = 1 / (1 + exp(-2u)): no cancellation for negative u, and a third of tanhf's instructions
     const float u = 0.7978845608028654f * (g + 0.044715f * g * g * g);
-    return 0.5f * g * (1.0f + tanhf(u));
+    return __fdividef(g, 1.0f + __expf(-2.0f * u));
   }
   if (act == 4) return 0.5f * g * (1.0f + erff(g * 0.7071067811865476f));     // gelu (exact), not gated
   const float r = fmaxf(g, 0.f);                                                 // relu^2 (codes 2 and 5)
@@ -292,61 +293,135 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
   }
 }
 
+// Columns c .. c + 3 (c % 4 == 0) of a token's activations in the streaming kernels' fragment order.
+__device__ __forceinline__ void moe_store_xr4(__half2* row, int c, const f2 (&q)[2]) {
+  float r[4];
+  f2_unpack(q[0], r[0], r[1]);
+  f2_unpack(q[1], r[2], r[3]);
+  // (xr_pos_trellis: columns c, c + 1 share a lane's 16 halfs, c + 2 and c + 3 sit 16 halfs on)
+  __half2* p = row + (((c & ~31) * XR_TRELLIS_EXPAND + xr_pos_trellis(c & 31)) >> 1);
+  const __half z = __float2half_rn(0.f);
+  p[0] = __halves2half2(__float2half_rn(r[0]), z);
+  p[2] = __halves2half2(__float2half_rn(r[1]), z);
+  p[8] = __halves2half2(__float2half_rn(r[2]), z);
+  p[10] = __halves2half2(__float2half_rn(r[3]), z);
+}
+
 // ---- 2: input transform per token (w13 side) -----------------------------------------------------------
-__global__ void __launch_bounds__(1024) moe_rht_in_kernel(const __grid_constant__ MoeDev M, const uint8_t* __restrict__ x,
-                                                          uint8_t* __restrict__ ws) {
-  extern __shared__ float fb[];
-  const int t = blockIdx.x;
-  for (int i = threadIdx.x; i < M.hidden; i += blockDim.x)
-    fb[i] = load_act(x, (long long)t * M.hidden + i, M.x_dtype) * __half2float(M.w13_sv[i]);
-  for (int b = 0; b < M.nb_n13; ++b) fht_smem(fb + M.off_n13[b], M.log_n13[b]);
-  __half2* out = reinterpret_cast<__half2*>(ws + M.o_xr1) + (long long)t * M.hidden;
+constexpr int MOE_XF_THREADS = FHT_THREADS;
+// One CTA takes `tt` consecutive tokens; store(t, c, logbs, n, v) gets a thread's finished groups of four: group k < n holds
+// columns c + fht_col(k, 128, logbs) .. + 3 of token t + fht_row(k, 128, logbs).
+template <class Store>
+__device__ __forceinline__ void moe_rht_in_body(const MoeDev& M, int T, int tt, const uint8_t* __restrict__ x, float* fb, Store store) {
+  const int t0 = blockIdx.x * tt, nt = min(tt, T - t0);
+  const bool vec = act_rows_aligned4(x, 0, M.hidden, M.x_dtype);
+  const int hidden = M.hidden;
   for (int b = 0; b < M.nb_n13; ++b) {
-    const float rs = rsqrtf((float)(1 << M.log_n13[b]));
-    for (int i = threadIdx.x; i < (1 << M.log_n13[b]); i += blockDim.x) {
-      const int col = M.off_n13[b] + i;
-      const int pos = (col & ~31) * XR_TRELLIS_EXPAND + xr_pos_trellis(col & 31);
-      out[pos >> 1] = __halves2half2(__float2half_rn(fb[col] * rs), __float2half_rn(0.f));
+    const int logbs = M.log_n13[b], off = M.off_n13[b], mask = (1 << logbs) - 1;
+    const float rs = rsqrtf((float)(1 << logbs));
+    const f2 rs2 = f2_pack(rs, rs);
+    const int step = min(nt, 8192 >> logbs);               // tokens per tile
+    for (int r0 = 0; r0 < nt; r0 += step) {
+      const int total = min(step, nt - r0) << logbs;
+      auto load = [&](int e0, f2 (&v)[8][2]) {
+        const int i0 = off + (e0 & mask);
+        const long long o0 = (long long)(t0 + r0 + (e0 >> logbs)) * hidden + i0;
+        const __half* sv = M.w13_sv + i0;
+        with_dtype(M.x_dtype, [&](auto dt) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            v[k][0] = v[k][1] = 0;
+            if (e0 + (k << 10) < total) {
+              const long long o = o0 + fht_row(k, 1024, logbs) * hidden + fht_col(k, 1024, logbs);
+              float q[4];
+              if (vec) load_act4(x, o, decltype(dt)::value, q);
+              else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) q[j] = load_act(x, o + j, decltype(dt)::value);
+              }
+              f2 s[2];
+              load_sign4(sv + fht_col(k, 1024, logbs), s);
+              v[k][0] = f2_mul(f2_pack(q[0], q[1]), s[0]);
+              v[k][1] = f2_mul(f2_pack(q[2], q[3]), s[1]);
+            }
+          }
+        });
+      };
+      auto store_all = [&](int e1, const f2 (&v)[8][2]) {
+        f2 r[8][2];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { r[k][0] = f2_mul(v[k][0], rs2); r[k][1] = f2_mul(v[k][1], rs2); }
+        if (e1 < total) store(t0 + r0 + (e1 >> logbs), off + (e1 & mask), logbs, min(8, (total - e1 + 127) >> 7), r);
+      };
+      fht_block_all(fb, logbs, total, load, store_all);
+      __syncthreads();
     }
   }
 }
 
-// 16 bytes (8 consecutive columns starting at col8 * 8) of padded row `trow` in a [tile][chunk] x (128 x 64) image
-__device__ __forceinline__ void moe_store_tile16(uint8_t* base, int trow, int kchunks, int col8, uint4 v) {
-  const int tile = trow / MOE_TN, r = trow % MOE_TN;
-  const int kc = col8 >> 3, e0 = (col8 & 7) * 8;
-  *reinterpret_cast<uint4*>(base + ((size_t)tile * kchunks + kc) * MOE_B_BYTES + sw128_offset(r, e0)) = v;
+__global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_rht_in_kernel(const __grid_constant__ MoeDev M, int T, int tt,
+                                                                       const uint8_t* __restrict__ x, uint8_t* __restrict__ ws) {
+  extern __shared__ __align__(16) float fb[];
+  const int hidden = M.hidden;
+  __half2* xr = reinterpret_cast<__half2*>(ws + M.o_xr1);
+  moe_rht_in_body(M, T, tt, x, fb, [&](int t, int c, int logbs, int n, const f2 (&v)[8][2]) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k < n) moe_store_xr4(xr + (long long)(t + fht_row(k, 128, logbs)) * hidden, c + fht_col(k, 128, logbs), v[k]);
+  });
 }
 
-__device__ __forceinline__ uint4 pack8_half(const float* f, float rs) {
-  __half2 h0 = __floats2half2_rn(f[0] * rs, f[1] * rs), h1 = __floats2half2_rn(f[2] * rs, f[3] * rs);
-  __half2 h2 = __floats2half2_rn(f[4] * rs, f[5] * rs), h3 = __floats2half2_rn(f[6] * rs, f[7] * rs);
-  return make_uint4(*reinterpret_cast<uint32_t*>(&h0), *reinterpret_cast<uint32_t*>(&h1),
-                    *reinterpret_cast<uint32_t*>(&h2), *reinterpret_cast<uint32_t*>(&h3));
+__device__ __forceinline__ uint2 pack4_half(const f2 (&q)[2]) {
+  float r[4];
+  f2_unpack(q[0], r[0], r[1]);
+  f2_unpack(q[1], r[2], r[3]);
+  const __half2 a = __floats2half2_rn(r[0], r[1]), b = __floats2half2_rn(r[2], r[3]);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+// place of columns col .. col + 3 of padded row `trow` in a [tile][chunk] x (128 x 64) image
+__device__ __forceinline__ uint8_t* moe_tile_at(uint8_t* base, int trow, int kchunks, int col) {
+  return base + ((size_t)(trow / MOE_TN) * kchunks + (col >> 6)) * MOE_B_BYTES + sw128_offset(trow % MOE_TN, col & 63);
 }
 
 // Input transform of one token, stored once per routing into the token tiles of the routed experts.
-__global__ void __launch_bounds__(1024) moe_rht_in_gemm_kernel(const __grid_constant__ MoeDev M, const uint8_t* __restrict__ x,
-                                                               uint8_t* __restrict__ ws) {
-  extern __shared__ float fb[];
-  const int t = blockIdx.x;
-  for (int i = threadIdx.x; i < M.hidden; i += blockDim.x)
-    fb[i] = load_act(x, (long long)t * M.hidden + i, M.x_dtype) * __half2float(M.w13_sv[i]);
-  for (int b = 0; b < M.nb_n13; ++b) fht_smem(fb + M.off_n13[b], M.log_n13[b]);
+__global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_rht_in_gemm_kernel(const __grid_constant__ MoeDev M, int T, int tt,
+                                                                            const uint8_t* __restrict__ x, uint8_t* __restrict__ ws) {
+  extern __shared__ __align__(16) float fb[];
   const int* slot_of = reinterpret_cast<const int*>(ws + M.o_slot_of);
   const int* trow = reinterpret_cast<const int*>(ws + M.o_trow);
   const int kchunks = M.hidden / GM_TILE_K;
-  for (int b = 0; b < M.nb_n13; ++b) {
-    const float rs = rsqrtf((float)(1 << M.log_n13[b]));
-    for (int i = threadIdx.x * 8; i < (1 << M.log_n13[b]); i += blockDim.x * 8) {
-      const int col = M.off_n13[b] + i;
-      const uint4 v = pack8_half(fb + col, rs);
-      for (int j = 0; j < M.top_k; ++j) {
-        const int slot = slot_of[t * M.top_k + j];
-        if (slot >= 0) moe_store_tile16(ws + M.o_xr1, trow[slot], kchunks, col >> 3, v);
-      }
-    }
+  int* rows = reinterpret_cast<int*>(fb + fht_words(8192));          // tile row of every routing of the CTA's tokens
+  const int t0 = blockIdx.x * tt, nr = min(tt, T - t0) * M.top_k;
+  for (int i = threadIdx.x; i < nr; i += blockDim.x) {
+    const int slot = slot_of[t0 * M.top_k + i];
+    rows[i] = slot >= 0 ? trow[slot] : -1;
   }
+  __syncthreads();
+  const int top_k = M.top_k;
+  uint8_t* xr = ws + M.o_xr1;
+  moe_rht_in_body(M, T, tt, x, fb, [&](int t, int c, int logbs, int n, const f2 (&v)[8][2]) {
+    uint2 h[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) h[k] = pack4_half(v[k]);
+    if (logbs >= 10) {               // a thread's groups are columns 128 apart of one token
+      for (int j = 0; j < top_k; ++j) {
+        const int r = rows[(t - t0) * top_k + j];
+        if (r < 0) continue;
+        uint8_t* p = moe_tile_at(xr, r, kchunks, c);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (k < n) *reinterpret_cast<uint2*>(p + k * 2 * MOE_B_BYTES) = h[k];
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k < n)
+          for (int j = 0; j < top_k; ++j) {
+            const int r = rows[(t + fht_row(k, 128, logbs) - t0) * top_k + j];
+            if (r >= 0) *reinterpret_cast<uint2*>(moe_tile_at(xr, r, kchunks, c + fht_col(k, 128, logbs))) = h[k];
+          }
+    }
+  });
 }
 
 // ---- 3 / 5: grouped decode + mma ------------------------------------------------------------------------
@@ -473,28 +548,82 @@ __global__ void __launch_bounds__(MV_THREADS, 2) trellis_moe_mv_kernel(const __g
   }
 }
 
-// Shared-memory words of `rows` arrays laid out block after block, each array padded by one word per 32
-// (the layout fht_tile works in): block b of row r starts at rows * pad_off[b] + r * row_words(b).
-__device__ __forceinline__ int moe_pad_words(int n) { return n + (n >> 5); }
-
-constexpr int MOE_XF_THREADS = 256;
-
-// 8 fp16 values (16-byte aligned) as floats
-__device__ __forceinline__ void load8_half(const __half* p, float (&f)[8]) {
-  const uint4 t = *reinterpret_cast<const uint4*>(p);
-  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&t.x));
-  const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&t.y));
-  const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&t.z));
-  const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&t.w));
-  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+// The transforms of the mid and combine kernels work on 1024-value chunks, one warp each (fht_warp).  `rows` arrays of a
+// block of 2^log values take moe_chunks(rows, log) chunks: value i of row r is value (r << log | i) & 1023 of chunk
+// (r << log | i) >> 10.  Blocks of more than 1024 values span chunks; what reads their results does the last stages.
+__host__ __device__ __forceinline__ int moe_chunks(int rows, int lg) { return ((rows << lg) + 1023) >> 10; }
+__host__ __device__ __forceinline__ int moe_chunks_all(int rows, int nb, const int* lg) {
+  int c = 0;
+  for (int b = 0; b < nb; ++b) c += moe_chunks(rows, lg[b]);
+  return c;
 }
+// block of chunk `ch`; `base` receives the block's first chunk
+__device__ __forceinline__ int moe_chunk_block(int ch, int rows, int nb, const int* lg, int& base) {
+  int b = 0;
+  base = 0;
+  for (; b + 1 < nb; ++b) {
+    const int n = moe_chunks(rows, lg[b]);
+    if (ch < base + n) break;
+    base += n;
+  }
+  return b;
+}
+// A chunk's values: sums of `cnt` partial sums `kstride` floats apart.  row_off(r): first value of row r (floats from
+// `src`, which points at the block's first column), negative for a row of zeros; rows from `nrow` on are zero.
+template <class RowOff>
+__device__ __forceinline__ void moe_load_chunk(f2 (&v)[8][2], int c, int logbs, int nrow, const float* __restrict__ src, int cnt,
+                                               long long kstride, RowOff row_off) {
+  const int e = (c << 10) | ((threadIdx.x & 31) << 2), i0 = e & ((1 << logbs) - 1);
+  const float* p[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int r = (e >> logbs) + fht_row(k, 128, logbs);
+    const long long o = r < nrow ? row_off(r) : -1;
+    p[k] = o >= 0 ? src + o + i0 + fht_col(k, 128, logbs) : nullptr;
+    v[k][0] = v[k][1] = 0;
+    if (p[k]) {
+      const ulonglong2 t = __ldcg(reinterpret_cast<const ulonglong2*>(p[k]));
+      v[k][0] = t.x; v[k][1] = t.y;
+    }
+  }
+  for (int s = 1; s < cnt; ++s) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (p[k]) {
+        const ulonglong2 t = __ldcg(reinterpret_cast<const ulonglong2*>(p[k] + s * kstride));
+        v[k][0] = f2_add(v[k][0], t.x);
+        v[k][1] = f2_add(v[k][1], t.y);
+      }
+  }
+}
+// values i .. i + 3 (i % 4 == 0) of row `row` of a block whose chunks start at `area`
+__device__ __forceinline__ void moe_read4(const float* area, int logbs, int row, int i, f2 (&v)[2]) {
+  if (logbs <= 10) {
+    fht_ld4(area + fht_pos((row << logbs) | i), v);
+    return;
+  }
+  v[0] = v[1] = 0;
+  const int top = logbs - 10;
+  for (int t = 0; t < (1 << top); ++t) {
+    f2 p[2];
+    fht_ld4(area + fht_pos((row << logbs) | (t << 10) | (i & 1023)), p);
+    const f2 sg = (__popc(t & (i >> 10)) & 1) ? F2_MINUS1 : F2_ONE;
+    v[0] = f2_fma(p[0], sg, v[0]);
+    v[1] = f2_fma(p[1], sg, v[1]);
+  }
+}
+
 __device__ __forceinline__ float round_half(float v) { return __half2float(__float2half_rn(v)); }
 
 // ---- 4: per slot  h = act(gate) * up  from w13 partials, then the w2 input transform ---------------------
-// One CTA handles `sg` consecutive slots (rows of the radix-32 tile transform).
+// One CTA handles `sg` consecutive slots.  Bound by memory (it reads a slot's w13 outputs as fp32 and writes its w2
+// inputs as fp16); chunk by chunk in one warp each, the gated activation is evaluated where the second transform
+// loads its values, so nothing but the two transforms' chunks passes through shared memory.  4096 tokens, top 8, 1536
+// and 768 columns: 243 -> 219 us (slots per CTA from 5 to 7 make no difference: latency and the one barrier are the
+// rest); the combine below 212 -> 116 us, the input transform 60 -> 45 us.
 __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_mid_kernel(const __grid_constant__ MoeDev M, int T, int sg,
                                                                     uint8_t* __restrict__ ws) {
-  extern __shared__ float fb[];              // sg x padded(max(w13_out, inter)) transform area, then sg x padded(inter)
+  extern __shared__ __align__(16) float fb[];   // chunks of sg w13 rows, then of sg w2 rows
   const int R = T * M.top_k;
   const int* g_count = reinterpret_cast<const int*>(ws + M.o_count);
   const int* g_base = reinterpret_cast<const int*>(ws + M.o_base);
@@ -502,202 +631,222 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_mid_kernel(const __grid
   const int slot0 = blockIdx.x * sg;
   if (slot0 >= used) return;
   const int nrow = min(sg, used - slot0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ int row_e[8];                   // expert of each row (sg <= 8)
   __shared__ float row_wsc[8];
+  __shared__ int row_t[8];
   if (threadIdx.x < nrow) {
     const int e = reinterpret_cast<const int*>(ws + M.o_route_exp)[slot0 + threadIdx.x];
     row_e[threadIdx.x] = e;
     row_wsc[threadIdx.x] = M.w13_wscale[e];
+    row_t[threadIdx.x] = M.gemm ? reinterpret_cast<const int*>(ws + M.o_trow)[slot0 + threadIdx.x] : 0;
+  }
+  const int inter = M.inter, w13_out = M.w13_out, kch = M.kch13;
+  const int n13 = moe_chunks_all(sg, M.nb_m13, M.log_m13), n2 = moe_chunks_all(sg, M.nb_n2, M.log_n2);
+  const long long kstride = (long long)R * w13_out;
+  const float* part1 = reinterpret_cast<const float*>(ws + M.o_part1) + (long long)slot0 * w13_out;
+
+  // -- output transform of w13; results stay in shared memory
+  for (int ch = warp; ch < n13; ch += MOE_XF_THREADS / 32) {
+    int base;
+    const int b = moe_chunk_block(ch, sg, M.nb_m13, M.log_m13, base);
+    f2 v[8][2];
+    moe_load_chunk(v, ch - base, M.log_m13[b], nrow, part1 + M.off_m13[b], kch, kstride,
+                   [&](int r) -> long long { return r * w13_out; });
+    fht_warp(fb + ch * FHT_CHUNK_WORDS, v, M.log_m13[b]);
   }
   __syncthreads();
-  const int hrw = moe_pad_words(M.inter);
-  float* hbuf = fb + sg * moe_pad_words(max(M.w13_out, M.inter));
-  const float* part1 = reinterpret_cast<const float*>(ws + M.o_part1);
-  const long long kstride = (long long)R * M.w13_out;
-  const int kch = M.kch13, w13_out = M.w13_out, inter = M.inter;
-
-  // -- output transform of w13 (Wscale applied on the way in); results stay in shared memory
-  int poff = 0;
-  for (int b = 0; b < M.nb_m13; ++b) {
-    const int logbs = M.log_m13[b], off = M.off_m13[b];
-    auto load32 = [&](int row, int i0, float (&v)[32]) {
-      const float wsc = row_wsc[row];
-      const float* src = part1 + (long long)(slot0 + row) * w13_out + off + i0;
+  // -- columns c .. c + 3 of the w13 output: Wscale, 1/sqrt(bs) and SU, fp16 rounding (the reference's w13 op returns
+  //    fp16: glq_vllm/fused_moe_method.py:412-421)
+  auto y13_4 = [&](int row, int c, float (&f)[4]) {
+    int base = 0, b = 0;
+    while (b + 1 < M.nb_m13 && c >= M.off_m13[b + 1]) { base += moe_chunks(sg, M.log_m13[b]); ++b; }
+    const float sc = rsqrtf((float)(1 << M.log_m13[b])) * row_wsc[row];
+    f2 p[2], s[2];
+    moe_read4(fb + base * FHT_CHUNK_WORDS, M.log_m13[b], row, c - M.off_m13[b], p);
+    load_sign4(M.w13_su + (long long)row_e[row] * w13_out + c, s);
+    const f2 sc2 = f2_pack(sc, sc);
+    f2_unpack(f2_mul(f2_mul(p[0], sc2), s[0]), f[0], f[1]);
+    f2_unpack(f2_mul(f2_mul(p[1], sc2), s[1]), f[2], f[3]);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int k = 0; k < kch; ++k) {
-          const float4 t4 = *reinterpret_cast<const float4*>(src + 4 * j + k * kstride);
-          a.x += t4.x; a.y += t4.y; a.z += t4.z; a.w += t4.w;
-        }
-        v[4 * j] = a.x * wsc; v[4 * j + 1] = a.y * wsc; v[4 * j + 2] = a.z * wsc; v[4 * j + 3] = a.w * wsc;
-      }
-    };
-    fht_tile_core(fb + sg * poff, logbs, nrow, load32);
-    poff += moe_pad_words(1 << logbs);
-  }
-  // -- 8 columns at a time: SU and 1/sqrt(bs), fp16 rounding (the reference's w13 op returns fp16:
-  //    glq_vllm/fused_moe_method.py:412-421), gated activation, fp16 rounding, SV of w2
-  auto y13_8 = [&](int row, int c, float (&f)[8]) {     // columns c .. c+7 of the w13 output (c % 8 == 0)
-    int po = 0, b = 0;
-    while (b + 1 < M.nb_m13 && c >= M.off_m13[b] + (1 << M.log_m13[b])) { po += moe_pad_words(1 << M.log_m13[b]); ++b; }
-    const int bs = 1 << M.log_m13[b];
-    const float rs = rsqrtf((float)bs);
-    const float* p = fb + sg * po + row * moe_pad_words(bs) + fht_pad(c - M.off_m13[b]);
-    float su[8];
-    load8_half(M.w13_su + (long long)row_e[row] * w13_out + c, su);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) f[k] = round_half(p[k] * rs * su[k]);
+    for (int k = 0; k < 4; ++k) f[k] = round_half(f[k]);
   };
-  const int per_row = inter >> 3;
-  for (int o = threadIdx.x; o < nrow * per_row; o += blockDim.x) {
-    const int row = o / per_row, i = (o - row * per_row) * 8;
-    float g[8], u[8], sv[8];
-    y13_8(row, i, g);
-    load8_half(M.w2_sv + i, sv);
-    if (M.gated) y13_8(row, inter + i, u);
-    float* dst = hbuf + row * hrw + fht_pad(i);
+  // -- input transform of w2 on act(gate) * up (fp16) times SV, stored from its chunks
+  float* area2 = fb + n13 * FHT_CHUNK_WORDS;
+  const int kchunks = inter / GM_TILE_K;
+  uint8_t* xr2 = ws + M.o_xr2;
+  __half2* xs2 = reinterpret_cast<__half2*>(xr2) + (long long)slot0 * inter;
+  const bool gemm = M.gemm != 0;
+  auto put = [&](int row, int c, const f2 (&v)[2], f2 rs2) {
+    const f2 r[2] = {f2_mul(v[0], rs2), f2_mul(v[1], rs2)};
+    if (gemm) *reinterpret_cast<uint2*>(moe_tile_at(xr2, row_t[row], kchunks, c)) = pack4_half(r);
+    else moe_store_xr4(xs2 + row * inter, c, r);
+  };
+  bool spans = false;                        // blocks of more than one chunk are finished when all chunks are done
+  for (int ch = warp; ch < n2; ch += MOE_XF_THREADS / 32) {
+    int base;
+    const int b = moe_chunk_block(ch, sg, M.nb_n2, M.log_n2, base);
+    const int logbs = M.log_n2[b], off = M.off_n2[b];
+    const int e = ((ch - base) << 10) | (lane << 2), row0 = e >> logbs, c0 = off + (e & ((1 << logbs) - 1));
+    f2 v[8][2];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const float a = moe_act(g[k], M.act);
-      dst[k] = round_half(M.gated ? a * u[k] : a) * sv[k];
-    }
-  }
-  __syncthreads();
-  // -- input transform of w2, back into the transform area, then 16-byte stores
-  poff = 0;
-  for (int b = 0; b < M.nb_n2; ++b) {
-    const int logbs = M.log_n2[b], off = M.off_n2[b];
-    auto load32 = [&](int row, int i0, float (&v)[32]) {
-      const float* src = hbuf + row * hrw + fht_pad(off + i0);    // off and i0 are multiples of 32
+      const int row = row0 + fht_row(k, 128, logbs), c = c0 + fht_col(k, 128, logbs);
+      v[k][0] = v[k][1] = 0;
+      if (row < nrow) {
+        float g[4], u[4];
+        f2 sv[2];
+        y13_4(row, c, g);
+        load_sign4(M.w2_sv + c, sv);
+        if (M.gated) y13_4(row, inter + c, u);
 #pragma unroll
-      for (int k = 0; k < 32; ++k) v[k] = src[k];
-    };
-    fht_tile_core(fb + sg * poff, logbs, nrow, load32);
-    poff += moe_pad_words(1 << logbs);
-  }
-  poff = 0;
-  const int* trow = reinterpret_cast<const int*>(ws + M.o_trow);
-  for (int b = 0; b < M.nb_n2; ++b) {
-    const int bs = 1 << M.log_n2[b], off = M.off_n2[b], rw = moe_pad_words(bs);
-    const float* reg = fb + sg * poff;
-    const float rs = rsqrtf((float)bs);
-    const int pr = bs >> 3;
-    for (int o = threadIdx.x; o < nrow * pr; o += blockDim.x) {
-      const int row = o / pr, i = (o - row * pr) * 8;
-      const float* src = reg + row * rw + fht_pad(i);
-      const int slot = slot0 + row, col = off + i;
-      if (M.gemm) {
-        moe_store_tile16(ws + M.o_xr2, trow[slot], inter / GM_TILE_K, col >> 3, pack8_half(src, rs));
-      } else {
-        __half2* out = reinterpret_cast<__half2*>(ws + M.o_xr2) + (long long)slot * inter;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int c = col + k;
-          const int pos = (c & ~31) * XR_TRELLIS_EXPAND + xr_pos_trellis(c & 31);
-          out[pos >> 1] = __halves2half2(__float2half_rn(src[k] * rs), __float2half_rn(0.f));
+        for (int j = 0; j < 4; ++j) {
+          const float a = moe_act(g[j], M.act);
+          g[j] = round_half(M.gated ? a * u[j] : a);
         }
+        v[k][0] = f2_mul(f2_pack(g[0], g[1]), sv[0]);
+        v[k][1] = f2_mul(f2_pack(g[2], g[3]), sv[1]);
       }
     }
-    poff += rw;
+    float* sm = area2 + ch * FHT_CHUNK_WORDS;
+    fht_warp(sm, v, logbs);
+    if (logbs > 10) { spans = true; continue; }
+    const float rs = rsqrtf((float)(1 << logbs));
+    const f2 rs2 = f2_pack(rs, rs);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int row = row0 + fht_row(k, 128, logbs);
+      if (row < nrow) {
+        fht_ld4(sm + (lane << 2) + k * 132, v[k]);
+        put(row, c0 + fht_col(k, 128, logbs), v[k], rs2);
+      }
+    }
+  }
+  if (!__syncthreads_or(spans)) return;
+  int base = 0;
+  for (int b = 0; b < M.nb_n2; ++b) {
+    const int logbs = M.log_n2[b], bs = 1 << logbs;
+    if (logbs > 10) {
+      const float rs = rsqrtf((float)bs);
+      const f2 rs2 = f2_pack(rs, rs);
+      for (int o = threadIdx.x * 4; o < nrow << logbs; o += MOE_XF_THREADS * 4) {
+        f2 v[2];
+        moe_read4(area2 + base * FHT_CHUNK_WORDS, logbs, o >> logbs, o & (bs - 1), v);
+        put(o >> logbs, M.off_n2[b] + (o & (bs - 1)), v, rs2);
+      }
+    }
+    base += moe_chunks(sg, logbs);
   }
 }
 
 // ---- 6: per token weighted combine ------------------------------------------------------------------------
-// The routings of a token are the rows of one tile transform (`rg` at a time); a thread then owns 8 output
-// columns and adds the routings' results in fixed j order.
+// The routings of a token are the rows of the transform (`rg` at a time), 1024 values per warp; a thread then owns groups
+// of four output columns, 1024 apart within a block, does the stages beyond the chunks and adds the routings' results
+// in fixed j order.
+template <int TOP>
+__device__ __forceinline__ void moe_combine_block(const MoeDev& M, const float* area, int logbs, int off, int nrow, bool first, bool last,
+                                                  const long long* row_off, const int* row_e, const float* row_wsc, const float* row_w,
+                                                  float* accs, uint8_t* y, long long y_row, bool y_vec) {
+  constexpr int N = 1 << TOP;
+  const float rs = rsqrtf((float)(1 << logbs));
+  const int span = 1 << (logbs - TOP);
+  for (int i = threadIdx.x * 4; i < span; i += MOE_XF_THREADS * 4) {
+    float a[N][4];
+#pragma unroll
+    for (int t = 0; t < N; ++t)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) a[t][j] = first ? 0.f : accs[off + (t << 10) + i + j];
+    for (int row = 0; row < nrow; ++row) {
+      if (row_off[row] < 0) continue;
+      const float w = row_w[row], sc = rs * row_wsc[row];
+      const f2 sc2 = f2_pack(sc, sc);
+      f2 v[N][2];
+#pragma unroll
+      for (int t = 0; t < N; ++t) fht_ld4(area + fht_pos((row << logbs) | (t << 10) | i), v[t]);
+#pragma unroll
+      for (int s = 0; s < TOP; ++s)
+#pragma unroll
+        for (int t = 0; t < N; ++t)
+          if (!(t & (1 << s))) { f2_butterfly(v[t][0], v[t | (1 << s)][0]); f2_butterfly(v[t][1], v[t | (1 << s)][1]); }
+      const __half* su = M.w2_su + (long long)row_e[row] * M.hidden + off + i;
+#pragma unroll
+      for (int t = 0; t < N; ++t) {
+        f2 s[2];
+        float r[4];
+        load_sign4(su + (t << 10), s);
+        f2_unpack(f2_mul(f2_mul(v[t][0], sc2), s[0]), r[0], r[1]);
+        f2_unpack(f2_mul(f2_mul(v[t][1], sc2), s[1]), r[2], r[3]);
+        // the reference's w2 op returns fp16 before the weighted sum
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a[t][j] += w * round_half(r[j]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      const int c = off + (t << 10) + i;
+      if (!last) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) accs[c + j] = a[t][j];
+      } else if (y_vec) {
+        store_act4(y, y_row + c, M.y_dtype, a[t]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) store_act(y, y_row + c + j, M.y_dtype, a[t][j]);
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_out_kernel(const __grid_constant__ MoeDev M, int T, int rg,
                                                                     const float* __restrict__ topk_w,
                                                                     const uint8_t* __restrict__ ws, uint8_t* __restrict__ y) {
-  extern __shared__ float fb[];              // rg x padded(hidden) (+ hidden floats when several passes are needed)
+  extern __shared__ __align__(16) float fb[];   // chunks of rg rows of hidden (+ hidden floats when several passes are needed)
   const int t = blockIdx.x;
   const int R = T * M.top_k;
   const int* slot_of = reinterpret_cast<const int*>(ws + M.o_slot_of);
   const int* route_exp = reinterpret_cast<const int*>(ws + M.o_route_exp);
   const float* part2 = reinterpret_cast<const float*>(ws + M.o_part2);
-  __shared__ int row_slot[64], row_e[64];    // per routing j of this token (top_k <= 64)
+  __shared__ long long row_off[64];          // per routing j of this token (top_k <= 64): its partial sums, or -1
+  __shared__ int row_e[64];
   __shared__ float row_wsc[64], row_w[64];
   if (threadIdx.x < M.top_k) {
     const int slot = slot_of[t * M.top_k + threadIdx.x];
     const int e = slot >= 0 ? route_exp[slot] : 0;
-    row_slot[threadIdx.x] = slot;
+    row_off[threadIdx.x] = slot >= 0 ? (long long)slot * M.hidden : -1;
     row_e[threadIdx.x] = e;
     row_wsc[threadIdx.x] = M.w2_wscale[e];
     row_w[threadIdx.x] = topk_w[t * M.top_k + threadIdx.x];
   }
   __syncthreads();
-  float* accs = fb + rg * moe_pad_words(M.hidden);   // running sums over the passes, hidden floats
-  const int hidden = M.hidden, kch = M.kch2;
+  const int hidden = M.hidden, kch = M.kch2, n2 = moe_chunks_all(rg, M.nb_m2, M.log_m2);
+  float* accs = fb + n2 * FHT_CHUNK_WORDS;   // running sums over the passes, hidden floats
   const long long kstride = (long long)R * hidden;
-  const bool y_vec = (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+  const bool y_vec = act_rows_aligned4(y, 0, hidden, M.y_dtype);
   for (int j0 = 0; j0 < M.top_k; j0 += rg) {
     const int nrow = min(rg, M.top_k - j0);
-    int poff = 0;
+    for (int ch = threadIdx.x >> 5; ch < n2; ch += MOE_XF_THREADS / 32) {
+      int base;
+      const int b = moe_chunk_block(ch, rg, M.nb_m2, M.log_m2, base);
+      f2 v[8][2];
+      moe_load_chunk(v, ch - base, M.log_m2[b], nrow, part2 + M.off_m2[b], kch, kstride,
+                     [&](int r) -> long long { return row_off[j0 + r]; });
+      fht_warp(fb + ch * FHT_CHUNK_WORDS, v, M.log_m2[b]);
+    }
+    __syncthreads();
+    const bool first = j0 == 0, last = j0 + rg >= M.top_k;
+    int base = 0;
     for (int b = 0; b < M.nb_m2; ++b) {
       const int logbs = M.log_m2[b], off = M.off_m2[b];
-      auto load32 = [&](int row, int i0, float (&v)[32]) {
-        const int slot = row_slot[j0 + row];
-        if (slot < 0) {
-#pragma unroll
-          for (int k = 0; k < 32; ++k) v[k] = 0.f;
-          return;
-        }
-        const float wsc = row_wsc[j0 + row];
-        const float* src = part2 + (long long)slot * hidden + off + i0;
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-          for (int k = 0; k < kch; ++k) {
-            const float4 t4 = *reinterpret_cast<const float4*>(src + 4 * jj + k * kstride);
-            a.x += t4.x; a.y += t4.y; a.z += t4.z; a.w += t4.w;
-          }
-          v[4 * jj] = a.x * wsc; v[4 * jj + 1] = a.y * wsc; v[4 * jj + 2] = a.z * wsc; v[4 * jj + 3] = a.w * wsc;
-        }
+      const float* area = fb + base * FHT_CHUNK_WORDS;
+      auto go = [&](auto top) {
+        moe_combine_block<decltype(top)::value>(M, area, logbs, off, nrow, first, last, row_off + j0, row_e + j0, row_wsc + j0,
+                                                row_w + j0, accs, y, (long long)t * hidden, y_vec);
       };
-      fht_tile_core(fb + rg * poff, logbs, nrow, load32);
-      poff += moe_pad_words(1 << logbs);
-    }
-    const bool first = j0 == 0, last = j0 + rg >= M.top_k;
-    for (int c = threadIdx.x * 8; c < hidden; c += blockDim.x * 8) {
-      int po = 0, b = 0;
-      while (b + 1 < M.nb_m2 && c >= M.off_m2[b] + (1 << M.log_m2[b])) { po += moe_pad_words(1 << M.log_m2[b]); ++b; }
-      const int bs = 1 << M.log_m2[b], rw = moe_pad_words(bs);
-      const float rs = rsqrtf((float)bs);
-      const float* reg = fb + rg * po + fht_pad(c - M.off_m2[b]);
-      float a[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) a[k] = first ? 0.f : accs[c + k];
-      for (int row = 0; row < nrow; ++row) {
-        if (row_slot[j0 + row] < 0) continue;
-        float su[8];
-        load8_half(M.w2_su + (long long)row_e[j0 + row] * hidden + c, su);
-        const float w = row_w[j0 + row];
-        const float* p = reg + row * rw;
-        // the reference's w2 op returns fp16 before the weighted sum
-#pragma unroll
-        for (int k = 0; k < 8; ++k) a[k] += w * round_half(p[k] * rs * su[k]);
-      }
-      if (!last) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) accs[c + k] = a[k];
-      } else if (y_vec && M.y_dtype != GLQB_DT_F32) {
-        uint4 o4;
-        if (M.y_dtype == GLQB_DT_F16) {
-          const __half2 h0 = __floats2half2_rn(a[0], a[1]), h1 = __floats2half2_rn(a[2], a[3]);
-          const __half2 h2 = __floats2half2_rn(a[4], a[5]), h3 = __floats2half2_rn(a[6], a[7]);
-          o4 = make_uint4(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1),
-                          *reinterpret_cast<const uint32_t*>(&h2), *reinterpret_cast<const uint32_t*>(&h3));
-        } else {
-          const __nv_bfloat162 h0 = __floats2bfloat162_rn(a[0], a[1]), h1 = __floats2bfloat162_rn(a[2], a[3]);
-          const __nv_bfloat162 h2 = __floats2bfloat162_rn(a[4], a[5]), h3 = __floats2bfloat162_rn(a[6], a[7]);
-          o4 = make_uint4(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1),
-                          *reinterpret_cast<const uint32_t*>(&h2), *reinterpret_cast<const uint32_t*>(&h3));
-        }
-        *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(y) + (long long)t * hidden + c) = o4;
-      } else {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) store_act(y, (long long)t * hidden + c + k, M.y_dtype, a[k]);
-      }
+      if (logbs <= 10) go(IntC<0>());
+      else if (logbs == 11) go(IntC<1>());
+      else if (logbs == 12) go(IntC<2>());
+      else go(IntC<3>());
+      base += moe_chunks(rg, logbs);
     }
     __syncthreads();
   }
@@ -822,6 +971,13 @@ static void moe_launch_group(const MoeDev& M, const void* ids, int tokens, uint8
   moe_count_kernel<<<nb, 1024, M.E * sizeof(int), st>>>(M, ids, tokens, ws);
   moe_group_kernel<<<1, 1024, sh, st>>>(M, ids, tokens, ws, 1);
   moe_place_kernel<<<nb, 1024, 2 * M.E * sizeof(int), st>>>(M, ids, tokens, ws);
+}
+
+// tokens per CTA of the input transform: one tile of 8192 values, fewer when that would leave SMs without work
+static int moe_in_tokens(const MoeDev& M, int tokens) {
+  int tt = std::max(1, std::min(8, 8192 / M.hidden));
+  while (tt > 1 && (tokens + tt - 1) / tt < 296) --tt;
+  return tt;
 }
 
 extern "C" {
@@ -974,19 +1130,20 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
     }
   }
   {
-    auto padw = [](size_t n) { return n + n / 32; };
-    const size_t budget = 74 * 1024;      // three CTAs per SM
-    const size_t mid_row = 4 * (padw(std::max(d->w13_out, d->inter)) + padw(d->inter)), out_row = 4 * padw(d->hidden);
-    P->mid_sg = (int)std::max<size_t>(1, std::min<size_t>(8, budget / mid_row));
-    P->out_rg = (int)std::max<size_t>(1, std::min<size_t>(std::min(8, d->top_k), budget / out_row));
-    // running sums between passes are only needed when one pass cannot hold all routings of a token
-    const size_t out_fixed = P->out_rg < d->top_k ? 4 * (size_t)d->hidden : 0;
-    P->mid_smem = P->mid_sg * mid_row;
-    P->out_smem = P->out_rg * out_row + out_fixed;
+    const size_t budget = 74 * 1024;      // three CTAs per SM (and the limit every plan sets: one plan never lowers another's)
+    auto mid_bytes = [&](int sg) { return (size_t)4 * FHT_CHUNK_WORDS * (moe_chunks_all(sg, M.nb_m13, M.log_m13) + moe_chunks_all(sg, M.nb_n2, M.log_n2)); };
+    auto out_bytes = [&](int rg) { return 4 * ((size_t)FHT_CHUNK_WORDS * moe_chunks_all(rg, M.nb_m2, M.log_m2) + (rg < d->top_k ? (size_t)d->hidden : 0)); };
+    P->mid_sg = 8;
+    while (P->mid_sg > 1 && mid_bytes(P->mid_sg) > budget) --P->mid_sg;
+    P->out_rg = std::min(8, d->top_k);
+    // (running sums between passes are only needed when one pass cannot hold all routings of a token)
+    while (P->out_rg > 1 && out_bytes(P->out_rg) > budget) --P->out_rg;
+    P->mid_smem = mid_bytes(P->mid_sg);
+    P->out_smem = out_bytes(P->out_rg);
     if (cudaFuncSetAttribute(moe_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)((4 * d->num_experts + 1) * sizeof(int))) != cudaSuccess ||
-        cudaFuncSetAttribute(moe_mid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P->mid_smem) != cudaSuccess ||
-        cudaFuncSetAttribute(moe_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P->out_smem) != cudaSuccess) {
+        cudaFuncSetAttribute(moe_mid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) != cudaSuccess ||
+        cudaFuncSetAttribute(moe_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) != cudaSuccess) {
       delete P;
       return moe_fail(GLQB_E_CUDA, "moe_plan_create: %s", cudaGetErrorString(cudaGetLastError()));
     }
@@ -1033,8 +1190,9 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
     const MoeDev& G = P->devg;
     const int R = tokens * G.top_k;
     moe_launch_group(G, topk_ids, tokens, ws, st);
-    moe_rht_in_gemm_kernel<<<tokens, std::max(64, std::min(1024, G.hidden / 8)), G.hidden * 4, st>>>(
-        G, reinterpret_cast<const uint8_t*>(x), ws);
+    const int tt = moe_in_tokens(G, tokens);
+    moe_rht_in_gemm_kernel<<<(tokens + tt - 1) / tt, MOE_XF_THREADS, (fht_words(8192) + tt * G.top_k) * 4, st>>>(
+        G, tokens, tt, reinterpret_cast<const uint8_t*>(x), ws);
     int* status = reinterpret_cast<int*>(ws + G.o_status);
     const int* nitems = reinterpret_cast<const int*>(ws + G.o_nitems);
     {
@@ -1059,8 +1217,9 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
   const MoeDev& M = P->dev;
   const int R = tokens * M.top_k;
   moe_launch_group(M, topk_ids, tokens, ws, st);
-  moe_rht_in_kernel<<<tokens, std::max(64, std::min(1024, M.hidden / 8)), M.hidden * 4, st>>>(
-      M, reinterpret_cast<const uint8_t*>(x), ws);
+  const int tt = moe_in_tokens(M, tokens);
+  moe_rht_in_kernel<<<(tokens + tt - 1) / tt, MOE_XF_THREADS, fht_words(8192) * 4, st>>>(M, tokens, tt,
+                                                                                       reinterpret_cast<const uint8_t*>(x), ws);
   MoeMvArgs A;
   memset(&A, 0, sizeof A);
   A.codes[0] = M.w13[0]; A.codes[1] = M.w13[1]; A.stride[0] = M.w13_stride[0]; A.stride[1] = M.w13_stride[1];

@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "glqb_kernels.cuh"
+#include "glqb_fht.cuh"
 
 namespace glqb {
 

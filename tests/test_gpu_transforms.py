@@ -1,0 +1,90 @@
+"""The Hadamard transforms at the edges of their tiles: every block length from 1 to 32768 (8192 is one tile), ragged token
+counts, padded and cut-off columns, rows that are not aligned for vector accesses, every activation type."""
+import numpy as np
+import pytest
+import torch
+
+from glq_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def fht64(v, blocks):
+    out, off = np.empty_like(v), 0
+    for b in blocks:
+        a, h = v[:, off:off + b].copy(), 1
+        while h < b:
+            a = a.reshape(len(v), b // (2 * h), 2, h)
+            a = np.stack((a[:, :, 0] + a[:, :, 1], a[:, :, 0] - a[:, :, 1]), 2).reshape(len(v), b)
+            h *= 2
+        out[:, off:off + b] = a / np.sqrt(b)
+        off += b
+    return out
+
+
+BLOCKS = [[1], [2], [4], [8, 4, 2, 1], [16], [32, 2], [64, 32, 8], [128], [256, 64], [1024, 512], [2048, 32], [4096], [8192, 256],
+          [16384, 1024], [32768]]
+ROUND = {torch.float32: 0.0, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("blocks", BLOCKS, ids=str)
+def test_transform_blocks(blocks, dtype):
+    g = torch.Generator(device="cuda").manual_seed(sum(blocks))
+    total = sum(blocks)
+    for tokens, cut, shift in ((1, 0, 0), (3, min(3, total - 1), 1), (67, 0, 3)):
+        feat = total - cut
+        signs = (torch.randint(0, 2, (total,), generator=g, device="cuda") * 2 - 1).half()
+        # rows of feat + shift values: with shift != 0 they are not aligned for vector loads
+        x = torch.randn(tokens, feat + shift, generator=g, device="cuda").to(dtype)[:, shift:]
+        out = torch.full((tokens, total), float("nan"), device="cuda")
+        ops.input_rht_blocks(x, signs, out, feat, total, blocks)
+        xp = np.zeros((tokens, total))
+        xp[:, :feat] = x.double().cpu().numpy()
+        ref = fht64(xp * signs.double().cpu().numpy(), blocks)
+        # at most 15 additions per value, each rounding to 2^-24 of a partial sum that stays below max |ref| * 16
+        assert np.abs(out.double().cpu().numpy() - ref).max() <= 15 * 16 * 2.0 ** -24 * max(1.0, np.abs(ref).max())
+        y = torch.full((tokens, feat + shift), float("nan"), dtype=dtype, device="cuda")
+        ops.output_rht_blocks(out, signs, y[:, shift:], feat, total, blocks)
+        ref = (fht64(out.double().cpu().numpy(), blocks) * signs.double().cpu().numpy())[:, :feat]
+        err = np.abs(y[:, shift:].double().cpu().numpy() - ref)
+        assert (err <= ROUND[dtype] * np.abs(ref) + 15 * 16 * 2.0 ** -24 * max(1.0, np.abs(ref).max())).all()
+
+
+@pytest.mark.parametrize("tokens", [1, 5, 9, 33, 65, 200])
+@pytest.mark.parametrize("shape", [(96, 160), (1312, 2080), (8224, 64), (64, 16416)], ids=str)
+def test_linear_is_the_transforms_around_the_matrix(shape, tokens):
+    """Whole linears whose block lists mix short, tile-sized and longer-than-tile blocks, through the streaming kernels'
+    and the tensor-core path's activation layouts."""
+    from glq_b200 import synth
+    from glq_b200.plan import block_decompose
+    m, n = shape
+    g = torch.Generator(device="cuda").manual_seed(m + n + tokens)
+    x = torch.randn(tokens, n, generator=g, device="cuda").half()
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda")
+    W = ops.glq_decompress_trellis_3inst_cuda(L.codes[0], m, n).double().cpu().numpy()
+    y = ops.fused_linear_trellis_3inst(x, L.sv, L.su, L.codes[0], None, None, None, None, L.wscale, n, m, n, m,
+                                       out_dtype=torch.float32)
+    _check(x, W, L, y, block_decompose(n), block_decompose(m))
+    if n % 64 == 0 or tokens <= 64:
+        table = synth.load_e8_table("cuda")
+        E = synth.e8_layer("e", m, n, 2, table, g, "cuda")
+        spec = E.spec(batch=ops.token_bucket(tokens), x_dtype=x.dtype, y_dtype=torch.float32)
+        from glq_b200.plan import Plan
+        plan = Plan([spec])
+        xb = x.new_zeros((spec.batch, n))
+        xb[:tokens] = x
+        yb = torch.empty(spec.batch, m, device="cuda")
+        plan.run(xb, yb)
+        nib = (table.cpu().numpy().view(np.uint32)[:, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15
+        cb = nib.astype(np.float64) * 0.5 - 3.0
+        W = sum(s * cb[q.cpu().numpy().view(np.uint16)].reshape(m, n) for q, s in zip(E.codes, [1.0] + list(E.stage_scale)))
+        _check(x, W, E, yb[:tokens], block_decompose(n), block_decompose(m))
+        plan.close()
+
+
+def _check(x, W, L, y, bn, bm):
+    xr = fht64(x.double().cpu().numpy() * L.sv.double().cpu().numpy(), bn)
+    ref = fht64((xr @ W.T) * L.wscale, bm) * L.su.double().cpu().numpy()
+    # the rotated activations (and, above 64 tokens, two-stage weights) are fp16: 2e-3 of the largest output
+    assert np.abs(y.double().cpu().numpy() - ref).max() <= 2e-3 * np.abs(ref).max()
