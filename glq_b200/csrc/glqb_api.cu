@@ -185,8 +185,15 @@ static E8SmemKernel pick_e8_smem_kernel(const Segment& s) {
 #endif
 static long long e8_smem_min_bytes() {
   const char* e = getenv("GLQB_E8_SMEM_MIN_BYTES");
-  // Filling the table costs every CTA about 224 KiB of L2 reads per launch (a few microseconds), so small
-  // launches keep the global-memory gathers.
+  // Filling the table costs every CTA about 224 KiB of L2 reads per launch (a few microseconds), so small launches
+  // keep the global-memory gathers.  Measured, whole linears, gathers / resident: two stages of 4096 x 4096 (8 MiB, 16
+  // tokens) 43 / 39 us, of 14336 x 4096 (28 MiB) one token 64 / 53, 16 tokens 79 / 63; 1024 x 4096 (2 MiB) 34 / 36.
+  return e ? atoll(e) : (6ll << 20);
+}
+// the same for the tile decode of the prefill path (two stages of 14336 x 4096: 57 us either way; three stages of
+// 5376 x 21504: 83 MiB of indices at 258 / 347 G indices per second)
+static long long e8_tiles_smem_min_bytes() {
+  const char* e = getenv("GLQB_E8_SMEM_MIN_BYTES");
   return e ? atoll(e) : (48ll << 20);
 }
 
@@ -226,6 +233,20 @@ static MvKernel pick_kernel(const Segment& s) {
 static int e8_two_phase_min_tokens() {
   const char* e = getenv("GLQB_E8_TWO_PHASE_MIN_TOKENS");
   return e ? atoi(e) : 129;     // measured on B200: above one 128-token tile the tile decode plus a copy-fed GEMM wins
+}
+
+// Trellis prefill decodes the weight tiles once instead of once per 256-token tile from this many flops per layer: the
+// tile decode costs a launch and a write of the fp16 weights (13 us at 11008 x 2048), the copy-fed GEMM saves a third of
+// the fused one's time.  Measured, whole linears, fused / two-phase: 4096 x 4096, 1024 tokens (34 GFLOP) 61 / 69 us,
+// 2048 tokens (69) 114 / 99; 11008 x 2048, 512 tokens (23) 60 / 66, 1024 (46) 93 / 88, 2048 (92) 156 / 141.
+static double trellis_two_phase_min_flops() {
+  const char* e = getenv("GLQB_TRELLIS_TWO_PHASE_MIN_FLOPS");
+  return e ? atof(e) : 40e9;
+}
+// ... and while the tiles of a launch stay below 2 GiB of workspace (a sweep over a whole model keeps the fused form)
+constexpr size_t TRELLIS_TILES_MAX_BYTES = 2ull << 30;
+static size_t tile_bytes(const GlqbLinearDesc& d) {
+  return (size_t)((d.m_pad + GM_TILE_M - 1) / GM_TILE_M) * ((d.n_pad + GM_TILE_K - 1) / GM_TILE_K) * GM_A_BYTES;
 }
 
 static int tn_for_batch(int batch) { return batch <= DECODE_MAX_BATCH ? 0 : (batch <= 128 ? 128 : 256); }
@@ -369,7 +390,8 @@ static int build_plan(GlqbPlan* P) {
     const int tn = tn_for_batch(d.batch);
     const int nb = tn ? 0 : nb_for_batch(d.batch);
     if (d.format == GLQB_FMT_TRELLIS_3INST)
-      k = Key(d.format, d.bits[0], d.n_stages > 1 ? d.bits[1] : 0, d.n_stages, nb, tn, 0);
+      k = Key(d.format, d.bits[0], d.n_stages > 1 ? d.bits[1] : 0, d.n_stages, nb, tn,
+              (tn && 2.0 * d.batch * d.m_pad * d.n_pad >= trellis_two_phase_min_flops()) ? 1 : 0);
     else
       k = Key(d.format, 0, 0, d.n_stages, nb, tn, (tn && d.batch >= e8_two_phase_min_tokens()) ? 1 : 0);
     if (!groups.count(k)) key_order.push_back(k);
@@ -385,6 +407,11 @@ static int build_plan(GlqbPlan* P) {
     s.first = (int)P->order.size();
     s.count = (int)groups[k].size();
     for (int i : groups[k]) P->order.push_back(i);
+    if (s.two_phase && s.format == GLQB_FMT_TRELLIS_3INST) {
+      size_t bytes = 0;
+      for (int i : groups[k]) bytes += tile_bytes(P->descs[i]);
+      if (bytes > TRELLIS_TILES_MAX_BYTES) s.two_phase = 0;
+    }
     if (s.tn ? !gemm_available(s) : !pick_kernel(s))
       return fail(GLQB_E_INVALID, "no kernel variant for format=%d K=%d+%d stages=%d token blocks=%d", s.format,
                   s.k1, s.k2, s.ns, s.nb);
@@ -600,14 +627,13 @@ static int build_plan(GlqbPlan* P) {
       s.total_groups = 0;
       s.per_warp = 1;
       CUDA_TRY(gemm_prepare(s));
-      if (s.two_phase) {
-        // tile decode with the codebook resident in shared memory, under the same conditions as the
-        // streaming kernel's resident form
+      if (s.two_phase && s.format == GLQB_FMT_E8_SHELL) {
+        // tile decode with the codebook resident in shared memory
         long long bytes = 0;
         const uint32_t* big = nullptr;
         const uint32_t* small = nullptr;
         int small_n = 0;
-        if (e8_uniform_tables(P->dev, s, &big, &small, &small_n, &bytes) && bytes >= e8_smem_min_bytes() &&
+        if (e8_uniform_tables(P->dev, s, &big, &small, &small_n, &bytes) && bytes >= e8_tiles_smem_min_bytes() &&
             tiles_smem_prepare(s.ns) == cudaSuccess) {
           s.smem_table = true;
           s.big_table = big;
@@ -1131,7 +1157,7 @@ size_t glqb_linear_workspace_bytes(const GlqbLinearDesc* desc) {
   // Upper bound that does not depend on the device, with the roundings build_plan applies: activations
   // (E8 batches are padded to 8 tokens; the GEMM path stores whole token tiles of whole 64-column chunks),
   // the largest possible number of partial-sum slots (one per work group of a strip, plus one), and for
-  // E8 above 128 tokens the decoded fp16 weight tiles.
+  // more than 128 tokens the decoded fp16 weight tiles.
   if (!desc) return 0;
   const size_t batch = (size_t)std::max(1, desc->batch);
   const int tn = tn_for_batch((int)batch);
@@ -1140,8 +1166,7 @@ size_t glqb_linear_workspace_bytes(const GlqbLinearDesc* desc) {
     const size_t n_tiles = (batch + tn - 1) / tn, kchunks = ((size_t)desc->n_pad + GM_TILE_K - 1) / GM_TILE_K;
     ws += align_up(n_tiles * kchunks * tn * 128, 1024);
     ws += align_up(16 * batch * desc->m_pad * 4, 1024);                      // at most 16 K splits
-    if (desc->format == GLQB_FMT_E8_SHELL)
-      ws += align_up((size_t)((desc->m_pad + GM_TILE_M - 1) / GM_TILE_M) * kchunks * GM_A_BYTES, 1024) + 1024;
+    ws += align_up(tile_bytes(*desc), 1024) + 1024;                          // (the two-phase forms)
   } else {
     const size_t gps = desc->format == GLQB_FMT_TRELLIS_3INST ? desc->n_pad / 32 : (desc->n_pad + 255) / 256;
     ws += align_up(((batch + 7) / 8 * 8) * desc->n_pad * 2 * XR_TRELLIS_EXPAND, 1024);

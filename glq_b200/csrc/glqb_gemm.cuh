@@ -222,29 +222,36 @@ static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_gemm_kern
 }
 
 // ---- weight producers ------------------------------------------------------------------------------
-// One trellis group (32 rows x 32 columns) -> its place in the 128 x 64 A tile.
-__device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-// Byte offsets (inside a swizzled 128 x 64 tile) of the 16 register pairs a lane stores per group:
-// entry q*4 + p with q = ni*2 + mi the 16x16 tile and p = c*2 + a the pair; fixed per thread.
-__device__ __forceinline__ void gemm_lane_offsets(int strip, int cg, int lane, uint32_t (&off)[16]) {
+// Where a lane's 16 register pairs of a 32 x 32 group go inside the 32-row slice of a swizzled 128 x 64 tile: pair
+// (ni, c, mi, a) at addr[ni * 2 + c] + mi * 2048 + a * 1024.  Only the 16-byte unit is swizzled, so four addresses and
+// immediate offsets cover all sixteen.
+__device__ __forceinline__ void gemm_lane_addrs(uint32_t slice, int cg, int lane, uint32_t (&addr)[4]) {
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      const int ni = q >> 1, mi = q & 1, c = p >> 1, a_ = p & 1;
-      off[q * 4 + p] = sw128_offset(strip * 32 + mi * 16 + 8 * a_ + g, cg * 32 + ni * 16 + 8 * c + 2 * t);
-    }
+  for (int u = 0; u < 4; ++u) addr[u] = slice + (uint32_t)(g * 128 + (((cg * 4 + u) ^ g) << 4) + t * 4);
+}
+template <int OFF>
+__device__ __forceinline__ void st_shared_u32_at(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.u32 [%0 + %2], %1;" ::"r"(addr), "r"(v), "n"(OFF) : "memory");
+}
+__device__ __forceinline__ void gemm_store_quad(const uint32_t (&addr)[4], int q, const uint32_t (&w)[4]) {
+  // q = ni * 2 + mi; w[p], p = c * 2 + a
+  const uint32_t a0 = addr[(q >> 1) * 2], a1 = addr[(q >> 1) * 2 + 1];
+  if (q & 1) {
+    st_shared_u32_at<2048>(a0, w[0]); st_shared_u32_at<3072>(a0, w[1]);
+    st_shared_u32_at<2048>(a1, w[2]); st_shared_u32_at<3072>(a1, w[3]);
+  } else {
+    st_shared_u32_at<0>(a0, w[0]); st_shared_u32_at<1024>(a0, w[1]);
+    st_shared_u32_at<0>(a1, w[2]); st_shared_u32_at<1024>(a1, w[3]);
+  }
 }
 
 template <int K1, int K2>
-__device__ __forceinline__ void gemm_store_group(uint32_t a_tile, const uint32_t (&off)[16], int lane, const Words<K1>& v,
+__device__ __forceinline__ void gemm_store_group(const uint32_t (&addr)[4], int lane, const Words<K1>& v,
                                                  const Words<(K2 > 0 ? K2 : 1)>& v2, __half2 s2) {
   const Words<K1> vn = shfl_words<K1>(v, (lane + 1) & 31);
   Words<K1> vn2 = vn;
@@ -256,25 +263,21 @@ __device__ __forceinline__ void gemm_store_group(uint32_t a_tile, const uint32_t
     if constexpr (K2 == 1) un2 = shfl_words<K2>(v2, (lane + 2) & 31);
   }
 #pragma unroll
-  for (int ni = 0; ni < 2; ++ni) {
+  for (int q = 0; q < 4; ++q) {
+    uint32_t a[8], b[8], w[4];
+    decode_tile<K1>(chunk_of<K1>(v, q), chunk_of<K1>(vn, q), chunk_of<K1>(vn2, q), a);
+    if constexpr (K2 > 0) decode_tile<K2>(chunk_of<K2>(v2, q), chunk_of<K2>(un, q), chunk_of<K2>(un2, q), b);
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi) {
-      const int q = ni * 2 + mi;
-      uint32_t a[8], b[8];
-      decode_tile<K1>(chunk_of<K1>(v, q), chunk_of<K1>(vn, q), chunk_of<K1>(vn2, q), a);
-      if constexpr (K2 > 0) decode_tile<K2>(chunk_of<K2>(v2, q), chunk_of<K2>(un, q), chunk_of<K2>(un2, q), b);
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        uint32_t w = __byte_perm(a[2 * p], a[2 * p + 1], 0x5410);        // (w_{2p}, w_{2p+1})
-        if constexpr (K2 > 0) {
-          // second stage folded into the fp16 operand: w = fp16(w1 + s2 * w2), one rounding
-          const uint32_t w2 = __byte_perm(b[2 * p], b[2 * p + 1], 0x5410);
-          const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&w2), s2, *reinterpret_cast<const __half2*>(&w));
-          w = *reinterpret_cast<const uint32_t*>(&r);
-        }
-        st_shared_u32(a_tile + off[q * 4 + p], w);
+    for (int p = 0; p < 4; ++p) {
+      w[p] = __byte_perm(a[2 * p], a[2 * p + 1], 0x5410);        // (w_{2p}, w_{2p+1})
+      if constexpr (K2 > 0) {
+        // second stage folded into the fp16 operand: w = fp16(w1 + s2 * w2), one rounding
+        const uint32_t w2 = __byte_perm(b[2 * p], b[2 * p + 1], 0x5410);
+        const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&w2), s2, *reinterpret_cast<const __half2*>(&w[p]));
+        w[p] = *reinterpret_cast<const uint32_t*>(&r);
       }
     }
+    gemm_store_quad(addr, q, w);
   }
 }
 
@@ -350,8 +353,8 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
         const uint8_t* p2 = nullptr;
         if constexpr (K2 > 0) p2 = L.codes[1] + ((long long)rp * gps) * (128 * K2) + lane * (4 * K2);
         const __half2 s2 = __float2half2_rn(L.stage_scale[1]);
-        uint32_t off[16];
-        gemm_lane_offsets(strip, cg, lane, off);
+        uint32_t lane_addr[4];                            // of stage 0
+        gemm_lane_addrs(smem_u32(a_base) + strip * 4096, cg, lane, lane_addr);
         Words<K1> nxt;
         Words<(K2 > 0 ? K2 : 1)> nxt2;
         auto fetch = [&](int kc) {
@@ -371,14 +374,17 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
           const bool valid = row_ok && (kc * 2 + cg) < gps;
           if (kc + 2 < it.k_end) fetch(kc + 2);
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
-          const uint32_t a_tile = smem_u32(a_base) + stage * GM_A_BYTES;
+          uint32_t addr[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) addr[u] = lane_addr[u] + stage * GM_A_BYTES;
           if (valid) {
-            gemm_store_group<K1, K2>(a_tile, off, lane, v, v2, s2);
+            gemm_store_group<K1, K2>(addr, lane, v, v2, s2);
           } else {
             // rows or columns past the matrix: zeros (validity is uniform per warp, so the shuffles
             // inside the decode always see all 32 lanes)
+            const uint32_t zero[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-            for (int i = 0; i < 16; ++i) st_shared_u32(a_tile + off[i], 0u);
+            for (int q4 = 0; q4 < 4; ++q4) gemm_store_quad(addr, q4, zero);
           }
           fence_async_smem();
           __syncwarp();
@@ -585,16 +591,20 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
 // For large token counts the fused kernel would decode every weight tile once per token tile; this
 // kernel decodes each 128 x 64 tile ONCE into the exact shared-memory image (K-major, 128-byte swizzle),
 // [m_tile][k_chunk] x 16 KiB, which glq_gemm_kernel<2,...> then fetches with one bulk copy per stage.
-// A CTA takes 128 rows x 4 consecutive chunks; thread (row = tid >> 1, half = tid & 1) reads the 16 indices
-// of two chunks with two 16-byte loads per stage (the two threads of a row read 64 contiguous bytes), keeps
-// all 16 * NS gathers in flight, and writes two full 128-byte tile rows.
-// TM = 0: table gathers from global memory, one unit per 256-thread CTA.  TM = 1: most of the table resident in
-// shared memory (see e8_gather), 512-thread CTA = two units side by side, one CTA per SM.
+// A warp takes 8 rows x 4 consecutive chunks.  Indices: one 16-byte load per lane and stage, requested a unit ahead, turned
+// through 512 bytes of shared memory so that lane (c, k) gets index k of chunk c, row after row: a row's four decoded
+// 128-byte tile rows are then one store of whole lines (a thread per row, 16 bytes of 32 different lines per store
+// instruction, spent more of the L1 pipe on stores than on the gathers).  8 x NS gathers are in flight per lane.
+// Bound by the gathers; two stages of 14336 x 4096 94 -> 57 us, three of 5376 x 21504 (resident) 157 -> 124 us.
+// TM = 0: table gathers from global memory.  TM = 1: most of the table resident in shared memory (see e8_gather), one
+// CTA per SM.
+constexpr int E8T_ROWS = 8;
+constexpr int E8T_RESIDENT = 54 * 1024;          // leaves 512 bytes per warp for the indices
 template <int NS, int TM>
 __device__ __forceinline__ void e8_tiles_body(const DevLinear* __restrict__ layers, int first, int count,
-                                              uint8_t* __restrict__ ws, const E8Tables& T, int unit0, int unit_stride,
-                                              int tid) {
-  const int row_l = tid >> 1, hf = tid & 1;
+                                              uint8_t* __restrict__ ws, const E8Tables& T, int warp0, int warps, uint4* buf) {
+  const int lane = threadIdx.x & 31, c = lane >> 3, k = lane & 7;
+  const uint16_t* mine = reinterpret_cast<const uint16_t*>(buf) + c * 8 + k;       // + 32 per row
   for (int li = first; li < first + count; ++li) {
     const DevLinear& L = layers[li];
     const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
@@ -615,61 +625,72 @@ __device__ __forceinline__ void e8_tiles_body(const DevLinear* __restrict__ laye
       sc[s] = __float2half2_rn(L.stage_scale[s]);
     }
     uint8_t* tiles = ws + L.atile_off;
-    for (int u = unit0; u < m_tiles * kgroups; u += unit_stride) {
-      const int mt = u / kgroups, kg = u - mt * kgroups;
-      const int row = mt * GM_TILE_M + row_l;
-      const bool row_ok = row < m;
-      const int kc0 = kg * 4 + hf * 2;
-      uint32_t ent[NS][2][8];
+    const int units = m_tiles * kgroups * (GM_TILE_M / E8T_ROWS);
+    uint4 nxt[NS];
+    auto fetch = [&](int u) {
+      const int t = u / (GM_TILE_M / E8T_ROWS), mt = t / kgroups;
+      const int row = mt * GM_TILE_M + (u % (GM_TILE_M / E8T_ROWS)) * E8T_ROWS + (lane >> 2);
+      const int i0 = ((t - mt * kgroups) * 4 + (lane & 3)) * 8;
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
-        const uint16_t* q = codes[s] + (long long)row * nidx;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int i0 = (kc0 + c) * 8;
+        nxt[s] = make_uint4(0u, 0u, 0u, 0u);
+        const uint16_t* q = codes[s] + (long long)row * nidx + i0;
+        if (row < m && vec_ok && i0 + 8 <= nidx) {
+          nxt[s] = ld_stream_v4(q);
+        } else if (row < m) {
           uint32_t w[4] = {0u, 0u, 0u, 0u};
-          if (row_ok && vec_ok && i0 + 8 <= nidx) {
-            const uint4 t = ld_stream_v4(q + i0);
-            w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
-          } else if (row_ok) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-              if (i0 + k < nidx) w[k >> 1] |= (uint32_t)q[i0 + k] << ((k & 1) * 16);
-          }
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            ent[s][c][k] = e8_gather<TM>(stg[s], ((w[k >> 1] >> ((k & 1) * 16)) & 0xFFFFu) & stg[s].mask);
+          for (int z = 0; z < 8; ++z)
+            if (i0 + z < nidx) w[z >> 1] |= (uint32_t)q[z] << ((z & 1) * 16);
+          nxt[s] = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
+    };
+    if (warp0 < units) fetch(warp0);
+    for (int u = warp0; u < units; u += warps) {
+      const int r8 = u % (GM_TILE_M / E8T_ROWS), t = u / (GM_TILE_M / E8T_ROWS);
+      const int mt = t / kgroups, kc = (t - mt * kgroups) * 4 + c;
+      const int row0 = r8 * E8T_ROWS;                             // first row inside the tile
+      uint32_t ent[NS][E8T_ROWS];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int kc = kc0 + c;
-        if (kc >= kchunks) continue;
-        uint8_t* tile = tiles + ((size_t)mt * kchunks + kc) * GM_A_BYTES;
+      for (int s = 0; s < NS; ++s) {
+        buf[lane] = nxt[s];
+        __syncwarp();
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          uint4 out = make_uint4(0u, 0u, 0u, 0u);
-          if (row_ok && kc * 8 + k < nidx) {
-            uint32_t h[4];
-            e8_entry_to_half2(ent[0][c][k], h);
+        for (int r = 0; r < E8T_ROWS; ++r) ent[s][r] = mine[r * 32];
+        __syncwarp();
+      }
+      if (u + warps < units) fetch(u + warps);
 #pragma unroll
-            for (int s = 1; s < NS; ++s) {
-              uint32_t h2[4];
-              e8_entry_to_half2(ent[s][c][k], h2);
+      for (int s = 0; s < NS; ++s)
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&h2[j]), sc[s], *reinterpret_cast<const __half2*>(&h[j]));
-                h[j] = *reinterpret_cast<const uint32_t*>(&r);
-              }
+        for (int r = 0; r < E8T_ROWS; ++r) ent[s][r] = e8_gather<TM, E8T_RESIDENT>(stg[s], ent[s][r] & stg[s].mask);
+      if (kc >= kchunks) continue;
+      const bool col_ok = kc * 8 + k < nidx;
+      uint8_t* tile = tiles + ((size_t)mt * kchunks + kc) * GM_A_BYTES + row0 * 128;
+#pragma unroll
+      for (int r = 0; r < E8T_ROWS; ++r) {
+        uint4 out = make_uint4(0u, 0u, 0u, 0u);
+        if (col_ok && mt * GM_TILE_M + row0 + r < m) {
+          uint32_t h[4];
+          e8_entry_to_half2(ent[0][r], h);
+#pragma unroll
+          for (int s = 1; s < NS; ++s) {
+            uint32_t h2[4];
+            e8_entry_to_half2(ent[s][r], h2);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const __half2 z = __hfma2(*reinterpret_cast<const __half2*>(&h2[j]), sc[s], *reinterpret_cast<const __half2*>(&h[j]));
+              h[j] = *reinterpret_cast<const uint32_t*>(&z);
             }
-            // natural column order inside the 16-byte chunk: (c0,c1),(c2,c3),(c4,c5),(c6,c7)
-            out.x = __byte_perm(h[0], h[1], 0x5410);
-            out.y = __byte_perm(h[2], h[3], 0x5410);
-            out.z = __byte_perm(h[0], h[1], 0x7632);
-            out.w = __byte_perm(h[2], h[3], 0x7632);
           }
-          *reinterpret_cast<uint4*>(tile + sw128_offset(row_l, k * 8)) = out;
+          // natural column order inside the 16-byte chunk: (c0,c1),(c2,c3),(c4,c5),(c6,c7)
+          out.x = __byte_perm(h[0], h[1], 0x5410);
+          out.y = __byte_perm(h[2], h[3], 0x5410);
+          out.z = __byte_perm(h[0], h[1], 0x7632);
+          out.w = __byte_perm(h[2], h[3], 0x7632);
         }
+        *reinterpret_cast<uint4*>(tile + r * 128 + ((k ^ r) << 4)) = out;        // (sw128_offset; row0 is a multiple of 8)
       }
     }
   }
@@ -678,26 +699,93 @@ __device__ __forceinline__ void e8_tiles_body(const DevLinear* __restrict__ laye
 template <int NS>
 __global__ void __launch_bounds__(256) e8_tiles_kernel(const DevLinear* __restrict__ layers, int first, int count,
                                                        uint8_t* __restrict__ ws) {
+  __shared__ uint4 idx[8][32];
   const E8Tables T = {0u, 0u};
-  e8_tiles_body<NS, 0>(layers, first, count, ws, T, blockIdx.x, gridDim.x, threadIdx.x);
+  e8_tiles_body<NS, 0>(layers, first, count, ws, T, blockIdx.x * 8 + (threadIdx.x >> 5), gridDim.x * 8, idx[threadIdx.x >> 5]);
 }
 
 constexpr int E8TS_THREADS = 512;
+constexpr int E8TS_SMEM_BYTES = E8T_RESIDENT * 4 + 256 * 4 + E8TS_THREADS / 32 * 512;
 template <int NS>
 __global__ void __launch_bounds__(E8TS_THREADS, 1)
 e8_tiles_smem_kernel(const DevLinear* __restrict__ layers, int first, int count, uint8_t* __restrict__ ws,
                      const uint32_t* __restrict__ big_table, const uint32_t* __restrict__ small_table, int small_entries) {
-  extern __shared__ __align__(16) uint32_t e8t_smem[];
+  extern __shared__ __align__(16) uint32_t e8t_smem[];    // table, small table, 512 bytes of indices per warp
   const uint4* src = reinterpret_cast<const uint4*>(big_table);
   uint4* dst = reinterpret_cast<uint4*>(e8t_smem);
-  for (int i = threadIdx.x; i < E8S_RESIDENT / 4; i += blockDim.x) dst[i] = __ldg(src + i);
-  for (int i = threadIdx.x; i < small_entries && i < 256; i += blockDim.x) e8t_smem[E8S_RESIDENT + i] = __ldg(small_table + i);
+  for (int i = threadIdx.x; i < E8T_RESIDENT / 4; i += blockDim.x) dst[i] = __ldg(src + i);
+  for (int i = threadIdx.x; i < small_entries && i < 256; i += blockDim.x) e8t_smem[E8T_RESIDENT + i] = __ldg(small_table + i);
   E8Tables T;
   const uint32_t local = (uint32_t)__cvta_generic_to_shared(e8t_smem);
   T.table_base = local;
-  T.small_base = local + E8S_RESIDENT * 4;
+  T.small_base = local + E8T_RESIDENT * 4;
   __syncthreads();
-  e8_tiles_body<NS, 1>(layers, first, count, ws, T, blockIdx.x * 2 + (threadIdx.x >> 8), gridDim.x * 2, threadIdx.x & 255);
+  const int warp = threadIdx.x >> 5;
+  e8_tiles_body<NS, 1>(layers, first, count, ws, T, blockIdx.x * (E8TS_THREADS / 32) + warp, gridDim.x * (E8TS_THREADS / 32),
+                       reinterpret_cast<uint4*>(e8t_smem + E8T_RESIDENT + 256) + warp * 32);
+}
+
+// ---- decode once: trellis bit-streams -> swizzled fp16 weight tiles ------------------------------------------
+// The counterpart of e8_tiles_kernel: a warp decodes a 32-row x 64-column slice (two 32 x 32 groups) into its own 4 KiB of
+// shared memory with the stores the GEMM's producers use — the slice is 4 KiB of the tile image in one piece — and
+// copies it out with whole-line 16-byte stores.  The codes of the next slice are in flight meanwhile.  Bound by the
+// state decode: 11008 x 2048 in 13 us; with the copy-fed GEMM behind it 97 us where the fused GEMM takes 117 (2048
+// tokens).
+constexpr int TT_THREADS = 256;
+template <int K1, int K2>
+__global__ void __launch_bounds__(TT_THREADS, 3)
+trellis_tiles_kernel(const DevLinear* __restrict__ layers, int first, int count, uint8_t* __restrict__ ws) {
+  __shared__ __align__(1024) uint8_t slices[TT_THREADS / 32][4096];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warp0 = blockIdx.x * (TT_THREADS / 32) + warp, warps = gridDim.x * (TT_THREADS / 32);
+  const uint32_t slice = smem_u32(slices[warp]);
+  uint32_t addr[2][4];
+  gemm_lane_addrs(slice, 0, lane, addr[0]);
+  gemm_lane_addrs(slice, 1, lane, addr[1]);
+  for (int li = first; li < first + count; ++li) {
+    const DevLinear& L = layers[li];
+    const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K, gps = L.groups_per_strip, strips = L.strips;
+    const int units = ((L.m + GM_TILE_M - 1) / GM_TILE_M) * 4 * kchunks;      // 32-row slices of whole tiles
+    const __half2 s2 = __float2half2_rn(L.stage_scale[1]);
+    uint8_t* tiles = ws + L.atile_off;
+    const uint8_t* p1 = L.codes[0] + lane * (4 * K1);
+    const uint8_t* p2 = K2 > 0 ? L.codes[1] + lane * (4 * K2) : nullptr;
+    Words<K1> v[2];
+    Words<(K2 > 0 ? K2 : 1)> v2[2];
+    auto fetch = [&](int u) {
+      const int strip = u / kchunks, kc = u - strip * kchunks;
+#pragma unroll
+      for (int cg = 0; cg < 2; ++cg)
+        if (strip < strips && kc * 2 + cg < gps) {
+          const long long g = (long long)strip * gps + kc * 2 + cg;
+          v[cg] = load_words<K1>(p1 + g * (128 * K1));
+          if constexpr (K2 > 0) v2[cg] = load_words<K2>(p2 + g * (128 * K2));
+        }
+    };
+    if (warp0 < units) fetch(warp0);
+    for (int u = warp0; u < units; u += warps) {
+      const int strip = u / kchunks, kc = u - strip * kchunks;
+      const Words<K1> cur[2] = {v[0], v[1]};
+      const Words<(K2 > 0 ? K2 : 1)> cur2[2] = {v2[0], v2[1]};
+      if (u + warps < units) fetch(u + warps);
+#pragma unroll
+      for (int cg = 0; cg < 2; ++cg) {
+        if (strip < strips && kc * 2 + cg < gps) {
+          gemm_store_group<K1, K2>(addr[cg], lane, cur[cg], cur2[cg], s2);
+        } else {                                             // rows or columns past the matrix: zeros
+          const uint32_t zero[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) gemm_store_quad(addr[cg], q, zero);
+        }
+      }
+      __syncwarp();
+      uint4* dst = reinterpret_cast<uint4*>(tiles + ((size_t)(strip >> 2) * kchunks + kc) * GM_A_BYTES + (strip & 3) * 4096) + lane;
+      const uint4* src = reinterpret_cast<const uint4*>(slices[warp]) + lane;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) dst[i * 32] = src[i * 32];
+      __syncwarp();
+    }
+  }
 }
 
 }  // namespace glqb

@@ -36,6 +36,18 @@ static TilesKernel pick_tiles_kernel(int ns) {
   return nullptr;
 }
 
+static TilesKernel pick_trellis_tiles_kernel(int k1, int k2) {
+#define T_CASE(A, B) if (k1 == A && k2 == B) return trellis_tiles_kernel<A, B>;
+#ifdef GLQB_FAST_BUILD
+  T_CASE(4, 0)
+#else
+  T_CASE(1, 0) T_CASE(2, 0) T_CASE(3, 0) T_CASE(4, 0)
+  T_CASE(4, 1) T_CASE(4, 2) T_CASE(4, 3) T_CASE(4, 4)
+#endif
+#undef T_CASE
+  return nullptr;
+}
+
 static GemmKernel pick_gemm_kernel(const Segment& s) {
   if (s.two_phase) return gemm_kernel_tn<2, 0, 0>(s.tn);
   if (s.format == GLQB_FMT_TRELLIS_3INST) {
@@ -70,13 +82,15 @@ cudaError_t gemm_prepare(const Segment& s) {
 }
 
 cudaError_t tiles_smem_prepare(int ns) {
-  return cudaFuncSetAttribute(pick_tiles_smem_kernel(ns), cudaFuncAttributeMaxDynamicSharedMemorySize, E8S_SMEM_BYTES);
+  return cudaFuncSetAttribute(pick_tiles_smem_kernel(ns), cudaFuncAttributeMaxDynamicSharedMemorySize, E8TS_SMEM_BYTES);
 }
 
 void gemm_launch(const Segment& s, const DevLinear* layers, const GemmItem* items, uint8_t* ws, int* status,
                  int sm_count, cudaStream_t stream) {
-  if (s.two_phase && s.smem_table)
-    pick_tiles_smem_kernel(s.ns)<<<sm_count, E8TS_THREADS, E8S_SMEM_BYTES, stream>>>(
+  if (s.two_phase && s.format == GLQB_FMT_TRELLIS_3INST)
+    pick_trellis_tiles_kernel(s.k1, s.k2)<<<sm_count * 3, TT_THREADS, 0, stream>>>(layers, s.first, s.count, ws);
+  else if (s.two_phase && s.smem_table)
+    pick_tiles_smem_kernel(s.ns)<<<sm_count, E8TS_THREADS, E8TS_SMEM_BYTES, stream>>>(
         layers, s.first, s.count, ws, s.big_table, s.small_table, s.small_entries);
   else if (s.two_phase)
     pick_tiles_kernel(s.ns)<<<sm_count * 8, 256, 0, stream>>>(layers, s.first, s.count, ws);

@@ -401,7 +401,7 @@ struct E8Stage {
 
 // The gathers are volatile so that they keep their place ahead of the (volatile) MMAs of the chunk being
 // consumed: that ordering is what keeps a whole chunk of gathers in flight.
-template <int TM>
+template <int TM, int RESIDENT = E8S_RESIDENT>
 __device__ __forceinline__ uint32_t e8_gather(const E8Stage& S, uint32_t idx) {
   uint32_t v;
   const uint32_t* gp = S.table + idx;
@@ -414,7 +414,7 @@ __device__ __forceinline__ uint32_t e8_gather(const E8Stage& S, uint32_t idx) {
                  "@!p ld.shared.u32 %0, [%3];\n\t"
                  "@p ld.global.nc.u32 %0, [%4];\n\t}"
                  : "=r"(v)
-                 : "r"(idx), "r"((uint32_t)E8S_RESIDENT), "r"(S.base + (idx << 2)), "l"(gp));
+                 : "r"(idx), "r"((uint32_t)RESIDENT), "r"(S.base + (idx << 2)), "l"(gp));
   }
   return v;
 }

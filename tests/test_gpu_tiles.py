@@ -1,0 +1,48 @@
+"""The decode-once forms of the prefill path against the fused one: the same fp16 weights, so the same bits."""
+import pytest
+import torch
+
+from glq_b200 import synth
+from glq_b200.plan import Plan
+
+pytestmark = pytest.mark.gpu
+
+
+def run(layer, x, monkeypatch, env):
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    y = torch.full((x.shape[0], layer.m), float("nan"), device="cuda")
+    plan = Plan([layer.spec(batch=x.shape[0], x_dtype=x.dtype, y_dtype=torch.float32)])
+    plan.run(x, y)
+    plan.check_status()
+    n = plan.launches
+    plan.close()
+    return y, n
+
+
+# rows that end inside a 128-row tile and a 32-row slice, columns that end inside a 64-column chunk
+@pytest.mark.parametrize("bits", [[1], [2], [3], [4], [4, 1], [4, 2], [4, 3], [4, 4]], ids=str)
+@pytest.mark.parametrize("shape", [(32, 32), (160, 96), (256, 64), (416, 1056)], ids=str)
+def test_trellis_tiles_equal_fused(shape, bits, monkeypatch):
+    m, n = shape
+    g = torch.Generator(device="cuda").manual_seed(m + n + sum(bits))
+    L = synth.trellis_layer("t", m, n, bits, g, "cuda")
+    x = torch.randn(300, n, generator=g, device="cuda").half()
+    a, na = run(L, x, monkeypatch, {"GLQB_TRELLIS_TWO_PHASE_MIN_FLOPS": "1"})
+    b, nb = run(L, x, monkeypatch, {"GLQB_TRELLIS_TWO_PHASE_MIN_FLOPS": "1e30"})
+    assert na == nb + 1
+    assert torch.equal(a, b)
+
+
+# index rows that are not 16-byte aligned, a last group of fewer than four chunks, a last chunk of fewer than eight
+@pytest.mark.parametrize("stages", [1, 2, 3, 4])
+@pytest.mark.parametrize("shape", [(24, 8), (136, 264), (256, 1024), (400, 1096)], ids=str)
+def test_e8_tiles_equal_fused(shape, stages, monkeypatch):
+    m, n = shape
+    g = torch.Generator(device="cuda").manual_seed(m + n + stages)
+    L = synth.e8_layer("e", m, n, stages, synth.load_e8_table("cuda"), g, "cuda")
+    x = torch.randn(300, n, generator=g, device="cuda").half()
+    fused, _ = run(L, x, monkeypatch, {"GLQB_E8_TWO_PHASE_MIN_TOKENS": "100000"})
+    for resident in ("0", str(1 << 40)):
+        tiles, _ = run(L, x, monkeypatch, {"GLQB_E8_TWO_PHASE_MIN_TOKENS": "65", "GLQB_E8_SMEM_MIN_BYTES": resident})
+        assert torch.equal(tiles, fused)
