@@ -619,7 +619,7 @@ static int build_plan(GlqbPlan* P) {
         for (int mt = 0; mt < m_tiles; ++mt)
           for (int nt = 0; nt < n_tiles; ++nt)
             for (int k = 0; k < ks; ++k)
-              P->gemm_items.push_back(GemmItem{s.first + i, mt, nt, k * per, std::min(kchunks, (k + 1) * per), k});
+              P->gemm_items.push_back(GemmItem{s.first + i, mt, nt, k * per, std::min(kchunks, (k + 1) * per), k, 0, 0, 0});
         P->max_batch_gemm = std::max(P->max_batch_gemm, L.batch);
       }
       s.item_count = (int)P->gemm_items.size() - s.item_first;

@@ -37,6 +37,8 @@ struct GemmItem {
   int k_begin;     // first 64-column chunk
   int k_end;       // one past the last chunk
   int slot;        // partial-sum slot this item writes
+  int tok0, ntok;  // variable token tiles (grouped experts): first token and tokens of the tile inside its layer,
+  int row0;        // and the 128-byte rows of activations in front of it, see glq_gemm_kernel
 };
 
 // ---- PTX wrappers ---------------------------------------------------------------------------------
@@ -285,6 +287,10 @@ __device__ __forceinline__ void gemm_store_group(const uint32_t (&addr)[4], int 
 // FORMAT 0: trellis (K1, K2 bits); FORMAT 1: E8 (K1 = number of stages, K2 unused);
 // FORMAT 2: the weight tiles were decoded beforehand (e8_tiles_kernel) and are fetched like the
 //           activation tiles, one bulk copy per stage; the producer warps have nothing to do
+// TN > 256: variable token tiles of up to TN tokens (a multiple of 64), for grouped experts.  A tile's activations are
+// rows of ntok rounded up to 16, [k chunk][row] behind the row0 rows of the tiles before it; an item multiplies exactly
+// that many columns (two MMAs beyond 256), so an expert's weights are decoded once for up to TN tokens and no time goes
+// into padding.  One accumulator (the columns of two would not fit): the stages run ahead while it is drained.
 template <int FORMAT, int K1, int K2, int TN, int STAGES>
 __global__ void __launch_bounds__(GM_THREADS, 1)
 glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict__ items, int n_items,
@@ -292,6 +298,8 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
   // work lists built on the device (grouped expert matmul) pass their length through memory
   if (n_items_dev) n_items = min(n_items, *n_items_dev);
   constexpr int B_BYTES = TN * 128;
+  constexpr bool VAR = TN > 256;
+  constexpr int TMEM_COLS = VAR ? 512 : 2 * TN;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* a_base = smem;                                   // STAGES x 16 KiB
@@ -322,7 +330,7 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
     fence_mbar_init();
   }
   if (warp == GM_MMA_WARP) {
-    tmem_alloc(tmem_slot, 2 * TN);
+    tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -480,12 +488,13 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0, seq = 0;
-      const uint32_t idesc = umma_idesc_f16(TN);
       bool ok = true;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
         const GemmItem it = items[item];
-        const uint32_t a = seq & 1u, a_phase = (seq >> 1) & 1u;     // accumulator and its use count parity
+        const uint32_t a = VAR ? 0u : seq & 1u, a_phase = (VAR ? seq : seq >> 1) & 1u;     // accumulator and its use count parity
         const uint32_t d_tmem = tmem_acc + a * TN;
+        const int cols = VAR ? (it.ntok + 15) & ~15 : TN, cols0 = VAR ? min(cols, 256) : TN;
+        const uint32_t idesc = umma_idesc_f16(cols0), idesc1 = VAR ? umma_idesc_f16(max(16, cols - cols0)) : 0u;
         if (!mbar_wait(&acc_empty[a], a_phase ^ 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         for (int kc = it.k_begin; kc < it.k_end; ++kc) {
@@ -496,6 +505,13 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
 #pragma unroll
           for (int k = 0; k < GM_TILE_K / 16; ++k)      // +32 bytes (2 x 16-byte units) per K step of 16
             umma_f16(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kc > it.k_begin || k > 0) ? 1u : 0u);
+          if constexpr (VAR) {
+            if (cols > 256) {                            // rows 256 on of the activation tile: 32 KiB further
+#pragma unroll
+              for (int k = 0; k < GM_TILE_K / 16; ++k)
+                umma_f16(d_tmem + 256, da + (uint64_t)(2 * k), db + (uint64_t)(2048 + 2 * k), idesc1, (kc > it.k_begin || k > 0) ? 1u : 0u);
+            }
+          }
           umma_commit(&empty[stage]);                    // stage reusable once these MMAs have read it
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -514,7 +530,8 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
         const GemmItem it = items[item];
         const DevLinear& L = layers[it.layer];
         const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
-        const uint8_t* src = ws + L.xr_off + ((size_t)it.n_tile * kchunks) * B_BYTES;
+        const uint32_t b_bytes = VAR ? (uint32_t)((it.ntok + 15) & ~15) * 128u : (uint32_t)B_BYTES;
+        const uint8_t* src = ws + L.xr_off + (VAR ? (size_t)it.row0 * kchunks * 128 : (size_t)it.n_tile * kchunks * B_BYTES);
         for (int kc = it.k_begin; kc < it.k_end; ++kc) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
           if constexpr (FORMAT == 2) {
@@ -522,9 +539,9 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
             bulk_g2s(a_base + stage * GM_A_BYTES,
                      ws + L.atile_off + ((size_t)it.m_tile * kchunks + kc) * GM_A_BYTES, GM_A_BYTES, &full_b[stage]);
           } else {
-            mbar_expect_tx(&full_b[stage], B_BYTES);
+            mbar_expect_tx(&full_b[stage], b_bytes);
           }
-          bulk_g2s(b_base + stage * B_BYTES, src + (size_t)kc * B_BYTES, B_BYTES, &full_b[stage]);
+          bulk_g2s(b_base + stage * B_BYTES, src + (size_t)kc * b_bytes, b_bytes, &full_b[stage]);
           ++loads_issued;
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -540,21 +557,27 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
       const GemmItem it = items[item];
       const DevLinear& L = layers[it.layer];
-      const uint32_t a = seq & 1u, a_phase = (seq >> 1) & 1u;
+      const uint32_t a = VAR ? 0u : seq & 1u, a_phase = (VAR ? seq : seq >> 1) & 1u;
       if (!mbar_wait(&acc_full[a], a_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const int row = it.m_tile * GM_TILE_M + quarter * 32 + lane;
-      float* part = reinterpret_cast<float*>(ws + L.part_off) + (long long)it.slot * L.batch * L.m;
+      const int m = L.m, first = VAR ? it.tok0 : it.n_tile * TN;
+      const int cols = VAR ? it.ntok : min(TN, L.batch - first);        // columns that are tokens
+      float* part = reinterpret_cast<float*>(ws + L.part_off) + ((long long)it.slot * L.batch + first) * m + row;
 #pragma unroll 1
-      for (int c0 = 0; c0 < TN; c0 += 32) {
+      for (int c0 = 0; c0 < cols; c0 += 32) {
         uint32_t r[32];
         tmem_ld32(tmem_acc + ((uint32_t)(quarter * 32) << 16) + a * TN + (uint32_t)c0, r);
         tmem_ld_wait();
-        if (row < L.m) {
+        if (row < m) {
+          float* p = part + (long long)c0 * m;
+          if (c0 + 32 <= cols) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int token = it.n_tile * TN + c0 + i;
-            if (token < L.batch) part[(long long)token * L.m + row] = __uint_as_float(r[i]);
+            for (int i = 0; i < 32; ++i) p[(long long)i * m] = __uint_as_float(r[i]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (c0 + i < cols) p[(long long)i * m] = __uint_as_float(r[i]);
           }
         }
       }
@@ -584,7 +607,7 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
     tc_fence_before();
     __syncthreads();
   }
-  if (warp == GM_MMA_WARP) tmem_dealloc(tmem_acc, 2 * TN);
+  if (warp == GM_MMA_WARP) tmem_dealloc(tmem_acc, TMEM_COLS);
 }
 
 // ---- decode once: E8 indices -> swizzled fp16 weight tiles in global memory ----------------------------

@@ -57,7 +57,7 @@ struct MoeDev {
   long long o_count, o_base, o_cursor, o_work, o_route_tok, o_route_exp, o_slot_of, o_xr1, o_part1, o_xr2, o_part2;
   // tensor-core form (gemm != 0): tile rows, device-built layer tables and work lists
   int gemm, k13a, k13b, k2a, k2b, max_items13, max_items2;
-  long long o_trow, o_tile0, o_layers13, o_layers2, o_items13, o_items2, o_nitems, o_status;
+  long long o_trow, o_row0, o_layers13, o_layers2, o_items13, o_items2, o_nitems, o_status;
   // E8 shell experts (format == GLQB_FMT_E8_SHELL; tensor-core form only): index matrices per stage,
   // expert-stacked, the packed tables, and the per-expert cumulative inverse residual scales of stages 2, 3
   int format, e8_ns;
@@ -69,8 +69,29 @@ struct MoeDev {
   const float* e8_w2_inv[2];
 };
 
-constexpr int MOE_TN = 128;                    // routed tokens per GEMM tile
-constexpr int MOE_B_BYTES = MOE_TN * 128;      // one 64-column chunk of a token tile
+// Routed tokens per GEMM tile: an expert's tokens are split evenly over ceil(count / MOE_TN) tiles, each padded to 16.
+// The kernels are bound by the weight decode, which every tile repeats, so a tile is as long as four stages of shared
+// memory allow (320 x 128 + 16 KiB each); 128-token tiles decoded an expert of 256 tokens two and a half times (4096
+// tokens, top 8 of 128: the two matmuls 489 + 265 -> 291 + 171 us).
+constexpr int MOE_TN = 320;
+__device__ __forceinline__ int moe_tile_tokens(int cnt) {           // tokens of an expert's tiles but the last
+  const int n = max(1, (cnt + MOE_TN - 1) / MOE_TN);
+  return max(16, ((cnt + n - 1) / n + 15) & ~15);
+}
+__device__ __forceinline__ int moe_tile_count(int cnt) {
+  const int tt = moe_tile_tokens(cnt);
+  return (cnt + tt - 1) / tt;
+}
+__device__ __forceinline__ int moe_tile_rows(int cnt) {             // 128-byte activation rows of an expert's tiles, per chunk
+  const int n = moe_tile_count(cnt);
+  return n ? (n - 1) * moe_tile_tokens(cnt) + ((cnt - (n - 1) * moe_tile_tokens(cnt) + 15) & ~15) : 0;
+}
+// where routing number i of an expert (activation rows from `row0` on) has its row: rows in front of its tile, and
+// rows of the tile << 16 | row inside it
+__device__ __forceinline__ int2 moe_tile_place(int cnt, int row0, int i) {
+  const int tt = moe_tile_tokens(cnt), j = i / tt, left = cnt - j * tt;
+  return make_int2(row0 + j * tt, (left >= tt ? tt : (left + 15) & ~15) << 16 | (i - j * tt));
+}
 
 __device__ __forceinline__ float moe_act(float g, int act) {
   if (act == GLQB_ACT_SILU || act == 3) return g / (1.0f + __expf(-g));
@@ -133,11 +154,12 @@ __global__ void __launch_bounds__(1024) moe_place_kernel(const __grid_constant__
   for (int e = threadIdx.x; e < M.E; e += blockDim.x) cur[e] = cnt[e] ? atomicAdd(&g_cursor[e], cnt[e]) : 0;
   __syncthreads();
   const int* g_base = reinterpret_cast<const int*>(ws + M.o_base);
-  const int* g_tile0 = reinterpret_cast<const int*>(ws + M.o_tile0);
+  const int* g_row0 = reinterpret_cast<const int*>(ws + M.o_row0);
+  const int* g_count = reinterpret_cast<const int*>(ws + M.o_count);
   int* route_tok = reinterpret_cast<int*>(ws + M.o_route_tok);
   int* route_exp = reinterpret_cast<int*>(ws + M.o_route_exp);
   int* slot_of = reinterpret_cast<int*>(ws + M.o_slot_of);
-  int* trow = reinterpret_cast<int*>(ws + M.o_trow);
+  int2* trow = reinterpret_cast<int2*>(ws + M.o_trow);
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const int i = i0 + u * 1024;
@@ -147,7 +169,7 @@ __global__ void __launch_bounds__(1024) moe_place_kernel(const __grid_constant__
         slot = atomicAdd(&cur[ev[u]], 1);
         route_tok[slot] = i / M.top_k;
         route_exp[slot] = ev[u];
-        if (M.gemm) trow[slot] = g_tile0[ev[u]] * MOE_TN + (slot - g_base[ev[u]]);
+        if (M.gemm) trow[slot] = moe_tile_place(g_count[ev[u]], g_row0[ev[u]], slot - g_base[ev[u]]);
       }
       slot_of[i] = slot;
     }
@@ -156,11 +178,12 @@ __global__ void __launch_bounds__(1024) moe_place_kernel(const __grid_constant__
 
 __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__ MoeDev M, const void* __restrict__ ids,
                                                          int T, uint8_t* __restrict__ ws, int phase) {
-  extern __shared__ int sh[];            // counts[E], cursor[E], first slot[E], first token tile[E + 1]
+  extern __shared__ int sh[];            // counts[E], cursor[E], first slot[E], first token tile[E + 1], first row[E]
   int* cnt = sh;
   int* cur = sh + M.E;
   int* base_s = sh + 2 * M.E;
   int* tile0 = sh + 3 * M.E;
+  int* row0 = sh + 4 * M.E + 1;
   int* g_count = reinterpret_cast<int*>(ws + M.o_count);
   int* g_base = reinterpret_cast<int*>(ws + M.o_base);
   int* g_work = reinterpret_cast<int*>(ws + M.o_work);
@@ -186,28 +209,39 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
     for (int e = threadIdx.x; e < M.E; e += blockDim.x) cnt[e] = g_count[e];
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0, tiles = 0;
-    for (int e = 0; e < M.E; ++e) {
-      cur[e] = run; base_s[e] = run; run += cnt[e];
-      tile0[e] = tiles; tiles += (cnt[e] + MOE_TN - 1) / MOE_TN;
+  if (threadIdx.x < 32) {
+    // running sums over the experts: slots, token tiles, activation rows
+    int run = 0, tiles = 0, rows = 0;
+    for (int e0 = 0; e0 < M.E; e0 += 32) {
+      const int e = e0 + threadIdx.x, c = e < M.E ? cnt[e] : 0;
+      const int nt = moe_tile_count(c), nr = moe_tile_rows(c);
+      int a = c, b = nt, d = nr;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int pa = __shfl_up_sync(0xffffffffu, a, o), pb = __shfl_up_sync(0xffffffffu, b, o), pd = __shfl_up_sync(0xffffffffu, d, o);
+        if ((int)threadIdx.x >= o) { a += pa; b += pb; d += pd; }
+      }
+      if (e < M.E) { cur[e] = base_s[e] = run + a - c; tile0[e] = tiles + b - nt; row0[e] = rows + d - nr; }
+      run += __shfl_sync(0xffffffffu, a, 31);
+      tiles += __shfl_sync(0xffffffffu, b, 31);
+      rows += __shfl_sync(0xffffffffu, d, 31);
     }
-    tile0[M.E] = tiles;
+    if (threadIdx.x == 0) tile0[M.E] = tiles;
   }
   __syncthreads();
   {
     int* g_cursor = reinterpret_cast<int*>(ws + M.o_cursor);
-    int* g_tile0 = reinterpret_cast<int*>(ws + M.o_tile0);
+    int* g_row0 = reinterpret_cast<int*>(ws + M.o_row0);
     for (int e = threadIdx.x; e < M.E; e += blockDim.x) {
-      g_base[e] = base_s[e]; g_count[e] = cnt[e]; g_cursor[e] = base_s[e]; g_tile0[e] = tile0[e];
+      g_base[e] = base_s[e]; g_count[e] = cnt[e]; g_cursor[e] = base_s[e]; g_row0[e] = row0[e];
     }
   }
-  int* trow = reinterpret_cast<int*>(ws + M.o_trow);
+  int2* trow = reinterpret_cast<int2*>(ws + M.o_trow);
   if (M.gemm) {
-    // Tensor-core form.  Expert e with c routings owns ceil(c / 128) token tiles; routing number i of the
-    // expert sits in row tile0[e] * 128 + i of the padded row space.  Every expert becomes a "layer" of the
-    // GEMM kernel (token count, activation tiles and partial-sum rows of this step), and the work list is
-    // ordered (token tile, row tile) so that the CTAs working at one moment share an activation tile in L2.
+    // Tensor-core form.  Expert e with c routings owns moe_tile_count(c) token tiles; routing number i of the expert
+    // sits where moe_tile_place says.  Every expert becomes a "layer" of the GEMM kernel (token count, activations and
+    // partial-sum rows of this step), and the work list is ordered (token tile, row tile) so that the CTAs working at
+    // one moment share an activation tile in L2.
     const int kc13 = M.hidden / GM_TILE_K, kc2 = M.inter / GM_TILE_K;
     const int mt13 = (M.w13_out + GM_TILE_M - 1) / GM_TILE_M, mt2 = (M.hidden + GM_TILE_M - 1) / GM_TILE_M;
     const int tiles = tile0[M.E];
@@ -219,38 +253,34 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
     }
     DevLinear* L13 = reinterpret_cast<DevLinear*>(ws + M.o_layers13);
     DevLinear* L2 = reinterpret_cast<DevLinear*>(ws + M.o_layers2);
-    for (int e = threadIdx.x; e < M.E; e += blockDim.x) {
-      DevLinear a;
-      memset(&a, 0, sizeof a);
-      a.format = M.format;
+    // (field by field: only what the GEMM kernel reads; thread 2e writes expert e's w13 entry, 2e + 1 its w2 entry)
+    for (int i = threadIdx.x; i < 2 * M.E; i += blockDim.x) {
+      const int e = i >> 1;
+      const bool second = i & 1;
+      DevLinear& a = (second ? L2 : L13)[e];
       a.batch = cnt[e];
-      DevLinear b = a;
+      a.m = second ? M.hidden : M.w13_out;
+      a.n = second ? M.inter : M.hidden;
+      a.strips = a.m / 32;
+      a.groups_per_strip = a.n / 32;
+      a.xr_off = (second ? M.o_xr2 : M.o_xr1) + (long long)row0[e] * (second ? kc2 : kc13) * 128;
+      a.part_off = (second ? M.o_part2 : M.o_part1) + (long long)base_s[e] * (second ? M.hidden : M.w13_out) * 4;
+      a.stage_scale[0] = 1.f;
       if (M.format == GLQB_FMT_E8_SHELL) {
-        a.n_stages = b.n_stages = M.e8_ns;
         for (int s = 0; s < M.e8_ns; ++s) {
-          a.codes[s] = M.e8_w13[s] + (long long)e * M.w13_stride[0];
-          b.codes[s] = M.e8_w2[s] + (long long)e * M.w2_stride[0];
-          a.table[s] = b.table[s] = M.e8_tab[s];
-          a.table_entries[s] = b.table_entries[s] = M.e8_ent[s];
-          a.stage_scale[s] = s ? M.e8_w13_inv[s - 1][e] : 1.f;
-          b.stage_scale[s] = s ? M.e8_w2_inv[s - 1][e] : 1.f;
+          a.codes[s] = (second ? M.e8_w2[s] : M.e8_w13[s]) + (long long)e * (second ? M.w2_stride[0] : M.w13_stride[0]);
+          a.table[s] = M.e8_tab[s];
+          a.table_entries[s] = M.e8_ent[s];
+          if (s) a.stage_scale[s] = (second ? M.e8_w2_inv : M.e8_w13_inv)[s - 1][e];
         }
       } else {
-        a.codes[0] = M.w13[0] + (long long)e * M.w13_stride[0];
-        a.codes[1] = M.w13[1] ? M.w13[1] + (long long)e * M.w13_stride[1] : nullptr;
-        a.stage_scale[0] = 1.f; a.stage_scale[1] = M.w13_inv2 ? M.w13_inv2[e] : 0.f;
-        b.codes[0] = M.w2[0] + (long long)e * M.w2_stride[0];
-        b.codes[1] = M.w2[1] ? M.w2[1] + (long long)e * M.w2_stride[1] : nullptr;
-        b.stage_scale[0] = 1.f; b.stage_scale[1] = M.w2_inv2 ? M.w2_inv2[e] : 0.f;
+        const uint8_t* const* w = second ? M.w2 : M.w13;
+        const long long* st = second ? M.w2_stride : M.w13_stride;
+        const float* inv = second ? M.w2_inv2 : M.w13_inv2;
+        a.codes[0] = w[0] + (long long)e * st[0];
+        a.codes[1] = w[1] ? w[1] + (long long)e * st[1] : nullptr;
+        a.stage_scale[1] = inv ? inv[e] : 0.f;
       }
-      a.m = M.w13_out; a.n = M.hidden; a.strips = M.w13_out / 32; a.groups_per_strip = M.hidden / 32;
-      a.xr_off = M.o_xr1 + (long long)tile0[e] * kc13 * MOE_B_BYTES;
-      a.part_off = M.o_part1 + (long long)base_s[e] * M.w13_out * 4;
-      b.m = M.hidden; b.n = M.inter; b.strips = M.hidden / 32; b.groups_per_strip = M.inter / 32;
-      b.xr_off = M.o_xr2 + (long long)tile0[e] * kc2 * MOE_B_BYTES;
-      b.part_off = M.o_part2 + (long long)base_s[e] * M.hidden * 4;
-      L13[e] = a;
-      L2[e] = b;
     }
     auto expert_of_tile = [&](int tile) -> int {       // last e with tile0[e] <= tile
       int lo = 0, hi = M.E - 1;
@@ -262,14 +292,12 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
     };
     GemmItem* I13 = reinterpret_cast<GemmItem*>(ws + M.o_items13);
     GemmItem* I2 = reinterpret_cast<GemmItem*>(ws + M.o_items2);
-    for (int idx = threadIdx.x; idx < min(tiles * mt13, M.max_items13); idx += blockDim.x) {
-      const int tile = idx / mt13, e = expert_of_tile(tile);
-      I13[idx] = GemmItem{e, idx - tile * mt13, tile - tile0[e], 0, kc13, 0};
-    }
-    for (int idx = threadIdx.x; idx < min(tiles * mt2, M.max_items2); idx += blockDim.x) {
-      const int tile = idx / mt2, e = expert_of_tile(tile);
-      I2[idx] = GemmItem{e, idx - tile * mt2, tile - tile0[e], 0, kc2, 0};
-    }
+    auto item = [&](int tile, int mt, int kc) -> GemmItem {
+      const int e = expert_of_tile(tile), j = tile - tile0[e], tt = moe_tile_tokens(cnt[e]);
+      return GemmItem{e, mt, j, 0, kc, 0, j * tt, min(tt, cnt[e] - j * tt), j * tt};
+    };
+    for (int idx = threadIdx.x; idx < min(tiles * mt13, M.max_items13); idx += blockDim.x) I13[idx] = item(idx / mt13, idx % mt13, kc13);
+    for (int idx = threadIdx.x; idx < min(tiles * mt2, M.max_items2); idx += blockDim.x) I2[idx] = item(idx / mt2, idx % mt2, kc2);
   }
   if (phase != 0) return;
   for (int i0 = threadIdx.x; i0 < R; i0 += 8 * blockDim.x) {
@@ -285,7 +313,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
           slot = atomicAdd(&cur[ev[u]], 1);
           route_tok[slot] = i / M.top_k;
           route_exp[slot] = ev[u];
-          if (M.gemm) trow[slot] = tile0[ev[u]] * MOE_TN + (slot - base_s[ev[u]]);
+          if (M.gemm) trow[slot] = moe_tile_place(cnt[ev[u]], row0[ev[u]], slot - base_s[ev[u]]);
         }
         slot_of[i] = slot;
       }
@@ -378,9 +406,9 @@ __device__ __forceinline__ uint2 pack4_half(const f2 (&q)[2]) {
   const __half2 a = __floats2half2_rn(r[0], r[1]), b = __floats2half2_rn(r[2], r[3]);
   return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
-// place of columns col .. col + 3 of padded row `trow` in a [tile][chunk] x (128 x 64) image
-__device__ __forceinline__ uint8_t* moe_tile_at(uint8_t* base, int trow, int kchunks, int col) {
-  return base + ((size_t)(trow / MOE_TN) * kchunks + (col >> 6)) * MOE_B_BYTES + sw128_offset(trow % MOE_TN, col & 63);
+// place of columns col .. col + 3 of the activation row `t` (moe_tile_place)
+__device__ __forceinline__ uint8_t* moe_tile_at(uint8_t* base, int2 t, int kchunks, int col) {
+  return base + ((size_t)t.x * kchunks + (size_t)(col >> 6) * (t.y >> 16)) * 128 + sw128_offset(t.y & 0xFFFF, col & 63);
 }
 
 // Input transform of one token, stored once per routing into the token tiles of the routed experts.
@@ -388,13 +416,13 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_rht_in_gemm_kernel(cons
                                                                             const uint8_t* __restrict__ x, uint8_t* __restrict__ ws) {
   extern __shared__ __align__(16) float fb[];
   const int* slot_of = reinterpret_cast<const int*>(ws + M.o_slot_of);
-  const int* trow = reinterpret_cast<const int*>(ws + M.o_trow);
+  const int2* trow = reinterpret_cast<const int2*>(ws + M.o_trow);
   const int kchunks = M.hidden / GM_TILE_K;
-  int* rows = reinterpret_cast<int*>(fb + fht_words(8192));          // tile row of every routing of the CTA's tokens
+  int2* rows = reinterpret_cast<int2*>(fb + fht_words(8192));        // activation row of every routing of the CTA's tokens
   const int t0 = blockIdx.x * tt, nr = min(tt, T - t0) * M.top_k;
   for (int i = threadIdx.x; i < nr; i += blockDim.x) {
     const int slot = slot_of[t0 * M.top_k + i];
-    rows[i] = slot >= 0 ? trow[slot] : -1;
+    rows[i] = slot >= 0 ? trow[slot] : make_int2(-1, 0);
   }
   __syncthreads();
   const int top_k = M.top_k;
@@ -405,20 +433,21 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_rht_in_gemm_kernel(cons
     for (int k = 0; k < 8; ++k) h[k] = pack4_half(v[k]);
     if (logbs >= 10) {               // a thread's groups are columns 128 apart of one token
       for (int j = 0; j < top_k; ++j) {
-        const int r = rows[(t - t0) * top_k + j];
-        if (r < 0) continue;
+        const int2 r = rows[(t - t0) * top_k + j];
+        if (r.x < 0) continue;
+        const int step = (r.y >> 16) * 256;                          // two chunks
         uint8_t* p = moe_tile_at(xr, r, kchunks, c);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          if (k < n) *reinterpret_cast<uint2*>(p + k * 2 * MOE_B_BYTES) = h[k];
+          if (k < n) *reinterpret_cast<uint2*>(p + k * step) = h[k];
       }
     } else {
 #pragma unroll
       for (int k = 0; k < 8; ++k)
         if (k < n)
           for (int j = 0; j < top_k; ++j) {
-            const int r = rows[(t + fht_row(k, 128, logbs) - t0) * top_k + j];
-            if (r >= 0) *reinterpret_cast<uint2*>(moe_tile_at(xr, r, kchunks, c + fht_col(k, 128, logbs))) = h[k];
+            const int2 r = rows[(t + fht_row(k, 128, logbs) - t0) * top_k + j];
+            if (r.x >= 0) *reinterpret_cast<uint2*>(moe_tile_at(xr, r, kchunks, c + fht_col(k, 128, logbs))) = h[k];
           }
     }
   });
@@ -634,12 +663,12 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_mid_kernel(const __grid
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ int row_e[8];                   // expert of each row (sg <= 8)
   __shared__ float row_wsc[8];
-  __shared__ int row_t[8];
+  __shared__ int2 row_t[8];
   if (threadIdx.x < nrow) {
     const int e = reinterpret_cast<const int*>(ws + M.o_route_exp)[slot0 + threadIdx.x];
     row_e[threadIdx.x] = e;
     row_wsc[threadIdx.x] = M.w13_wscale[e];
-    row_t[threadIdx.x] = M.gemm ? reinterpret_cast<const int*>(ws + M.o_trow)[slot0 + threadIdx.x] : 0;
+    row_t[threadIdx.x] = M.gemm ? reinterpret_cast<const int2*>(ws + M.o_trow)[slot0 + threadIdx.x] : make_int2(0, 0);
   }
   const int inter = M.inter, w13_out = M.w13_out, kch = M.kch13;
   const int n13 = moe_chunks_all(sg, M.nb_m13, M.log_m13), n2 = moe_chunks_all(sg, M.nb_n2, M.log_n2);
@@ -879,7 +908,7 @@ static MoeGemmKernel moe_gemm_pick_e8(int ns) {
   return nullptr;
 }
 static size_t moe_gemm_smem_bytes() {
-  return (size_t)MOE_GEMM_STAGES * (GM_A_BYTES + (size_t)MOE_B_BYTES) + (3 * MOE_GEMM_STAGES + 5) * 8 + 16 + 1024;
+  return (size_t)MOE_GEMM_STAGES * (GM_A_BYTES + (size_t)MOE_TN * 128) + (3 * MOE_GEMM_STAGES + 5) * 8 + 16 + 1024;
 }
 // routed tokens per expert (average) from which the tensor-core form is used
 static int moe_gemm_min_avg() {
@@ -961,7 +990,7 @@ static int fill_blocks(const int32_t* blocks, int nb, int total, int* off, int* 
 // grouping: one CTA for small steps; count / tables / place kernels (many CTAs) for large ones
 static void moe_launch_group(const MoeDev& M, const void* ids, int tokens, uint8_t* ws, cudaStream_t st) {
   const int R = tokens * M.top_k;
-  const size_t sh = (4 * (size_t)M.E + 1) * sizeof(int);
+  const size_t sh = (5 * (size_t)M.E + 1) * sizeof(int);
   if (R < MOE_GROUP_SPLIT_MIN) {
     moe_group_kernel<<<1, 1024, sh, st>>>(M, ids, tokens, ws, 0);
     return;
@@ -1085,7 +1114,7 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
   M.o_count = o; o = al(o + 4 * (size_t)M.E);
   M.o_base = o; o = al(o + 4 * (size_t)M.E);
   M.o_cursor = o; o = al(o + 4 * (size_t)M.E);
-  M.o_tile0 = o; o = al(o + 4 * ((size_t)M.E + 1));
+  M.o_row0 = o; o = al(o + 4 * (size_t)M.E);
   M.o_work = o; o = al(o + 16);
   M.o_route_tok = o; o = al(o + 4 * R);
   M.o_route_exp = o; o = al(o + 4 * R);
@@ -1111,11 +1140,12 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
     G.max_items2 = (int)(tiles * mt2);
     auto al1k = [](size_t v) { return (v + 1023) / 1024 * 1024; };
     size_t g = al1k((size_t)M.o_xr1);
-    G.o_xr1 = g; g = al1k(g + tiles * (d->hidden / GM_TILE_K) * MOE_B_BYTES);
+    const size_t rows = R + 16 * tiles;                        // every tile rounds its tokens up to 16
+    G.o_xr1 = g; g = al1k(g + rows * (d->hidden / GM_TILE_K) * 128);
     G.o_part1 = g; g = al1k(g + R * d->w13_out * 4);
-    G.o_xr2 = g; g = al1k(g + tiles * (d->inter / GM_TILE_K) * MOE_B_BYTES);
+    G.o_xr2 = g; g = al1k(g + rows * (d->inter / GM_TILE_K) * 128);
     G.o_part2 = g; g = al1k(g + R * d->hidden * 4);
-    G.o_trow = g; g = al1k(g + 4 * R);
+    G.o_trow = g; g = al1k(g + 8 * R);
     G.o_layers13 = g; g = al1k(g + sizeof(DevLinear) * M.E);
     G.o_layers2 = g; g = al1k(g + sizeof(DevLinear) * M.E);
     G.o_items13 = g; g = al1k(g + sizeof(GemmItem) * G.max_items13);
@@ -1141,7 +1171,7 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
     P->mid_smem = mid_bytes(P->mid_sg);
     P->out_smem = out_bytes(P->out_rg);
     if (cudaFuncSetAttribute(moe_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)((4 * d->num_experts + 1) * sizeof(int))) != cudaSuccess ||
+                             (int)((5 * 4096 + 1) * sizeof(int))) != cudaSuccess ||
         cudaFuncSetAttribute(moe_mid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) != cudaSuccess ||
         cudaFuncSetAttribute(moe_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) != cudaSuccess) {
       delete P;
@@ -1191,7 +1221,7 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
     const int R = tokens * G.top_k;
     moe_launch_group(G, topk_ids, tokens, ws, st);
     const int tt = moe_in_tokens(G, tokens);
-    moe_rht_in_gemm_kernel<<<(tokens + tt - 1) / tt, MOE_XF_THREADS, (fht_words(8192) + tt * G.top_k) * 4, st>>>(
+    moe_rht_in_gemm_kernel<<<(tokens + tt - 1) / tt, MOE_XF_THREADS, (fht_words(8192) + 2 * tt * G.top_k) * 4, st>>>(
         G, tokens, tt, reinterpret_cast<const uint8_t*>(x), ws);
     int* status = reinterpret_cast<int*>(ws + G.o_status);
     const int* nitems = reinterpret_cast<const int*>(ws + G.o_nitems);
