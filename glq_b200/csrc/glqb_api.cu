@@ -12,6 +12,7 @@
 #include "glqb_kernels.cuh"
 #include "glqb_fused.cuh"
 #include "glqb_gemm.cuh"
+#include "glqb_tgemm.cuh"
 #include "glqb_launch.h"
 
 namespace glqb {
@@ -235,21 +236,29 @@ static int e8_two_phase_min_tokens() {
   return e ? atoi(e) : 129;     // measured on B200: above one 128-token tile the tile decode plus a copy-fed GEMM wins
 }
 
-// Trellis prefill decodes the weight tiles once instead of once per 256-token tile from this many flops per layer: the
-// tile decode costs a launch and a write of the fp16 weights (13 us at 11008 x 2048), the copy-fed GEMM saves a third of
-// the fused one's time.  Measured, whole linears, fused / two-phase: 4096 x 4096, 1024 tokens (34 GFLOP) 61 / 69 us,
-// 2048 tokens (69) 114 / 99; 11008 x 2048, 512 tokens (23) 60 / 66, 1024 (46) 93 / 88, 2048 (92) 156 / 141.
+// Trellis prefill decodes the weight tiles once, for the copy-fed GEMM, instead of once per 192-token tile into tensor
+// memory (trellis_gemm_kernel), from this many flops per layer: the tile decode costs a launch and a write of the fp16
+// weights (13 us at 11008 x 2048).  Measured, whole linears, tensor memory / tiles: 4096 x 4096, 1024 tokens (34 GFLOP)
+// 65 / 65 us, 2048 tokens (69) 106 / 99; 11008 x 2048, 1024 tokens (46) 81 / 84, 2048 (92) 145 / 141; 2048 x 11008,
+// 1024 tokens 94 / 103, 2048 tokens 186 / 149.
 static double trellis_two_phase_min_flops() {
   const char* e = getenv("GLQB_TRELLIS_TWO_PHASE_MIN_FLOPS");
-  return e ? atof(e) : 40e9;
+  return e ? atof(e) : 60e9;
 }
-// ... and while the tiles of a launch stay below 2 GiB of workspace (a sweep over a whole model keeps the fused form)
+// ... and while the tiles of a launch stay below 2 GiB of workspace (a sweep over a whole model keeps decoding into tensor memory)
 constexpr size_t TRELLIS_TILES_MAX_BYTES = 2ull << 30;
 static size_t tile_bytes(const GlqbLinearDesc& d) {
   return (size_t)((d.m_pad + GM_TILE_M - 1) / GM_TILE_M) * ((d.n_pad + GM_TILE_K - 1) / GM_TILE_K) * GM_A_BYTES;
 }
 
-static int tn_for_batch(int batch) { return batch <= DECODE_MAX_BATCH ? 0 : (batch <= 128 ? 128 : 256); }
+// token tile of the tensor-core forms.  Pre-decoded tiles and E8: 128 or 256; trellis codes: at most 192, the tokens split
+// evenly, in steps of 16.
+static int tn_for_batch(int batch, bool codes) {
+  if (batch <= DECODE_MAX_BATCH) return 0;
+  if (!codes) return batch <= 128 ? 128 : 256;
+  const int tiles = (batch + TG_TN - 1) / TG_TN;
+  return ((batch + tiles - 1) / tiles + 15) & ~15;
+}
 
 static int nb_for_batch(int batch) {
   if (batch <= 8) return 1;
@@ -382,18 +391,25 @@ static int build_plan(GlqbPlan* P) {
 
   // ---- segments: layers with the same kernel variant, in caller order inside a segment
   typedef std::tuple<int, int, int, int, int, int, int> Key;   // format, k1, k2, ns, nb, tn, two-phase
+  const double tiles_min = trellis_two_phase_min_flops();
+  auto by_flops = [&](const GlqbLinearDesc& d) { return 2.0 * d.batch * d.m_pad * d.n_pad >= tiles_min; };
+  size_t trellis_tile_bytes = 0;
+  for (const GlqbLinearDesc& d : P->descs)
+    if (d.format == GLQB_FMT_TRELLIS_3INST && d.batch > DECODE_MAX_BATCH && by_flops(d)) trellis_tile_bytes += tile_bytes(d);
+  auto trellis_tiles_once = [&](const GlqbLinearDesc& d) { return by_flops(d) && trellis_tile_bytes <= TRELLIS_TILES_MAX_BYTES; };
   std::map<Key, std::vector<int>> groups;
   std::vector<Key> key_order;
   for (int i = 0; i < n; ++i) {
     const GlqbLinearDesc& d = P->descs[i];
     Key k;
-    const int tn = tn_for_batch(d.batch);
+    const bool trellis = d.format == GLQB_FMT_TRELLIS_3INST;
+    const bool tiles = d.batch > DECODE_MAX_BATCH && (trellis ? trellis_tiles_once(d) : d.batch >= e8_two_phase_min_tokens());
+    const int tn = tn_for_batch(d.batch, trellis && !tiles);
     const int nb = tn ? 0 : nb_for_batch(d.batch);
-    if (d.format == GLQB_FMT_TRELLIS_3INST)
-      k = Key(d.format, d.bits[0], d.n_stages > 1 ? d.bits[1] : 0, d.n_stages, nb, tn,
-              (tn && 2.0 * d.batch * d.m_pad * d.n_pad >= trellis_two_phase_min_flops()) ? 1 : 0);
+    if (trellis)
+      k = Key(d.format, d.bits[0], d.n_stages > 1 ? d.bits[1] : 0, d.n_stages, nb, tn, tiles ? 1 : 0);
     else
-      k = Key(d.format, 0, 0, d.n_stages, nb, tn, (tn && d.batch >= e8_two_phase_min_tokens()) ? 1 : 0);
+      k = Key(d.format, 0, 0, d.n_stages, nb, tn, tiles ? 1 : 0);
     if (!groups.count(k)) key_order.push_back(k);
     groups[k].push_back(i);
   }
@@ -407,11 +423,6 @@ static int build_plan(GlqbPlan* P) {
     s.first = (int)P->order.size();
     s.count = (int)groups[k].size();
     for (int i : groups[k]) P->order.push_back(i);
-    if (s.two_phase && s.format == GLQB_FMT_TRELLIS_3INST) {
-      size_t bytes = 0;
-      for (int i : groups[k]) bytes += tile_bytes(P->descs[i]);
-      if (bytes > TRELLIS_TILES_MAX_BYTES) s.two_phase = 0;
-    }
     if (s.tn ? !gemm_available(s) : !pick_kernel(s))
       return fail(GLQB_E_INVALID, "no kernel variant for format=%d K=%d+%d stages=%d token blocks=%d", s.format,
                   s.k1, s.k2, s.ns, s.nb);
@@ -619,7 +630,8 @@ static int build_plan(GlqbPlan* P) {
         for (int mt = 0; mt < m_tiles; ++mt)
           for (int nt = 0; nt < n_tiles; ++nt)
             for (int k = 0; k < ks; ++k)
-              P->gemm_items.push_back(GemmItem{s.first + i, mt, nt, k * per, std::min(kchunks, (k + 1) * per), k, 0, 0, 0});
+              P->gemm_items.push_back(GemmItem{s.first + i, mt, nt, k * per, std::min(kchunks, (k + 1) * per), k,
+                                               nt * s.tn, std::min(s.tn, L.batch - nt * s.tn), nt * s.tn});
         P->max_batch_gemm = std::max(P->max_batch_gemm, L.batch);
       }
       s.item_count = (int)P->gemm_items.size() - s.item_first;
@@ -1160,7 +1172,7 @@ size_t glqb_linear_workspace_bytes(const GlqbLinearDesc* desc) {
   // more than 128 tokens the decoded fp16 weight tiles.
   if (!desc) return 0;
   const size_t batch = (size_t)std::max(1, desc->batch);
-  const int tn = tn_for_batch((int)batch);
+  const int tn = tn_for_batch((int)batch, false);         // (the larger of the tiles a layer may take)
   size_t ws = 1024;
   if (tn) {
     const size_t n_tiles = (batch + tn - 1) / tn, kchunks = ((size_t)desc->n_pad + GM_TILE_K - 1) / GM_TILE_K;

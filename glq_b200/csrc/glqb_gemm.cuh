@@ -4,8 +4,8 @@
 // Warp roles (GM_THREADS = 704):
 //   warps 0-15 decode producers in two groups of eight; group 0 produces the even 128x64 weight chunks,
 //              group 1 the odd ones (two stages are always being filled).  Inside a group every warp
-//              decodes one 32x32 trellis group (or 16 rows x 64 columns of E8 indices) into the stage's
-//              A tile, K-major with the 128-byte swizzle the tensor core expects
+//              decodes 16 rows x 64 columns of E8 indices into the stage's A tile, K-major with the 128-byte
+//              swizzle the tensor core expects
 //   warps 18-21 epilogue: tcgen05.ld of the finished accumulator (two accumulators alternate, so the
 //              next tile's MMAs run while these warps write the previous tile's partial sums)
 //   warp  16   one thread issues tcgen05.mma (4 per chunk: K = 16 each) and tcgen05.commit
@@ -116,6 +116,12 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
+// one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(ok));
+  return ok != 0;
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // K-major operand tile with 128-byte swizzle: rows of 128 bytes, 8-row atoms of 1024 bytes stacked along
@@ -149,15 +155,18 @@ static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_gemm_kern
   extern __shared__ __align__(16) float fbuf[];
   const RhtItem it = items[blockIdx.x];
   const DevLinear& L = layers[it.layer];
-  const int tn = L.gemm_tn, tn_log = tn == 128 ? 7 : 8;
+  const int tn = L.gemm_tn;
+  const bool steps = L.format == GLQB_FMT_TRELLIS_3INST && tn < 256;   // trellis_gemm_kernel: the last tile ends on 16 rows
   const int off = L.bn_off[it.block];
   const int logbs = L.bn_log[it.block];
   const int bs = 1 << logbs;
   const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
   const float rs = L.x_is_rotated ? 1.0f : rsqrtf((float)bs);
   uint8_t* xr = ws + L.xr_off;
+  auto tile_rows = [&](int tile) -> int { return steps ? min(tn, (L.batch - tile * tn + 15) & ~15) : tn; };
   auto place = [&](int token, int col) -> uint8_t* {
-    return xr + (((size_t)(token >> tn_log) * kchunks + (col >> 6)) << (tn_log + 7)) + sw128_offset(token & (tn - 1), col & 63);
+    const int tile = token / tn;
+    return xr + ((size_t)tile * tn * kchunks + (size_t)(col >> 6) * tile_rows(tile)) * 128 + sw128_offset(token - tile * tn, col & 63);
   };
   auto store1 = [&](int row, int i, float v) { *reinterpret_cast<__half*>(place(it.tok0 + row, off + i)) = __float2half_rn(v); };
   auto load1 = [&](int row, int i) -> float {
@@ -181,7 +190,9 @@ static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_gemm_kern
       auto load_plain = [&](int e0, f2 (&v)[8][2]) { rht_load_x_plain(L, it, x_base, off, log_t, total, S, e0, v); };
       auto store_plain = [&](int e1, const f2 (&v)[8][2]) {
         const f2 rs2 = f2_pack(rs, rs);
-        uint8_t* p = place(it.tok0 + (e1 >> log_t), off + run0 + (e1 & ((1 << log_t) - 1)));
+        const int token = it.tok0 + (e1 >> log_t);
+        const size_t step = (size_t)tile_rows(token / tn) * 256;
+        uint8_t* p = place(token, off + run0 + (e1 & ((1 << log_t) - 1)));
 #pragma unroll
         for (int k = 0; k < 8; ++k)
           if (e1 + (k << 7) < total) {
@@ -189,7 +200,7 @@ static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_gemm_kern
             f2_unpack(f2_mul(v[k][0], rs2), r[0], r[1]);
             f2_unpack(f2_mul(v[k][1], rs2), r[2], r[3]);
             const __half2 a = __floats2half2_rn(r[0], r[1]), b = __floats2half2_rn(r[2], r[3]);
-            *reinterpret_cast<uint2*>(p + ((size_t)k << (tn_log + 8))) =
+            *reinterpret_cast<uint2*>(p + k * step) =
                 make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
           }
       };
@@ -284,21 +295,19 @@ __device__ __forceinline__ void gemm_store_group(const uint32_t (&addr)[4], int 
 }
 
 // ---- the GEMM kernel -------------------------------------------------------------------------------
-// FORMAT 0: trellis (K1, K2 bits); FORMAT 1: E8 (K1 = number of stages, K2 unused);
-// FORMAT 2: the weight tiles were decoded beforehand (e8_tiles_kernel) and are fetched like the
-//           activation tiles, one bulk copy per stage; the producer warps have nothing to do
-// TN > 256: variable token tiles of up to TN tokens (a multiple of 64), for grouped experts.  A tile's activations are
-// rows of ntok rounded up to 16, [k chunk][row] behind the row0 rows of the tiles before it; an item multiplies exactly
-// that many columns (two MMAs beyond 256), so an expert's weights are decoded once for up to TN tokens and no time goes
-// into padding.  One accumulator (the columns of two would not fit): the stages run ahead while it is drained.
-template <int FORMAT, int K1, int K2, int TN, int STAGES>
+// FORMAT 1: E8 (K1 = number of stages); FORMAT 2: the weight tiles were decoded beforehand (e8_tiles_kernel,
+//           trellis_tiles_kernel) and are fetched like the activation tiles, one bulk copy per stage; the producer warps
+//           have nothing to do.  (Trellis codes are decoded by trellis_gemm_kernel.)
+// TN = 192: variable token tiles, for grouped experts.  A tile's activations are rows of ntok rounded up to 16, [k chunk]
+// [row] behind the row0 rows of the tiles before it; an item multiplies exactly that many columns.
+template <int FORMAT, int K1, int TN, int STAGES>
 __global__ void __launch_bounds__(GM_THREADS, 1)
 glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict__ items, int n_items,
                 uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev) {
   // work lists built on the device (grouped expert matmul) pass their length through memory
   if (n_items_dev) n_items = min(n_items, *n_items_dev);
   constexpr int B_BYTES = TN * 128;
-  constexpr bool VAR = TN > 256;
+  constexpr bool VAR = TN == 192;
   constexpr int TMEM_COLS = VAR ? 512 : 2 * TN;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -352,52 +361,6 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
       const int first = it.k_begin + (int)((grp - q0) & 1u);       // this group's first chunk of the item
       if constexpr (FORMAT == 2) {
         (void)first; (void)wl; (void)L;
-      } else if constexpr (FORMAT == 0) {
-        const int strip = wl >> 1, cg = wl & 1;
-        const int rp = it.m_tile * 4 + strip;
-        const int gps = L.groups_per_strip;
-        const bool row_ok = rp < L.strips;
-        const uint8_t* p1 = L.codes[0] + ((long long)rp * gps) * (128 * K1) + lane * (4 * K1);
-        const uint8_t* p2 = nullptr;
-        if constexpr (K2 > 0) p2 = L.codes[1] + ((long long)rp * gps) * (128 * K2) + lane * (4 * K2);
-        const __half2 s2 = __float2half2_rn(L.stage_scale[1]);
-        uint32_t lane_addr[4];                            // of stage 0
-        gemm_lane_addrs(smem_u32(a_base) + strip * 4096, cg, lane, lane_addr);
-        Words<K1> nxt;
-        Words<(K2 > 0 ? K2 : 1)> nxt2;
-        auto fetch = [&](int kc) {
-          const int cp = kc * 2 + cg;
-          if (row_ok && cp < gps) {
-            nxt = load_words<K1>(p1 + (long long)cp * (128 * K1));
-            if constexpr (K2 > 0) nxt2 = load_words<K2>(p2 + (long long)cp * (128 * K2));
-          }
-        };
-        if (first < it.k_end) fetch(first);
-        for (int kc = first; kc < it.k_end; kc += 2) {
-          const uint32_t q = q0 + (uint32_t)(kc - it.k_begin);
-          const int stage = (int)(q % STAGES);
-          const uint32_t phase = (q / STAGES) & 1u;
-          const Words<K1> v = nxt;
-          const Words<(K2 > 0 ? K2 : 1)> v2 = nxt2;
-          const bool valid = row_ok && (kc * 2 + cg) < gps;
-          if (kc + 2 < it.k_end) fetch(kc + 2);
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
-          uint32_t addr[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) addr[u] = lane_addr[u] + stage * GM_A_BYTES;
-          if (valid) {
-            gemm_store_group<K1, K2>(addr, lane, v, v2, s2);
-          } else {
-            // rows or columns past the matrix: zeros (validity is uniform per warp, so the shuffles
-            // inside the decode always see all 32 lanes)
-            const uint32_t zero[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) gemm_store_quad(addr, q4, zero);
-          }
-          fence_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&full_a[stage]);
-        }
       } else {
         // E8: 128 rows x 8 indices per chunk; thread (row = tid >> 1, half = tid & 1) expands 4 indices
         const int tid = threadIdx.x & 255;                // thread inside the producer group
@@ -485,41 +448,39 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
     if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_PRODUCER); }
   } else if (warp == GM_MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0, seq = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
-        const GemmItem it = items[item];
-        const uint32_t a = VAR ? 0u : seq & 1u, a_phase = (VAR ? seq : seq >> 1) & 1u;     // accumulator and its use count parity
-        const uint32_t d_tmem = tmem_acc + a * TN;
-        const int cols = VAR ? (it.ntok + 15) & ~15 : TN, cols0 = VAR ? min(cols, 256) : TN;
-        const uint32_t idesc = umma_idesc_f16(cols0), idesc1 = VAR ? umma_idesc_f16(max(16, cols - cols0)) : 0u;
-        if (!mbar_wait(&acc_empty[a], a_phase ^ 1, abort_flag)) { ok = false; break; }
+    // The whole warp walks the chunks and one elected lane issues: warp-uniform control flow keeps descriptors and
+    // addresses in uniform registers (under a lane == 0 branch this loop itself took longer than the MMAs).
+    const uint32_t d0 = __shfl_sync(0xffffffffu, tmem_acc, 0);
+    const uint32_t a0 = smem_u32(a_base), b0 = smem_u32(b_base);
+    int stage = 0;
+    uint32_t phase = 0, seq = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
+      const int chunks = __shfl_sync(0xffffffffu, items[item].k_end - items[item].k_begin, 0);
+      const uint32_t idesc = umma_idesc_f16(VAR ? (__shfl_sync(0xffffffffu, items[item].ntok, 0) + 15) & ~15 : TN);
+      const uint32_t a = seq & 1u, a_phase = (seq >> 1) & 1u;     // accumulator and its use count parity
+      const uint32_t d_tmem = d0 + a * TN;
+      if (!mbar_wait(&acc_empty[a], a_phase ^ 1, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      for (int c = 0; c < chunks; ++c) {
+        if ((FORMAT != 2 && !mbar_wait(&full_a[stage], phase, abort_flag)) || !mbar_wait(&full_b[stage], phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        for (int kc = it.k_begin; kc < it.k_end; ++kc) {
-          if ((FORMAT != 2 && !mbar_wait(&full_a[stage], phase, abort_flag)) || !mbar_wait(&full_b[stage], phase, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint64_t da = umma_desc_sw128(smem_u32(a_base + stage * GM_A_BYTES));
-          const uint64_t db = umma_desc_sw128(smem_u32(b_base + stage * B_BYTES));
+        const uint64_t da = umma_desc_sw128(a0 + stage * GM_A_BYTES);
+        const uint64_t db = umma_desc_sw128(b0 + stage * B_BYTES);
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < GM_TILE_K / 16; ++k)      // +32 bytes (2 x 16-byte units) per K step of 16
-            umma_f16(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kc > it.k_begin || k > 0) ? 1u : 0u);
-          if constexpr (VAR) {
-            if (cols > 256) {                            // rows 256 on of the activation tile: 32 KiB further
-#pragma unroll
-              for (int k = 0; k < GM_TILE_K / 16; ++k)
-                umma_f16(d_tmem + 256, da + (uint64_t)(2 * k), db + (uint64_t)(2048 + 2 * k), idesc1, (kc > it.k_begin || k > 0) ? 1u : 0u);
-            }
-          }
+            umma_f16(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (c > 0 || k > 0) ? 1u : 0u);
           umma_commit(&empty[stage]);                    // stage reusable once these MMAs have read it
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if (!ok) break;
-        umma_commit(&acc_full[a]);
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
-      if (!ok) { *abort_flag = 1; atomicCAS(status, 0, (int)ST_GAVE_UP_MMA); }
+      if (!ok) break;
+      if (elect_one()) umma_commit(&acc_full[a]);
+      __syncwarp();
     }
+    if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_MMA); }
   } else if (warp == GM_LOAD_WARP) {
     // ------------------------------------------------------------------ activation loader
     if (lane == 0) {
@@ -557,7 +518,7 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
       const GemmItem it = items[item];
       const DevLinear& L = layers[it.layer];
-      const uint32_t a = VAR ? 0u : seq & 1u, a_phase = (VAR ? seq : seq >> 1) & 1u;
+      const uint32_t a = seq & 1u, a_phase = (seq >> 1) & 1u;
       if (!mbar_wait(&acc_full[a], a_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const int row = it.m_tile * GM_TILE_M + quarter * 32 + lane;
@@ -600,7 +561,8 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
         mbar_wait(&full_b[q % STAGES], (q / STAGES) & 1u);
       }
     }
-    if (warp == GM_MMA_WARP && lane == 0) {
+    // (commit tracks the MMAs of the issuing thread: the lane elect.sync picks)
+    if (warp == GM_MMA_WARP && elect_one()) {
       umma_commit(drain);
       mbar_wait(drain, 0);
     }

@@ -1,6 +1,7 @@
 // Instantiations and launches of the tensor-core GEMM kernels and the E8 tile decode (see glqb_gemm.cuh).
 #include "glqb_kernels.cuh"
 #include "glqb_gemm.cuh"
+#include "glqb_tgemm.cuh"
 #include "glqb_launch.h"
 
 namespace glqb {
@@ -18,10 +19,10 @@ static TilesSmemKernel pick_tiles_smem_kernel(int ns) {
 
 typedef void (*GemmKernel)(const DevLinear*, const GemmItem*, int, uint8_t*, int*, const int*);
 
-template <int FORMAT, int K1, int K2>
+template <int FORMAT, int K1>
 static GemmKernel gemm_kernel_tn(int tn) {
-  if (tn == 128) return glq_gemm_kernel<FORMAT, K1, K2, 128, GEMM_STAGES>;
-  if (tn == 256) return glq_gemm_kernel<FORMAT, K1, K2, 256, GEMM_STAGES>;
+  if (tn == 128) return glq_gemm_kernel<FORMAT, K1, 128, GEMM_STAGES>;
+  if (tn == 256) return glq_gemm_kernel<FORMAT, K1, 256, GEMM_STAGES>;
   return nullptr;
 }
 
@@ -49,23 +50,23 @@ static TilesKernel pick_trellis_tiles_kernel(int k1, int k2) {
 }
 
 static GemmKernel pick_gemm_kernel(const Segment& s) {
-  if (s.two_phase) return gemm_kernel_tn<2, 0, 0>(s.tn);
+  if (s.two_phase) return gemm_kernel_tn<2, 0>(s.tn);
   if (s.format == GLQB_FMT_TRELLIS_3INST) {
-#define G_CASE(A, B) if (s.k1 == A && s.k2 == B) return gemm_kernel_tn<0, A, B>(s.tn);
+#define G_CASE(A, B) if (s.k1 == A && s.k2 == B) return trellis_gemm_kernel<A, B>;
 #ifdef GLQB_FAST_BUILD   /* developer builds for kernel experiments: the 4-bit single-stage rate only */
     G_CASE(4, 0)
 #else
     G_CASE(1, 0) G_CASE(2, 0) G_CASE(3, 0) G_CASE(4, 0)
     G_CASE(4, 1) G_CASE(4, 2) G_CASE(4, 3) G_CASE(4, 4)
 #endif
-  #undef G_CASE
+#undef G_CASE
     return nullptr;
   }
   switch (s.ns) {
-    case 1: return gemm_kernel_tn<1, 1, 0>(s.tn);
-    case 2: return gemm_kernel_tn<1, 2, 0>(s.tn);
-    case 3: return gemm_kernel_tn<1, 3, 0>(s.tn);
-    case 4: return gemm_kernel_tn<1, 4, 0>(s.tn);
+    case 1: return gemm_kernel_tn<1, 1>(s.tn);
+    case 2: return gemm_kernel_tn<1, 2>(s.tn);
+    case 3: return gemm_kernel_tn<1, 3>(s.tn);
+    case 4: return gemm_kernel_tn<1, 4>(s.tn);
   }
   return nullptr;
 }
@@ -75,10 +76,13 @@ static size_t gemm_smem_bytes(int tn) {
 }
 
 
+static bool trellis_form(const Segment& s) { return s.format == GLQB_FMT_TRELLIS_3INST && !s.two_phase; }
+static size_t segment_smem(const Segment& s) { return trellis_form(s) ? (size_t)TG_SMEM_BYTES : gemm_smem_bytes(s.tn); }
+
 bool gemm_available(const Segment& s) { return pick_gemm_kernel(s) != nullptr; }
 
 cudaError_t gemm_prepare(const Segment& s) {
-  return cudaFuncSetAttribute(pick_gemm_kernel(s), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem_bytes(s.tn));
+  return cudaFuncSetAttribute(pick_gemm_kernel(s), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)segment_smem(s));
 }
 
 cudaError_t tiles_smem_prepare(int ns) {
@@ -94,7 +98,7 @@ void gemm_launch(const Segment& s, const DevLinear* layers, const GemmItem* item
         layers, s.first, s.count, ws, s.big_table, s.small_table, s.small_entries);
   else if (s.two_phase)
     pick_tiles_kernel(s.ns)<<<sm_count * 8, 256, 0, stream>>>(layers, s.first, s.count, ws);
-  pick_gemm_kernel(s)<<<s.grid, GM_THREADS, gemm_smem_bytes(s.tn), stream>>>(layers, items, s.item_count, ws, status, nullptr);
+  pick_gemm_kernel(s)<<<s.grid, trellis_form(s) ? TG_THREADS : GM_THREADS, segment_smem(s), stream>>>(layers, items, s.item_count, ws, status, nullptr);
 }
 
 }  // namespace glqb

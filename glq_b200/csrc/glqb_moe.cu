@@ -33,6 +33,7 @@
 
 #include "glqb_kernels.cuh"
 #include "glqb_gemm.cuh"
+#include "glqb_tgemm.cuh"
 
 namespace glqb {
 
@@ -70,10 +71,7 @@ struct MoeDev {
 };
 
 // Routed tokens per GEMM tile: an expert's tokens are split evenly over ceil(count / MOE_TN) tiles, each padded to 16.
-// The kernels are bound by the weight decode, which every tile repeats, so a tile is as long as four stages of shared
-// memory allow (320 x 128 + 16 KiB each); 128-token tiles decoded an expert of 256 tokens two and a half times (4096
-// tokens, top 8 of 128: the two matmuls 489 + 265 -> 291 + 171 us).
-constexpr int MOE_TN = 320;
+constexpr int MOE_TN = TG_TN;
 __device__ __forceinline__ int moe_tile_tokens(int cnt) {           // tokens of an expert's tiles but the last
   const int n = max(1, (cnt + MOE_TN - 1) / MOE_TN);
   return max(16, ((cnt + n - 1) / n + 15) & ~15);
@@ -894,26 +892,28 @@ static MoeMvKernel moe_mv_pick(int k1, int k2) {
 typedef void (*MoeGemmKernel)(const DevLinear*, const GemmItem*, int, uint8_t*, int*, const int*);
 constexpr int MOE_GEMM_STAGES = 4;
 static MoeGemmKernel moe_gemm_pick(int k1, int k2) {
-#define M_CASE(A, B) if (k1 == A && k2 == B) return glq_gemm_kernel<0, A, B, MOE_TN, MOE_GEMM_STAGES>;
+#define M_CASE(A, B) if (k1 == A && k2 == B) return trellis_gemm_kernel<A, B>;
   M_CASE(2, 0) M_CASE(3, 0) M_CASE(4, 0) M_CASE(4, 1) M_CASE(4, 2) M_CASE(4, 3) M_CASE(4, 4)
 #undef M_CASE
   return nullptr;
 }
 static MoeGemmKernel moe_gemm_pick_e8(int ns) {
   switch (ns) {
-    case 1: return glq_gemm_kernel<1, 1, 0, MOE_TN, MOE_GEMM_STAGES>;
-    case 2: return glq_gemm_kernel<1, 2, 0, MOE_TN, MOE_GEMM_STAGES>;
-    case 3: return glq_gemm_kernel<1, 3, 0, MOE_TN, MOE_GEMM_STAGES>;
+    case 1: return glq_gemm_kernel<1, 1, MOE_TN, MOE_GEMM_STAGES>;
+    case 2: return glq_gemm_kernel<1, 2, MOE_TN, MOE_GEMM_STAGES>;
+    case 3: return glq_gemm_kernel<1, 3, MOE_TN, MOE_GEMM_STAGES>;
   }
   return nullptr;
 }
-static size_t moe_gemm_smem_bytes() {
+static size_t moe_gemm_smem_bytes(bool e8) {
+  if (!e8) return TG_SMEM_BYTES;
   return (size_t)MOE_GEMM_STAGES * (GM_A_BYTES + (size_t)MOE_TN * 128) + (3 * MOE_GEMM_STAGES + 5) * 8 + 16 + 1024;
 }
-// routed tokens per expert (average) from which the tensor-core form is used
+// routed tokens per expert (average) from which the tensor-core form is used (measured, 128 experts, top 8, streaming /
+// tensor-core: 64 tokens 260 / 263 us, 128 tokens 283 / 264, 256 tokens 333 / 271, 512 tokens 518 / 325)
 static int moe_gemm_min_avg() {
   const char* e = getenv("GLQB_MOE_GEMM_MIN_AVG");
-  return e ? atoi(e) : 64;
+  return e ? atoi(e) : 6;
 }
 
 }  // namespace glqb
@@ -1153,8 +1153,8 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
     G.o_nitems = g; g = al1k(g + 16);
     G.o_status = g; g = al1k(g + 16);
     P->ws_bytes = std::max(P->ws_bytes, g);
-    if (cudaFuncSetAttribute(P->g13, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)moe_gemm_smem_bytes()) != cudaSuccess ||
-        cudaFuncSetAttribute(P->g2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)moe_gemm_smem_bytes()) != cudaSuccess) {
+    if (cudaFuncSetAttribute(P->g13, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)moe_gemm_smem_bytes(e8)) != cudaSuccess ||
+        cudaFuncSetAttribute(P->g2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)moe_gemm_smem_bytes(e8)) != cudaSuccess) {
       cudaGetLastError();
       P->gemm_ok = false;
     }
@@ -1223,18 +1223,20 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
     const int tt = moe_in_tokens(G, tokens);
     moe_rht_in_gemm_kernel<<<(tokens + tt - 1) / tt, MOE_XF_THREADS, (fht_words(8192) + 2 * tt * G.top_k) * 4, st>>>(
         G, tokens, tt, reinterpret_cast<const uint8_t*>(x), ws);
+    const bool g_e8 = G.format == GLQB_FMT_E8_SHELL;
+    const int g_threads = g_e8 ? GM_THREADS : TG_THREADS;
     int* status = reinterpret_cast<int*>(ws + G.o_status);
     const int* nitems = reinterpret_cast<const int*>(ws + G.o_nitems);
     {
       MoeTimer t(P, st);
-      P->g13<<<std::min(P->sm_count, G.max_items13), GM_THREADS, moe_gemm_smem_bytes(), st>>>(
+      P->g13<<<std::min(P->sm_count, G.max_items13), g_threads, moe_gemm_smem_bytes(g_e8), st>>>(
           reinterpret_cast<const DevLinear*>(ws + G.o_layers13), reinterpret_cast<const GemmItem*>(ws + G.o_items13),
           G.max_items13, ws, status, nitems);
     }
     moe_mid_kernel<<<(R + P->mid_sg - 1) / P->mid_sg, MOE_XF_THREADS, P->mid_smem, st>>>(G, tokens, P->mid_sg, ws);
     {
       MoeTimer t(P, st);
-      P->g2<<<std::min(P->sm_count, G.max_items2), GM_THREADS, moe_gemm_smem_bytes(), st>>>(
+      P->g2<<<std::min(P->sm_count, G.max_items2), g_threads, moe_gemm_smem_bytes(g_e8), st>>>(
           reinterpret_cast<const DevLinear*>(ws + G.o_layers2), reinterpret_cast<const GemmItem*>(ws + G.o_items2),
           G.max_items2, ws, status, nitems + 1);
     }

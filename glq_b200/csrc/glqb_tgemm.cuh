@@ -1,0 +1,305 @@
+// Prefill and grouped experts on trellis weights: states decoded straight into tensor memory as the A operand of
+// tcgen05.mma, activations streamed through shared memory.
+//
+// Why A goes to tensor memory: with A and B both in shared memory the 128 bytes per clock of an SM were the limit — per
+// 128 x 64 x 256 chunk 48 KiB of operand reads, 16 KiB of producer stores and 32 KiB of copies are 768 clocks, the tensor
+// pipe needs 512 (measured: 1010 clocks per chunk, the MMA thread waiting for neither operand).  A lane of a decoding
+// warp holds exactly the fragment layout of tcgen05.st.16x128b (row g and g + 8, columns 2t and 2t + 1 of every 16 x 8
+// block), so two stores replace sixteen and the chunk leaves 64 KiB of shared-memory traffic.
+//
+// One CTA computes 128 weight rows x up to 192 tokens: two accumulators of 192 columns and four 64-column chunks of A
+// (32 columns each) fill the 512 columns of tensor memory.  Warp roles: warp 0 issues MMAs, warp 1 the bulk copies (TMA
+// without multicast) of the activation tiles, warps 4-7 drain accumulators, 24 producer warps in three groups of eight
+// (group q % 3 decodes chunk q, warp w of a group the 32 x 32 trellis group at rows 32 (w % 4), columns 32 (w / 4)).
+// Stages hand over through mbarriers; every wait is bounded as in glq_gemm_kernel.
+#pragma once
+#include "glqb_gemm.cuh"
+
+namespace glqb {
+
+constexpr int TG_TN = 192;                       // most tokens of a tile (multiples of 16)
+// a stage is a pair of 64-column chunks: 64 columns of tensor memory, one copy of the two chunks' activations
+constexpr int TG_A_STAGES = 2, TG_A_COLS = 32;   // columns per chunk
+constexpr int TG_B_STAGES = 4;
+constexpr int TG_B_BYTES = 2 * TG_TN * 128;
+constexpr int TG_GROUPS = 3;
+constexpr int TG_MMA_WARP = 0, TG_LOAD_WARP = 1, TG_EPI_WARP0 = 4, TG_PROD_WARP0 = 8;   // (2 and 3 only keep warp % 4 aligned)
+constexpr int TG_THREADS = (TG_PROD_WARP0 + TG_GROUPS * 8) * 32;
+constexpr int TG_SMEM_BYTES = TG_B_STAGES * TG_B_BYTES + (2 * TG_A_STAGES + 2 * TG_B_STAGES + 5) * 8 + 16 + 1024;
+
+__device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// A from tensor memory, B from shared memory
+__device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// One trellis group -> the A fragments of its two 16-row halves: r[mi][(ni * 2 + c) * 2 + a] = weights (2t, 2t + 1) of
+// row g + 8 a in the 16 x 8 block (ni, c).
+template <int K1, int K2>
+__device__ __forceinline__ void tg_decode_group(int lane, const Words<K1>& v, const Words<(K2 > 0 ? K2 : 1)>& v2, __half2 s2,
+                                                uint32_t (&r)[2][8]) {
+  const Words<K1> vn = shfl_words<K1>(v, (lane + 1) & 31);
+  Words<K1> vn2 = vn;
+  if constexpr (K1 == 1) vn2 = shfl_words<K1>(v, (lane + 2) & 31);
+  Words<(K2 > 0 ? K2 : 1)> un, un2;
+  if constexpr (K2 > 0) {
+    un = shfl_words<K2>(v2, (lane + 1) & 31);
+    un2 = un;
+    if constexpr (K2 == 1) un2 = shfl_words<K2>(v2, (lane + 2) & 31);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {                  // q = ni * 2 + mi
+    uint32_t a[8], b[8];
+    decode_tile<K1>(chunk_of<K1>(v, q), chunk_of<K1>(vn, q), chunk_of<K1>(vn2, q), a);
+    if constexpr (K2 > 0) decode_tile<K2>(chunk_of<K2>(v2, q), chunk_of<K2>(un, q), chunk_of<K2>(un2, q), b);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {                // p = c * 2 + a
+      uint32_t w = __byte_perm(a[2 * p], a[2 * p + 1], 0x5410);
+      if constexpr (K2 > 0) {
+        // second stage folded into the fp16 operand: w = fp16(w1 + s2 * w2), one rounding
+        const uint32_t w2 = __byte_perm(b[2 * p], b[2 * p + 1], 0x5410);
+        const __half2 z = __hfma2(*reinterpret_cast<const __half2*>(&w2), s2, *reinterpret_cast<const __half2*>(&w));
+        w = *reinterpret_cast<const uint32_t*>(&z);
+      }
+      r[q & 1][(q >> 1) * 4 + p] = w;
+    }
+  }
+}
+
+// Activations of a tile: ntok rounded up to 16 rows of 128 bytes per 64-column chunk, [k chunk][row], behind the row0
+// rows of the tiles before it.  An item multiplies exactly the columns it has.
+template <int K1, int K2>
+__global__ void __launch_bounds__(TG_THREADS, 1)
+trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict__ items, int n_items,
+                    uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev) {
+  // work lists built on the device (grouped expert matmul) pass their length through memory
+  if (n_items_dev) n_items = min(n_items, *n_items_dev);
+  constexpr int MMA_WARP = TG_MMA_WARP, LOAD_WARP = TG_LOAD_WARP;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* b_base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(b_base + TG_B_STAGES * TG_B_BYTES);
+  uint64_t* full_a = bars;
+  uint64_t* empty_a = full_a + TG_A_STAGES;
+  uint64_t* full_b = empty_a + TG_A_STAGES;
+  uint64_t* empty_b = full_b + TG_B_STAGES;
+  uint64_t* acc_full = empty_b + TG_B_STAGES;      // [2]
+  uint64_t* acc_empty = acc_full + 2;              // [2]
+  uint64_t* drain = acc_empty + 2;                 // give-up path only: completion of the MMAs issued so far
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < TG_A_STAGES; ++s) { mbar_init(&full_a[s], 16); mbar_init(&empty_a[s], 1); }
+    for (int s = 0; s < TG_B_STAGES; ++s) { mbar_init(&full_b[s], 1); mbar_init(&empty_b[s], 1); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 4); }
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == MMA_WARP) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot, tmem_a = tmem + 2 * TG_TN;
+  uint32_t loads_issued = 0;                       // loader thread: stages armed so far
+
+  if (warp == MMA_WARP) {
+    // ------------------------------------------------------------------ MMA issuer
+    // The whole warp walks the chunks and one elected lane issues: with warp-uniform control flow descriptors and
+    // addresses stay in uniform registers, and one wait per pair is left (a producer warp hands A over only after it
+    // has seen B arrive).  This loop, not the operands, was the limit: 1040 clocks per chunk with two waits per chunk
+    // under a lane == 0 branch, whatever the number of tokens, 740 in this form chunk by chunk; hence pairs.
+    const uint32_t d0 = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t b0 = smem_u32(b_base);
+    uint32_t q = 0, seq = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
+      const int chunks = __shfl_sync(0xffffffffu, items[item].k_end - items[item].k_begin, 0);
+      const int cols = (__shfl_sync(0xffffffffu, items[item].ntok, 0) + 15) & ~15;
+      const uint32_t idesc = umma_idesc_f16(cols), half = (uint32_t)cols * 8u;     // (16-byte units of a chunk's activations)
+      const uint32_t a = seq & 1u;                 // accumulator
+      const uint32_t d_tmem = d0 + a * TG_TN;
+      if (!mbar_wait(&acc_empty[a], ((seq >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      for (int c = 0; c < chunks; c += 2, ++q) {           // q numbers pairs here
+        const uint32_t sa = q % TG_A_STAGES, sb = q % TG_B_STAGES;
+        if (!mbar_wait(&full_a[sa], (q / TG_A_STAGES) & 1u, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t ta = d0 + 2 * TG_TN + sa * (2 * TG_A_COLS);
+        const uint64_t db = umma_desc_sw128(b0 + sb * TG_B_BYTES);
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < GM_TILE_K / 16; ++k)        // K step of 16: 8 columns of A, 32 bytes of B
+            umma_f16_ta(d_tmem, ta + (uint32_t)(8 * k), db + (uint64_t)(2 * k), idesc, (c > 0 || k > 0) ? 1u : 0u);
+          if (c + 1 < chunks) {
+#pragma unroll
+            for (int k = 0; k < GM_TILE_K / 16; ++k)
+              umma_f16_ta(d_tmem, ta + (uint32_t)(TG_A_COLS + 8 * k), db + (uint64_t)(half + 2 * k), idesc, 1u);
+          }
+          umma_commit(&empty_a[sa]);                       // stages reusable once these MMAs have read them
+          umma_commit(&empty_b[sb]);
+        }
+        __syncwarp();
+      }
+      if (!ok) break;
+      if (elect_one()) umma_commit(&acc_full[a]);
+      __syncwarp();
+    }
+    if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_MMA); }
+  } else if (warp == LOAD_WARP) {
+    // ------------------------------------------------------------------ activation loader
+    if (lane == 0) {
+      uint32_t q = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        const GemmItem it = items[item];
+        const DevLinear& L = layers[it.layer];
+        const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
+        const uint32_t bytes = (uint32_t)((it.ntok + 15) & ~15) * 128u;
+        const uint8_t* src = ws + L.xr_off + (size_t)it.row0 * kchunks * 128;
+        for (int kc = it.k_begin; kc < it.k_end; kc += 2, ++q) {
+          const uint32_t sb = q % TG_B_STAGES, n = kc + 1 < it.k_end ? 2u * bytes : bytes;
+          if (!mbar_wait(&empty_b[sb], ((q / TG_B_STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          mbar_expect_tx(&full_b[sb], n);
+          bulk_g2s(b_base + sb * TG_B_BYTES, src + (size_t)kc * bytes, n, &full_b[sb]);
+          ++loads_issued;
+        }
+      }
+      if (!ok) { *abort_flag = 1; atomicCAS(status, 0, (int)ST_GAVE_UP_LOADER); }
+    }
+  } else if (warp >= TG_PROD_WARP0) {
+    // ------------------------------------------------------------------ producers
+    // q numbers the chunks of this CTA over all its items, every item rounded up to pairs (the second half of a last odd
+    // pair is handed over without being written or multiplied); chunk q is half q & 1 of pair q >> 1
+    const int grp = (warp - TG_PROD_WARP0) >> 3, strip = warp & 3, cg = (warp >> 2) & 1;
+    const uint32_t lanes = tmem_a + ((uint32_t)(strip * 32) << 16) + (uint32_t)(cg * 16);
+    uint32_t q0 = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+      const GemmItem it = items[item];
+      const DevLinear& L = layers[it.layer];
+      const int first = it.k_begin + (int)(((uint32_t)(grp + TG_GROUPS) - q0 % (uint32_t)TG_GROUPS) % (uint32_t)TG_GROUPS);
+      const int rp = it.m_tile * 4 + strip, gps = L.groups_per_strip, k_end = it.k_end;
+      const int k_pad = it.k_begin + ((k_end - it.k_begin + 1) & ~1);
+      const bool row_ok = rp < L.strips;
+      const uint8_t* p1 = L.codes[0] + ((long long)rp * gps) * (128 * K1) + lane * (4 * K1);
+      const uint8_t* p2 = nullptr;
+      if constexpr (K2 > 0) p2 = L.codes[1] + ((long long)rp * gps) * (128 * K2) + lane * (4 * K2);
+      const __half2 s2 = __float2half2_rn(L.stage_scale[1]);
+      Words<K1> nxt;
+      Words<(K2 > 0 ? K2 : 1)> nxt2;
+      auto fetch = [&](int kc) {
+        const int cp = kc * 2 + cg;
+        if (row_ok && cp < gps) {
+          nxt = load_words<K1>(p1 + (long long)cp * (128 * K1));
+          if constexpr (K2 > 0) nxt2 = load_words<K2>(p2 + (long long)cp * (128 * K2));
+        }
+      };
+      if (first < k_end) fetch(first);
+      for (int kc = first; kc < k_pad; kc += TG_GROUPS) {
+        const uint32_t q = q0 + (uint32_t)(kc - it.k_begin);
+        const uint32_t pair = q >> 1;
+        const int stage = (int)(pair % TG_A_STAGES);
+        const Words<K1> v = nxt;
+        const Words<(K2 > 0 ? K2 : 1)> v2 = nxt2;
+        uint32_t r[2][8];
+        if (row_ok && kc * 2 + cg < gps && kc < k_end) {         // (uniform per warp: the shuffles inside see all lanes)
+          tg_decode_group<K1, K2>(lane, v, v2, s2, r);
+        } else {                                   // rows or columns past the matrix: zeros
+#pragma unroll
+          for (int i = 0; i < 16; ++i) r[i >> 3][i & 7] = 0u;
+        }
+        if (kc + TG_GROUPS < k_end) fetch(kc + TG_GROUPS);
+        if (!mbar_wait(&empty_a[stage], ((pair / TG_A_STAGES) & 1u) ^ 1u, abort_flag) ||
+            ((warp & 7) == 0 && !mbar_wait(&full_b[pair % TG_B_STAGES], (pair / TG_B_STAGES) & 1u, abort_flag))) { ok = false; break; }
+        __syncwarp();
+        tc_fence_after();
+        const uint32_t cols = (uint32_t)((stage * 2 + (int)(q & 1u)) * TG_A_COLS);
+        tmem_st_16x128b_x4(lanes + cols, r[0]);
+        tmem_st_16x128b_x4(lanes + (16u << 16) + cols, r[1]);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full_a[stage]);
+      }
+      q0 += (uint32_t)(k_pad - it.k_begin);
+    }
+    if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_PRODUCER); }
+  } else if (warp >= TG_EPI_WARP0) {
+    // ------------------------------------------------------------------ epilogue warps
+    const int quarter = warp & 3;                          // TMEM lanes 32*quarter .. 32*quarter + 31
+    uint32_t seq = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
+      const GemmItem it = items[item];
+      const DevLinear& L = layers[it.layer];
+      const uint32_t a = seq & 1u;
+      if (!mbar_wait(&acc_full[a], (seq >> 1) & 1u, abort_flag)) { ok = false; break; }
+      __syncwarp();
+      tc_fence_after();
+      const int row = it.m_tile * GM_TILE_M + quarter * 32 + lane, m = L.m, cols = it.ntok;
+      float* part = reinterpret_cast<float*>(ws + L.part_off) + ((long long)it.slot * L.batch + it.tok0) * m + row;
+#pragma unroll 1
+      for (int c0 = 0; c0 < cols; c0 += 32) {
+        uint32_t r[32];
+        tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + a * TG_TN + (uint32_t)c0, r);
+        tmem_ld_wait();
+        if (row < m) {
+          float* p = part + (long long)c0 * m;
+          if (c0 + 32 <= cols) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) p[(long long)i * m] = __uint_as_float(r[i]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (c0 + i < cols) p[(long long)i * m] = __uint_as_float(r[i]);
+          }
+        }
+        __syncwarp();
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[a]);
+    }
+    if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_EPILOGUE); }
+  }
+  // ---- teardown: every thread arrives here (also after a wait gave up)
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    // A role gave up.  Before shared memory and tensor memory are released, wait (bounded again) for what may still be
+    // in flight: the bulk copies into the stages armed last, and the MMAs issued so far.
+    if (warp == LOAD_WARP && lane == 0) {
+      const uint32_t n = loads_issued < (uint32_t)TG_B_STAGES ? loads_issued : (uint32_t)TG_B_STAGES;
+      for (uint32_t i = 0; i < n; ++i) {
+        const uint32_t q = loads_issued - 1 - i;
+        mbar_wait(&full_b[q % TG_B_STAGES], (q / TG_B_STAGES) & 1u);
+      }
+    }
+    // (commit tracks the MMAs of the issuing thread: the lane elect.sync picks)
+    if (warp == MMA_WARP && elect_one()) {
+      umma_commit(drain);
+      mbar_wait(drain, 0);
+    }
+    tc_fence_before();
+    __syncthreads();
+  }
+  if (warp == MMA_WARP) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+}  // namespace glqb
