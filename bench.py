@@ -250,7 +250,8 @@ def kernel_name(W):
     if T > 64:
         tn = 128 if T <= 128 else 256
         if fmt == "trellis":
-            return f"glq_gemm_kernel<trellis,{par[0]},{par[1] if len(par) > 1 else 0},{tn},4>"
+            rate = f"{par[0]},{par[1] if len(par) > 1 else 0}"
+            return (f"trellis_gemm_kernel<{rate}> (layers of 60 GFLOP and more: trellis_tiles_kernel<{rate}> + glq_gemm_kernel<tiles,256,4>)")
         if T >= 129:
             return f"e8_tiles_smem_kernel<{ns}> + glq_gemm_kernel<tiles,{tn},4> (weight tiles decoded once, then the copy-fed GEMM)"
         return f"glq_gemm_kernel<e8,{ns},{tn},4>"
@@ -473,7 +474,7 @@ def run_moe_bench(name, D: Dist, args, steps, tokens=None):
     hbm, tens, kind = measured_peaks()
     gbs = W["code_bytes"] / (ms * 1e-3) / 1e9
     tf = W["flops"] / (ms * 1e-3) / 1e12
-    gemm = T * 8 >= 128 * 64
+    gemm = T * 8 >= 128 * 64             # enough routed tokens per expert for the tensor pipe to be the bound
     rec = {"workload": name, "metric": "MoE grouped expert matmul: compressed-byte GB/s and TFLOP/s", "value": gbs,
            "unit": "GB/s", "tflops": tf, "ms_per_step": ms, "n_gpus": D.world,
            "config": f"128 experts top-8, hidden 2048, expert intermediate 768, trellis 4 bpw, {T} tokens, "
@@ -485,13 +486,14 @@ def run_moe_bench(name, D: Dist, args, steps, tokens=None):
            "gpu_launches": (6 if T * 8 < 8192 else 8) * steps}
     if gemm:     # tensor-core form: the two grouped GEMMs against the tensor peak
         ach = W["flops"] / D.world / (kern_ms * 1e-3) / 1e12
-        rec["roofline"] = {"bound": "tensor", "kernel": "glq_gemm_kernel<trellis,4,0,128,4> (w13 + w2 grouped GEMMs)",
+        rec["roofline"] = {"bound": "tensor", "kernel": "trellis_gemm_kernel<4,0> (w13 + w2 grouped GEMMs)",
                            "achieved": ach, "peak": tens, "peak_kind": f"of {kind}", "unit": "TFLOP/s", "frac": ach / tens,
                            "kernel_ms": kern_ms, "flops_per_launch": W["flops"] // D.world,
                            "whole_step_frac": tf / (tens * D.world), "traffic": None}
-    else:        # streaming form: expert codes read once by the two grouped decode kernels
+    else:        # few routed tokens per expert: bound by the expert codes
         ach = W["code_bytes"] / D.world / (kern_ms * 1e-3) / 1e9
-        rec["roofline"] = {"bound": "hbm", "kernel": "trellis_moe_mv_kernel<4,0,4> (w13 + w2)", "achieved": ach, "peak": hbm,
+        kern = "trellis_gemm_kernel<4,0>" if T * 8 >= 128 * 6 else "trellis_moe_mv_kernel<4,0,4>"
+        rec["roofline"] = {"bound": "hbm", "kernel": kern + " (w13 + w2)", "achieved": ach, "peak": hbm,
                            "peak_kind": f"of {kind}", "unit": "GB/s", "frac": ach / hbm, "kernel_ms": kern_ms,
                            "bytes_per_launch": W["code_bytes"] // D.world, "whole_step_frac": gbs / (hbm * D.world),
                            "traffic": None}

@@ -1172,11 +1172,13 @@ size_t glqb_linear_workspace_bytes(const GlqbLinearDesc* desc) {
   // more than 128 tokens the decoded fp16 weight tiles.
   if (!desc) return 0;
   const size_t batch = (size_t)std::max(1, desc->batch);
-  const int tn = tn_for_batch((int)batch, false);         // (the larger of the tiles a layer may take)
+  const int tn = tn_for_batch((int)batch, false);
   size_t ws = 1024;
   if (tn) {
-    const size_t n_tiles = (batch + tn - 1) / tn, kchunks = ((size_t)desc->n_pad + GM_TILE_K - 1) / GM_TILE_K;
-    ws += align_up(n_tiles * kchunks * tn * 128, 1024);
+    const size_t kchunks = ((size_t)desc->n_pad + GM_TILE_K - 1) / GM_TILE_K;
+    const size_t tc = tn_for_batch((int)batch, true);       // either token tile may be the one: whole tiles of tn, or even ones
+    const size_t rows = std::max((batch + tn - 1) / tn * tn, (batch + tc - 1) / tc * tc);
+    ws += align_up(rows * kchunks * 128, 1024);
     ws += align_up(16 * batch * desc->m_pad * 4, 1024);                      // at most 16 K splits
     ws += align_up(tile_bytes(*desc), 1024) + 1024;                          // (the two-phase forms)
   } else {
