@@ -625,6 +625,7 @@ static int build_plan(GlqbPlan* P) {
         L.fixed_slots = ks;
         L.slots = ks;
         L.gemm_tn = s.tn;
+        L.gemm_even = trellis_form(s) ? 1 : 0;
         L.per_warp = 1;
         L.atile_off = s.two_phase ? -1 : 0;      // -1: allocate below
         for (int mt = 0; mt < m_tiles; ++mt)
@@ -769,7 +770,7 @@ static int build_plan(GlqbPlan* P) {
       if (layer_fused[q]) continue;
       const DevLinear& Q = P->dev[q];
       const GlqbLinearDesc& e = P->descs[P->order[q]];
-      if (Q.format == L.format && Q.gemm_tn == L.gemm_tn && Q.n == L.n && Q.in_f == L.in_f && Q.sv == L.sv &&
+      if (Q.format == L.format && Q.gemm_tn == L.gemm_tn && Q.gemm_even == L.gemm_even && Q.n == L.n && Q.in_f == L.in_f && Q.sv == L.sv &&
           Q.batch == L.batch &&
           Q.x_off == L.x_off && Q.x_stride == L.x_stride && Q.x_dtype == L.x_dtype && Q.nbn == L.nbn &&
           Q.x_is_rotated == L.x_is_rotated && Q.in_norm_w == L.in_norm_w && Q.in_norm_dtype == L.in_norm_dtype &&

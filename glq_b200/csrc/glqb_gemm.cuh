@@ -156,7 +156,7 @@ static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_gemm_kern
   const RhtItem it = items[blockIdx.x];
   const DevLinear& L = layers[it.layer];
   const int tn = L.gemm_tn;
-  const bool steps = L.format == GLQB_FMT_TRELLIS_3INST && tn < 256;   // trellis_gemm_kernel: the last tile ends on 16 rows
+  const bool steps = L.gemm_even != 0;             // the last tile ends on 16 rows
   const int off = L.bn_off[it.block];
   const int logbs = L.bn_log[it.block];
   const int bs = 1 << logbs;

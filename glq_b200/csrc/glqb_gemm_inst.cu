@@ -76,7 +76,6 @@ static size_t gemm_smem_bytes(int tn) {
 }
 
 
-static bool trellis_form(const Segment& s) { return s.format == GLQB_FMT_TRELLIS_3INST && !s.two_phase; }
 static size_t segment_smem(const Segment& s) { return trellis_form(s) ? (size_t)TG_SMEM_BYTES : gemm_smem_bytes(s.tn); }
 
 bool gemm_available(const Segment& s) { return pick_gemm_kernel(s) != nullptr; }

@@ -33,6 +33,8 @@ struct DevLinear {
   int per_warp;          // work groups handed to each warp of the segment's launch
   int fixed_slots;       // > 0: every strip has exactly this many partial sums (GEMM path: K splits)
   int gemm_tn;           // token tile of the GEMM path (0: streaming decode path)
+  int gemm_even;         // 1: the activations of the last token tile end on a step of 16 rows (trellis_gemm_kernel),
+                         // 0: every tile has gemm_tn rows (glq_gemm_kernel with 128 / 256 tokens)
   int ticket_base;       // single-launch form: first completion ticket of this layer (one per output Hadamard block)
   const void* in_norm_w; // optional fusions (single-launch form): RMSNorm weight, its dtype and epsilon,
   int in_norm_dtype;     // gated activation of a [gate | up] input (0 none, 1 + GLQB_ACT_*), residual accumulate

@@ -46,3 +46,17 @@ def test_e8_tiles_equal_fused(shape, stages, monkeypatch):
     for resident in ("0", str(1 << 40)):
         tiles, _ = run(L, x, monkeypatch, {"GLQB_E8_TWO_PHASE_MIN_TOKENS": "65", "GLQB_E8_SMEM_MIN_BYTES": resident})
         assert torch.equal(tiles, fused)
+
+
+# every token tile of the two forms: below, at and just above a step of 16, one 128-token tile, the first of 256, the
+# first even split (193 tokens are two tiles of 112), with several chunks of 64 columns
+@pytest.mark.parametrize("bits", [[4], [4, 2]], ids=str)
+@pytest.mark.parametrize("tokens", [65, 72, 100, 112, 113, 128, 129, 192, 193])
+def test_trellis_tiles_equal_fused_token_counts(tokens, bits, monkeypatch):
+    m, n = 160, 1056
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    L = synth.trellis_layer("t", m, n, bits, g, "cuda")
+    x = torch.randn(tokens, n, generator=g, device="cuda").half()
+    a, _ = run(L, x, monkeypatch, {"GLQB_TRELLIS_TWO_PHASE_MIN_FLOPS": "1"})
+    b, _ = run(L, x, monkeypatch, {"GLQB_TRELLIS_TWO_PHASE_MIN_FLOPS": "1e30"})
+    assert torch.equal(a, b)
