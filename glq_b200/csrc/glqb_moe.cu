@@ -1160,7 +1160,10 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
     }
   }
   {
-    const size_t budget = 74 * 1024;      // three CTAs per SM (and the limit every plan sets: one plan never lowers another's)
+    // Slots per CTA and routings per pass are chosen for three CTAs per SM; one row may need more: a block shorter than
+    // 1024 values takes a whole chunk, and 16 blocks per side at the largest served sizes come to 156,288 bytes (mid kernel).  The limit is a
+    // property of the kernels, not of a plan, so every plan sets the same one.
+    const size_t budget = 74 * 1024, limit = 200 * 1024;
     auto mid_bytes = [&](int sg) { return (size_t)4 * FHT_CHUNK_WORDS * (moe_chunks_all(sg, M.nb_m13, M.log_m13) + moe_chunks_all(sg, M.nb_n2, M.log_n2)); };
     auto out_bytes = [&](int rg) { return 4 * ((size_t)FHT_CHUNK_WORDS * moe_chunks_all(rg, M.nb_m2, M.log_m2) + (rg < d->top_k ? (size_t)d->hidden : 0)); };
     P->mid_sg = 8;
@@ -1170,10 +1173,14 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
     while (P->out_rg > 1 && out_bytes(P->out_rg) > budget) --P->out_rg;
     P->mid_smem = mid_bytes(P->mid_sg);
     P->out_smem = out_bytes(P->out_rg);
+    if (P->mid_smem > limit || P->out_smem > limit) {
+      delete P;
+      return moe_fail(GLQB_E_INVALID, "moe_plan_create: one row of the expert transforms needs more than %zu bytes of shared memory", limit);
+    }
     if (cudaFuncSetAttribute(moe_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)((5 * 4096 + 1) * sizeof(int))) != cudaSuccess ||
-        cudaFuncSetAttribute(moe_mid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) != cudaSuccess ||
-        cudaFuncSetAttribute(moe_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) != cudaSuccess) {
+        cudaFuncSetAttribute(moe_mid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit) != cudaSuccess ||
+        cudaFuncSetAttribute(moe_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit) != cudaSuccess) {
       delete P;
       return moe_fail(GLQB_E_CUDA, "moe_plan_create: %s", cudaGetErrorString(cudaGetLastError()));
     }

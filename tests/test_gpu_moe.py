@@ -195,3 +195,24 @@ def test_moe_large_step_uses_split_grouping():
     err = np.abs(y.float().cpu().numpy() - ref).max() / np.abs(ref).max()
     assert err <= 5e-3, err
     ops.clear_caches()
+
+
+# sizes whose rows need more shared memory than the three-CTAs-per-SM budget (many short blocks: 8160, 8128, 4064), blocks
+# of several 1024-value chunks on either side (8192, 4096, 3136 = 2048 + 1024 + 64, 1056), with routings in several passes
+@pytest.mark.parametrize("form", ["1", "1000000"], ids=["gemm", "stream"])
+@pytest.mark.parametrize("hidden,inter", [(8160, 64), (8128, 64), (8192, 64), (128, 4064), (128, 4096), (256, 3136), (4096, 1056)])
+def test_moe_block_lists(hidden, inter, form, monkeypatch):
+    from glq_b200 import ops
+    monkeypatch.setenv("GLQB_MOE_GEMM_MIN_AVG", form)       # (sizes that are not multiples of 64 stream either way)
+    E, k, T = 3, 2, 5
+    rng = np.random.default_rng(hidden + inter)
+    d, w13_out = _make(rng, E, hidden, inter, 2)
+    x_t = cuda(rng.standard_normal((T, hidden)).astype(np.float32), torch.float16)
+    ids = np.stack([rng.permutation(E)[:k] for _ in range(T)]).astype(np.int64)
+    w = rng.random((T, k)).astype(np.float32)
+    ops.clear_caches()
+    y = _run(ops, d, x_t, cuda(ids), cuda(w), E, hidden, inter, w13_out, 0, 1)
+    ref = _oracle(d, x_t.float().cpu().numpy(), ids, w, E, hidden, inter, w13_out, 2, 0, O.ACT_CODES[1])
+    err = np.abs(y.float().cpu().numpy() - ref).max() / np.abs(ref).max()
+    ops.clear_caches()
+    assert err <= 5e-3, err      # as above: two chained layers with fp16 hand-offs
