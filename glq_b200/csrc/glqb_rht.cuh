@@ -384,7 +384,9 @@ __device__ __forceinline__ void rht_out_body(const DevLinear& L, const RhtItem i
       }
       return;
     }
-    // all eight loads of a slot are issued together; element offsets fit 32 bits (at most 65535 tokens x 32768 rows)
+    // all eight loads of a slot are issued together; offsets inside the tile (at most 64 tokens x 524288 rows) fit 32
+    // bits, those of the tile itself do not (65535 tokens x 131072 rows)
+    const float* tile = src + (long long)it.tok0 * m;
     for (int kk = 0; kk < S; ++kk) {
       unsigned idx[8];
       int cnt[8];
@@ -393,13 +395,13 @@ __device__ __forceinline__ void rht_out_body(const DevLinear& L, const RhtItem i
       for (int k = 0; k < 8; ++k) {
         const int e = e0 + (k << 10);
         const int row = off + (kk << FHT_LOG) + (e & ((1 << log_t) - 1));
-        idx[k] = (unsigned)(it.tok0 + (e >> log_t)) * (unsigned)m + (unsigned)row;
+        idx[k] = (unsigned)(e >> log_t) * (unsigned)m + (unsigned)row;
         cnt[k] = e < total ? (fixed_slots > 0 ? fixed_slots : slots_of(row)) : 0;
         most = max(most, cnt[k]);
       }
       const f2 sg2 = (__popc(max(it.sub, 0) & kk) & 1) ? F2_MINUS1 : F2_ONE;
       for (int s = 0; s < most; ++s) {
-        const float* p = src + s * slot_stride;
+        const float* p = tile + s * slot_stride;
         ulonglong2 t[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k)

@@ -88,3 +88,23 @@ def _check(x, W, L, y, bn, bm):
     ref = fht64((xr @ W.T) * L.wscale, bm) * L.su.double().cpu().numpy()
     # the rotated activations (and, above 64 tokens, two-stage weights) are fp16: 2e-3 of the largest output
     assert np.abs(y.double().cpu().numpy() - ref).max() <= 2e-3 * np.abs(ref).max()
+
+
+def test_output_transform_beyond_32_bit_offsets():
+    """131073 rows of 32768 sums: the last row starts 2^32 elements in.  Only its sums are written and only its result is
+    looked at (six of the columns, so that the general body runs)."""
+    tokens, m, out = 131073, 32768, 6
+    if torch.cuda.mem_get_info()[0] < 20 << 30:
+        pytest.skip("needs 17 GiB")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    src = torch.empty(tokens, m, device="cuda")
+    src[0] = 1.0
+    src[-1] = torch.randn(m, generator=g, device="cuda")
+    signs = (torch.randint(0, 2, (m,), generator=g, device="cuda") * 2 - 1).half()
+    y = torch.empty(tokens, out, device="cuda")
+    ops.output_rht_blocks(src, signs, y, out, m, [8192] * 4)
+    ref = (fht64(src[-1:].double().cpu().numpy(), [8192] * 4) * signs.double().cpu().numpy())[:, :out]
+    err = np.abs(y[-1:].double().cpu().numpy() - ref).max()
+    del src
+    torch.cuda.empty_cache()
+    assert err <= 13 * 16 * 2.0 ** -24 * max(1.0, np.abs(ref).max())      # as in test_transform_blocks, 13 stages
