@@ -910,10 +910,12 @@ static size_t moe_gemm_smem_bytes(bool e8) {
   return (size_t)MOE_GEMM_STAGES * (GM_A_BYTES + (size_t)MOE_TN * 128) + (3 * MOE_GEMM_STAGES + 5) * 8 + 16 + 1024;
 }
 // routed tokens per expert (average) from which the tensor-core form is used (measured, 128 experts, top 8, streaming /
-// tensor-core: 64 tokens 260 / 263 us, 128 tokens 283 / 264, 256 tokens 333 / 271, 512 tokens 518 / 325)
-static int moe_gemm_min_avg() {
+// tensor-core: 64 tokens 260 / 263 us, 128 tokens 283 / 264, 256 tokens 333 / 271, 512 tokens 518 / 325).  With two
+// stages the GEMM multiplies fp16(w1 + s * w2), where the streaming kernel keeps exact weights and an fp32 sum per stage:
+// steps below 64 routed tokens per expert keep that precision.
+static int moe_gemm_min_avg(bool two_stages) {
   const char* e = getenv("GLQB_MOE_GEMM_MIN_AVG");
-  return e ? atoi(e) : 6;
+  return e ? atoi(e) : (two_stages ? 64 : 6);
 }
 
 }  // namespace glqb
@@ -931,7 +933,7 @@ struct GlqbMoePlan {
   int mid_sg = 1, out_rg = 1;          // slots per CTA of the mid kernel, routings per pass of the combine
   size_t mid_smem = 0, out_smem = 0;
   // tensor-core form
-  bool gemm_ok = false;
+  bool gemm_ok = false, two_stages = false;
   MoeDev devg;             // same weights, workspace laid out for the GEMM kernels
   MoeGemmKernel g13 = nullptr, g2 = nullptr;
   // optional timing of the two expert matmuls (event pairs around each, on the launching stream)
@@ -1124,11 +1126,12 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
   M.o_xr2 = o; o = al(o + R * d->inter * 2 * XR_TRELLIS_EXPAND);
   M.o_part2 = o; o = al(o + (size_t)M.kch2 * R * d->hidden * 4);
   P->ws_bytes = o;
+  P->two_stages = k13b || k2b;
   // tensor-core form: its buffers overlay the decode form's (a step runs one or the other)
   P->g13 = e8 ? moe_gemm_pick_e8(d->e8_stages) : moe_gemm_pick(k13a, k13b);
   P->g2 = e8 ? moe_gemm_pick_e8(d->e8_stages) : moe_gemm_pick(k2a, k2b);
   P->gemm_ok = P->g13 && P->g2 && d->hidden % GM_TILE_K == 0 && d->inter % GM_TILE_K == 0 && M.E <= 4096 &&
-               (e8 || R >= (size_t)M.E * moe_gemm_min_avg());
+               (e8 || R >= (size_t)M.E * moe_gemm_min_avg(P->two_stages));
   if (P->gemm_ok) {
     MoeDev& G = P->devg;
     G = M;
@@ -1223,7 +1226,7 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_);
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
   if (P->gemm_ok && (P->dev.format == GLQB_FMT_E8_SHELL ||
-                     (long long)tokens * P->dev.top_k >= (long long)P->dev.E * moe_gemm_min_avg())) {
+                     (long long)tokens * P->dev.top_k >= (long long)P->dev.E * moe_gemm_min_avg(P->two_stages))) {
     const MoeDev& G = P->devg;
     const int R = tokens * G.top_k;
     moe_launch_group(G, topk_ids, tokens, ws, st);

@@ -216,3 +216,28 @@ def test_moe_block_lists(hidden, inter, form, monkeypatch):
     err = np.abs(y.float().cpu().numpy() - ref).max() / np.abs(ref).max()
     ops.clear_caches()
     assert err <= 5e-3, err      # as above: two chained layers with fp16 hand-offs
+
+
+@pytest.mark.parametrize("T", [13, 40, 255])
+def test_moe_two_stages_keep_a_sum_per_stage(T, monkeypatch):
+    """Below 64 routed tokens per expert two-stage experts run the streaming kernels, whose weights are exact and whose
+    stages are summed in fp32 each (the GEMM multiplies fp16(w1 + s * w2)): the same bits as with that form forced."""
+    from glq_b200 import ops
+    E, hidden, inter, k = 8, 256, 128, 2
+    rng = np.random.default_rng(8000 + T)
+    d, w13_out = _make(rng, E, hidden, inter, 4, 2)
+    x_t = cuda(rng.standard_normal((T, hidden)).astype(np.float32), torch.float16)
+    ids = np.stack([rng.permutation(E)[:k] for _ in range(T)]).astype(np.int64)
+    w = rng.random((T, k)).astype(np.float32)
+    w /= w.sum(1, keepdims=True)
+    outs = []
+    for forced in (None, "1000000"):
+        monkeypatch.delenv("GLQB_MOE_GEMM_MIN_AVG", raising=False)
+        if forced:
+            monkeypatch.setenv("GLQB_MOE_GEMM_MIN_AVG", forced)
+        ops.clear_caches()
+        outs.append(_run(ops, d, x_t, cuda(ids), cuda(w), E, hidden, inter, w13_out, 2, 1))
+    ops.clear_caches()
+    assert torch.equal(outs[0], outs[1])
+    ref = _oracle(d, x_t.float().cpu().numpy(), ids, w, E, hidden, inter, w13_out, 4, 2, O.ACT_CODES[1])
+    assert np.abs(outs[0].float().cpu().numpy() - ref).max() <= 5e-3 * np.abs(ref).max()
