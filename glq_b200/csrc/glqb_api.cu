@@ -260,6 +260,17 @@ static int tn_for_batch(int batch, bool codes) {
   return ((batch + tiles - 1) / tiles + 15) & ~15;
 }
 
+// Two-stage trellis layers (whose weight decode costs twice as much) take 256-token tiles, decoded into shared memory by
+// glq_gemm_kernel, where that saves a pass over the weights and there are 8 M of them.  Measured with 4 + 2 bits, whole
+// plans, 192 / 256 tokens per tile: 256 tokens, 4096 x 4096 45 / 38 us, 11008 x 2048 57 / 42, 14336 x 4096 99 / 64,
+// 2048 x 2048 21.4 / 22.1; 384 tokens (two passes either way) 48 / 49, 60 / 62, 104 / 107; 512 tokens 59 / 50, 63 / 65,
+// 144 / 108; 1024 tokens of 2048 x 11008 143 / 127.
+static bool trellis_two_stage_256(const GlqbLinearDesc& d) {
+  const char* e = getenv("GLQB_TRELLIS_256_MIN_WEIGHTS");
+  return d.n_stages > 1 && (d.batch + 255) / 256 < (d.batch + TG_TN - 1) / TG_TN &&
+         (long long)d.m_pad * d.n_pad >= (e ? atoll(e) : (8ll << 20));
+}
+
 static int nb_for_batch(int batch) {
   if (batch <= 8) return 1;
   if (batch <= 16) return 2;
@@ -404,7 +415,7 @@ static int build_plan(GlqbPlan* P) {
     Key k;
     const bool trellis = d.format == GLQB_FMT_TRELLIS_3INST;
     const bool tiles = d.batch > DECODE_MAX_BATCH && (trellis ? trellis_tiles_once(d) : d.batch >= e8_two_phase_min_tokens());
-    const int tn = tn_for_batch(d.batch, trellis && !tiles);
+    const int tn = tn_for_batch(d.batch, trellis && !tiles && !trellis_two_stage_256(d));
     const int nb = tn ? 0 : nb_for_batch(d.batch);
     if (trellis)
       k = Key(d.format, d.bits[0], d.n_stages > 1 ? d.bits[1] : 0, d.n_stages, nb, tn, tiles ? 1 : 0);

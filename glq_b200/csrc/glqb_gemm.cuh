@@ -295,12 +295,12 @@ __device__ __forceinline__ void gemm_store_group(const uint32_t (&addr)[4], int 
 }
 
 // ---- the GEMM kernel -------------------------------------------------------------------------------
-// FORMAT 1: E8 (K1 = number of stages); FORMAT 2: the weight tiles were decoded beforehand (e8_tiles_kernel,
+// FORMAT 0: two-stage trellis codes (K1, K2 bits), 256 tokens per tile; FORMAT 1: E8 (K1 = number of stages); FORMAT 2: the weight tiles were decoded beforehand (e8_tiles_kernel,
 //           trellis_tiles_kernel) and are fetched like the activation tiles, one bulk copy per stage; the producer warps
-//           have nothing to do.  (Trellis codes are decoded by trellis_gemm_kernel.)
+//           have nothing to do.  (Other trellis layers are decoded by trellis_gemm_kernel.)
 // TN = 192: variable token tiles, for grouped experts.  A tile's activations are rows of ntok rounded up to 16, [k chunk]
 // [row] behind the row0 rows of the tiles before it; an item multiplies exactly that many columns.
-template <int FORMAT, int K1, int TN, int STAGES>
+template <int FORMAT, int K1, int K2, int TN, int STAGES>
 __global__ void __launch_bounds__(GM_THREADS, 1)
 glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict__ items, int n_items,
                 uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev) {
@@ -361,6 +361,45 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
       const int first = it.k_begin + (int)((grp - q0) & 1u);       // this group's first chunk of the item
       if constexpr (FORMAT == 2) {
         (void)first; (void)wl; (void)L;
+      } else if constexpr (FORMAT == 0) {
+        // warp wl of a group decodes the 32 x 32 trellis group at rows 32 (wl >> 1), columns 32 (wl & 1) of the chunk
+        const int strip = wl >> 1, cg = wl & 1;
+        const int rp = it.m_tile * 4 + strip, gps = L.groups_per_strip;
+        const bool row_ok = rp < L.strips;
+        const uint8_t* p1 = L.codes[0] + (long long)rp * gps * (128 * K1) + lane * (4 * K1);
+        const uint8_t* p2 = L.codes[1] + (long long)rp * gps * (128 * K2) + lane * (4 * K2);
+        const __half2 s2 = __float2half2_rn(L.stage_scale[1]);
+        Words<K1> nxt;
+        Words<K2> nxt2;
+        auto fetch = [&](int kc) {
+          const int cp = kc * 2 + cg;
+          if (row_ok && cp < gps) {
+            nxt = load_words<K1>(p1 + (long long)cp * (128 * K1));
+            nxt2 = load_words<K2>(p2 + (long long)cp * (128 * K2));
+          }
+        };
+        if (first < it.k_end) fetch(first);
+        for (int kc = first; kc < it.k_end; kc += 2) {
+          const uint32_t q = q0 + (uint32_t)(kc - it.k_begin);
+          const int stage = (int)(q % STAGES);
+          const Words<K1> v = nxt;
+          const Words<K2> v2 = nxt2;
+          if (kc + 2 < it.k_end) fetch(kc + 2);
+          if (!mbar_wait(&empty[stage], ((q / STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          __syncwarp();
+          uint32_t addr[4];
+          gemm_lane_addrs(smem_u32(a_base) + stage * GM_A_BYTES + strip * 4096, cg, lane, addr);
+          if (row_ok && kc * 2 + cg < gps) {                 // (uniform per warp: the shuffles inside see all lanes)
+            gemm_store_group<K1, K2>(addr, lane, v, v2, s2);
+          } else {                                           // rows or columns past the matrix: zeros
+            const uint32_t zero[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int p = 0; p < 4; ++p) gemm_store_quad(addr, p, zero);
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&full_a[stage]);
+        }
       } else {
         // E8: 128 rows x 8 indices per chunk; thread (row = tid >> 1, half = tid & 1) expands 4 indices
         const int tid = threadIdx.x & 255;                // thread inside the producer group

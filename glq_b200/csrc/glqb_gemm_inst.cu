@@ -21,8 +21,8 @@ typedef void (*GemmKernel)(const DevLinear*, const GemmItem*, int, uint8_t*, int
 
 template <int FORMAT, int K1>
 static GemmKernel gemm_kernel_tn(int tn) {
-  if (tn == 128) return glq_gemm_kernel<FORMAT, K1, 128, GEMM_STAGES>;
-  if (tn == 256) return glq_gemm_kernel<FORMAT, K1, 256, GEMM_STAGES>;
+  if (tn == 128) return glq_gemm_kernel<FORMAT, K1, 0, 128, GEMM_STAGES>;
+  if (tn == 256) return glq_gemm_kernel<FORMAT, K1, 0, 256, GEMM_STAGES>;
   return nullptr;
 }
 
@@ -52,6 +52,14 @@ static TilesKernel pick_trellis_tiles_kernel(int k1, int k2) {
 static GemmKernel pick_gemm_kernel(const Segment& s) {
   if (s.two_phase) return gemm_kernel_tn<2, 0>(s.tn);
   if (s.format == GLQB_FMT_TRELLIS_3INST) {
+    if (!trellis_form(s)) {
+#ifndef GLQB_FAST_BUILD
+#define G_CASE(A, B) if (s.k1 == A && s.k2 == B) return glq_gemm_kernel<0, A, B, 256, GEMM_STAGES>;
+      G_CASE(4, 1) G_CASE(4, 2) G_CASE(4, 3) G_CASE(4, 4)
+#undef G_CASE
+#endif
+      return nullptr;
+    }
 #define G_CASE(A, B) if (s.k1 == A && s.k2 == B) return trellis_gemm_kernel<A, B>;
 #ifdef GLQB_FAST_BUILD   /* developer builds for kernel experiments: the 4-bit single-stage rate only */
     G_CASE(4, 0)

@@ -33,8 +33,9 @@ struct Segment {
   int res_entries = 0;       // single-launch E8 form: table entries kept in shared memory (0: all gathers go to L1 / L2)
 };
 
-// does trellis_gemm_kernel run the segment's GEMM (and not glq_gemm_kernel)?  The activation layout follows from it.
-inline bool trellis_form(const Segment& s) { return s.tn && s.format == GLQB_FMT_TRELLIS_3INST && !s.two_phase; }
+// does trellis_gemm_kernel run the segment's GEMM?  (Else glq_gemm_kernel: decoded tiles, E8, two stages with 256-token
+// tiles.)  The activation layout follows from it.
+inline bool trellis_form(const Segment& s) { return s.tn && s.tn < 256 && s.format == GLQB_FMT_TRELLIS_3INST && !s.two_phase; }
 
 constexpr int GEMM_STAGES = 4;
 

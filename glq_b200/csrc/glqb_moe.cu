@@ -918,9 +918,9 @@ static MoeGemmKernel moe_gemm_pick(int k1, int k2) {
 }
 static MoeGemmKernel moe_gemm_pick_e8(int ns) {
   switch (ns) {
-    case 1: return glq_gemm_kernel<1, 1, MOE_TN, MOE_GEMM_STAGES>;
-    case 2: return glq_gemm_kernel<1, 2, MOE_TN, MOE_GEMM_STAGES>;
-    case 3: return glq_gemm_kernel<1, 3, MOE_TN, MOE_GEMM_STAGES>;
+    case 1: return glq_gemm_kernel<1, 1, 0, MOE_TN, MOE_GEMM_STAGES>;
+    case 2: return glq_gemm_kernel<1, 2, 0, MOE_TN, MOE_GEMM_STAGES>;
+    case 3: return glq_gemm_kernel<1, 3, 0, MOE_TN, MOE_GEMM_STAGES>;
   }
   return nullptr;
 }

@@ -60,3 +60,17 @@ def test_trellis_tiles_equal_fused_token_counts(tokens, bits, monkeypatch):
     a, _ = run(L, x, monkeypatch, {"GLQB_TRELLIS_TWO_PHASE_MIN_FLOPS": "1"})
     b, _ = run(L, x, monkeypatch, {"GLQB_TRELLIS_TWO_PHASE_MIN_FLOPS": "1e30"})
     assert torch.equal(a, b)
+
+
+# two-stage layers with 256-token tiles decoded into shared memory: one tile, its edge, the first sizes of two and three
+@pytest.mark.parametrize("bits", [[4, 1], [4, 2], [4, 3], [4, 4]], ids=str)
+@pytest.mark.parametrize("shape", [(32, 32), (160, 1056), (416, 96)], ids=str)
+def test_two_stage_256_token_tiles(shape, bits, monkeypatch):
+    m, n = shape
+    g = torch.Generator(device="cuda").manual_seed(m + n + sum(bits))
+    L = synth.trellis_layer("t", m, n, bits, g, "cuda")
+    for tokens in (193, 256, 385, 577):
+        x = torch.randn(tokens, n, generator=g, device="cuda").half()
+        a, _ = run(L, x, monkeypatch, {"GLQB_TRELLIS_256_MIN_WEIGHTS": "1"})
+        b, _ = run(L, x, monkeypatch, {"GLQB_TRELLIS_256_MIN_WEIGHTS": str(1 << 60)})
+        assert torch.equal(a, b)
