@@ -370,28 +370,45 @@ static bool out_plain(const GlqbPlan* P, const uint8_t* y_base) {
 
 static int rht_smem(int max_elems) { return fht_words(max_elems) * 4 + 64; }
 
-// one item per (layer, block, tile of tokens); tracks the largest tile (floats) for the launch's smem.
+// Tokens per CTA of the transform kernels: a tile of 8192 values (fht_block), less when the launch, with `blocks` Hadamard
+// blocks in all its layers, would leave SMs without work.
+static int rht_tile_tokens(int block_size, int batch, long long blocks, int sm_count) {
+  int t = std::min(std::max(1, std::min(64, 8192 / block_size)), batch);
+  while (t > 1 && blocks * ((batch + t - 1) / t) < sm_count) t = (t + 1) / 2;
+  return t;
+}
+
+// The blocks of one layer that a transform launch takes: those of at least 2^min_log values (the single-launch kernel
+// transforms the shorter output blocks itself).
+struct RhtLayer {
+  int layer, nblocks;
+  const int* logs;
+  int batch, min_log;
+};
+// One item per (layer, block, tile of tokens); tracks the largest tile (floats) for the launch's smem.
 // A block of more than 8192 values is shared by S = bs / 8192 CTAs per token, each producing one run of 8192 outputs
-// (RhtItem::sub).  `min_log`: only blocks of at least 2^min_log values get items (the single-launch kernel transforms
-// the shorter output blocks itself).
-static void add_rht_items(std::vector<RhtItem>& items, int layer, int nblocks, const int* logs, int batch,
-                          int& max_elems, int min_log = 0) {
-  for (int b = 0; b < nblocks; ++b) {
-    if (logs[b] < min_log) continue;
-    const int bs = 1 << logs[b];
-    if (logs[b] > FHT_LOG) {
-      for (int t = 0; t < batch; ++t)
-        for (int k = 0; k < (bs >> FHT_LOG); ++k) items.push_back(RhtItem{layer, b, t, 1, k});
-      max_elems = std::max(max_elems, 1 << FHT_LOG);
-      continue;
+// (RhtItem::sub).
+static void add_rht_items(std::vector<RhtItem>& items, const std::vector<RhtLayer>& layers, int sm_count, int& max_elems) {
+  long long blocks = 0;
+  for (const RhtLayer& r : layers)
+    for (int b = 0; b < r.nblocks; ++b) blocks += r.logs[b] >= r.min_log;
+  for (const RhtLayer& r : layers)
+    for (int b = 0; b < r.nblocks; ++b) {
+      if (r.logs[b] < r.min_log) continue;
+      const int bs = 1 << r.logs[b];
+      if (r.logs[b] > FHT_LOG) {
+        for (int t = 0; t < r.batch; ++t)
+          for (int k = 0; k < (bs >> FHT_LOG); ++k) items.push_back(RhtItem{r.layer, b, t, 1, k});
+        max_elems = std::max(max_elems, 1 << FHT_LOG);
+        continue;
+      }
+      const int tt = rht_tile_tokens(bs, r.batch, blocks, sm_count);
+      for (int t0 = 0; t0 < r.batch; t0 += tt) {
+        const int nt = std::min(tt, r.batch - t0);
+        items.push_back(RhtItem{r.layer, b, t0, nt, -1});
+        max_elems = std::max(max_elems, nt * bs);
+      }
     }
-    const int tt = rht_tile_tokens(bs, batch, nblocks);
-    for (int t0 = 0; t0 < batch; t0 += tt) {
-      const int nt = std::min(tt, batch - t0);
-      items.push_back(RhtItem{layer, b, t0, nt, -1});
-      max_elems = std::max(max_elems, nt * bs);
-    }
-  }
 }
 
 static int build_plan(GlqbPlan* P) {
@@ -751,6 +768,7 @@ static int build_plan(GlqbPlan* P) {
                   "layer %d: the fused norm / activation / residual steps are served by the single-launch decode form only "
                   "(at most %d tokens, all layers of the call reading one input)", P->order[pos], FUSED_MAX_TOKENS);
   }
+  std::vector<RhtLayer> rht_in, rht_in_gemm, rht_out;      // what the three transform launches of a run take
   for (int pos = 0; pos < n; ++pos) {
     DevLinear& L = P->dev[pos];
     const GlqbLinearDesc& d = P->descs[P->order[pos]];
@@ -764,7 +782,7 @@ static int build_plan(GlqbPlan* P) {
         if (first == pos) {
           L.xr_off = (long long)ws;
           ws = align_up(ws + (size_t)L.batch * L.n * sizeof(__half) * XR_TRELLIS_EXPAND, 1024);
-          add_rht_items(P->items_in, pos, L.nbn, L.bn_log, L.batch, P->max_elems_in);
+          rht_in.push_back({pos, L.nbn, L.bn_log, L.batch, 0});
         } else {
           L.xr_off = P->dev[first].xr_off;
         }
@@ -773,7 +791,7 @@ static int build_plan(GlqbPlan* P) {
       ws = align_up(ws + (size_t)L.slots * L.batch * L.m * sizeof(float), 256);
       L.rstd_off = (long long)ws;
       ws += 256;
-      add_rht_items(P->items_out, pos, L.nbm, L.bm_log, L.batch, P->max_elems_out, L.stop_at_yrht ? 64 : L.out_split_log);
+      rht_out.push_back({pos, L.nbm, L.bm_log, L.batch, L.stop_at_yrht ? 64 : L.out_split_log});
       continue;
     }
     int same = -1;
@@ -798,13 +816,13 @@ static int build_plan(GlqbPlan* P) {
       if (L.gemm_tn) {
         const size_t n_tiles = (L.batch + L.gemm_tn - 1) / L.gemm_tn, kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
         ws = align_up(ws + n_tiles * kchunks * L.gemm_tn * 128, 256);
-        add_rht_items(P->items_in_gemm, pos, L.nbn, L.bn_log, L.batch, P->max_elems_in);
+        rht_in_gemm.push_back({pos, L.nbn, L.bn_log, L.batch, 0});
       } else {
         // E8 with several tokens interleaves groups of 8 tokens: round the token count up
         const size_t xr_tokens = (L.format == GLQB_FMT_E8_SHELL && L.batch > 1) ? (size_t)((L.batch + 7) / 8 * 8) : (size_t)L.batch;
         ws = align_up(ws + xr_tokens * L.n * sizeof(__half) *
                                (L.format == GLQB_FMT_TRELLIS_3INST ? XR_TRELLIS_EXPAND : 1), 256);
-        add_rht_items(P->items_in, pos, L.nbn, L.bn_log, L.batch, P->max_elems_in);
+        rht_in.push_back({pos, L.nbn, L.bn_log, L.batch, 0});
       }
     }
     L.part_off = (long long)ws;
@@ -814,8 +832,11 @@ static int build_plan(GlqbPlan* P) {
       L.atile_off = (long long)ws;
       ws += (size_t)((L.m + GM_TILE_M - 1) / GM_TILE_M) * ((L.n + GM_TILE_K - 1) / GM_TILE_K) * GM_A_BYTES;
     }
-    add_rht_items(P->items_out, pos, L.nbm, L.bm_log, L.batch, P->max_elems_out);
+    rht_out.push_back({pos, L.nbm, L.bm_log, L.batch, 0});
   }
+  add_rht_items(P->items_in, rht_in, P->sm_count, P->max_elems_in);
+  add_rht_items(P->items_in_gemm, rht_in_gemm, P->sm_count, P->max_elems_in);
+  add_rht_items(P->items_out, rht_out, P->sm_count, P->max_elems_out);
   P->ws_bytes = ws;
   P->out_plain_static = true;
   for (const RhtItem& it : P->items_out) {
@@ -1117,7 +1138,9 @@ static int run_rht_single(bool input, const void* src, int src_dtype, int64_t sr
   memset(&L, 0, sizeof L);
   RhtSingle S;
   memset(&S, 0, sizeof S);
-  int off = 0, max_elems = 32, ctas = 0;
+  int off = 0, max_elems = 32, ctas = 0, dev_id = 0, sm_count = 0;
+  CUDA_TRY(cudaGetDevice(&dev_id));
+  CUDA_TRY(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev_id));
   for (int i = 0; i < n_blocks; ++i) {
     const int b = blocks[i];
     if (b < 1 || (b & (b - 1)) || b > 32768) return fail(GLQB_E_INVALID, "rht: block %d", b);
@@ -1125,7 +1148,7 @@ static int run_rht_single(bool input, const void* src, int src_dtype, int64_t sr
     if (o < 0 || o + b > pad) return fail(GLQB_E_INVALID, "rht: block %d at column %d exceeds %d columns", b, o, pad);
     if (input) { L.bn_off[i] = o; L.bn_log[i] = ilog2(b); } else { L.bm_off[i] = o; L.bm_log[i] = ilog2(b); }
     off += b;
-    const int tt = rht_tile_tokens(b, batch, n_blocks);
+    const int tt = rht_tile_tokens(b, batch, n_blocks, sm_count);
     S.first_cta[i] = ctas;
     S.tile_tokens[i] = tt;
     S.runs[i] = std::max(1, b >> FHT_LOG);

@@ -65,17 +65,6 @@ struct RhtItem {
                // the short factor applied while loading, so S CTAs share a long block without talking
 };
 
-// Tokens per CTA of the transform kernels: a tile of 8192 values (fht_block), less when that would leave SMs without
-// work (`ctas` is what the launch has besides, at one token per CTA and block).
-static inline int rht_tile_tokens(int block_size, int batch, int blocks) {
-  int t = 8192 / block_size;
-  if (t < 1) t = 1;
-  if (t > 64) t = 64;
-  if (t > batch) t = batch;
-  while (t > 1 && (long long)blocks * ((batch + t - 1) / t) < 148) t = (t + 1) / 2;
-  return t;
-}
-
 // Stores the message glqb_last_error() returns for the calling thread (defined in glqb_api.cu).
 void set_error_message(const char* msg);
 

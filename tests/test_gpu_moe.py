@@ -241,3 +241,22 @@ def test_moe_two_stages_keep_a_sum_per_stage(T, monkeypatch):
     assert torch.equal(outs[0], outs[1])
     ref = _oracle(d, x_t.float().cpu().numpy(), ids, w, E, hidden, inter, w13_out, 4, 2, O.ACT_CODES[1])
     assert np.abs(outs[0].float().cpu().numpy() - ref).max() <= 5e-3 * np.abs(ref).max()
+
+
+def test_moe_even_tiles():
+    """Routed tokens per expert at the edges of the token tiles of the tensor-core form: none, one, one step of 16 and one
+    more, one whole tile of 192 and one more (two even tiles of 112 and 81), three tiles."""
+    from glq_b200 import ops
+    counts = [0, 1, 16, 17, 192, 193, 385, 0]
+    E, hidden, inter, T = len(counts), 128, 64, sum(counts)
+    rng = np.random.default_rng(77)
+    d, w13_out = _make(rng, E, hidden, inter, 4)
+    x_t = cuda(rng.standard_normal((T, hidden)).astype(np.float32), torch.float16)
+    ids = rng.permutation(np.repeat(np.arange(E), counts)).astype(np.int64)[:, None]
+    w = rng.random((T, 1)).astype(np.float32)
+    ops.clear_caches()
+    y = _run(ops, d, x_t, cuda(ids), cuda(w), E, hidden, inter, w13_out, 0, 1)
+    assert torch.equal(y, _run(ops, d, x_t, cuda(ids), cuda(w), E, hidden, inter, w13_out, 0, 1))
+    ref = _oracle(d, x_t.float().cpu().numpy(), ids, w, E, hidden, inter, w13_out, 4, 0, O.ACT_CODES[1])
+    ops.clear_caches()
+    assert np.abs(y.float().cpu().numpy() - ref).max() <= 5e-3 * np.abs(ref).max()
