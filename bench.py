@@ -251,9 +251,13 @@ def kernel_name(W):
         tn = 128 if T <= 128 else 256
         if fmt == "trellis":
             rate = f"{par[0]},{par[1] if len(par) > 1 else 0}"
-            return (f"trellis_gemm_kernel<{rate}> (layers of 60 GFLOP and more: trellis_tiles_kernel<{rate}> + glq_gemm_kernel<tiles,256,4>)")
+            wide = (f", glq_gemm_kernel<trellis,{rate},256,4> where 256-token tiles save a pass over 8 M weights or more"
+                    if len(par) > 1 else "")
+            return (f"trellis_gemm_kernel<{rate}> (layers of 60 GFLOP and more: trellis_tiles_kernel<{rate}> + glq_gemm_kernel<tiles,256,4>{wide})")
         if T >= 129:
-            return f"e8_tiles_smem_kernel<{ns}> + glq_gemm_kernel<tiles,{tn},4> (weight tiles decoded once, then the copy-fed GEMM)"
+            resident = W["code_bytes"] >= int(os.environ.get("GLQB_E8_SMEM_MIN_BYTES", str(48 << 20)))
+            tiles = "e8_tiles_smem_kernel" if resident else "e8_tiles_kernel"
+            return f"{tiles}<{ns}> + glq_gemm_kernel<tiles,{tn},4> (weight tiles decoded once, then the copy-fed GEMM)"
         return f"glq_gemm_kernel<e8,{ns},{tn},4>"
     nb = 1 if T <= 8 else 2 if T <= 16 else 4 if T <= 32 else 8
     if fmt == "trellis":

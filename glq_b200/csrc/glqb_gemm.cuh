@@ -1,11 +1,11 @@
-// Prefill path: decoded weight tiles -> swizzled shared memory -> tcgen05.mma with fp32 accumulators in
-// tensor memory (TMEM).  One CTA computes D[128 weight rows x TN tokens] = W~[128 x K] * X~[TN x K]^T.
+// Prefill path with both operands in swizzled shared memory (E8 layers, weight tiles decoded beforehand, two-stage trellis
+// codes; the other trellis layers: glqb_tgemm.cuh) -> tcgen05.mma with fp32 accumulators in tensor memory (TMEM).  One CTA computes D[128 weight rows x TN tokens] = W~[128 x K] * X~[TN x K]^T.
 //
 // Warp roles (GM_THREADS = 704):
 //   warps 0-15 decode producers in two groups of eight; group 0 produces the even 128x64 weight chunks,
 //              group 1 the odd ones (two stages are always being filled).  Inside a group every warp
-//              decodes 16 rows x 64 columns of E8 indices into the stage's A tile, K-major with the 128-byte
-//              swizzle the tensor core expects
+//              decodes 16 rows x 64 columns of E8 indices, or a 32 x 32 trellis group, into the stage's A tile,
+//              K-major with the 128-byte swizzle the tensor core expects
 //   warps 18-21 epilogue: tcgen05.ld of the finished accumulator (two accumulators alternate, so the
 //              next tile's MMAs run while these warps write the previous tile's partial sums)
 //   warp  16   one thread issues tcgen05.mma (4 per chunk: K = 16 each) and tcgen05.commit
@@ -753,8 +753,8 @@ e8_tiles_smem_kernel(const DevLinear* __restrict__ layers, int first, int count,
 // The counterpart of e8_tiles_kernel: a warp decodes a 32-row x 64-column slice (two 32 x 32 groups) into its own 4 KiB of
 // shared memory with the stores the GEMM's producers use — the slice is 4 KiB of the tile image in one piece — and
 // copies it out with whole-line 16-byte stores.  The codes of the next slice are in flight meanwhile.  Bound by the
-// state decode: 11008 x 2048 in 13 us; with the copy-fed GEMM behind it 97 us where the fused GEMM takes 117 (2048
-// tokens).
+// state decode: 11008 x 2048 in 13 us.  Whole linears of 2048 tokens with the copy-fed GEMM behind it / with
+// trellis_gemm_kernel: 11008 x 2048 138 / 146 us, 14336 x 4096 272 / 288, two stages (4 + 2 bits) 142 / 207, 279 / 438.
 constexpr int TT_THREADS = 256;
 template <int K1, int K2>
 __global__ void __launch_bounds__(TT_THREADS, 3)

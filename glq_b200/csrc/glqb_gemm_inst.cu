@@ -1,4 +1,4 @@
-// Instantiations and launches of the tensor-core GEMM kernels and the E8 tile decode (see glqb_gemm.cuh).
+// Instantiations and launches of the tensor-core GEMM kernels and the tile decodes (see glqb_gemm.cuh, glqb_tgemm.cuh).
 #include "glqb_kernels.cuh"
 #include "glqb_gemm.cuh"
 #include "glqb_tgemm.cuh"

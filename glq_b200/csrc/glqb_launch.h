@@ -1,5 +1,5 @@
 // Host-side launch interface between the plan builder (glqb_api.cu) and the translation units that
-// instantiate the large kernel families (glqb_gemm_inst.cu: tensor-core GEMM and E8 tile decode;
+// instantiate the large kernel families (glqb_gemm_inst.cu: tensor-core GEMMs and tile decodes;
 // glqb_fused.cu: single-launch decode).  Splitting them keeps every unit's compile time in check.
 #pragma once
 #include "glqb_internal.h"
@@ -13,8 +13,9 @@ struct GemmItem;
 // token-column blocks, contiguous in the device table.
 struct Segment {
   int format, k1, k2, ns, nb;
-  int tn;                    // 0: streaming decode kernel; 128 / 256: tensor-core GEMM with that token tile
-  int two_phase = 0;         // E8 GEMM with many tokens: weight tiles decoded once beforehand
+  int tn;                    // 0: streaming decode kernel; else tensor-core GEMM with that token tile (glq_gemm_kernel: 128
+                             // or 256, trellis_gemm_kernel: a multiple of 16 up to 192)
+  int two_phase = 0;         // GEMM with many tokens: weight tiles decoded once beforehand (E8, large trellis layers)
   // single-launch form (input transform + decode + output transform in one kernel): all layers read one input
   bool fused = false;
   int total_units = 0, scratch_elems = 0;
@@ -43,7 +44,7 @@ constexpr int GEMM_STAGES = 4;
 bool gemm_available(const Segment& s);                       // is there a kernel for the segment's format / rates?
 cudaError_t gemm_prepare(const Segment& s);                  // raises the kernel's dynamic shared-memory limit
 cudaError_t tiles_smem_prepare(int ns);                      // same for the resident-table tile decode
-// the segment's launches: (two-phase E8: tile decode, then) the GEMM over `items`
+// the segment's launches: (two-phase: tile decode, then) the GEMM over `items`
 void gemm_launch(const Segment& s, const DevLinear* layers, const GemmItem* items, uint8_t* ws, int* status,
                  int sm_count, cudaStream_t stream);
 

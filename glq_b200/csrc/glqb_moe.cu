@@ -20,11 +20,12 @@
 // Integer atomics decide only WHERE a routing is stored, never a numeric value: outputs are
 // bit-identical run to run.
 //
-// Steps with many routed tokens per expert take the tensor-core form instead: launches 3 and 5 become the
-// tcgen05 GEMM kernel (glq_gemm_kernel, trellis producers) over a work list that the grouping kernel builds
+// Steps with enough routed tokens per expert (moe_gemm_min_avg) take the tensor-core form instead, E8 experts always:
+// launches 3 and 5 become trellis_gemm_kernel (E8: glq_gemm_kernel) over a work list that the grouping kernel builds
 // on the device from the expert counts — every expert is a "layer" whose token count, activation tiles and
-// partial-sum rows are patched in each run; experts' routings are padded to whole 128-token tiles.  The
-// transforms write the activations straight into the swizzled tile images the GEMM's bulk copies fetch.
+// partial-sum rows are patched in each run; an expert's routings are split evenly over tiles of at most 192, each
+// padded to a multiple of 16.  The transforms write the activations straight into the swizzled tile images the GEMM's
+// bulk copies fetch.
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>

@@ -1,11 +1,11 @@
 // Prefill and grouped experts on trellis weights: states decoded straight into tensor memory as the A operand of
 // tcgen05.mma, activations streamed through shared memory.
 //
-// Why A goes to tensor memory: with A and B both in shared memory the 128 bytes per clock of an SM were the limit — per
-// 128 x 64 x 256 chunk 48 KiB of operand reads, 16 KiB of producer stores and 32 KiB of copies are 768 clocks, the tensor
-// pipe needs 512 (measured: 1010 clocks per chunk, the MMA thread waiting for neither operand).  A lane of a decoding
-// warp holds exactly the fragment layout of tcgen05.st.16x128b (row g and g + 8, columns 2t and 2t + 1 of every 16 x 8
-// block), so two stores replace sixteen and the chunk leaves 64 KiB of shared-memory traffic.
+// Why A goes to tensor memory: a lane of a decoding warp holds exactly the fragment layout of tcgen05.st.16x128b (row g
+// and g + 8, columns 2t and 2t + 1 of every 16 x 8 block), so two stores replace sixteen and a 128 x 64 x 256 chunk leaves
+// 64 KiB of shared-memory traffic instead of 96 (768 clocks at 128 bytes, where the tensor pipe needs 512).  That alone
+// changed nothing (1010 -> 1045 clocks per chunk): the limit was the issuing thread's own loop, see the MMA issuer below,
+// and with that loop warp-uniform a chunk takes 742.
 //
 // One CTA computes 128 weight rows x up to 192 tokens: two accumulators of 192 columns and four 64-column chunks of A
 // (32 columns each) fill the 512 columns of tensor memory.  Warp roles: warp 0 issues MMAs, warp 1 the bulk copies (TMA
@@ -182,7 +182,7 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
   } else if (warp >= TG_PROD_WARP0) {
     // ------------------------------------------------------------------ producers
     // q numbers the chunks of this CTA over all its items, every item rounded up to pairs (the second half of a last odd
-    // pair is handed over without being written or multiplied); chunk q is half q & 1 of pair q >> 1
+    // pair is filled with zeros and not multiplied); chunk q is half q & 1 of pair q >> 1
     const int grp = (warp - TG_PROD_WARP0) >> 3, strip = warp & 3, cg = (warp >> 2) & 1;
     const uint32_t lanes = tmem_a + ((uint32_t)(strip * 32) << 16) + (uint32_t)(cg * 16);
     uint32_t q0 = 0;
