@@ -539,7 +539,7 @@ static int build_plan(GlqbPlan* P) {
       // the extra launch); so is a fused RMSNorm whose output block is too long for the in-kernel transform
       static const int in_max_n = [] { const char* e = getenv("GLQB_FUSED_IN_MAX_N"); return e ? atoi(e) : 4096; }();
       bool xr_global = d0.n_pad > in_max_n;
-      for (int i = 0; i < d0.n_blocks_n; ++i) xr_global = xr_global || d0.blocks_n[i] > (1 << FUSED_IN_MAX_LOG);
+      for (int i = 0; i < d0.n_blocks_n; ++i) xr_global = xr_global || d0.blocks_n[i] > (1 << fused_in_max_log(e8));
       // Output blocks of at least 2^out_split_log rows are left to rht_out_kernel; shorter
       // ones are transformed inside the decode kernel by the CTA that completes them.  Measured on B200 (decoder
       // chain, SmolLM3-3B shapes): an extra launch costs more than the 8192-row transform it takes out of the

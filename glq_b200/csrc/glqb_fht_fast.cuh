@@ -31,8 +31,12 @@ __device__ __forceinline__ void fht_regs(float (&v)[1 << R]) {
 //   call of `store` the lanes of a warp hold consecutive i.
 // `smem` needs bs + bs / 32 floats (index i lives at i + i / 32).  All 256 threads must call; `load(i0, v)` fills v[0..E) with values
 // i0 .. i0 + E - 1.
+// What `store` needs besides the transformed value (a sign) is requested by `pre(i)` for exactly the indices the thread
+// will store: up front, so that it arrives while the transform runs, or, with LATE values per thread and more, once the
+// values sit in shared memory and have left their registers free.  PACK: `pre` gives fp16 and two are kept per register,
+// else fp32.  (Both kinds of register cost spills in kernels that hold prefetched codes, see fused_out_block.)
 // ---------------------------------------------------------------------------------------------------
-template <int E, class Load, class Pre, class Store>
+template <int E, int LATE, bool PACK, class Load, class Pre, class Store>
 __device__ __forceinline__ void fht_fast_e(float* smem, int logbs, Load& load, Pre& pre, Store& store) {
   constexpr int LOGE = E == 1 ? 0 : E == 2 ? 1 : E == 4 ? 2 : E == 8 ? 3 : E == 16 ? 4 : 5;
   constexpr int QMAX = E >= 8 ? E / 8 : 1;         // rounds of the final loop (values per warp / 256)
@@ -42,22 +46,39 @@ __device__ __forceinline__ void fht_fast_e(float* smem, int logbs, Load& load, P
   const int W = nthreads >> 5;                     // warps that hold values (1 .. 8)
   const bool active = t < nthreads;
   const int span = 32 << LOGE;                     // values per warp = distance between the W partners
-  // What `store` needs besides the transformed value (a sign, the old output, ...) is requested first by
-  // `pre(i)`, for exactly the indices this thread will store, so that it arrives while the transform runs.
-  float aux[QMAX][8];
-  if (W == 1) {
-    if (active) {
+  uint32_t aux[QMAX][PACK ? 4 : 8];
+  auto aux_of = [](const uint32_t (&a)[PACK ? 4 : 8], int w) -> float {
+    if constexpr (PACK) return __half2float(__ushort_as_half((unsigned short)(a[w >> 1] >> ((w & 1) * 16))));
+    else return __uint_as_float(a[w]);
+  };
+  auto request = [&]() {
+    if (W == 1) {
+      if (active) {
 #pragma unroll
-      for (int j = 0; j < E; ++j) aux[0][j] = pre(t * E + j);        // E <= 1 here (32 values, one warp)
+        for (int j = 0; j < E; ++j) {                                  // E <= 1 here (32 values, one warp)
+          if constexpr (PACK) aux[0][0] = __half_as_ushort(pre(t * E + j));
+          else aux[0][j & 7] = __float_as_uint(pre(t * E + j));
+        }
+      }
+      return;
     }
-  } else {
 #pragma unroll
     for (int q = 0; q < QMAX; ++q) {
       const int r = t + 256 * q;
 #pragma unroll
-      for (int w = 0; w < 8; ++w) aux[q][w] = (r < span && w < W) ? pre(w * span + r) : 0.f;
+      for (int w = 0; w < 8; ++w) {
+        if constexpr (PACK) {
+          if (w & 1) continue;
+          const __half z = __ushort_as_half(0), lo = (r < span && w < W) ? pre(w * span + r) : z;
+          const __half hi = (r < span && w + 1 < W) ? pre((w + 1) * span + r) : z;
+          aux[q][w >> 1] = (uint32_t)__half_as_ushort(lo) | ((uint32_t)__half_as_ushort(hi) << 16);
+        } else {
+          aux[q][w] = __float_as_uint((r < span && w < W) ? pre(w * span + r) : 0.f);
+        }
+      }
     }
-  }
+  };
+  if constexpr (E < LATE) request();
   float v[E];
   if (active) {
     load(t * E, v);
@@ -75,7 +96,7 @@ __device__ __forceinline__ void fht_fast_e(float* smem, int logbs, Load& load, P
   if (W == 1) {
     if (active) {
 #pragma unroll
-      for (int j = 0; j < E; ++j) store(t * E + j, v[j], aux[0][j]);
+      for (int j = 0; j < E; ++j) store(t * E + j, v[j], aux_of(aux[0], j & 7));
     }
     return;
   }
@@ -83,6 +104,7 @@ __device__ __forceinline__ void fht_fast_e(float* smem, int logbs, Load& load, P
 #pragma unroll
     for (int j = 0; j < E; ++j) smem[fht_pad(t * E + j)] = v[j];
   }
+  if constexpr (E >= LATE) request();
   __syncthreads();
   const int logw = W == 2 ? 1 : W == 4 ? 2 : 3;
 #pragma unroll
@@ -104,16 +126,16 @@ __device__ __forceinline__ void fht_fast_e(float* smem, int logbs, Load& load, P
       }
 #pragma unroll
       for (int w = 0; w < 8; ++w)
-        if (w < W) store(w * span + r, u[w], aux[q][w]);
+        if (w < W) store(w * span + r, u[w], aux_of(aux[q], w));
     }
   }
 }
 
 // dispatch on the array length (2^logbs, 32 .. 8192)
-template <int MAXLOG = 13, class Load1, class Load4, class Pre, class Store>
+template <int MAXLOG, int LATE, bool PACK, class Load1, class Load4, class Pre, class Store>
 __device__ __forceinline__ void fht_fast(float* smem, int logbs, Load1 load1, Load4 load4, Pre pre, Store store) {
   // load1(i) -> value i;  load4(i0, float (&q)[4]) -> values i0 .. i0 + 3 (i0 a multiple of 4);
-  // pre(i) -> float handed back to store(i, value, that float)
+  // pre(i) -> what store(i, value, x) gets as x (fp32; PACK: given as fp16)
   auto ld1 = [&](int i0, float (&v)[1]) { v[0] = load1(i0); };
   auto ld2 = [&](int i0, float (&v)[2]) { v[0] = load1(i0); v[1] = load1(i0 + 1); };
   auto ld4 = [&](int i0, float (&v)[4]) { load4(i0, v); };
@@ -133,12 +155,12 @@ __device__ __forceinline__ void fht_fast(float* smem, int logbs, Load1 load1, Lo
     for (int k = 0; k < 8; ++k) { load4(i0 + 4 * k, q); v[4 * k] = q[0]; v[4 * k + 1] = q[1]; v[4 * k + 2] = q[2]; v[4 * k + 3] = q[3]; }
   };
   // arrays longer than 2^MAXLOG never reach this instantiation (their cases are not compiled)
-  if (logbs == 9) { fht_fast_e<2>(smem, logbs, ld2, pre, store); return; }
-  if (logbs == 10) { fht_fast_e<4>(smem, logbs, ld4, pre, store); return; }
-  if constexpr (MAXLOG >= 11) if (logbs == 11) { fht_fast_e<8>(smem, logbs, ld8, pre, store); return; }
-  if constexpr (MAXLOG >= 12) if (logbs == 12) { fht_fast_e<16>(smem, logbs, ld16, pre, store); return; }
-  if constexpr (MAXLOG >= 13) if (logbs == 13) { fht_fast_e<32>(smem, logbs, ld32, pre, store); return; }
-  fht_fast_e<1>(smem, logbs, ld1, pre, store);                        // 32 .. 256 values
+  if (logbs == 9) { fht_fast_e<2, LATE, PACK>(smem, logbs, ld2, pre, store); return; }
+  if (logbs == 10) { fht_fast_e<4, LATE, PACK>(smem, logbs, ld4, pre, store); return; }
+  if constexpr (MAXLOG >= 11) if (logbs == 11) { fht_fast_e<8, LATE, PACK>(smem, logbs, ld8, pre, store); return; }
+  if constexpr (MAXLOG >= 12) if (logbs == 12) { fht_fast_e<16, LATE, PACK>(smem, logbs, ld16, pre, store); return; }
+  if constexpr (MAXLOG >= 13) if (logbs == 13) { fht_fast_e<32, LATE, PACK>(smem, logbs, ld32, pre, store); return; }
+  fht_fast_e<1, LATE, PACK>(smem, logbs, ld1, pre, store);                        // 32 .. 256 values
 }
 constexpr int FHT_FAST_MAX_LOG = 13;
 

@@ -46,14 +46,20 @@ __host__ __device__ __forceinline__ size_t fused_smem_bytes(int n, int batch, in
   return xs + ((size_t)scratch_elems + scratch_elems / 32) * 4 + 8 * 256 * 4 + 64;
 }
 
-// Output transform of one (layer, Hadamard block, token) by the CTA that completed the block, with the
-// low-latency transform.  Blocks of up to 8192 rows (longer ones are left to rht_out_kernel).
-constexpr int FUSED_IN_MAX_LOG = 13;             // longest input block of the in-kernel shuffle transform: 8192
+// longest input block of the in-kernel shuffle transform (8192; E8, whose prefetched indices leave fewer registers, 4096)
+__host__ __device__ constexpr int fused_in_max_log(bool e8) { return e8 ? 12 : 13; }
 constexpr int FUSED_OUT_MAX_LOG = 13;            // longest output block the kernel can transform itself: 8192 (see out_split_log)
 
+// Output transform of one (layer, Hadamard block, token) by the CTA that completed the block, with the
+// low-latency transform.  Blocks of up to 8192 rows (longer ones are left to rht_out_kernel).
 // `C` (tensor-parallel ranks, row-parallel layer): instead of being written to y, the block's transformed values are
 // stored into every rank's receive area at float offset `piece` (this rank's source slot of epoch `comm_e`); the
 // caller exchanges flags and adds the ranks' blocks afterwards.
+// Registers are short here (128 per thread, two CTAs per SM, the next unit's codes may be in flight): one offset instead
+// of a pointer per rank, signs packed (E8) and requested late by threads with LATE values or more (fht_fast_e).  E8 kernels
+// without that spilled 51 words instead of 22 and took 17.5 us for two stages of 2048 x 2048 (one token, in a graph) instead
+// of 16.8, 14.2 instead of 12.6 for 4096 x 512.
+template <bool E8FMT, int LATE>
 __device__ __forceinline__ void fused_out_block(const DevLinear& L, int b, int tok, float in_scale,
                                                 const uint8_t* __restrict__ ws, uint8_t* __restrict__ y_base, float* fbuf,
                                                 const CommDev* C = nullptr, int comm_e = 0, long long piece = 0) {
@@ -91,7 +97,9 @@ __device__ __forceinline__ void fused_out_block(const DevLinear& L, int b, int t
   const float rs = rsqrtf((float)(1 << logbs));
   const __half* su = L.su + off;
   const bool accumulate = L.y_accumulate != 0;
-  auto pre = [&](int i) -> float { return __half2float(su[i]); };      // the sign, requested before the partial sums
+  auto pre = [&](int i) {                                              // the sign, requested before the partial sums
+    if constexpr (E8FMT) return su[i]; else return __half2float(su[i]);
+  };
   auto store = [&](int i, float val, float sign) {
     if (off + i < out_f) {
       float r = val * rs * sign;
@@ -100,20 +108,18 @@ __device__ __forceinline__ void fused_out_block(const DevLinear& L, int b, int t
     }
   };
   if (C) {
-    float* dst[COMM_MAX_RANKS];
-#pragma unroll
-    for (int r = 0; r < COMM_MAX_RANKS; ++r) dst[r] = r < C->world ? comm_slot(*C, r, comm_e, C->rank) + piece : nullptr;
     const int world = C->world;
+    const size_t at = (size_t)(comm_slot(*C, 0, comm_e, C->rank) - C->data[0]) + (size_t)piece;      // the same in every area
     auto push = [&](int i, float val, float sign) {                    // consecutive threads, consecutive i
       const float r = val * rs * sign;
 #pragma unroll
       for (int k = 0; k < COMM_MAX_RANKS; ++k)
-        if (k < world) dst[k][i] = r;
+        if (k < world) C->data[k][at + i] = r;
     };
-    fht_fast<FUSED_OUT_MAX_LOG>(fbuf, logbs, load1, load4, pre, push);
+    fht_fast<FUSED_OUT_MAX_LOG, LATE, E8FMT>(fbuf, logbs, load1, load4, pre, push);
     return;
   }
-  fht_fast<FUSED_OUT_MAX_LOG>(fbuf, logbs, load1, load4, pre, store);
+  fht_fast<FUSED_OUT_MAX_LOG, LATE, E8FMT>(fbuf, logbs, load1, load4, pre, store);
 }
 
 // Phase 1 of the single-launch decode kernels: the transformed activations of the shared input, in shared memory
@@ -187,7 +193,7 @@ __device__ __forceinline__ void fused_phase1(const DevLinear& L0, int batch, con
             for (int k = 0; k < 4; ++k) q[k] = load1(off + i0 + k);
           }
         };
-        fht_fast<FUSED_IN_MAX_LOG>(fbuf, logbs, ld1, load4, none, put3);
+        fht_fast<fused_in_max_log(E8FMT), 64, false>(fbuf, logbs, ld1, load4, none, put3);
         __syncthreads();
       }
       if (nw) {                                              // every value of the token was loaded exactly once
@@ -209,6 +215,7 @@ __device__ __forceinline__ void fused_phase1(const DevLinear& L0, int batch, con
 
 // Phase 3 of the single-launch decode kernels: output transforms of the blocks this CTA completed (`todo` entries
 // are (layer << 8) | block), with the sum over tensor-parallel ranks when the layer asks for it.
+template <bool E8FMT, int LATE>
 __device__ __forceinline__ void fused_phase3(const DevLinear* layers, const int* todo, int nt, int batch, const float* rstd_s,
                                              const uint8_t* __restrict__ ws, uint8_t* __restrict__ y_base, float* fbuf,
                                              int scratch_elems, const CommDev& C, int comm_e) {
@@ -223,7 +230,7 @@ __device__ __forceinline__ void fused_phase3(const DevLinear* layers, const int*
       const int logbs = L.bm_log[b], bs = 1 << logbs, off = L.bm_off[b];
       const long long piece = (long long)L.comm_off + (long long)off * batch;            // floats; a multiple of 32
       for (int tok = 0; tok < batch; ++tok) {
-        fused_out_block(L, b, tok, rstd_s[tok], ws, y_base, fbuf, &C, comm_e, piece + ((long long)tok << logbs));
+        fused_out_block<E8FMT, LATE>(L, b, tok, rstd_s[tok], ws, y_base, fbuf, &C, comm_e, piece + ((long long)tok << logbs));
         __syncthreads();
       }
       comm_signal_and_wait(C, comm_e, L.comm_unit_base + b);
@@ -249,7 +256,7 @@ __device__ __forceinline__ void fused_phase3(const DevLinear* layers, const int*
       __syncthreads();
     } else {
       for (int tok = 0; tok < batch; ++tok) {
-        fused_out_block(L, b, tok, rstd_s[tok], ws, y_base, fbuf);
+        fused_out_block<E8FMT, LATE>(L, b, tok, rstd_s[tok], ws, y_base, fbuf);
         __syncthreads();
       }
     }
@@ -406,7 +413,7 @@ trellis_fused_kernel(const __grid_constant__ FusedLayers T, int n_layers, int to
   __syncthreads();
 
   // ---- phase 3: output transforms of the blocks this CTA completed
-  fused_phase3(layers, todo, n_todo, batch, rstd_s, ws, y_base, fbuf, scratch_elems, C, comm_e);
+  fused_phase3<false, 32>(layers, todo, n_todo, batch, rstd_s, ws, y_base, fbuf, scratch_elems, C, comm_e);
   if (C.world > 1) comm_cta_done(C, comm_e);
 }
 
@@ -625,7 +632,7 @@ e8_fused_kernel(const __grid_constant__ FusedLayers T, int n_layers, int total_u
   __syncthreads();
 
   // ---- phase 3: output transforms of the blocks this CTA completed
-  fused_phase3(layers, todo, n_todo, batch, rstd_s, ws, y_base, fbuf, scratch_elems, C, comm_e);
+  fused_phase3<true, RES ? 64 : 16>(layers, todo, n_todo, batch, rstd_s, ws, y_base, fbuf, scratch_elems, C, comm_e);
   if (C.world > 1) comm_cta_done(C, comm_e);
 }
 
