@@ -2,6 +2,7 @@
 #pragma once
 #include "glqb_kernels.cuh"
 #include "glqb_fht.cuh"
+#include "glqb_fht_fast.cuh"
 
 namespace glqb {
 
@@ -569,14 +570,34 @@ __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_out_kernel(const De
   rht_out_body<FROM_F32>(layers[it.layer], it, ws, y_base, yrht_in, fbuf);
 }
 
+// One array of 32 to 1024 values of the unfused op: the shuffle transform (one token of 1024 values 2.3 us; fht_block, whose
+// second pass is one warp's at that size, 3.7; 64 tokens, a CTA each, 2.4 and 4.0).
+__device__ __forceinline__ void rht_out_short(const DevLinear& L, const RhtItem it, const float* __restrict__ src,
+                                              uint8_t* __restrict__ y_base, float* fbuf) {
+  const int off = L.bm_off[it.block], logbs = L.bm_log[it.block];
+  const float* p = src + (long long)it.tok0 * L.m + off;
+  const __half* su = L.su + off;
+  const long long o = L.y_off + (long long)it.tok0 * L.y_stride + off;
+  const float rs = rsqrtf((float)(1 << logbs));
+  auto load4 = [&](int i, float (&q)[4]) {
+    const float4 t = __ldcg(reinterpret_cast<const float4*>(p + i));
+    q[0] = t.x; q[1] = t.y; q[2] = t.z; q[3] = t.w;
+  };
+  fht_fast<10, 64, false>(fbuf, logbs, [&](int i) { return __ldcg(p + i); }, load4, [&](int i) { return __half2float(su[i]); },
+                          [&](int i, float v, float sign) { store_act(y_base, o + i, L.y_dtype, v * rs * sign); });
+}
+
 static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_out_single_kernel(const __grid_constant__ DevLinear L,
                                                                      const __grid_constant__ RhtSingle S,
                                                                      uint8_t* __restrict__ y_base,
                                                                      const float* __restrict__ yrht_in) {
   extern __shared__ __align__(16) float fbuf[];
   const RhtItem it = rht_single_item(S, L.batch);
-  if (rht_out_is_plain<true>(L, it, y_base, yrht_in)) rht_out_plain<true>(L, it, yrht_in, y_base, fbuf);
-  else rht_out_body<true>(L, it, nullptr, y_base, yrht_in, fbuf);
+  const int logbs = L.bm_log[it.block];
+  if (rht_out_is_plain<true>(L, it, y_base, yrht_in)) {
+    if (it.ntok == 1 && logbs >= 5 && logbs <= 10) rht_out_short(L, it, yrht_in, y_base, fbuf);
+    else rht_out_plain<true>(L, it, yrht_in, y_base, fbuf);
+  } else rht_out_body<true>(L, it, nullptr, y_base, yrht_in, fbuf);
 }
 
 }  // namespace glqb
