@@ -108,3 +108,29 @@ def test_output_transform_beyond_32_bit_offsets():
     del src
     torch.cuda.empty_cache()
     assert err <= 13 * 16 * 2.0 ** -24 * max(1.0, np.abs(ref).max())      # as in test_transform_blocks, 13 stages
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("tokens", [1, 8, 9])
+def test_wide_inputs_of_decode_steps(tokens, shift):
+    """Input blocks of 8192 and 4096 values in front of the single-launch kernel (up to 8 tokens) and of the streaming ones
+    (9), rows aligned for vector loads and not, both formats' activation layouts."""
+    from glq_b200 import synth
+    from glq_b200.plan import Plan, block_decompose
+    m, n = 64, 12352                                        # 8192 + 4096 + 64
+    g = torch.Generator(device="cuda").manual_seed(tokens + shift)
+    x = torch.randn(tokens, n + shift, generator=g, device="cuda").half()[:, shift:]
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda")
+    W = ops.glq_decompress_trellis_3inst_cuda(L.codes[0], m, n).double().cpu().numpy()
+    y = ops.fused_linear_trellis_3inst(x, L.sv, L.su, L.codes[0], None, None, None, None, L.wscale, n, m, n, m,
+                                       out_dtype=torch.float32)
+    _check(x, W, L, y, block_decompose(n), block_decompose(m))
+    table = synth.load_e8_table("cuda")
+    E = synth.e8_layer("e", m, n, 1, table, g, "cuda")
+    plan = Plan([E.spec(batch=tokens, x_dtype=x.dtype, y_dtype=torch.float32, x_stride=x.stride(0))])
+    yb = torch.empty(tokens, m, device="cuda")
+    plan.run(x, yb)
+    plan.close()
+    nib = (table.cpu().numpy().view(np.uint32)[:, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15
+    W = (nib.astype(np.float64) * 0.5 - 3.0)[E.codes[0].cpu().numpy().view(np.uint16)].reshape(m, n)
+    _check(x, W, E, yb, block_decompose(n), block_decompose(m))
