@@ -930,8 +930,9 @@ static size_t moe_gemm_smem_bytes(bool e8) {
   return (size_t)MOE_GEMM_STAGES * (GM_A_BYTES + (size_t)MOE_TN * 128) + (3 * MOE_GEMM_STAGES + 5) * 8 + 16 + 1024;
 }
 // routed tokens per expert (average) from which the tensor-core form is used (measured, 128 experts, top 8, streaming /
-// tensor-core: 64 tokens 260 / 263 us, 128 tokens 283 / 264, 256 tokens 333 / 271, 512 tokens 518 / 325).  With two
-// stages the GEMM multiplies fp16(w1 + s * w2), where the streaming kernel keeps exact weights and an fp32 sum per stage:
+// tensor-core: 64 tokens 260 / 263 us, 128 tokens 283 / 264, 256 tokens 333 / 271, 512 tokens 518 / 325; at an average of 8:
+// 64 experts, 1024 x 512, 3 bits 84 / 85; 32 experts, 2048 x 768, 2 bits 113 / 98, 2048 x 1536, 4 bits 167 / 150; 8 experts,
+// 4096 x 2048 120 / 115).  With two stages the GEMM multiplies fp16(w1 + s * w2), where the streaming kernel keeps exact weights and an fp32 sum per stage:
 // steps below 64 routed tokens per expert keep that precision.
 static int moe_gemm_min_avg(bool two_stages) {
   const char* e = getenv("GLQB_MOE_GEMM_MIN_AVG");
