@@ -67,6 +67,7 @@ struct GlqbPlan {
   size_t ws_bytes = 0;
   int max_batch = 1;
   bool out_plain_static = false; // every output item takes the plain transform when the output is aligned
+  bool out_wide = false;         // some layer has 2^32 partial sums per slot or more
   int max_elems_in = 32, max_elems_out = 32;    // floats of shared memory the transform CTAs need
   int sm_count = 0;
   int64_t code_bytes = 0, flops = 0;
@@ -838,6 +839,8 @@ static int build_plan(GlqbPlan* P) {
   add_rht_items(P->items_in_gemm, rht_in_gemm, P->sm_count, P->max_elems_in);
   add_rht_items(P->items_out, rht_out, P->sm_count, P->max_elems_out);
   P->ws_bytes = ws;
+  P->out_wide = false;
+  for (const DevLinear& L : P->dev) P->out_wide = P->out_wide || (long long)L.batch * L.m > 0xFFFFFFFFll;
   P->out_plain_static = true;
   for (const RhtItem& it : P->items_out) {
     const DevLinear& L = P->dev[it.layer];
@@ -994,7 +997,7 @@ int glqb_plan_run(GlqbPlan* P, const void* x_base, void* y_base, void* workspace
     uint8_t* yb = reinterpret_cast<uint8_t*>(y_base);
     const float* none = nullptr;
     if (out_plain(P, yb)) CUDA_TRY(cudaLaunchKernelEx(&cfg, rht_out_plain_kernel, dl, di, cws, yb));
-    else CUDA_TRY(cudaLaunchKernelEx(&cfg, rht_out_kernel<false>, dl, di, cws, yb, none));
+    else CUDA_TRY(cudaLaunchKernelEx(&cfg, P->out_wide ? rht_out_kernel<true> : rht_out_kernel<false>, dl, di, cws, yb, none));
   }
   CUDA_TRY(cudaGetLastError());
   return GLQB_OK;

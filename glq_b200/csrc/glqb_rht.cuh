@@ -341,8 +341,10 @@ static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_single_ke
 // wscale (and the optional per-row scale), the block Hadamard, 1/sqrt(bs) and SU, and writes
 // y[:, :out_features] (reference: glq_output_rht_multiblock_kernel, glq/csrc/glq_cuda.cu:2151).
 // FROM_F32: input is a plain fp32 (batch, m) matrix (the unfused output_rht op).
+// WIDE: batch * m may be 2^32 or more.  The tile's first token is then part of the pointer; elsewhere it is part of the
+// 32-bit offsets, which is 3 % faster where there are many slots (16 tokens of 2048 x 2048: 37.4 / 39.0 us).
 // ---------------------------------------------------------------------------------------------
-template <bool FROM_F32>
+template <bool FROM_F32, bool WIDE>
 __device__ __forceinline__ void rht_out_body(const DevLinear& L, const RhtItem it, const uint8_t* __restrict__ ws,
                                              uint8_t* __restrict__ y_base, const float* __restrict__ yrht_in,
                                              float* fbuf) {
@@ -356,9 +358,9 @@ __device__ __forceinline__ void rht_out_body(const DevLinear& L, const RhtItem i
   const long long slot_stride = (long long)L.batch * m;
   const float wscale = L.wscale;
   const float* row_scale = L.row_scale;
-  // the tile's first token (its offset needs 64 bits: 65535 tokens x 131072 rows; as a second pointer beside the layer's the
-  // loads of the vector path were not kept in flight, 14.2 instead of 12.7 us for one token of 14336 rows)
-  const float* src = (FROM_F32 ? yrht_in : reinterpret_cast<const float*>(ws + L.part_off)) + (long long)it.tok0 * m;
+  const float* src = FROM_F32 ? yrht_in : reinterpret_cast<const float*>(ws + L.part_off);
+  if constexpr (WIDE) src += (long long)it.tok0 * m;
+  const int tok0 = WIDE ? 0 : it.tok0;             // first token of the tile, counted from `src`
   // partial sums of a row: a property of its strip (the warps whose group ranges touch the strip)
   auto slots_of = [&](int row) -> int {
     if (fixed_slots > 0) return fixed_slots;
@@ -368,7 +370,7 @@ __device__ __forceinline__ void rht_out_body(const DevLinear& L, const RhtItem i
   };
   auto load1 = [&](int trow, int i) -> float {
     const int row = off + i;
-    const float* p = src + (long long)trow * m + row;
+    const float* p = src + (long long)(tok0 + trow) * m + row;
     if constexpr (FROM_F32) return *p;
     if (row >= m) return 0.f;
     const int cnt = slots_of(row);
@@ -407,7 +409,7 @@ __device__ __forceinline__ void rht_out_body(const DevLinear& L, const RhtItem i
       }
       return;
     }
-    // all eight loads of a slot are issued together; offsets inside the tile (at most 64 tokens x 524288 rows) fit 32 bits
+    // all eight loads of a slot are issued together; element offsets fit 32 bits (a tile: at most 64 tokens x 524288 rows)
     for (int kk = 0; kk < S; ++kk) {
       unsigned idx[8];
       int cnt[8];
@@ -416,7 +418,7 @@ __device__ __forceinline__ void rht_out_body(const DevLinear& L, const RhtItem i
       for (int k = 0; k < 8; ++k) {
         const int e = e0 + (k << 10);
         const int row = off + (kk << FHT_LOG) + (e & ((1 << log_t) - 1));
-        idx[k] = (unsigned)(e >> log_t) * (unsigned)m + (unsigned)row;
+        idx[k] = (unsigned)(tok0 + (e >> log_t)) * (unsigned)m + (unsigned)row;
         cnt[k] = e < total ? (fixed_slots > 0 ? fixed_slots : slots_of(row)) : 0;
         most = max(most, cnt[k]);
       }
@@ -555,7 +557,7 @@ static __global__ void __launch_bounds__(RHT_THREADS, 4) rht_out_plain_kernel(co
   rht_out_plain<false>(L, it, reinterpret_cast<const float*>(ws + L.part_off), y_base, fbuf);
 }
 
-template <bool FROM_F32>
+template <bool WIDE>
 __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_out_kernel(const DevLinear* __restrict__ layers,
                                                               const RhtItem* __restrict__ items,
                                                               const uint8_t* __restrict__ ws,
@@ -567,7 +569,7 @@ __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_out_kernel(const De
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const RhtItem it = items[blockIdx.x];
-  rht_out_body<FROM_F32>(layers[it.layer], it, ws, y_base, yrht_in, fbuf);
+  rht_out_body<false, WIDE>(layers[it.layer], it, ws, y_base, yrht_in, fbuf);
 }
 
 // One array of 32 to 1024 values of the unfused op: the shuffle transform (one token of 1024 values 2.3 us; fht_block, whose
@@ -597,7 +599,7 @@ static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_out_single_k
   if (rht_out_is_plain<true>(L, it, y_base, yrht_in)) {
     if (it.ntok == 1 && logbs >= 5 && logbs <= 10) rht_out_short(L, it, yrht_in, y_base, fbuf);
     else rht_out_plain<true>(L, it, yrht_in, y_base, fbuf);
-  } else rht_out_body<true>(L, it, nullptr, y_base, yrht_in, fbuf);
+  } else rht_out_body<true, true>(L, it, nullptr, y_base, yrht_in, fbuf);
 }
 
 }  // namespace glqb

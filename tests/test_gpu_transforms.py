@@ -134,3 +134,36 @@ def test_wide_inputs_of_decode_steps(tokens, shift):
     nib = (table.cpu().numpy().view(np.uint32)[:, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15
     W = (nib.astype(np.float64) * 0.5 - 3.0)[E.codes[0].cpu().numpy().view(np.uint16)].reshape(m, n)
     _check(x, W, E, yb, block_decompose(n), block_decompose(m))
+
+
+def test_plan_output_beyond_32_bit_offsets():
+    """32769 tokens of a layer of 131072 rows: the last token's partial sums start 2^32 elements in (rows of the result are
+    not aligned, so the general body runs).  Against the same token alone."""
+    from glq_b200 import synth
+    from glq_b200.plan import Plan
+    tokens, m, n = 32769, 131072, 32
+    if torch.cuda.mem_get_info()[0] < 40 << 30:
+        pytest.skip("needs 27 GiB")
+    g = torch.Generator(device="cuda").manual_seed(9)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda")
+    x = torch.zeros(tokens, n, device="cuda", dtype=torch.float16)
+    x[0] = 1.0
+    x[-1] = torch.randn(n, generator=g, device="cuda").half()
+    spec = L.spec(batch=tokens, x_dtype=x.dtype, y_dtype=torch.float16, y_stride=m + 1)
+    spec.blocks_m = [32768] * 4
+    plan = Plan([spec])
+    y = torch.empty(tokens * (m + 1), device="cuda", dtype=torch.float16)
+    plan.run(x, y)
+    last = y[(tokens - 1) * (m + 1):(tokens - 1) * (m + 1) + m].float()
+    plan.check_status()
+    plan.close()
+    del plan, y
+    torch.cuda.empty_cache()
+    spec = L.spec(batch=1, x_dtype=x.dtype, y_dtype=torch.float32)
+    spec.blocks_m = [32768] * 4
+    plan = Plan([spec])
+    one = torch.empty(1, m, device="cuda")
+    plan.run(x[-1:].contiguous(), one)
+    plan.close()
+    # the result's fp16 rounding, and fp32 sums in another order
+    assert (last - one[0]).abs().max() <= (2.0 ** -11 + 1e-4) * one.abs().max()
