@@ -5,12 +5,16 @@
 // and g + 8, columns 2t and 2t + 1 of every 16 x 8 block), so two stores replace sixteen and a 128 x 64 x 256 chunk leaves
 // 64 KiB of shared-memory traffic instead of 96 (768 clocks at 128 bytes, where the tensor pipe needs 512).  That alone
 // changed nothing (1010 -> 1045 clocks per chunk): the limit was the issuing thread's own loop, see the MMA issuer below,
-// and with that loop warp-uniform a chunk takes 742.
+// and with that loop warp-uniform a chunk took 742.
 //
 // One CTA computes 128 weight rows x up to 192 tokens: two accumulators of 192 columns and four 64-column chunks of A
 // (32 columns each) fill the 512 columns of tensor memory.  Warp roles: warp 0 issues MMAs, warp 1 the bulk copies (TMA
-// without multicast) of the activation tiles, warps 4-7 drain accumulators, 24 producer warps in three groups of eight
-// (group q % 3 decodes chunk q, warp w of a group the 32 x 32 trellis group at rows 32 (w % 4), columns 32 (w / 4)).
+// without multicast) of the activation tiles, warps 4-7 drain accumulators, 16 producer warps in two groups of eight
+// (group p % 2 decodes pair p; warp w of a group rows 32 (w % 4) and chunk w / 4 of the pair: two 32 x 32 trellis groups).
+// Bound by the instructions of the state decode (issue slots 74 % busy at 256 routed tokens per expert): with a loop
+// turn per pair instead of per chunk a trellis group takes 229 instructions instead of 263, and 80 registers hold both
+// decoded groups until the stage is free.  24 producer warps, a chunk per turn / this: experts of 256 tokens 273 / 257 us,
+// 333 tokens of 2048 x 11008 80 / 76 us.
 // Stages hand over through mbarriers; every wait is bounded as in glq_gemm_kernel.
 #pragma once
 #include "glqb_gemm.cuh"
@@ -22,7 +26,7 @@ constexpr int TG_TN = 192;                       // most tokens of a tile (multi
 constexpr int TG_A_STAGES = 2, TG_A_COLS = 32;   // columns per chunk
 constexpr int TG_B_STAGES = 4;
 constexpr int TG_B_BYTES = 2 * TG_TN * 128;
-constexpr int TG_GROUPS = 3;
+constexpr int TG_GROUPS = TG_A_STAGES;           // producer groups: one per stage of A
 constexpr int TG_MMA_WARP = 0, TG_LOAD_WARP = 1, TG_EPI_WARP0 = 4, TG_PROD_WARP0 = 8;   // (2 and 3 only keep warp % 4 aligned)
 constexpr int TG_THREADS = (TG_PROD_WARP0 + TG_GROUPS * 8) * 32;
 constexpr int TG_SMEM_BYTES = TG_B_STAGES * TG_B_BYTES + (2 * TG_A_STAGES + 2 * TG_B_STAGES + 5) * 8 + 16 + 1024;
@@ -98,7 +102,7 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < TG_A_STAGES; ++s) { mbar_init(&full_a[s], 16); mbar_init(&empty_a[s], 1); }
+    for (int s = 0; s < TG_A_STAGES; ++s) { mbar_init(&full_a[s], 8); mbar_init(&empty_a[s], 1); }
     for (int s = 0; s < TG_B_STAGES; ++s) { mbar_init(&full_b[s], 1); mbar_init(&empty_b[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 4); }
     mbar_init(drain, 1);
@@ -181,60 +185,82 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
     }
   } else if (warp >= TG_PROD_WARP0) {
     // ------------------------------------------------------------------ producers
-    // q numbers the chunks of this CTA over all its items, every item rounded up to pairs (the second half of a last odd
-    // pair is filled with zeros and not multiplied); chunk q is half q & 1 of pair q >> 1
-    const int grp = (warp - TG_PROD_WARP0) >> 3, strip = warp & 3, cg = (warp >> 2) & 1;
-    const uint32_t lanes = tmem_a + ((uint32_t)(strip * 32) << 16) + (uint32_t)(cg * 16);
-    uint32_t q0 = 0;
+    // Group g takes pairs g, g + 2, ... of this CTA (counted over all its items) and always fills A stage g.  A warp
+    // decodes both 32 x 32 groups of one chunk of the pair before it asks for the stage, so that a stage is held for
+    // the stores alone.
+    const int grp = (warp - TG_PROD_WARP0) >> 3, strip = warp & 3, half = (warp >> 2) & 1;
+    const bool waits_b = (warp & 7) == 0;
+    const uint32_t dst = tmem_a + ((uint32_t)(strip * 32) << 16) + (uint32_t)((grp * 2 + half) * TG_A_COLS);
+    uint32_t p0 = 0, mine = 0;                     // pairs of the items before; pairs this group has filled
     bool ok = true;
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       const GemmItem it = items[item];
       const DevLinear& L = layers[it.layer];
-      const int first = it.k_begin + (int)(((uint32_t)(grp + TG_GROUPS) - q0 % (uint32_t)TG_GROUPS) % (uint32_t)TG_GROUPS);
       const int rp = it.m_tile * 4 + strip, gps = L.groups_per_strip, k_end = it.k_end;
-      const int k_pad = it.k_begin + ((k_end - it.k_begin + 1) & ~1);
       const bool row_ok = rp < L.strips;
-      const uint8_t* p1 = L.codes[0] + ((long long)rp * gps) * (128 * K1) + lane * (4 * K1);
+      // chunks below k_both have two groups, chunk k_both may have one (columns past the matrix are zeros)
+      const int k_both = row_ok ? min(k_end, gps >> 1) : 0, k_any = row_ok ? k_end : 0;
+      int kc = it.k_begin + 2 * (int)((grp ^ p0) & 1u) + half;
+      const uint8_t* p1 = L.codes[0] + ((long long)rp * gps + 2 * kc) * (128 * K1) + lane * (4 * K1);
       const uint8_t* p2 = nullptr;
-      if constexpr (K2 > 0) p2 = L.codes[1] + ((long long)rp * gps) * (128 * K2) + lane * (4 * K2);
+      if constexpr (K2 > 0) p2 = L.codes[1] + ((long long)rp * gps + 2 * kc) * (128 * K2) + lane * (4 * K2);
       const __half2 s2 = __float2half2_rn(L.stage_scale[1]);
-      Words<K1> nxt;
-      Words<(K2 > 0 ? K2 : 1)> nxt2;
-      auto fetch = [&](int kc) {
-        const int cp = kc * 2 + cg;
-        if (row_ok && cp < gps) {
-          nxt = load_words<K1>(p1 + (long long)cp * (128 * K1));
-          if constexpr (K2 > 0) nxt2 = load_words<K2>(p2 + (long long)cp * (128 * K2));
-        }
+      Words<K1> v[2];
+      Words<(K2 > 0 ? K2 : 1)> v2[2];
+      auto fetch = [&](int g) {
+        v[g] = load_words<K1>(p1 + g * (128 * K1));
+        if constexpr (K2 > 0) v2[g] = load_words<K2>(p2 + g * (128 * K2));
       };
-      if (first < k_end) fetch(first);
-      for (int kc = first; kc < k_pad; kc += TG_GROUPS) {
-        const uint32_t q = q0 + (uint32_t)(kc - it.k_begin);
-        const uint32_t pair = q >> 1;
-        const int stage = (int)(pair % TG_A_STAGES);
-        const Words<K1> v = nxt;
-        const Words<(K2 > 0 ? K2 : 1)> v2 = nxt2;
-        uint32_t r[2][8];
-        if (row_ok && kc * 2 + cg < gps && kc < k_end) {         // (uniform per warp: the shuffles inside see all lanes)
-          tg_decode_group<K1, K2>(lane, v, v2, s2, r);
-        } else {                                   // rows or columns past the matrix: zeros
+      if (kc < k_any) fetch(0);
+      if (kc < k_both) fetch(1);
+      const int pairs = (k_end - it.k_begin + 1) >> 1;
+      for (int pair = (int)((grp ^ p0) & 1u); pair < pairs; pair += 2, kc += 4, ++mine) {
+        p1 += 8 * (128 * K1);                      // the codes of this warp's next chunk
+        if constexpr (K2 > 0) p2 += 8 * (128 * K2);
+        auto decode = [&](int g, int k_lim, uint32_t (&r)[2][8]) {
+          if (kc < k_lim) {                        // (uniform per warp: the shuffles inside see all lanes)
+            tg_decode_group<K1, K2>(lane, v[g], v2[g], s2, r);
+            if (kc + 4 < k_lim) fetch(g);
+          } else {                                 // rows or columns past the matrix: zeros
 #pragma unroll
-          for (int i = 0; i < 16; ++i) r[i >> 3][i & 7] = 0u;
+            for (int i = 0; i < 16; ++i) r[i >> 3][i & 7] = 0u;
+          }
+        };
+        auto wait = [&]() -> bool {
+          if (!mbar_wait(&empty_a[grp], (mine & 1u) ^ 1u, abort_flag)) return false;
+          if (waits_b) {                           // (the MMA warp waits for A alone)
+            const uint32_t q = p0 + (uint32_t)pair;
+            if (!mbar_wait(&full_b[q % TG_B_STAGES], (q / TG_B_STAGES) & 1u, abort_flag)) return false;
+          }
+          __syncwarp();
+          tc_fence_after();
+          return true;
+        };
+        auto put = [&](int g, const uint32_t (&r)[2][8]) {
+          tmem_st_16x128b_x4(dst + (uint32_t)(g * 16), r[0]);
+          tmem_st_16x128b_x4(dst + (16u << 16) + (uint32_t)(g * 16), r[1]);
+        };
+        if constexpr (K2 == 0) {
+          uint32_t r[2][2][8];
+          decode(0, k_any, r[0]);
+          decode(1, k_both, r[1]);
+          if (!wait()) { ok = false; break; }
+          put(0, r[0]);
+          put(1, r[1]);
+        } else {                                   // (two stages: no registers for both groups)
+          uint32_t r[2][8];
+          decode(0, k_any, r);
+          if (!wait()) { ok = false; break; }
+          put(0, r);
+          decode(1, k_both, r);
+          put(1, r);
         }
-        if (kc + TG_GROUPS < k_end) fetch(kc + TG_GROUPS);
-        if (!mbar_wait(&empty_a[stage], ((pair / TG_A_STAGES) & 1u) ^ 1u, abort_flag) ||
-            ((warp & 7) == 0 && !mbar_wait(&full_b[pair % TG_B_STAGES], (pair / TG_B_STAGES) & 1u, abort_flag))) { ok = false; break; }
-        __syncwarp();
-        tc_fence_after();
-        const uint32_t cols = (uint32_t)((stage * 2 + (int)(q & 1u)) * TG_A_COLS);
-        tmem_st_16x128b_x4(lanes + cols, r[0]);
-        tmem_st_16x128b_x4(lanes + (16u << 16) + cols, r[1]);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full_a[stage]);
+        if (lane == 0) mbar_arrive(&full_a[grp]);
       }
-      q0 += (uint32_t)(k_pad - it.k_begin);
+      p0 += (uint32_t)pairs;
     }
     if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_PRODUCER); }
   } else if (warp >= TG_EPI_WARP0) {
