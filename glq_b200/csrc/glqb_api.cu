@@ -59,6 +59,12 @@ struct GlqbPlan {
   RhtItem* d_items_in_gemm = nullptr;
   RhtItem* d_items_out = nullptr;
   GemmItem* d_gemm_items = nullptr;
+  // A run of at most `few_tokens` tokens needs one token tile fewer than the plan's bucket (trellis_gemm_kernel): work list,
+  // K splits and the layer table that names them are kept for both.  0: there is one schedule only.
+  int few_tokens = 0;
+  std::vector<Segment> few_segs;
+  DevLinear* d_few_layers = nullptr;
+  GemmItem* d_few_items = nullptr;
   int* d_status = nullptr;
   int* d_tickets = nullptr;      // completion tickets of the single-launch form, all zero between runs
   const GlqbComm* comm = nullptr;  // tensor-parallel ranks whose outputs the single-launch kernel sums (glqb_plan_set_comm)
@@ -81,7 +87,7 @@ namespace glqb {
 // ------------------------------------------------------------------------------------------
 // kernel variant tables
 // ------------------------------------------------------------------------------------------
-typedef void (*MvKernel)(const DevLinear*, int, long long, int, uint8_t*);
+typedef void (*MvKernel)(const DevLinear*, int, long long, int, uint8_t*, int);
 
 template <int K1, int K2>
 static MvKernel trellis_kernel_nb(int nb) {
@@ -160,7 +166,7 @@ static bool same_input(const GlqbLinearDesc& a, const GlqbLinearDesc& b) {
          memcmp(a.blocks_n, b.blocks_n, sizeof(int32_t) * a.n_blocks_n) == 0;
 }
 
-typedef void (*E8SmemKernel)(const DevLinear*, int, long long, int, uint8_t*, const uint32_t*, const uint32_t*, int);
+typedef void (*E8SmemKernel)(const DevLinear*, int, long long, int, uint8_t*, const uint32_t*, const uint32_t*, int, int);
 
 template <int NS>
 static E8SmemKernel e8_smem_kernel_nb(int nb) {
@@ -256,9 +262,50 @@ static size_t tile_bytes(const GlqbLinearDesc& d) {
 // evenly, in steps of 16.
 static int tn_for_batch(int batch, bool codes) {
   if (batch <= DECODE_MAX_BATCH) return 0;
-  if (!codes) return batch <= 128 ? 128 : 256;
-  const int tiles = (batch + TG_TN - 1) / TG_TN;
-  return ((batch + tiles - 1) / tiles + 15) & ~15;
+  return codes ? tile_tokens(batch) : batch <= 128 ? 128 : 256;
+}
+
+// Work of a segment's GEMM for at most `limit` tokens per layer: items (layer, 128-row tile, token tile, K range), and the
+// K splits of every layer (`dev`: fixed_slots).  The SMs take the items in turn, so a split is chosen by the rounds it
+// takes, in 64-column chunks (about 0.3 us each), plus the fp32 partial sums it writes and reads back at 5 TB/s.
+// Splits for as many items as SMs, rounded up / by this rule, with the tokens rounded up to 512 / taken as they are: 333
+// tokens of 2048 x 11008 80 / 43 us (192 items in two rounds of 148 / 128 in one).
+static void gemm_schedule(Segment& s, int limit, int sm_count, std::vector<DevLinear>& dev, std::vector<GemmItem>& items) {
+  auto tokens_of = [&](const DevLinear& L) { return std::min(L.batch, limit); };
+  auto tile_of = [&](const DevLinear& L) { return trellis_form(s) ? tile_tokens(tokens_of(L)) : s.tn; };
+  auto splits = [](int kchunks, int ks, int& per) { per = (kchunks + ks - 1) / ks; return (kchunks + per - 1) / per; };
+  int best = 1;
+  double best_cost = 0;
+  for (int ks = 1; ks <= 16; ++ks) {
+    long long n = 0;
+    int longest = 0, per = 0;
+    double sums = 0;
+    bool ok = true;
+    for (int i = 0; i < s.count; ++i) {
+      const DevLinear& L = dev[s.first + i];
+      const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
+      ok = ok && ks <= std::max(1, kchunks / 8);
+      const int k = splits(kchunks, ks, per);
+      longest = std::max(longest, per);
+      n += (long long)((L.m + GM_TILE_M - 1) / GM_TILE_M) * ((tokens_of(L) + tile_of(L) - 1) / tile_of(L)) * k;
+      sums += (double)k * tokens_of(L) * L.m;
+    }
+    const double cost = (double)((n + sm_count - 1) / sm_count) * longest + sums * 8 / 5e12 / 0.3e-6;
+    if (ks == 1 || (ok && cost < best_cost)) { best = ks; best_cost = cost; }
+  }
+  s.item_first = (int)items.size();
+  for (int i = 0; i < s.count; ++i) {
+    DevLinear& L = dev[s.first + i];
+    const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K, tn = tile_of(L), n_tiles = (tokens_of(L) + tn - 1) / tn;
+    int per;
+    L.fixed_slots = splits(kchunks, std::min(best, std::max(1, kchunks / 8)), per);
+    for (int mt = 0; mt < (L.m + GM_TILE_M - 1) / GM_TILE_M; ++mt)
+      for (int nt = 0; nt < n_tiles; ++nt)
+        for (int k = 0; k < L.fixed_slots; ++k)
+          items.push_back(GemmItem{s.first + i, mt, nt, k * per, std::min(kchunks, (k + 1) * per), k, 0, 0, 0});
+  }
+  s.item_count = (int)items.size() - s.item_first;
+  s.grid = std::min(s.item_count, sm_count);
 }
 
 // Two-stage trellis layers (whose weight decode costs twice as much) take 256-token tiles, decoded into shared memory by
@@ -634,38 +681,16 @@ static int build_plan(GlqbPlan* P) {
       }
     }
     if (s.tn) {
-      // tensor-core GEMM: work items = (layer, 128-row tile, token tile[, K split]); the K range is
-      // split only when there are too few tiles to occupy the SMs
-      long long tiles = 0;
-      for (int i = 0; i < s.count; ++i) {
-        const DevLinear& L = P->dev[s.first + i];
-        tiles += (long long)((L.m + GM_TILE_M - 1) / GM_TILE_M) * ((L.batch + s.tn - 1) / s.tn);
-      }
-      s.item_first = (int)P->gemm_items.size();
       for (int i = 0; i < s.count; ++i) {
         DevLinear& L = P->dev[s.first + i];
-        const int m_tiles = (L.m + GM_TILE_M - 1) / GM_TILE_M, n_tiles = (L.batch + s.tn - 1) / s.tn;
-        const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
-        int ks = 1;
-        if (tiles < P->sm_count) ks = (int)std::min<long long>(std::max(1, kchunks / 8), (P->sm_count + tiles - 1) / tiles);
-        ks = std::max(1, std::min(ks, 16));
-        const int per = (kchunks + ks - 1) / ks;
-        ks = (kchunks + per - 1) / per;
-        L.fixed_slots = ks;
-        L.slots = ks;
         L.gemm_tn = s.tn;
         L.gemm_even = trellis_form(s) ? 1 : 0;
         L.per_warp = 1;
         L.atile_off = s.two_phase ? -1 : 0;      // -1: allocate below
-        for (int mt = 0; mt < m_tiles; ++mt)
-          for (int nt = 0; nt < n_tiles; ++nt)
-            for (int k = 0; k < ks; ++k)
-              P->gemm_items.push_back(GemmItem{s.first + i, mt, nt, k * per, std::min(kchunks, (k + 1) * per), k,
-                                               nt * s.tn, std::min(s.tn, L.batch - nt * s.tn), nt * s.tn});
         P->max_batch_gemm = std::max(P->max_batch_gemm, L.batch);
       }
-      s.item_count = (int)P->gemm_items.size() - s.item_first;
-      s.grid = std::min(s.item_count, P->sm_count);
+      gemm_schedule(s, P->max_batch, P->sm_count, P->dev, P->gemm_items);
+      for (int i = 0; i < s.count; ++i) P->dev[s.first + i].slots = P->dev[s.first + i].fixed_slots;
       s.total_groups = 0;
       s.per_warp = 1;
       CUDA_TRY(gemm_prepare(s));
@@ -748,6 +773,22 @@ static int build_plan(GlqbPlan* P) {
       L.per_warp = s.per_warp;
       L.slots = (L.groups_per_strip - 1) / s.per_warp + 2;
     }
+  }
+
+  // ---- the schedule of runs that need one token tile fewer (plans of one token count)
+  std::vector<DevLinear> few;
+  std::vector<GemmItem> few_items;
+  P->few_tokens = 0;
+  bool one_count = true, codes_in_gemm = false;
+  for (const DevLinear& L : P->dev) { one_count = one_count && L.batch == P->max_batch; codes_in_gemm = codes_in_gemm || L.gemm_even; }
+  const int tiles_most = (P->max_batch + TG_TN - 1) / TG_TN;
+  if (one_count && codes_in_gemm && tiles_most > 1) {
+    P->few_tokens = (tiles_most - 1) * TG_TN;
+    P->few_segs = P->segs;
+    few = P->dev;
+    for (Segment& s : P->few_segs)
+      if (s.tn) gemm_schedule(s, trellis_form(s) ? P->few_tokens : P->max_batch, P->sm_count, few, few_items);
+    for (int pos = 0; pos < n; ++pos) P->dev[pos].slots = std::max(P->dev[pos].slots, few[pos].fixed_slots);
   }
 
   // ---- workspace: rotated activations (shared by layers with the same input) + partial sums
@@ -850,6 +891,17 @@ static int build_plan(GlqbPlan* P) {
   }
 
   // ---- upload
+  if (P->few_tokens) {
+    for (int pos = 0; pos < n; ++pos) {                    // the plan's buffers, the schedule's K splits
+      const int slots = few[pos].fixed_slots;
+      few[pos] = P->dev[pos];
+      few[pos].fixed_slots = slots;
+    }
+    CUDA_TRY(cudaMalloc(&P->d_few_layers, sizeof(DevLinear) * n));
+    CUDA_TRY(cudaMemcpy(P->d_few_layers, few.data(), sizeof(DevLinear) * n, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMalloc(&P->d_few_items, sizeof(GemmItem) * std::max<size_t>(1, few_items.size())));
+    CUDA_TRY(cudaMemcpy(P->d_few_items, few_items.data(), sizeof(GemmItem) * few_items.size(), cudaMemcpyHostToDevice));
+  }
   CUDA_TRY(cudaMalloc(&P->d_layers, sizeof(DevLinear) * n));
   CUDA_TRY(cudaMemcpy(P->d_layers, P->dev.data(), sizeof(DevLinear) * n, cudaMemcpyHostToDevice));
   CUDA_TRY(cudaMalloc(&P->d_items_in, sizeof(RhtItem) * std::max<size_t>(1, P->items_in.size())));
@@ -932,8 +984,21 @@ int glqb_plan_kernel_ms(GlqbPlan* plan, double* total_ms_out, int32_t* runs_out)
 }
 
 int glqb_plan_run(GlqbPlan* P, const void* x_base, void* y_base, void* workspace, size_t workspace_bytes,
-                  void* stream_) {
+                  void* stream) {
+  return glqb_plan_run_tokens(P, x_base, y_base, INT32_MAX, workspace, workspace_bytes, stream);
+}
+
+int glqb_plan_run_tokens(GlqbPlan* P, const void* x_base, void* y_base, int32_t tokens, void* workspace,
+                         size_t workspace_bytes, void* stream_) {
   if (!P || !x_base || !y_base) return fail(GLQB_E_INVALID, "plan_run: null argument");
+  if (tokens < 1) return fail(GLQB_E_INVALID, "plan_run: %d tokens", tokens);
+  for (const Segment& s : P->segs)
+    if (s.fused && tokens < P->dev[s.first].batch)
+      return fail(GLQB_E_INVALID, "plan_run: a plan of the single-launch form takes its %d tokens, not %d", P->dev[s.first].batch, tokens);
+  const bool few = tokens <= P->few_tokens;
+  const std::vector<Segment>& segs = few ? P->few_segs : P->segs;
+  const DevLinear* d_layers = few ? P->d_few_layers : P->d_layers;
+  const GemmItem* d_gemm_items = few ? P->d_few_items : P->d_gemm_items;
   if (P->ws_bytes && (!workspace || workspace_bytes < P->ws_bytes))
     return fail(GLQB_E_WORKSPACE, "workspace of %zu bytes needed, %zu given", P->ws_bytes, workspace_bytes);
   if (reinterpret_cast<uintptr_t>(workspace) & 255)
@@ -942,11 +1007,11 @@ int glqb_plan_run(GlqbPlan* P, const void* x_base, void* y_base, void* workspace
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
   if (!P->items_in.empty()) {
     rht_in_kernel<false><<<(unsigned)P->items_in.size(), RHT_THREADS, rht_smem(P->max_elems_in), stream>>>(
-        P->d_layers, P->d_items_in, reinterpret_cast<const uint8_t*>(x_base), ws);
+        d_layers, P->d_items_in, reinterpret_cast<const uint8_t*>(x_base), ws, tokens);
   }
   if (!P->items_in_gemm.empty()) {
     rht_in_gemm_kernel<<<(unsigned)P->items_in_gemm.size(), RHT_THREADS, rht_smem(P->max_elems_in), stream>>>(
-        P->d_layers, P->d_items_in_gemm, reinterpret_cast<const uint8_t*>(x_base), ws);
+        d_layers, P->d_items_in_gemm, reinterpret_cast<const uint8_t*>(x_base), ws, tokens);
   }
   if (P->timing) {
     while (P->ev.size() < P->ev_used + 2) {
@@ -956,22 +1021,22 @@ int glqb_plan_run(GlqbPlan* P, const void* x_base, void* y_base, void* workspace
     }
     CUDA_TRY(cudaEventRecord(P->ev[P->ev_used], stream));
   }
-  for (const Segment& s : P->segs) {
+  for (const Segment& s : segs) {
     if (s.fused) {
       fused_launch(s, P->dev.data() + s.first, reinterpret_cast<const uint8_t*>(x_base), reinterpret_cast<uint8_t*>(y_base),
                    ws, P->d_tickets, P->comm ? comm_dev(P->comm) : nullptr, stream);
     } else if (s.tn) {
-      gemm_launch(s, P->d_layers, P->d_gemm_items + s.item_first, ws, P->d_status, P->sm_count, stream);
+      gemm_launch(s, d_layers, d_gemm_items + s.item_first, ws, P->d_status, P->sm_count, tokens, stream);
     } else if (s.smem_table) {
       pick_e8_smem_kernel(s)<<<s.grid, E8S_THREADS, E8S_SMEM_BYTES, stream>>>(
-          P->d_layers + s.first, s.count, s.total_groups, s.per_warp, ws, s.big_table, s.small_table, s.small_entries);
+          d_layers + s.first, s.count, s.total_groups, s.per_warp, ws, s.big_table, s.small_table, s.small_entries, tokens);
     } else {
       MvKernel kern = pick_kernel(s);
       if (s.lut_table)
-        trellis_lut_kernel(s.k1)<<<s.grid, MV_LUT_THREADS, MV_LUT_SMEM_BYTES, stream>>>(P->d_layers + s.first, s.count,
-                                                                                       s.total_groups, s.per_warp, ws);
+        trellis_lut_kernel(s.k1)<<<s.grid, MV_LUT_THREADS, MV_LUT_SMEM_BYTES, stream>>>(d_layers + s.first, s.count, s.total_groups,
+                                                                                       s.per_warp, ws, tokens);
       else
-        kern<<<s.grid, MV_THREADS, 0, stream>>>(P->d_layers + s.first, s.count, s.total_groups, s.per_warp, ws);
+        kern<<<s.grid, MV_THREADS, 0, stream>>>(d_layers + s.first, s.count, s.total_groups, s.per_warp, ws, tokens);
     }
   }
   if (P->timing) {
@@ -991,13 +1056,14 @@ int glqb_plan_run(GlqbPlan* P, const void* x_base, void* y_base, void* workspace
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const DevLinear* dl = P->d_layers;
+    const DevLinear* dl = d_layers;
     const RhtItem* di = P->d_items_out;
     const uint8_t* cws = ws;
     uint8_t* yb = reinterpret_cast<uint8_t*>(y_base);
     const float* none = nullptr;
-    if (out_plain(P, yb)) CUDA_TRY(cudaLaunchKernelEx(&cfg, rht_out_plain_kernel, dl, di, cws, yb));
-    else CUDA_TRY(cudaLaunchKernelEx(&cfg, P->out_wide ? rht_out_kernel<true> : rht_out_kernel<false>, dl, di, cws, yb, none));
+    if (out_plain(P, yb)) CUDA_TRY(cudaLaunchKernelEx(&cfg, rht_out_plain_kernel, dl, di, cws, yb, (int)tokens));
+    else CUDA_TRY(cudaLaunchKernelEx(&cfg, P->out_wide ? rht_out_kernel<true> : rht_out_kernel<false>, dl, di, cws, yb, none,
+                                     (int)tokens));
   }
   CUDA_TRY(cudaGetLastError());
   return GLQB_OK;
@@ -1052,6 +1118,8 @@ int glqb_plan_status(GlqbPlan* plan, int32_t* status_out) {
 void glqb_plan_destroy(GlqbPlan* plan) {
   if (!plan) return;
   if (plan->d_layers) cudaFree(plan->d_layers);
+  if (plan->d_few_layers) cudaFree(plan->d_few_layers);
+  if (plan->d_few_items) cudaFree(plan->d_few_items);
   if (plan->d_items_in) cudaFree(plan->d_items_in);
   if (plan->d_items_out) cudaFree(plan->d_items_out);
   if (plan->d_items_in_gemm) cudaFree(plan->d_items_in_gemm);

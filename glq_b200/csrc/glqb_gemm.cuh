@@ -37,9 +37,17 @@ struct GemmItem {
   int k_begin;     // first 64-column chunk
   int k_end;       // one past the last chunk
   int slot;        // partial-sum slot this item writes
-  int tok0, ntok;  // variable token tiles (grouped experts): first token and tokens of the tile inside its layer,
-  int row0;        // and the 128-byte rows of activations in front of it, see glq_gemm_kernel
+  int tok0, ntok;  // lists built on the device (grouped experts): first token and tokens of the tile inside its layer,
+  int row0;        // and the 128-byte rows of activations in front of it; other lists: see tile_tokens and glq_gemm_kernel
 };
+
+// Token tiles of the layers whose codes are decoded in the GEMM (trellis_gemm_kernel): as few as possible of at most 192
+// tokens, the tokens split evenly in steps of 16.
+constexpr int TG_TN = 192;
+__host__ __device__ __forceinline__ int tile_tokens(int tokens) {
+  const int tiles = (tokens + TG_TN - 1) / TG_TN;
+  return ((tokens + tiles - 1) / tiles + 15) & ~15;
+}
 
 // ---- PTX wrappers ---------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -151,19 +159,20 @@ __device__ __forceinline__ uint32_t sw128_offset(int r, int e) {
 static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_gemm_kernel(const DevLinear* __restrict__ layers,
                                                                   const RhtItem* __restrict__ items,
                                                                   const uint8_t* __restrict__ x_base,
-                                                                  uint8_t* __restrict__ ws) {
+                                                                  uint8_t* __restrict__ ws, int tokens) {
   extern __shared__ __align__(16) float fbuf[];
-  const RhtItem it = items[blockIdx.x];
+  RhtItem it = items[blockIdx.x];
+  if (!rht_item_trim(it, tokens)) return;
   const DevLinear& L = layers[it.layer];
-  const int tn = L.gemm_tn;
-  const bool steps = L.gemm_even != 0;             // the last tile ends on 16 rows
+  const bool steps = L.gemm_even != 0;             // tiles of the tokens of this run, the last one ends on 16 rows
+  const int used = min(L.batch, tokens), tn = steps ? tile_tokens(used) : L.gemm_tn;
   const int off = L.bn_off[it.block];
   const int logbs = L.bn_log[it.block];
   const int bs = 1 << logbs;
   const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
   const float rs = L.x_is_rotated ? 1.0f : rsqrtf((float)bs);
   uint8_t* xr = ws + L.xr_off;
-  auto tile_rows = [&](int tile) -> int { return steps ? min(tn, (L.batch - tile * tn + 15) & ~15) : tn; };
+  auto tile_rows = [&](int tile) -> int { return steps ? min(tn, (used - tile * tn + 15) & ~15) : tn; };
   auto place = [&](int token, int col) -> uint8_t* {
     const int tile = token / tn;
     return xr + ((size_t)tile * tn * kchunks + (size_t)(col >> 6) * tile_rows(tile)) * 128 + sw128_offset(token - tile * tn, col & 63);
@@ -303,12 +312,16 @@ __device__ __forceinline__ void gemm_store_group(const uint32_t (&addr)[4], int 
 template <int FORMAT, int K1, int K2, int TN, int STAGES>
 __global__ void __launch_bounds__(GM_THREADS, 1)
 glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict__ items, int n_items,
-                uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev) {
+                uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev, int tokens) {
   // work lists built on the device (grouped expert matmul) pass their length through memory
   if (n_items_dev) n_items = min(n_items, *n_items_dev);
   constexpr int B_BYTES = TN * 128;
   constexpr bool VAR = TN == 192;
   constexpr int TMEM_COLS = VAR ? 512 : 2 * TN;
+  // tokens of an item's tile (none: every role skips the item); an MMA takes them rounded up to 16
+  auto cols_of = [&](const GemmItem& it, const DevLinear& L) -> int {
+    return VAR ? it.ntok : min(TN, min(L.batch, tokens) - it.n_tile * TN);
+  };
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* a_base = smem;                                   // STAGES x 16 KiB
@@ -358,6 +371,7 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       const GemmItem it = items[item];
       const DevLinear& L = layers[it.layer];
+      if (cols_of(it, L) <= 0) continue;
       const int first = it.k_begin + (int)((grp - q0) & 1u);       // this group's first chunk of the item
       if constexpr (FORMAT == 2) {
         (void)first; (void)wl; (void)L;
@@ -494,9 +508,11 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
     int stage = 0;
     uint32_t phase = 0, seq = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       const int chunks = __shfl_sync(0xffffffffu, items[item].k_end - items[item].k_begin, 0);
-      const uint32_t idesc = umma_idesc_f16(VAR ? (__shfl_sync(0xffffffffu, items[item].ntok, 0) + 15) & ~15 : TN);
+      const int cols = __shfl_sync(0xffffffffu, cols_of(items[item], layers[items[item].layer]), 0);
+      if (cols <= 0) continue;
+      const uint32_t idesc = umma_idesc_f16((cols + 15) & ~15);
       const uint32_t a = seq & 1u, a_phase = (seq >> 1) & 1u;     // accumulator and its use count parity
       const uint32_t d_tmem = d0 + a * TN;
       if (!mbar_wait(&acc_empty[a], a_phase ^ 1, abort_flag)) { ok = false; break; }
@@ -518,6 +534,7 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
       if (!ok) break;
       if (elect_one()) umma_commit(&acc_full[a]);
       __syncwarp();
+      ++seq;
     }
     if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_MMA); }
   } else if (warp == GM_LOAD_WARP) {
@@ -530,18 +547,21 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
         const GemmItem it = items[item];
         const DevLinear& L = layers[it.layer];
         const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
-        const uint32_t b_bytes = VAR ? (uint32_t)((it.ntok + 15) & ~15) * 128u : (uint32_t)B_BYTES;
+        const int cols = cols_of(it, L);
+        if (cols <= 0) continue;
+        // (tiles of VAR hold just these rows, the others TN)
+        const uint32_t b_bytes = (uint32_t)((cols + 15) & ~15) * 128u, b_step = VAR ? b_bytes : (uint32_t)B_BYTES;
         const uint8_t* src = ws + L.xr_off + (VAR ? (size_t)it.row0 * kchunks * 128 : (size_t)it.n_tile * kchunks * B_BYTES);
         for (int kc = it.k_begin; kc < it.k_end; ++kc) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
           if constexpr (FORMAT == 2) {
-            mbar_expect_tx(&full_b[stage], B_BYTES + GM_A_BYTES);
+            mbar_expect_tx(&full_b[stage], b_bytes + GM_A_BYTES);
             bulk_g2s(a_base + stage * GM_A_BYTES,
                      ws + L.atile_off + ((size_t)it.m_tile * kchunks + kc) * GM_A_BYTES, GM_A_BYTES, &full_b[stage]);
           } else {
             mbar_expect_tx(&full_b[stage], b_bytes);
           }
-          bulk_g2s(b_base + stage * B_BYTES, src + (size_t)kc * b_bytes, b_bytes, &full_b[stage]);
+          bulk_g2s(b_base + stage * B_BYTES, src + (size_t)kc * b_step, b_bytes, &full_b[stage]);
           ++loads_issued;
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -554,15 +574,16 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
     const int quarter = warp & 3;                          // TMEM lanes 32*quarter .. 32*quarter + 31
     uint32_t seq = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       const GemmItem it = items[item];
       const DevLinear& L = layers[it.layer];
+      const int cols = cols_of(it, L);                                  // columns that are tokens
+      if (cols <= 0) continue;
       const uint32_t a = seq & 1u, a_phase = (seq >> 1) & 1u;
       if (!mbar_wait(&acc_full[a], a_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const int row = it.m_tile * GM_TILE_M + quarter * 32 + lane;
       const int m = L.m, first = VAR ? it.tok0 : it.n_tile * TN;
-      const int cols = VAR ? it.ntok : min(TN, L.batch - first);        // columns that are tokens
       float* part = reinterpret_cast<float*>(ws + L.part_off) + ((long long)it.slot * L.batch + first) * m + row;
 #pragma unroll 1
       for (int c0 = 0; c0 < cols; c0 += 32) {
@@ -584,6 +605,7 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[a]);
+      ++seq;
     }
     if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_EPILOGUE); }
   }

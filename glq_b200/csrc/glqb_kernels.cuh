@@ -217,7 +217,7 @@ constexpr int MV_LUT_SMEM_BYTES = 65536 * 2;
 template <int K1, int K2, int NB, int LUT = 0>
 __global__ void __launch_bounds__(LUT ? MV_LUT_THREADS : MV_THREADS, LUT ? 1 : ((NB == 1 && K2 == 0) ? GLQB_MINB : 1))
 trellis_mv_kernel(const DevLinear* __restrict__ layers, int n_layers, long long total_groups,
-                  int per_warp, uint8_t* __restrict__ ws) {
+                  int per_warp, uint8_t* __restrict__ ws, int tokens) {
   uint32_t lut_base = 0u;
   if constexpr (LUT > 0) {
     extern __shared__ __align__(16) unsigned short lut3[];
@@ -250,7 +250,7 @@ trellis_mv_kernel(const DevLinear* __restrict__ layers, int n_layers, long long 
     const int strip = (int)(local / gps);
     const int c0 = (int)(local - (long long)strip * gps);
     const int c1 = (int)min((long long)gps, c0 + (gend - g));
-    const int batch = L.batch;
+    const int batch = L.batch, used = min(batch, tokens);    // rows of the buffers; rows of this run
 
     float acc[NB][2][4];
     float acc2[K2 ? NB : 1][2][4];
@@ -265,13 +265,13 @@ trellis_mv_kernel(const DevLinear* __restrict__ layers, int n_layers, long long 
     const uint8_t* p2 = nullptr;
     if constexpr (K2 > 0) p2 = L.codes[1] + ((long long)strip * gps + c0) * (128 * K2) + lane * (4 * K2);
     const __half* xr = reinterpret_cast<const __half*>(ws + L.xr_off);
-    // MMA column gq of block nb carries token 8*nb + gq.  Columns past the batch read the last
+    // MMA column gq of block nb carries token 8*nb + gq.  Columns past the tokens of the run read the last
     // token again: their products land in accumulator columns that are never stored, which saves the
     // predicate and the zero fill on every group.
     const uint4* xq[NB];
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
-      const int token = min(nb * 8 + gq, batch - 1);
+      const int token = min(nb * 8 + gq, used - 1);
       xq[nb] = reinterpret_cast<const uint4*>(xr + ((long long)token * L.n + c0 * 32) * XR_TRELLIS_EXPAND + tq * 16);
     }
 
@@ -355,7 +355,7 @@ trellis_mv_kernel(const DevLinear* __restrict__ layers, int n_layers, long long 
           for (int i = 0; i < 4; ++i) {
             const int token = nb * 8 + tq * 2 + (i & 1);
             const int row = strip * 32 + mi * 16 + gq + ((i >> 1) ? 8 : 0);
-            if (token < batch) {
+            if (token < used) {
               float v = acc[nb][mi][i];
               if constexpr (K2 > 0) v = __fadd_rn(v, __fmul_rn(s2, acc2[nb][mi][i]));
               part[(long long)token * L.m + row] = v;
@@ -428,7 +428,7 @@ __device__ __forceinline__ uint32_t e8_gather(const E8Stage& S, uint32_t idx) {
 template <int NS, int NB, int TM>
 __device__ __forceinline__ void e8_mv_body(const DevLinear* __restrict__ layers, int n_layers, long long total_groups,
                                            int per_warp, uint8_t* __restrict__ ws, const E8Tables& T,
-                                           int warps_per_cta) {
+                                           int warps_per_cta, int tokens) {
   const int lane = threadIdx.x & 31;
   const long long w = (long long)blockIdx.x * warps_per_cta + (threadIdx.x >> 5);
   long long g = w * per_warp;
@@ -449,7 +449,7 @@ __device__ __forceinline__ void e8_mv_body(const DevLinear* __restrict__ layers,
     const int strip = (int)(local / gps);
     const int c0 = (int)(local - (long long)strip * gps);
     const int c1 = (int)min((long long)gps, c0 + (gend - g));
-    const int batch = L.batch;
+    const int batch = L.batch, used = min(batch, tokens);    // rows of the buffers; rows of this run
     const int nidx = L.n >> 3;                 // indices per row
     bool vec_ok = (nidx & 7) == 0;             // rows (and the matrices themselves) start 16-byte aligned
 #pragma unroll
@@ -523,12 +523,12 @@ __device__ __forceinline__ void e8_mv_body(const DevLinear* __restrict__ layers,
           eb[s][k] = e8_gather<TM>(stg[s], (qb[s][k >> 1] >> ((k & 1) * 16)) & stg[s].mask);
         }
     };
-    // columns past the batch read the last token again (their accumulator columns are never stored)
+    // columns past the tokens of the run read the last token again (their accumulator columns are never stored)
     const uint4* xrow[NB];
     const int xstep = batch == 1 ? 1 : 8;      // 16-byte units between consecutive 8-column blocks
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
-      const int tok = min(nb * 8 + gq, batch - 1);
+      const int tok = min(nb * 8 + gq, used - 1);
       xrow[nb] = reinterpret_cast<const uint4*>(xr) + (batch == 1 ? 0 : (long long)(tok >> 3) * nidx * 8 + (tok & 7));
     }
     auto consume = [&](int cc, const uint32_t (&ea)[NS][KC], const uint32_t (&eb)[NS][KC]) {
@@ -589,7 +589,7 @@ __device__ __forceinline__ void e8_mv_body(const DevLinear* __restrict__ layers,
         for (int i = 0; i < 4; ++i) {
           const int token = nb * 8 + tq * 2 + (i & 1);
           const int row = (i >> 1) ? rowB : rowA;
-          if (token < batch && row < L.m) {
+          if (token < used && row < L.m) {
             float v = acc[0][nb][i];
 #pragma unroll
             for (int s = 1; s < NS; ++s) v = __fadd_rn(v, __fmul_rn(L.stage_scale[s], acc[s][nb][i]));
@@ -606,9 +606,9 @@ __device__ __forceinline__ void e8_mv_body(const DevLinear* __restrict__ layers,
 template <int NS, int NB>
 __global__ void __launch_bounds__(MV_THREADS, (NB <= 2 ? GLQB_E8_MINB : 1))
 e8_mv_kernel(const DevLinear* __restrict__ layers, int n_layers, long long total_groups,
-             int per_warp, uint8_t* __restrict__ ws) {
+             int per_warp, uint8_t* __restrict__ ws, int tokens) {
   const E8Tables T = {0u, 0u};
-  e8_mv_body<NS, NB, 0>(layers, n_layers, total_groups, per_warp, ws, T, MV_WARPS);
+  e8_mv_body<NS, NB, 0>(layers, n_layers, total_groups, per_warp, ws, T, MV_WARPS, tokens);
 }
 
 // Resident-table form: one CTA per SM keeps most of the 65,536-entry table in shared memory.
@@ -622,7 +622,7 @@ template <int NS, int NB>
 __global__ void __launch_bounds__(E8S_THREADS, 1)
 e8_mv_smem_kernel(const DevLinear* __restrict__ layers, int n_layers, long long total_groups, int per_warp,
                   uint8_t* __restrict__ ws, const uint32_t* __restrict__ big_table,
-                  const uint32_t* __restrict__ small_table, int small_entries) {
+                  const uint32_t* __restrict__ small_table, int small_entries, int tokens) {
   extern __shared__ __align__(16) uint32_t e8_smem[];
   const uint4* src = reinterpret_cast<const uint4*>(big_table);
   uint4* dst = reinterpret_cast<uint4*>(e8_smem);
@@ -633,7 +633,7 @@ e8_mv_smem_kernel(const DevLinear* __restrict__ layers, int n_layers, long long 
   T.table_base = local;
   T.small_base = local + E8S_RESIDENT * 4;
   __syncthreads();
-  e8_mv_body<NS, NB, 1>(layers, n_layers, total_groups, per_warp, ws, T, E8S_THREADS / 32);
+  e8_mv_body<NS, NB, 1>(layers, n_layers, total_groups, per_warp, ws, T, E8S_THREADS / 32, tokens);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -44,9 +44,9 @@ constexpr int GEMM_STAGES = 4;
 bool gemm_available(const Segment& s);                       // is there a kernel for the segment's format / rates?
 cudaError_t gemm_prepare(const Segment& s);                  // raises the kernel's dynamic shared-memory limit
 cudaError_t tiles_smem_prepare(int ns);                      // same for the resident-table tile decode
-// the segment's launches: (two-phase: tile decode, then) the GEMM over `items`
+// the segment's launches: (two-phase: tile decode, then) the GEMM over `items`, for at most `tokens` tokens per layer
 void gemm_launch(const Segment& s, const DevLinear* layers, const GemmItem* items, uint8_t* ws, int* status,
-                 int sm_count, cudaStream_t stream);
+                 int sm_count, int tokens, cudaStream_t stream);
 
 // ---- glqb_fused.cu
 bool fused_available(const Segment& s);                      // is there a single-launch kernel for the segment's format / rates?

@@ -907,7 +907,7 @@ static MoeMvKernel moe_mv_pick(int k1, int k2) {
   return nullptr;
 }
 
-typedef void (*MoeGemmKernel)(const DevLinear*, const GemmItem*, int, uint8_t*, int*, const int*);
+typedef void (*MoeGemmKernel)(const DevLinear*, const GemmItem*, int, uint8_t*, int*, const int*, int);
 // E8 experts: three stages of 40 KiB leave the codebook gathers of the producers as much L1 as 128-token tiles with four
 // did.  8 experts, top 2, 4096 x 2048, two stages, four / three: 8 tokens 318 / 281 us, 1024 tokens 672 / 618.
 constexpr int MOE_GEMM_STAGES = 3;
@@ -1263,14 +1263,14 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
       MoeTimer t(P, st);
       P->g13<<<std::min(P->sm_count, G.max_items13), g_threads, moe_gemm_smem_bytes(g_e8), st>>>(
           reinterpret_cast<const DevLinear*>(ws + G.o_layers13), reinterpret_cast<const GemmItem*>(ws + G.o_items13),
-          G.max_items13, ws, status, nitems);
+          G.max_items13, ws, status, nitems, tokens);
     }
     moe_mid_kernel<<<(R + P->mid_sg - 1) / P->mid_sg, MOE_XF_THREADS, P->mid_smem, st>>>(G, tokens, P->mid_sg, ws);
     {
       MoeTimer t(P, st);
       P->g2<<<std::min(P->sm_count, G.max_items2), g_threads, moe_gemm_smem_bytes(g_e8), st>>>(
           reinterpret_cast<const DevLinear*>(ws + G.o_layers2), reinterpret_cast<const GemmItem*>(ws + G.o_items2),
-          G.max_items2, ws, status, nitems + 1);
+          G.max_items2, ws, status, nitems + 1, tokens);
     }
     moe_out_kernel<<<tokens, MOE_XF_THREADS, P->out_smem, st>>>(G, tokens, P->out_rg, topk_weights, ws,
                                                                reinterpret_cast<uint8_t*>(y));

@@ -298,17 +298,23 @@ __device__ __forceinline__ void rht_in_body(const DevLinear& L, const RhtItem it
   fht_block(fbuf, log_t, total, load, store);
 }
 
+// the tile of an item that lies below `tokens`, the tokens of this run; false: none of it does
+__device__ __forceinline__ bool rht_item_trim(RhtItem& it, int tokens) {
+  it.ntok = min(it.ntok, tokens - it.tok0);
+  return it.ntok > 0;
+}
+
 template <bool PLAIN_F32>
 __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_kernel(const DevLinear* __restrict__ layers,
                                                              const RhtItem* __restrict__ items,
                                                              const uint8_t* __restrict__ x_base,
-                                                             uint8_t* __restrict__ ws) {
+                                                             uint8_t* __restrict__ ws, int tokens) {
   extern __shared__ __align__(16) float fbuf[];
   // a successor launched with programmatic stream serialization (the single-launch decode kernel) may start
   // its prologue now; it waits for this kernel's completion before it reads the activations
   asm volatile("griddepcontrol.launch_dependents;");
-  const RhtItem it = items[blockIdx.x];
-  rht_in_body<PLAIN_F32>(layers[it.layer], it, x_base, ws, fbuf);
+  RhtItem it = items[blockIdx.x];
+  if (rht_item_trim(it, tokens)) rht_in_body<PLAIN_F32>(layers[it.layer], it, x_base, ws, fbuf);
 }
 
 // One layer described entirely in kernel-parameter space (no device table, nothing to allocate or copy):
@@ -548,11 +554,12 @@ __device__ __forceinline__ void rht_out_plain(const DevLinear& L, const RhtItem 
 static __global__ void __launch_bounds__(RHT_THREADS, 4) rht_out_plain_kernel(const DevLinear* __restrict__ layers,
                                                               const RhtItem* __restrict__ items,
                                                               const uint8_t* __restrict__ ws,
-                                                              uint8_t* __restrict__ y_base) {
+                                                              uint8_t* __restrict__ y_base, int tokens) {
   extern __shared__ __align__(16) float fbuf[];
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const RhtItem it = items[blockIdx.x];
+  RhtItem it = items[blockIdx.x];
+  if (!rht_item_trim(it, tokens)) return;
   const DevLinear& L = layers[it.layer];
   rht_out_plain<false>(L, it, reinterpret_cast<const float*>(ws + L.part_off), y_base, fbuf);
 }
@@ -562,14 +569,14 @@ __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_out_kernel(const De
                                                               const RhtItem* __restrict__ items,
                                                               const uint8_t* __restrict__ ws,
                                                               uint8_t* __restrict__ y_base,
-                                                              const float* __restrict__ yrht_in) {
+                                                              const float* __restrict__ yrht_in, int tokens) {
   extern __shared__ __align__(16) float fbuf[];
   // launched with programmatic stream serialization behind the decode kernels: wait for them here; the next
   // kernel of the stream may start its prologue
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const RhtItem it = items[blockIdx.x];
-  rht_out_body<false, WIDE>(layers[it.layer], it, ws, y_base, yrht_in, fbuf);
+  RhtItem it = items[blockIdx.x];
+  if (rht_item_trim(it, tokens)) rht_out_body<false, WIDE>(layers[it.layer], it, ws, y_base, yrht_in, fbuf);
 }
 
 // One array of 32 to 1024 values of the unfused op: the shuffle transform (one token of 1024 values 2.3 us; fht_block, whose

@@ -21,7 +21,6 @@
 
 namespace glqb {
 
-constexpr int TG_TN = 192;                       // most tokens of a tile (multiples of 16)
 // a stage is a pair of 64-column chunks: 64 columns of tensor memory, one copy of the two chunks' activations
 constexpr int TG_A_STAGES = 2, TG_A_COLS = 32;   // columns per chunk
 constexpr int TG_B_STAGES = 4;
@@ -83,9 +82,16 @@ __device__ __forceinline__ void tg_decode_group(int lane, const Words<K1>& v, co
 template <int K1, int K2>
 __global__ void __launch_bounds__(TG_THREADS, 1)
 trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict__ items, int n_items,
-                    uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev) {
+                    uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev, int tokens) {
   // work lists built on the device (grouped expert matmul) pass their length through memory
   if (n_items_dev) n_items = min(n_items, *n_items_dev);
+  // first token and tokens of an item's tile (none: every role skips the item), and the activation rows in front of it
+  struct Tile { int tok0, ntok, row0; };
+  auto tile_of = [&](const GemmItem& it, const DevLinear& L) -> Tile {
+    if (n_items_dev) return Tile{it.tok0, it.ntok, it.row0};
+    const int used = min(L.batch, tokens), tt = tile_tokens(used);
+    return Tile{it.n_tile * tt, min(tt, used - it.n_tile * tt), it.n_tile * tt};
+  };
   constexpr int MMA_WARP = TG_MMA_WARP, LOAD_WARP = TG_LOAD_WARP;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* b_base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -129,9 +135,11 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
     const uint32_t b0 = smem_u32(b_base);
     uint32_t q = 0, seq = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       const int chunks = __shfl_sync(0xffffffffu, items[item].k_end - items[item].k_begin, 0);
-      const int cols = (__shfl_sync(0xffffffffu, items[item].ntok, 0) + 15) & ~15;
+      const int ntok = __shfl_sync(0xffffffffu, tile_of(items[item], layers[items[item].layer]).ntok, 0);
+      if (ntok <= 0) continue;
+      const int cols = (ntok + 15) & ~15;
       const uint32_t idesc = umma_idesc_f16(cols), half = (uint32_t)cols * 8u;     // (16-byte units of a chunk's activations)
       const uint32_t a = seq & 1u;                 // accumulator
       const uint32_t d_tmem = d0 + a * TG_TN;
@@ -160,6 +168,7 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
       if (!ok) break;
       if (elect_one()) umma_commit(&acc_full[a]);
       __syncwarp();
+      ++seq;
     }
     if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_MMA); }
   } else if (warp == LOAD_WARP) {
@@ -171,8 +180,10 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
         const GemmItem it = items[item];
         const DevLinear& L = layers[it.layer];
         const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
-        const uint32_t bytes = (uint32_t)((it.ntok + 15) & ~15) * 128u;
-        const uint8_t* src = ws + L.xr_off + (size_t)it.row0 * kchunks * 128;
+        const Tile t = tile_of(it, L);
+        if (t.ntok <= 0) continue;
+        const uint32_t bytes = (uint32_t)((t.ntok + 15) & ~15) * 128u;
+        const uint8_t* src = ws + L.xr_off + (size_t)t.row0 * kchunks * 128;
         for (int kc = it.k_begin; kc < it.k_end; kc += 2, ++q) {
           const uint32_t sb = q % TG_B_STAGES, n = kc + 1 < it.k_end ? 2u * bytes : bytes;
           if (!mbar_wait(&empty_b[sb], ((q / TG_B_STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
@@ -196,6 +207,7 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       const GemmItem it = items[item];
       const DevLinear& L = layers[it.layer];
+      if (tile_of(it, L).ntok <= 0) continue;
       const int rp = it.m_tile * 4 + strip, gps = L.groups_per_strip, k_end = it.k_end;
       const bool row_ok = rp < L.strips;
       // chunks below k_both have two groups, chunk k_both may have one (columns past the matrix are zeros)
@@ -268,15 +280,17 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
     const int quarter = warp & 3;                          // TMEM lanes 32*quarter .. 32*quarter + 31
     uint32_t seq = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++seq) {
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       const GemmItem it = items[item];
       const DevLinear& L = layers[it.layer];
+      const Tile t = tile_of(it, L);
+      if (t.ntok <= 0) continue;
       const uint32_t a = seq & 1u;
       if (!mbar_wait(&acc_full[a], (seq >> 1) & 1u, abort_flag)) { ok = false; break; }
       __syncwarp();
       tc_fence_after();
-      const int row = it.m_tile * GM_TILE_M + quarter * 32 + lane, m = L.m, cols = it.ntok;
-      float* part = reinterpret_cast<float*>(ws + L.part_off) + ((long long)it.slot * L.batch + it.tok0) * m + row;
+      const int row = it.m_tile * GM_TILE_M + quarter * 32 + lane, m = L.m, cols = t.ntok;
+      float* part = reinterpret_cast<float*>(ws + L.part_off) + ((long long)it.slot * L.batch + t.tok0) * m + row;
 #pragma unroll 1
       for (int c0 = 0; c0 < cols; c0 += 32) {
         uint32_t r[32];
@@ -298,6 +312,7 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[a]);
+      ++seq;
     }
     if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_EPILOGUE); }
   }

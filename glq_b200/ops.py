@@ -74,8 +74,7 @@ def e8_packed_table(codebook: torch.Tensor) -> torch.Tensor:
 
 def token_bucket(b: int) -> int:
     """Token count a plan is built for when ``b`` tokens arrive: exact up to 8, multiples of 8 up to 64
-    (the streaming kernels), 128, then multiples of 256 (the tensor-core path).  Inputs are zero-padded to
-    the bucket and the extra output rows dropped."""
+    (the streaming kernels), 128, then multiples of 256 (the tensor-core path).  A run takes the tokens there are."""
     if b <= 8:
         return b
     if b <= DECODE_MAX_TOKENS:
@@ -139,30 +138,21 @@ def clear_caches() -> None:
 
 
 def _run_sliced(x2d: torch.Tensor, out: torch.Tensor, key_base, make_spec, max_tokens=DECODE_MAX_TOKENS,
-                y_offset: int = 0, out_cols: Optional[int] = None, accumulate: bool = False, comm=None) -> None:
-    """Run a single-layer op over x2d (B, in) into out[:, y_offset : y_offset + out_cols].  Up to 64 tokens go
-    through the streaming kernels in slices of <= max_tokens, more through one tensor-core plan; token counts
-    are rounded up to ``token_bucket`` sizes (zero-padded copy in, extra rows dropped)."""
+                y_offset: int = 0, comm=None) -> None:
+    """Run a single-layer op over x2d (B, in) into the columns of out from y_offset on.  Up to 64 tokens go
+    through the streaming kernels in slices of <= max_tokens, more through one tensor-core plan; plans are built
+    for ``token_bucket`` sizes and take the tokens there are."""
     B = x2d.shape[0]
-    cols = out_cols if out_cols is not None else out.shape[1]
 
-    def run(xs, b, dst_rows):
+    def run(xin, b, yout):
         bb = token_bucket(b)
-        if bb == b:
-            xin, yout, yoff = xs, dst_rows, y_offset
-        else:
-            xin = xs.new_zeros((bb, xs.shape[1]))
-            xin[:b] = xs
-            yout, yoff = torch.empty((bb, cols), dtype=out.dtype, device=out.device), 0
-            if accumulate:
-                yout[:b] = dst_rows[:b, y_offset:y_offset + cols]
-        key = key_base + (bb, xin.dtype, yout.dtype, xin.stride(0), yout.stride(0), yoff, id(comm) if comm is not None else 0)
+        key = key_base + (bb, xin.dtype, yout.dtype, xin.stride(0), yout.stride(0), y_offset, id(comm) if comm is not None else 0)
         refused = _REFUSED.get(key)
         if refused is not None:                       # the library refused this form before: do not build the plan again
             raise RuntimeError(refused)
         fresh = key not in _PLAN_CACHE
         try:
-            plan = _cached_plan(key, lambda: [make_spec(bb, xin.stride(0), yout.stride(0), yoff)])
+            plan = _cached_plan(key, lambda: [make_spec(bb, xin.stride(0), yout.stride(0), y_offset)])
             if fresh and comm is not None:
                 try:
                     plan.set_comm(comm)
@@ -175,9 +165,7 @@ def _run_sliced(x2d: torch.Tensor, out: torch.Tensor, key_base, make_spec, max_t
             if "single-launch" in str(e) or "plan_set_comm" in str(e):
                 _REFUSED[key] = str(e)
             raise
-        plan.run(xin, yout, workspace=shared_workspace(xin.device, plan.workspace_bytes))
-        if bb != b:
-            dst_rows[:b, y_offset:y_offset + cols] = yout[:b]
+        plan.run(xin, yout, workspace=shared_workspace(xin.device, plan.workspace_bytes), tokens=b)
 
     if B > DECODE_MAX_TOKENS:
         run(x2d, B, out)
@@ -304,8 +292,7 @@ def _fused_trellis(x, sv, su, packed, packed2, blocks_n, blocks_m, wscale, inv_r
            accumulate_into is not None)
     # two decoded stages keep two accumulator sets: 32 tokens per pass instead of 64
     try:
-        _run_sliced(x2d, tgt, key, make_spec, 32 if has2 else DECODE_MAX_TOKENS, y_offset=yoff,
-                    out_cols=m_pad if stop else out_features, accumulate=accumulate_into is not None, comm=comm)
+        _run_sliced(x2d, tgt, key, make_spec, 32 if has2 else DECODE_MAX_TOKENS, y_offset=yoff, comm=comm)
     except RuntimeError as e:
         if comm is not None or not extras or "single-launch" not in str(e):
             raise
@@ -384,10 +371,7 @@ def fused_linear_trellis_3inst_shards(x, sv, shards, blocks_n=None, out_dtype=No
     bn = _blocks(blocks_n, n)
     bb = token_bucket(B)
     xin = x2d
-    if bb != B:
-        xin = x2d.new_zeros((bb, n))
-        xin[:B] = x2d
-    out = torch.empty((bb, total_m), dtype=odt, device=x2d.device)
+    out = torch.empty((B, total_m), dtype=odt, device=x2d.device)
     key = ("trellis_shards", tuple(sh[1].data_ptr() for sh in shards), sv.data_ptr(), tuple(float(sh[3]) for sh in shards),
            bb, xin.dtype, odt, xin.stride(0), in_norm_weight.data_ptr() if in_norm_weight is not None else 0, float(in_norm_eps))
 
@@ -405,8 +389,8 @@ def fused_linear_trellis_3inst_shards(x, sv, shards, blocks_n=None, out_dtype=No
             col += int(m)
         return specs
     plan = _cached_plan(key, make_specs)
-    plan.run(xin, out, workspace=shared_workspace(xin.device, plan.workspace_bytes))
-    return out[:B]
+    plan.run(xin, out, workspace=shared_workspace(xin.device, plan.workspace_bytes), tokens=B)
+    return out
 
 
 def fused_linear_e8_shards(x, sv, shards, codebook, codebook2=None, blocks_n=None, out_dtype=None, in_norm_weight=None,
@@ -429,10 +413,7 @@ def fused_linear_e8_shards(x, sv, shards, codebook, codebook2=None, blocks_n=Non
     bn = _blocks(blocks_n, n)
     bb = token_bucket(B)
     xin = x2d
-    if bb != B:
-        xin = x2d.new_zeros((bb, n))
-        xin[:B] = x2d
-    out = torch.empty((bb, total_m), dtype=odt, device=x2d.device)
+    out = torch.empty((B, total_m), dtype=odt, device=x2d.device)
     t1 = e8_packed_table(codebook)
     t2 = e8_packed_table(codebook2) if codebook2 is not None else t1
     key = ("e8_shards", tuple(sh[1][0].data_ptr() for sh in shards), sv.data_ptr(), tuple(float(sh[3]) for sh in shards),
@@ -451,8 +432,8 @@ def fused_linear_e8_shards(x, sv, shards, codebook, codebook2=None, blocks_n=Non
             col += int(m)
         return specs
     plan = _cached_plan(key, make_specs)
-    plan.run(xin, out, workspace=shared_workspace(xin.device, plan.workspace_bytes))
-    return out[:B]
+    plan.run(xin, out, workspace=shared_workspace(xin.device, plan.workspace_bytes), tokens=B)
+    return out
 
 
 _ONES: dict = {}
@@ -569,8 +550,7 @@ def _fused_e8(x, sv, su, codes, tables, scales, wscale, in_features, out_feature
            su.data_ptr(), sv.data_ptr(), float(wscale), m_pad, n_pad, in_features, out_features, stop, x_is_rotated,
            in_norm_weight.data_ptr() if in_norm_weight is not None else 0, float(in_norm_eps), gated_act,
            accumulate_into is not None)
-    _run_sliced(x2d, out, key, make_spec, 32 if len(codes) > 2 else DECODE_MAX_TOKENS,
-                accumulate=accumulate_into is not None, comm=comm)
+    _run_sliced(x2d, out, key, make_spec, 32 if len(codes) > 2 else DECODE_MAX_TOKENS, comm=comm)
     return accumulate_into if accumulate_into is not None else out
 
 

@@ -137,14 +137,15 @@ class Plan:
         self.launches = int(self.lib.glqb_plan_launches(handle))
 
     def run(self, x: torch.Tensor, y: torch.Tensor, stream: Optional[torch.cuda.Stream] = None,
-            workspace: Optional[torch.Tensor] = None) -> None:
-        """Enqueue on ``stream`` (default: the current torch stream); does not synchronise."""
+            workspace: Optional[torch.Tensor] = None, tokens: int = 2 ** 31 - 1) -> None:
+        """Enqueue on ``stream`` (default: the current torch stream); does not synchronise.  ``tokens``: rows of x and y
+        to process when they are fewer than the plan was built for."""
         st = stream if stream is not None else torch.cuda.current_stream(self.device)
         ws = workspace if workspace is not None else self.workspace
         if ws is None:
             raise RuntimeError("glq_b200: this plan owns no workspace; pass one to run()")
-        _lib.check(self.lib.glqb_plan_run(self.handle, x.data_ptr(), y.data_ptr(), ws.data_ptr(), ws.numel(),
-                                          st.cuda_stream), "plan_run")
+        _lib.check(self.lib.glqb_plan_run_tokens(self.handle, x.data_ptr(), y.data_ptr(), tokens, ws.data_ptr(),
+                                                 ws.numel(), st.cuda_stream), "plan_run")
 
     def set_timing(self, on: bool) -> None:
         _lib.check(self.lib.glqb_plan_set_timing(self.handle, 1 if on else 0), "plan_set_timing")

@@ -107,6 +107,11 @@ int32_t glqb_plan_launches(const GlqbPlan* plan);
  * descriptors' offsets are applied to. */
 int glqb_plan_run(GlqbPlan* plan, const void* x_base, void* y_base,
                   void* workspace, size_t workspace_bytes, void* stream);
+/* The same for the first `tokens` tokens (>= 1; layers of fewer take all of theirs): no other row of x is read, no other
+ * row of y is written, and the work shrinks with the tokens.  A plan of the single-launch decode form takes its own
+ * number of tokens or more. */
+int glqb_plan_run_tokens(GlqbPlan* plan, const void* x_base, void* y_base, int32_t tokens,
+                         void* workspace, size_t workspace_bytes, void* stream);
 /* With timing enabled every run brackets its decode kernels with a CUDA event pair on the launching
  * stream.  glqb_plan_kernel_ms waits for those events and returns the summed kernel time (ms) and the
  * number of runs recorded since timing was (re-)enabled. */

@@ -74,3 +74,33 @@ def test_two_stage_256_token_tiles(shape, bits, monkeypatch):
         a, _ = run(L, x, monkeypatch, {"GLQB_TRELLIS_256_MIN_WEIGHTS": "1"})
         b, _ = run(L, x, monkeypatch, {"GLQB_TRELLIS_256_MIN_WEIGHTS": str(1 << 60)})
         assert torch.equal(a, b)
+
+
+# fewer tokens than the plan was built for: edges of the 16-row steps, of the token tiles (192, 256) and of the two schedules
+# of a plan; rows past the tokens are neither read (NaN) nor written.  The same products in fp32, split over K in another
+# order: n 2^-24 = 6e-5 of a row's absolute sum, about sqrt(n) of which is its largest value (2e-6), with a margin of ten.
+@pytest.mark.parametrize("kind", ["trellis", "two stages", "tiles", "e8", "e8 fused"])
+@pytest.mark.parametrize("bucket,tokens", [(16, 9), (32, 27), (64, 57), (128, 65), (128, 113), (256, 129), (256, 192), (256, 193),
+                                           (512, 257), (512, 384), (512, 385), (512, 20)])
+def test_run_of_fewer_tokens(kind, bucket, tokens, monkeypatch):
+    m, n = 160, 1056
+    monkeypatch.setenv("GLQB_TRELLIS_TWO_PHASE_MIN_FLOPS", "1" if kind == "tiles" else "1e30")
+    monkeypatch.setenv("GLQB_E8_TWO_PHASE_MIN_TOKENS", "65" if kind == "e8" else "100000")
+    if kind == "two stages" and bucket == 64:
+        pytest.skip("two stages take 32 tokens per pass")
+    g = torch.Generator(device="cuda").manual_seed(bucket + tokens)
+    if kind.startswith("e8"):
+        L = synth.e8_layer("e", m, n, 2, synth.load_e8_table("cuda"), g, "cuda")
+    else:
+        L = synth.trellis_layer("t", m, n, [4, 2] if kind == "two stages" else [4], g, "cuda")
+    x = torch.randn(bucket, n, generator=g, device="cuda").half()
+    plan = Plan([L.spec(batch=bucket, x_dtype=x.dtype, y_dtype=torch.float32)])
+    full = torch.empty(bucket, m, device="cuda")
+    plan.run(x, full)
+    x[tokens:] = float("nan")
+    y = torch.full((bucket, m), -7.0, device="cuda")
+    plan.run(x, y, tokens=tokens)
+    plan.check_status()
+    plan.close()
+    assert (y[tokens:] == -7.0).all()
+    assert (y[:tokens] - full[:tokens]).abs().max() <= 2e-5 * full.abs().max()
