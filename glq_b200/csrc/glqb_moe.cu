@@ -3,7 +3,7 @@
 // (reference: glq_fused_moe_trellis_3inst_cuda, glq/csrc/glq_cuda.cu:5042; eager loop
 // glq_vllm/fused_moe_method.py:393-440; storage glq_vllm/moe_shapes.py:56-72).
 //
-// Six launches (eight kernels and a memset from 8192 routings, see moe_launch_group), fixed grids, no host
+// Six launches (eight kernels and a memset from 65536 routings, see moe_launch_group), fixed grids, no host
 // synchronisation (capture-safe):
 //   1 moe_group_kernel     count tokens per expert, prefix sums, place every (token, j) routing in a slot
 //                          (tensor-core form: also the per-expert layer entries and the GEMM work lists)
@@ -106,10 +106,13 @@ __device__ __forceinline__ float moe_act(float g, int act) {
 }
 
 // ---- 1: grouping ------------------------------------------------------------------------------------
-// phase 0: everything in this one CTA (small steps).  phase 1: the counts were made by moe_count_kernel and the
+// phase 0: one launch of up to 32 CTAs.  Every CTA counts all routings (their ids come from L2), so that each knows the
+// counts, the prefix sums and how many routings of an expert lie in front of its own share; tables and placements are
+// shared out, and nothing has to be cleared first.  phase 1: the counts were made by moe_count_kernel and the
 // routings are placed by moe_place_kernel (many CTAs each); this kernel only does the prefix sums and tables.
 constexpr int MOE_GROUP_CHUNK = 8192;          // routings per CTA of the count / place kernels
-constexpr int MOE_GROUP_SPLIT_MIN = 8192;      // routings from which the three-kernel form is used
+constexpr int MOE_GROUP_SPLIT_MIN = 65536;     // routings from which the three-kernel form is used
+constexpr int MOE_GROUP_SHARE = 256, MOE_GROUP_CTAS = 32;      // routings per CTA of the one-launch form, most CTAs
 
 __device__ __forceinline__ int moe_expert_of(const MoeDev& M, const void* ids, int i) {
   const long long v = M.ids_i64 ? reinterpret_cast<const long long*>(ids)[i] : (long long)reinterpret_cast<const int*>(ids)[i];
@@ -178,12 +181,13 @@ __global__ void __launch_bounds__(1024) moe_place_kernel(const __grid_constant__
 
 __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__ MoeDev M, const void* __restrict__ ids,
                                                          int T, uint8_t* __restrict__ ws, int phase) {
-  extern __shared__ int sh[];            // counts[E], cursor[E], first slot[E], first token tile[E + 1], first row[E]
+  extern __shared__ int sh[];            // counts[E], cursor[E], first slot[E], first token tile[E + 1], first row[E], in front[E]
   int* cnt = sh;
   int* cur = sh + M.E;
   int* base_s = sh + 2 * M.E;
   int* tile0 = sh + 3 * M.E;
   int* row0 = sh + 4 * M.E + 1;
+  int* front = sh + 5 * M.E + 1;         // routings of the expert in front of this CTA's share
   int* g_count = reinterpret_cast<int*>(ws + M.o_count);
   int* g_base = reinterpret_cast<int*>(ws + M.o_base);
   int* g_work = reinterpret_cast<int*>(ws + M.o_work);
@@ -191,8 +195,10 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
   int* route_exp = reinterpret_cast<int*>(ws + M.o_route_exp);
   int* slot_of = reinterpret_cast<int*>(ws + M.o_slot_of);
   const int R = T * M.top_k;
-  for (int e = threadIdx.x; e < M.E; e += blockDim.x) cnt[e] = 0;
-  if (threadIdx.x < 2) g_work[threadIdx.x] = 0;
+  const int share = (R + (int)gridDim.x - 1) / (int)gridDim.x, lo = (int)blockIdx.x * share, hi = min(R, lo + share);
+  const int tid = (int)(blockIdx.x * blockDim.x + threadIdx.x), step = (int)(gridDim.x * blockDim.x);
+  for (int e = threadIdx.x; e < M.E; e += blockDim.x) cnt[e] = front[e] = 0;
+  if (tid < 2) g_work[tid] = 0;
   __syncthreads();
   auto expert_of = [&](int i) -> int { return moe_expert_of(M, ids, i); };
   if (phase == 0) {
@@ -202,7 +208,11 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
 #pragma unroll
       for (int u = 0; u < 8; ++u) { const int i = i0 + u * blockDim.x; ev[u] = i < R ? expert_of(i) : -1; }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) if (ev[u] >= 0) atomicAdd(&cnt[ev[u]], 1);
+      for (int u = 0; u < 8; ++u)
+        if (ev[u] >= 0) {
+          atomicAdd(&cnt[ev[u]], 1);
+          if (i0 + u * (int)blockDim.x < lo) atomicAdd(&front[ev[u]], 1);
+        }
     }
   } else {
     __syncthreads();
@@ -221,7 +231,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
         const int pa = __shfl_up_sync(0xffffffffu, a, o), pb = __shfl_up_sync(0xffffffffu, b, o), pd = __shfl_up_sync(0xffffffffu, d, o);
         if ((int)threadIdx.x >= o) { a += pa; b += pb; d += pd; }
       }
-      if (e < M.E) { cur[e] = base_s[e] = run + a - c; tile0[e] = tiles + b - nt; row0[e] = rows + d - nr; }
+      if (e < M.E) { base_s[e] = run + a - c; cur[e] = base_s[e] + front[e]; tile0[e] = tiles + b - nt; row0[e] = rows + d - nr; }
       run += __shfl_sync(0xffffffffu, a, 31);
       tiles += __shfl_sync(0xffffffffu, b, 31);
       rows += __shfl_sync(0xffffffffu, d, 31);
@@ -229,7 +239,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
     if (threadIdx.x == 0) tile0[M.E] = tiles;
   }
   __syncthreads();
-  {
+  if (blockIdx.x == 0) {
     int* g_cursor = reinterpret_cast<int*>(ws + M.o_cursor);
     int* g_row0 = reinterpret_cast<int*>(ws + M.o_row0);
     for (int e = threadIdx.x; e < M.E; e += blockDim.x) {
@@ -245,7 +255,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
     const int kc13 = M.hidden / GM_TILE_K, kc2 = M.inter / GM_TILE_K;
     const int mt13 = (M.w13_out + GM_TILE_M - 1) / GM_TILE_M, mt2 = (M.hidden + GM_TILE_M - 1) / GM_TILE_M;
     const int tiles = tile0[M.E];
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
       int* nitems = reinterpret_cast<int*>(ws + M.o_nitems);
       nitems[0] = min(tiles * mt13, M.max_items13);
       nitems[1] = min(tiles * mt2, M.max_items2);
@@ -254,7 +264,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
     DevLinear* L13 = reinterpret_cast<DevLinear*>(ws + M.o_layers13);
     DevLinear* L2 = reinterpret_cast<DevLinear*>(ws + M.o_layers2);
     // (field by field: only what the GEMM kernel reads; thread 2e writes expert e's w13 entry, 2e + 1 its w2 entry)
-    for (int i = threadIdx.x; i < 2 * M.E; i += blockDim.x) {
+    for (int i = tid; i < 2 * M.E; i += step) {
       const int e = i >> 1;
       const bool second = i & 1;
       DevLinear& a = (second ? L2 : L13)[e];
@@ -296,18 +306,18 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
       const int e = expert_of_tile(tile), j = tile - tile0[e], tt = moe_tile_tokens(cnt[e]);
       return GemmItem{e, mt, j, 0, kc, 0, j * tt, min(tt, cnt[e] - j * tt), j * tt};
     };
-    for (int idx = threadIdx.x; idx < min(tiles * mt13, M.max_items13); idx += blockDim.x) I13[idx] = item(idx / mt13, idx % mt13, kc13);
-    for (int idx = threadIdx.x; idx < min(tiles * mt2, M.max_items2); idx += blockDim.x) I2[idx] = item(idx / mt2, idx % mt2, kc2);
+    for (int idx = tid; idx < min(tiles * mt13, M.max_items13); idx += step) I13[idx] = item(idx / mt13, idx % mt13, kc13);
+    for (int idx = tid; idx < min(tiles * mt2, M.max_items2); idx += step) I2[idx] = item(idx / mt2, idx % mt2, kc2);
   }
   if (phase != 0) return;
-  for (int i0 = threadIdx.x; i0 < R; i0 += 8 * blockDim.x) {
+  for (int i0 = lo + (int)threadIdx.x; i0 < hi; i0 += 8 * blockDim.x) {
     int ev[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) { const int i = i0 + u * blockDim.x; ev[u] = i < R ? expert_of(i) : -1; }
+    for (int u = 0; u < 8; ++u) { const int i = i0 + u * blockDim.x; ev[u] = i < hi ? expert_of(i) : -1; }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int i = i0 + u * blockDim.x;
-      if (i < R) {
+      if (i < hi) {
         int slot = -1;
         if (ev[u] >= 0) {
           slot = atomicAdd(&cur[ev[u]], 1);
@@ -597,6 +607,10 @@ __device__ __forceinline__ int moe_chunk_block(int ch, int rows, int nb, const i
   }
   return b;
 }
+// 16 bytes from global to shared memory, past the registers (complete after cp.async.wait_group, for the issuing thread)
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
 // A chunk's values: sums of `cnt` partial sums `kstride` floats apart.  row_off(r): first value of row r (floats from
 // `src`, which points at the block's first column), negative for a row of zeros; rows from `nrow` on are zero.
 template <class RowOff>
@@ -784,6 +798,151 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_mid_kernel(const __grid
   }
 }
 
+// The same for blocks of up to 1024 values on both sides: a warp takes two consecutive slots by itself, no block barrier.
+// The w13 outputs of its slots pass through shared memory as the fp16 values they are rounded to, in column order, so
+// Wscale, SU and the rounding are done once per value and gate and up are one 8-byte load each; the partial sums of the
+// next chunk are in flight while one is transformed.  4096 tokens, top 8, 1536 and 768 columns: 190 us by
+// the kernel above, 175 us by this (104 and 91 M warp instructions; tanhf and the roundings are a third of them).
+constexpr int MIDW_ROWS = 2, MIDW_WARPS = 4;
+__host__ __device__ __forceinline__ size_t moe_midw_warp_bytes(int w13_out) { return FHT_CHUNK_WORDS * 4 + (size_t)MIDW_ROWS * w13_out * 2; }
+template <class F>
+__device__ __forceinline__ void with_act(int act, F f) {
+  switch (act) {
+    case 0: f(IntC<0>()); break;
+    case 1: f(IntC<1>()); break;
+    case 2: f(IntC<2>()); break;
+    case 3: f(IntC<3>()); break;
+    case 4: f(IntC<4>()); break;
+    default: f(IntC<5>()); break;
+  }
+}
+__global__ void __launch_bounds__(MIDW_WARPS * 32, 4) moe_mid_warp_kernel(const __grid_constant__ MoeDev M, int T,
+                                                                          uint8_t* __restrict__ ws) {
+  extern __shared__ __align__(16) uint8_t fb8[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int R = T * M.top_k;
+  const int used = reinterpret_cast<const int*>(ws + M.o_base)[M.E - 1] + reinterpret_cast<const int*>(ws + M.o_count)[M.E - 1];
+  const int slot0 = (blockIdx.x * MIDW_WARPS + warp) * MIDW_ROWS;
+  if (slot0 >= used) return;
+  const int nrow = min(MIDW_ROWS, used - slot0);
+  const int inter = M.inter, w13_out = M.w13_out, kch = M.kch13;
+  float* sm = reinterpret_cast<float*>(fb8 + warp * moe_midw_warp_bytes(w13_out));
+  __half* h13 = reinterpret_cast<__half*>(sm + FHT_CHUNK_WORDS);          // [row][w13_out]
+  int ex[MIDW_ROWS];
+  float wsc[MIDW_ROWS];
+  int2 tr[MIDW_ROWS];
+#pragma unroll
+  for (int r = 0; r < MIDW_ROWS; ++r) {
+    const int slot = slot0 + min(r, nrow - 1);
+    ex[r] = reinterpret_cast<const int*>(ws + M.o_route_exp)[slot];
+    wsc[r] = M.w13_wscale[ex[r]];
+    tr[r] = M.gemm ? reinterpret_cast<const int2*>(ws + M.o_trow)[slot] : make_int2(0, 0);
+  }
+  const long long kstride = (long long)R * w13_out;
+  const float* part1 = reinterpret_cast<const float*>(ws + M.o_part1) + (long long)slot0 * w13_out + (lane << 2);
+  // -- output transform of w13, chunk by chunk (chunk c of block b holds values c << 10 .. of the block's rows)
+  auto load = [&](int b, int c, f2 (&v)[8][2]) {
+    const int logbs = M.log_m13[b], mask = (1 << logbs) - 1;
+    const float* src = part1 + M.off_m13[b];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int e = (c << 10) | (k << 7), r = (e | (lane << 2)) >> logbs;
+      v[k][0] = v[k][1] = 0;
+      if (r < nrow) {
+        // (a block of less than 128 values: the row changes within the warp's 128 values)
+        const float* p = src + (logbs >= 7 ? r * w13_out + (e & mask) : r * w13_out + ((e | (lane << 2)) & mask) - (lane << 2));
+        ulonglong2 t = __ldcg(reinterpret_cast<const ulonglong2*>(p));
+        v[k][0] = t.x; v[k][1] = t.y;
+        for (int s = 1; s < kch; ++s) {
+          t = __ldcg(reinterpret_cast<const ulonglong2*>(p + s * kstride));
+          v[k][0] = f2_add(v[k][0], t.x);
+          v[k][1] = f2_add(v[k][1], t.y);
+        }
+      }
+    }
+  };
+  int b = 0, c = 0;
+  f2 nxt[8][2];
+  load(0, 0, nxt);
+  while (b < M.nb_m13) {
+    const int logbs = M.log_m13[b], off = M.off_m13[b], mask = (1 << logbs) - 1, base = c << 10;
+    f2 v[8][2];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { v[k][0] = nxt[k][0]; v[k][1] = nxt[k][1]; }
+    if (++c >= moe_chunks(MIDW_ROWS, logbs)) { c = 0; ++b; }
+    if (b < M.nb_m13) load(b, c, nxt);
+    fht_warp(sm, v, logbs);
+    const float rs = rsqrtf((float)(1 << logbs));
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int e = base | (k << 7) | (lane << 2), r = e >> logbs, col = off + (e & mask);
+      if (r < nrow) {
+        f2 p[2], sg[2];
+        float f[4];
+        fht_ld4(sm + (lane << 2) + k * 132, p);
+        load_sign4(M.w13_su + (long long)(r ? ex[1] : ex[0]) * w13_out + col, sg);
+        const float sc = rs * (r ? wsc[1] : wsc[0]);
+        const f2 sc2 = f2_pack(sc, sc);
+        f2_unpack(f2_mul(f2_mul(p[0], sc2), sg[0]), f[0], f[1]);
+        f2_unpack(f2_mul(f2_mul(p[1], sc2), sg[1]), f[2], f[3]);
+        const __half2 lo = __floats2half2_rn(f[0], f[1]), hi = __floats2half2_rn(f[2], f[3]);
+        *reinterpret_cast<uint2*>(h13 + r * w13_out + col) =
+            make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+      }
+    }
+    __syncwarp();
+  }
+  // -- gated activation (fp16), SV and the input transform of w2
+  const int kchunks = inter / GM_TILE_K;
+  uint8_t* xr2 = ws + M.o_xr2;
+  __half2* xs2 = reinterpret_cast<__half2*>(xr2) + (long long)slot0 * inter;
+  const bool gated = M.gated != 0, gemm = M.gemm != 0;
+  auto unpack4 = [](const __half* p, float (&f)[4]) {
+    const uint2 t = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&t.x)), d = __half22float2(*reinterpret_cast<const __half2*>(&t.y));
+    f[0] = a.x; f[1] = a.y; f[2] = d.x; f[3] = d.y;
+  };
+  for (int b2 = 0; b2 < M.nb_n2; ++b2) {
+    const int logbs = M.log_n2[b2], off = M.off_n2[b2], mask = (1 << logbs) - 1;
+    const float rs = rsqrtf((float)(1 << logbs));
+    const f2 rs2 = f2_pack(rs, rs);
+    for (int c2 = 0; c2 < moe_chunks(MIDW_ROWS, logbs); ++c2) {
+      f2 v[8][2];
+      with_act(M.act, [&](auto act) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int e = (c2 << 10) | (k << 7) | (lane << 2), r = e >> logbs, col = off + (e & mask);
+          v[k][0] = v[k][1] = 0;
+          if (r < nrow) {
+            float g[4], u[4] = {1.f, 1.f, 1.f, 1.f};
+            f2 sv[2];
+            unpack4(h13 + r * w13_out + col, g);
+            if (gated) unpack4(h13 + r * w13_out + inter + col, u);
+            load_sign4(M.w2_sv + col, sv);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) g[j] = round_half(moe_act(g[j], decltype(act)::value) * u[j]);
+            v[k][0] = f2_mul(f2_pack(g[0], g[1]), sv[0]);
+            v[k][1] = f2_mul(f2_pack(g[2], g[3]), sv[1]);
+          }
+        }
+      });
+      fht_warp(sm, v, logbs);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int e = (c2 << 10) | (k << 7) | (lane << 2), r = e >> logbs, col = off + (e & mask);
+        if (r < nrow) {
+          f2 q[2];
+          fht_ld4(sm + (lane << 2) + k * 132, q);
+          const f2 o[2] = {f2_mul(q[0], rs2), f2_mul(q[1], rs2)};
+          if (gemm) *reinterpret_cast<uint2*>(moe_tile_at(xr2, r ? tr[1] : tr[0], kchunks, col)) = pack4_half(o);
+          else moe_store_xr4(xs2 + r * inter, col, o);
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
 // ---- 6: per token weighted combine ------------------------------------------------------------------------
 // The routings of a token are the rows of the transform (`rg` at a time), 1024 values per warp; a thread then owns groups
 // of four output columns, 1024 apart within a block, does the stages beyond the chunks and adds the routings' results
@@ -846,7 +1005,7 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_out_kernel(const __grid
                                                                     const float* __restrict__ topk_w,
                                                                     const uint8_t* __restrict__ ws, uint8_t* __restrict__ y) {
   extern __shared__ __align__(16) float fb[];   // chunks of rg rows of hidden (+ hidden floats when several passes are needed)
-  const int t = blockIdx.x;
+  const int t = blockIdx.x, lane = threadIdx.x & 31;
   const int R = T * M.top_k;
   const int* slot_of = reinterpret_cast<const int*>(ws + M.o_slot_of);
   const int* route_exp = reinterpret_cast<const int*>(ws + M.o_route_exp);
@@ -869,11 +1028,31 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_out_kernel(const __grid
   const bool y_vec = act_rows_aligned4(y, 0, hidden, M.y_dtype);
   for (int j0 = 0; j0 < M.top_k; j0 += rg) {
     const int nrow = min(rg, M.top_k - j0);
+    if (kch == 1) {
+      // one partial sum per value: all chunks of a warp travel at once, each lane to where it will read them
+      for (int ch = threadIdx.x >> 5; ch < n2; ch += MOE_XF_THREADS / 32) {
+        int base;
+        const int b = moe_chunk_block(ch, rg, M.nb_m2, M.log_m2, base), logbs = M.log_m2[b];
+        const int e = ((ch - base) << 10) | (lane << 2), i0 = M.off_m2[b] + (e & ((1 << logbs) - 1));
+        float* dst = fb + ch * FHT_CHUNK_WORDS + (lane << 2);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = (e >> logbs) + fht_row(k, 128, logbs);
+          const long long o = r < nrow ? row_off[j0 + r] : -1;
+          if (o >= 0) cp_async16(dst + k * 132, part2 + o + i0 + fht_col(k, 128, logbs));
+          else *reinterpret_cast<float4*>(dst + k * 132) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+      asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    }
     for (int ch = threadIdx.x >> 5; ch < n2; ch += MOE_XF_THREADS / 32) {
       int base;
       const int b = moe_chunk_block(ch, rg, M.nb_m2, M.log_m2, base);
       f2 v[8][2];
-      moe_load_chunk(v, ch - base, M.log_m2[b], nrow, part2 + M.off_m2[b], kch, kstride,
+      if (kch == 1) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) fht_ld4(fb + ch * FHT_CHUNK_WORDS + (lane << 2) + k * 132, v[k]);
+      } else moe_load_chunk(v, ch - base, M.log_m2[b], nrow, part2 + M.off_m2[b], kch, kstride,
                      [&](int r) -> long long { return row_off[j0 + r]; });
       fht_warp(fb + ch * FHT_CHUNK_WORDS, v, M.log_m2[b]);
     }
@@ -952,6 +1131,7 @@ struct GlqbMoePlan {
   MoeMvKernel k13 = nullptr, k2 = nullptr;
   int grid13 = 0, grid2 = 0;
   int mid_sg = 1, out_rg = 1;          // slots per CTA of the mid kernel, routings per pass of the combine
+  bool mid_warp = false;               // moe_mid_warp_kernel instead of moe_mid_kernel
   size_t mid_smem = 0, out_smem = 0;
   // tensor-core form
   bool gemm_ok = false, two_stages = false;
@@ -1010,12 +1190,15 @@ static int fill_blocks(const int32_t* blocks, int nb, int total, int* off, int* 
   return GLQB_OK;
 }
 
-// grouping: one CTA for small steps; count / tables / place kernels (many CTAs) for large ones
+// grouping: one launch; count / tables / place kernels (many CTAs) for steps in which counting all routings in every CTA
+// would take longer than three launches.  128 experts, top 8, one CTA or three launches / one launch of many: 256 tokens
+// 24 / 19 us, 4096 tokens 56 / 25 us (cold, by ncu).
 static void moe_launch_group(const MoeDev& M, const void* ids, int tokens, uint8_t* ws, cudaStream_t st) {
   const int R = tokens * M.top_k;
-  const size_t sh = (5 * (size_t)M.E + 1) * sizeof(int);
+  const size_t sh = (6 * (size_t)M.E + 1) * sizeof(int);
   if (R < MOE_GROUP_SPLIT_MIN) {
-    moe_group_kernel<<<1, 1024, sh, st>>>(M, ids, tokens, ws, 0);
+    const int ctas = std::max(1, std::min(MOE_GROUP_CTAS, (R + MOE_GROUP_SHARE - 1) / MOE_GROUP_SHARE));
+    moe_group_kernel<<<ctas, 1024, sh, st>>>(M, ids, tokens, ws, 0);
     return;
   }
   const int nb = (R + MOE_GROUP_CHUNK - 1) / MOE_GROUP_CHUNK;
@@ -1023,6 +1206,12 @@ static void moe_launch_group(const MoeDev& M, const void* ids, int tokens, uint8
   moe_count_kernel<<<nb, 1024, M.E * sizeof(int), st>>>(M, ids, tokens, ws);
   moe_group_kernel<<<1, 1024, sh, st>>>(M, ids, tokens, ws, 1);
   moe_place_kernel<<<nb, 1024, 2 * M.E * sizeof(int), st>>>(M, ids, tokens, ws);
+}
+
+static void moe_launch_mid(const GlqbMoePlan* P, const MoeDev& M, int tokens, uint8_t* ws, cudaStream_t st) {
+  const int R = tokens * M.top_k, per = P->mid_warp ? MIDW_ROWS * MIDW_WARPS : P->mid_sg;
+  if (P->mid_warp) moe_mid_warp_kernel<<<(R + per - 1) / per, MIDW_WARPS * 32, P->mid_smem, st>>>(M, tokens, ws);
+  else moe_mid_kernel<<<(R + per - 1) / per, MOE_XF_THREADS, P->mid_smem, st>>>(M, tokens, per, ws);
 }
 
 // tokens per CTA of the input transform: one tile of 8192 values, fewer when that would leave SMs without work
@@ -1197,14 +1386,18 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
     // (running sums between passes are only needed when one pass cannot hold all routings of a token)
     while (P->out_rg > 1 && out_bytes(P->out_rg) > budget) --P->out_rg;
     P->mid_smem = mid_bytes(P->mid_sg);
+    P->mid_warp = !M.wide_m13 && MIDW_WARPS * moe_midw_warp_bytes(d->w13_out) <= limit;
+    for (int b = 0; b < M.nb_n2; ++b) P->mid_warp = P->mid_warp && M.log_n2[b] <= 10;
+    if (P->mid_warp) P->mid_smem = MIDW_WARPS * moe_midw_warp_bytes(d->w13_out);
     P->out_smem = out_bytes(P->out_rg);
     if (P->mid_smem > limit || P->out_smem > limit) {
       delete P;
       return moe_fail(GLQB_E_INVALID, "moe_plan_create: one row of the expert transforms needs more than %zu bytes of shared memory", limit);
     }
     if (cudaFuncSetAttribute(moe_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)((5 * 4096 + 1) * sizeof(int))) != cudaSuccess ||
+                             (int)((6 * 4096 + 1) * sizeof(int))) != cudaSuccess ||
         cudaFuncSetAttribute(moe_mid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit) != cudaSuccess ||
+        cudaFuncSetAttribute(moe_mid_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit) != cudaSuccess ||
         cudaFuncSetAttribute(moe_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit) != cudaSuccess) {
       delete P;
       return moe_fail(GLQB_E_CUDA, "moe_plan_create: %s", cudaGetErrorString(cudaGetLastError()));
@@ -1265,7 +1458,7 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
           reinterpret_cast<const DevLinear*>(ws + G.o_layers13), reinterpret_cast<const GemmItem*>(ws + G.o_items13),
           G.max_items13, ws, status, nitems, tokens);
     }
-    moe_mid_kernel<<<(R + P->mid_sg - 1) / P->mid_sg, MOE_XF_THREADS, P->mid_smem, st>>>(G, tokens, P->mid_sg, ws);
+    moe_launch_mid(P, G, tokens, ws, st);
     {
       MoeTimer t(P, st);
       P->g2<<<std::min(P->sm_count, G.max_items2), g_threads, moe_gemm_smem_bytes(g_e8), st>>>(
@@ -1300,7 +1493,7 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
     MoeTimer t(P, st);
     P->k13<<<P->grid13, MV_THREADS, 0, st>>>(A);
   }
-  moe_mid_kernel<<<(R + P->mid_sg - 1) / P->mid_sg, MOE_XF_THREADS, P->mid_smem, st>>>(M, tokens, P->mid_sg, ws);
+  moe_launch_mid(P, M, tokens, ws, st);
   A.codes[0] = M.w2[0]; A.codes[1] = M.w2[1]; A.stride[0] = M.w2_stride[0]; A.stride[1] = M.w2_stride[1];
   A.inv2 = M.w2_inv2;
   A.row_map = nullptr;

@@ -260,3 +260,23 @@ def test_moe_even_tiles():
     ref = _oracle(d, x_t.float().cpu().numpy(), ids, w, E, hidden, inter, w13_out, 4, 0, O.ACT_CODES[1])
     ops.clear_caches()
     assert np.abs(y.float().cpu().numpy() - ref).max() <= 5e-3 * np.abs(ref).max()
+
+
+# routings around the share of a grouping CTA (256), of many CTAs (32 x 256), and past the one-launch form (65536): a token's
+# result does not depend on the tokens around it.  inter 736 = 512 + 128 + 64 + 32: blocks of fewer values than a warp's chunk.
+@pytest.mark.parametrize("T", [127, 128, 129, 4096, 4097, 32767, 32768])
+def test_moe_grouping_sizes(T, monkeypatch):
+    from glq_b200 import ops
+    monkeypatch.setenv("GLQB_MOE_GEMM_MIN_AVG", "0")
+    E, hidden, inter, k = 8, 128, 736 if T < 5000 else 64, 2
+    rng = np.random.default_rng(T)
+    d, w13_out = _make(rng, E, hidden, inter, 4, 0)
+    x_t = cuda(rng.standard_normal((T, hidden)).astype(np.float32), torch.float16)
+    ids = np.argsort(rng.random((T, E)), axis=1)[:, :k].astype(np.int64)
+    w = cuda(rng.random((T, k)).astype(np.float32))
+    run = lambda a, b: _run(ops, d, x_t[a:b].contiguous(), cuda(ids[a:b]), w[a:b].contiguous(), E, hidden, inter, w13_out, 0, 1)
+    ops.clear_caches()
+    y = run(0, T)
+    cut = T // 2 + 3
+    assert torch.equal(y, torch.cat([run(0, cut), run(cut, T)]))
+    ops.clear_caches()
