@@ -641,7 +641,9 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
 // through 512 bytes of shared memory so that lane (c, k) gets index k of chunk c, row after row: a row's four decoded
 // 128-byte tile rows are then one store of whole lines (a thread per row, 16 bytes of 32 different lines per store
 // instruction, spent more of the L1 pipe on stores than on the gathers).  8 x NS gathers are in flight per lane.
-// Bound by the gathers; two stages of 14336 x 4096 94 -> 57 us, three of 5376 x 21504 (resident) 157 -> 124 us.
+// Bound by the gathers and the expansion, which alternate row by row: the entries of a unit are requested while the unit
+// before it is expanded.  All of a unit's gathers first / this: whole calls of 2048 tokens of 14336 x 4096 346 / 336 us, of
+// 700 tokens of 5376 x 21504 (three stages, resident) 313 / 301 us.
 // TM = 0: table gathers from global memory.  TM = 1: most of the table resident in shared memory (see e8_gather), one
 // CTA per SM.
 constexpr int E8T_ROWS = 8;
@@ -692,26 +694,40 @@ __device__ __forceinline__ void e8_tiles_body(const DevLinear* __restrict__ laye
         }
       }
     };
-    if (warp0 < units) fetch(warp0);
-    for (int u = warp0; u < units; u += warps) {
-      const int r8 = u % (GM_TILE_M / E8T_ROWS), t = u / (GM_TILE_M / E8T_ROWS);
-      const int mt = t / kgroups, kc = (t - mt * kgroups) * 4 + c;
-      const int row0 = r8 * E8T_ROWS;                             // first row inside the tile
-      uint32_t ent[NS][E8T_ROWS];
+    // the indices in `nxt`, two rows per register, for lane (c, k)
+    uint32_t ix[NS][E8T_ROWS / 2], ent[NS][E8T_ROWS];
+    auto turn = [&]() {
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
         buf[lane] = nxt[s];
         __syncwarp();
 #pragma unroll
-        for (int r = 0; r < E8T_ROWS; ++r) ent[s][r] = mine[r * 32];
+        for (int r = 0; r < E8T_ROWS; r += 2) ix[s][r >> 1] = (uint32_t)mine[r * 32] | ((uint32_t)mine[r * 32 + 32] << 16);
         __syncwarp();
       }
-      if (u + warps < units) fetch(u + warps);
+    };
+    auto gather = [&](int r) {
 #pragma unroll
-      for (int s = 0; s < NS; ++s)
+      for (int s = 0; s < NS; ++s) ent[s][r] = e8_gather<TM, E8T_RESIDENT>(stg[s], (ix[s][r >> 1] >> ((r & 1) * 16)) & stg[s].mask);
+    };
+    if (warp0 < units) {
+      fetch(warp0);
+      turn();
+      if (warp0 + warps < units) fetch(warp0 + warps);
 #pragma unroll
-        for (int r = 0; r < E8T_ROWS; ++r) ent[s][r] = e8_gather<TM, E8T_RESIDENT>(stg[s], ent[s][r] & stg[s].mask);
-      if (kc >= kchunks) continue;
+      for (int r = 0; r < E8T_ROWS; ++r) gather(r);
+    }
+    for (int u = warp0; u < units; u += warps) {
+      // (the entries of row r of the next unit are requested as soon as row r of this one is expanded: gathers and arithmetic
+      // alternate, and a unit's gathers have the arithmetic of another one to arrive)
+      const bool more = u + warps < units;
+      if (more) {
+        turn();
+        if (u + 2 * warps < units) fetch(u + 2 * warps);
+      }
+      const int r8 = u % (GM_TILE_M / E8T_ROWS), t = u / (GM_TILE_M / E8T_ROWS);
+      const int mt = t / kgroups, kc = (t - mt * kgroups) * 4 + c;
+      const int row0 = r8 * E8T_ROWS;                             // first row inside the tile
       const bool col_ok = kc * 8 + k < nidx;
       uint8_t* tile = tiles + ((size_t)mt * kchunks + kc) * GM_A_BYTES + row0 * 128;
 #pragma unroll
@@ -736,7 +752,8 @@ __device__ __forceinline__ void e8_tiles_body(const DevLinear* __restrict__ laye
           out.z = __byte_perm(h[0], h[1], 0x7632);
           out.w = __byte_perm(h[2], h[3], 0x7632);
         }
-        *reinterpret_cast<uint4*>(tile + r * 128 + ((k ^ r) << 4)) = out;        // (sw128_offset; row0 is a multiple of 8)
+        if (kc < kchunks) *reinterpret_cast<uint4*>(tile + r * 128 + ((k ^ r) << 4)) = out;  // (sw128_offset; row0 is a multiple of 8)
+        if (more) gather(r);
       }
     }
   }
