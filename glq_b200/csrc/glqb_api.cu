@@ -270,29 +270,36 @@ static int tn_for_batch(int batch, bool codes) {
 // takes, in 64-column chunks (about 0.3 us each), plus the fp32 partial sums it writes and reads back at 5 TB/s.
 // Splits for as many items as SMs, rounded up / by this rule, with the tokens rounded up to 512 / taken as they are: 333
 // tokens of 2048 x 11008 80 / 43 us (192 items in two rounds of 148 / 128 in one).
+//
+// trellis_gemm_kernel may take two token tiles per item and decode their weights once; a chunk of such an item takes about 1.6
+// times as long as one tile's (experts of two tiles of 128 tokens: 270 us a tile at a time, 215 us two), and there are half as
+// many items: the same costs decide.
 static void gemm_schedule(Segment& s, int limit, int sm_count, std::vector<DevLinear>& dev, std::vector<GemmItem>& items) {
   auto tokens_of = [&](const DevLinear& L) { return std::min(L.batch, limit); };
   auto tile_of = [&](const DevLinear& L) { return trellis_form(s) ? tile_tokens(tokens_of(L)) : s.tn; };
   auto splits = [](int kchunks, int ks, int& per) { per = (kchunks + ks - 1) / ks; return (kchunks + per - 1) / per; };
   int best = 1;
+  bool pairs = false;                            // an item takes two token tiles
   double best_cost = 0;
-  for (int ks = 1; ks <= 16; ++ks) {
-    long long n = 0;
-    int longest = 0, per = 0;
-    double sums = 0;
-    bool ok = true;
-    for (int i = 0; i < s.count; ++i) {
-      const DevLinear& L = dev[s.first + i];
-      const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K;
-      ok = ok && ks <= std::max(1, kchunks / 8);
-      const int k = splits(kchunks, ks, per);
-      longest = std::max(longest, per);
-      n += (long long)((L.m + GM_TILE_M - 1) / GM_TILE_M) * ((tokens_of(L) + tile_of(L) - 1) / tile_of(L)) * k;
-      sums += (double)k * tokens_of(L) * L.m;
+  for (int ks = 1; ks <= 16; ++ks)
+    for (int two = 0; two <= (trellis_form(s) ? 1 : 0); ++two) {
+      long long n = 0;
+      int longest = 0, per = 0;
+      double sums = 0;
+      bool ok = true, paired = false;
+      for (int i = 0; i < s.count; ++i) {
+        const DevLinear& L = dev[s.first + i];
+        const int kchunks = (L.n + GM_TILE_K - 1) / GM_TILE_K, n_tiles = (tokens_of(L) + tile_of(L) - 1) / tile_of(L);
+        ok = ok && ks <= std::max(1, kchunks / 8);
+        const int k = splits(kchunks, ks, per);
+        longest = std::max(longest, per);
+        n += (long long)((L.m + GM_TILE_M - 1) / GM_TILE_M) * (two ? (n_tiles + 1) / 2 : n_tiles) * k;
+        sums += (double)k * tokens_of(L) * L.m;
+        paired = paired || (two && n_tiles > 1);
+      }
+      const double cost = (double)((n + sm_count - 1) / sm_count) * longest * (paired ? 1.6 : 1.0) + sums * 8 / 5e12 / 0.3e-6;
+      if ((ks == 1 && !two) || (ok && cost < best_cost)) { best = ks; pairs = two; best_cost = cost; }
     }
-    const double cost = (double)((n + sm_count - 1) / sm_count) * longest + sums * 8 / 5e12 / 0.3e-6;
-    if (ks == 1 || (ok && cost < best_cost)) { best = ks; best_cost = cost; }
-  }
   s.item_first = (int)items.size();
   for (int i = 0; i < s.count; ++i) {
     DevLinear& L = dev[s.first + i];
@@ -300,9 +307,9 @@ static void gemm_schedule(Segment& s, int limit, int sm_count, std::vector<DevLi
     int per;
     L.fixed_slots = splits(kchunks, std::min(best, std::max(1, kchunks / 8)), per);
     for (int mt = 0; mt < (L.m + GM_TILE_M - 1) / GM_TILE_M; ++mt)
-      for (int nt = 0; nt < n_tiles; ++nt)
+      for (int nt = 0; nt < n_tiles; nt += pairs ? 2 : 1)
         for (int k = 0; k < L.fixed_slots; ++k)
-          items.push_back(GemmItem{s.first + i, mt, nt, k * per, std::min(kchunks, (k + 1) * per), k, 0, 0, 0});
+          items.push_back(GemmItem{s.first + i, mt, nt, k * per, std::min(kchunks, (k + 1) * per), k, 0, 0, 0, pairs && nt + 1 < n_tiles});
   }
   s.item_count = (int)items.size() - s.item_first;
   s.grid = std::min(s.item_count, sm_count);

@@ -39,6 +39,7 @@ struct GemmItem {
   int slot;        // partial-sum slot this item writes
   int tok0, ntok;  // lists built on the device (grouped experts): first token and tokens of the tile inside its layer,
   int row0;        // and the 128-byte rows of activations in front of it; other lists: see tile_tokens and glq_gemm_kernel
+  int ntok2;       // trellis_gemm_kernel: tokens of the tile behind it, which the item takes as well (other lists: 1), or 0
 };
 
 // Token tiles of the layers whose codes are decoded in the GEMM (trellis_gemm_kernel): as few as possible of at most 192

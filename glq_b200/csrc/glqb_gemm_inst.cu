@@ -60,7 +60,7 @@ static GemmKernel pick_gemm_kernel(const Segment& s) {
 #endif
       return nullptr;
     }
-#define G_CASE(A, B) if (s.k1 == A && s.k2 == B) return trellis_gemm_kernel<A, B>;
+#define G_CASE(A, B) if (s.k1 == A && s.k2 == B) return trellis_gemm_kernel<A, B, TG_TN>;
 #ifdef GLQB_FAST_BUILD   /* developer builds for kernel experiments: the 4-bit single-stage rate only */
     G_CASE(4, 0)
 #else
@@ -84,7 +84,7 @@ static size_t gemm_smem_bytes(int tn) {
 }
 
 
-static size_t segment_smem(const Segment& s) { return trellis_form(s) ? (size_t)TG_SMEM_BYTES : gemm_smem_bytes(s.tn); }
+static size_t segment_smem(const Segment& s) { return trellis_form(s) ? (size_t)TgShape<TG_TN>::SMEM_BYTES : gemm_smem_bytes(s.tn); }
 
 bool gemm_available(const Segment& s) { return pick_gemm_kernel(s) != nullptr; }
 

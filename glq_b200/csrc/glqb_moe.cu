@@ -23,7 +23,7 @@
 // Steps with enough routed tokens per expert (moe_gemm_min_avg) take the tensor-core form instead, E8 experts always:
 // launches 3 and 5 become trellis_gemm_kernel (E8: glq_gemm_kernel) over a work list that the grouping kernel builds
 // on the device from the expert counts — every expert is a "layer" whose token count, activation tiles and
-// partial-sum rows are patched in each run; an expert's routings are split evenly over tiles of at most 192, each
+// partial-sum rows are patched in each run; an expert's routings are split evenly over tiles of at most 160 (E8: 192), each
 // padded to a multiple of 16.  The transforms write the activations straight into the swizzled tile images the GEMM's
 // bulk copies fetch.
 #include <algorithm>
@@ -59,7 +59,7 @@ struct MoeDev {
   // workspace offsets (bytes)
   long long o_count, o_base, o_cursor, o_work, o_route_tok, o_route_exp, o_slot_of, o_xr1, o_part1, o_xr2, o_part2;
   // tensor-core form (gemm != 0): tile rows, device-built layer tables and work lists
-  int gemm, k13a, k13b, k2a, k2b, max_items13, max_items2;
+  int gemm, tile_tn, k13a, k13b, k2a, k2b, max_items13, max_items2;
   long long o_trow, o_row0, o_layers13, o_layers2, o_items13, o_items2, o_nitems, o_status;
   // E8 shell experts (format == GLQB_FMT_E8_SHELL; tensor-core form only): index matrices per stage,
   // expert-stacked, the packed tables, and the per-expert cumulative inverse residual scales of stages 2, 3
@@ -72,24 +72,26 @@ struct MoeDev {
   const float* e8_w2_inv[2];
 };
 
-// Routed tokens per GEMM tile: an expert's tokens are split evenly over ceil(count / MOE_TN) tiles, each padded to 16.
-constexpr int MOE_TN = TG_TN;
-__device__ __forceinline__ int moe_tile_tokens(int cnt) {           // tokens of an expert's tiles but the last
-  const int n = max(1, (cnt + MOE_TN - 1) / MOE_TN);
+// Routed tokens per GEMM tile: an expert's tokens are split evenly over ceil(count / tn) tiles, each padded to 16.  Trellis
+// experts: 160, of which an item takes two, so that 320 tokens are one pass over the weights and tensor memory has a third
+// stage of weights; E8 experts: 192.
+constexpr int MOE_TN = 160, MOE_TN_E8 = 192;
+__device__ __forceinline__ int moe_tile_tokens(int cnt, int tn) {           // tokens of an expert's tiles but the last
+  const int n = max(1, (cnt + tn - 1) / tn);
   return max(16, ((cnt + n - 1) / n + 15) & ~15);
 }
-__device__ __forceinline__ int moe_tile_count(int cnt) {
-  const int tt = moe_tile_tokens(cnt);
+__device__ __forceinline__ int moe_tile_count(int cnt, int tn) {
+  const int tt = moe_tile_tokens(cnt, tn);
   return (cnt + tt - 1) / tt;
 }
-__device__ __forceinline__ int moe_tile_rows(int cnt) {             // 128-byte activation rows of an expert's tiles, per chunk
-  const int n = moe_tile_count(cnt);
-  return n ? (n - 1) * moe_tile_tokens(cnt) + ((cnt - (n - 1) * moe_tile_tokens(cnt) + 15) & ~15) : 0;
+__device__ __forceinline__ int moe_tile_rows(int cnt, int tn) {             // 128-byte activation rows of an expert's tiles, per chunk
+  const int n = moe_tile_count(cnt, tn), tt = moe_tile_tokens(cnt, tn);
+  return n ? (n - 1) * tt + ((cnt - (n - 1) * tt + 15) & ~15) : 0;
 }
 // where routing number i of an expert (activation rows from `row0` on) has its row: rows in front of its tile, and
 // rows of the tile << 16 | row inside it
-__device__ __forceinline__ int2 moe_tile_place(int cnt, int row0, int i) {
-  const int tt = moe_tile_tokens(cnt), j = i / tt, left = cnt - j * tt;
+__device__ __forceinline__ int2 moe_tile_place(int cnt, int tn, int row0, int i) {
+  const int tt = moe_tile_tokens(cnt, tn), j = i / tt, left = cnt - j * tt;
   return make_int2(row0 + j * tt, (left >= tt ? tt : (left + 15) & ~15) << 16 | (i - j * tt));
 }
 
@@ -172,7 +174,7 @@ __global__ void __launch_bounds__(1024) moe_place_kernel(const __grid_constant__
         slot = atomicAdd(&cur[ev[u]], 1);
         route_tok[slot] = i / M.top_k;
         route_exp[slot] = ev[u];
-        if (M.gemm) trow[slot] = moe_tile_place(g_count[ev[u]], g_row0[ev[u]], slot - g_base[ev[u]]);
+        if (M.gemm) trow[slot] = moe_tile_place(g_count[ev[u]], M.tile_tn, g_row0[ev[u]], slot - g_base[ev[u]]);
       }
       slot_of[i] = slot;
     }
@@ -195,6 +197,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
   int* route_exp = reinterpret_cast<int*>(ws + M.o_route_exp);
   int* slot_of = reinterpret_cast<int*>(ws + M.o_slot_of);
   const int R = T * M.top_k;
+  const int per_item = M.format == GLQB_FMT_E8_SHELL ? 1 : 2;        // token tiles of a work item
   const int share = (R + (int)gridDim.x - 1) / (int)gridDim.x, lo = (int)blockIdx.x * share, hi = min(R, lo + share);
   const int tid = (int)(blockIdx.x * blockDim.x + threadIdx.x), step = (int)(gridDim.x * blockDim.x);
   for (int e = threadIdx.x; e < M.E; e += blockDim.x) cnt[e] = front[e] = 0;
@@ -224,7 +227,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
     int run = 0, tiles = 0, rows = 0;
     for (int e0 = 0; e0 < M.E; e0 += 32) {
       const int e = e0 + threadIdx.x, c = e < M.E ? cnt[e] : 0;
-      const int nt = moe_tile_count(c), nr = moe_tile_rows(c);
+      const int nt = (moe_tile_count(c, M.tile_tn) + per_item - 1) / per_item, nr = moe_tile_rows(c, M.tile_tn);
       int a = c, b = nt, d = nr;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -303,8 +306,8 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
     GemmItem* I13 = reinterpret_cast<GemmItem*>(ws + M.o_items13);
     GemmItem* I2 = reinterpret_cast<GemmItem*>(ws + M.o_items2);
     auto item = [&](int tile, int mt, int kc) -> GemmItem {
-      const int e = expert_of_tile(tile), j = tile - tile0[e], tt = moe_tile_tokens(cnt[e]);
-      return GemmItem{e, mt, j, 0, kc, 0, j * tt, min(tt, cnt[e] - j * tt), j * tt};
+      const int e = expert_of_tile(tile), j = (tile - tile0[e]) * per_item, tt = moe_tile_tokens(cnt[e], M.tile_tn), left = cnt[e] - j * tt;
+      return GemmItem{e, mt, j, 0, kc, 0, j * tt, min(tt, left), j * tt, per_item > 1 ? max(0, min(tt, left - tt)) : 0};
     };
     for (int idx = tid; idx < min(tiles * mt13, M.max_items13); idx += step) I13[idx] = item(idx / mt13, idx % mt13, kc13);
     for (int idx = tid; idx < min(tiles * mt2, M.max_items2); idx += step) I2[idx] = item(idx / mt2, idx % mt2, kc2);
@@ -323,7 +326,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__
           slot = atomicAdd(&cur[ev[u]], 1);
           route_tok[slot] = i / M.top_k;
           route_exp[slot] = ev[u];
-          if (M.gemm) trow[slot] = moe_tile_place(cnt[ev[u]], row0[ev[u]], slot - base_s[ev[u]]);
+          if (M.gemm) trow[slot] = moe_tile_place(cnt[ev[u]], M.tile_tn, row0[ev[u]], slot - base_s[ev[u]]);
         }
         slot_of[i] = slot;
       }
@@ -1091,22 +1094,22 @@ typedef void (*MoeGemmKernel)(const DevLinear*, const GemmItem*, int, uint8_t*, 
 // did.  8 experts, top 2, 4096 x 2048, two stages, four / three: 8 tokens 318 / 281 us, 1024 tokens 672 / 618.
 constexpr int MOE_GEMM_STAGES = 3;
 static MoeGemmKernel moe_gemm_pick(int k1, int k2) {
-#define M_CASE(A, B) if (k1 == A && k2 == B) return trellis_gemm_kernel<A, B>;
+#define M_CASE(A, B) if (k1 == A && k2 == B) return trellis_gemm_kernel<A, B, MOE_TN>;
   M_CASE(2, 0) M_CASE(3, 0) M_CASE(4, 0) M_CASE(4, 1) M_CASE(4, 2) M_CASE(4, 3) M_CASE(4, 4)
 #undef M_CASE
   return nullptr;
 }
 static MoeGemmKernel moe_gemm_pick_e8(int ns) {
   switch (ns) {
-    case 1: return glq_gemm_kernel<1, 1, 0, MOE_TN, MOE_GEMM_STAGES>;
-    case 2: return glq_gemm_kernel<1, 2, 0, MOE_TN, MOE_GEMM_STAGES>;
-    case 3: return glq_gemm_kernel<1, 3, 0, MOE_TN, MOE_GEMM_STAGES>;
+    case 1: return glq_gemm_kernel<1, 1, 0, MOE_TN_E8, MOE_GEMM_STAGES>;
+    case 2: return glq_gemm_kernel<1, 2, 0, MOE_TN_E8, MOE_GEMM_STAGES>;
+    case 3: return glq_gemm_kernel<1, 3, 0, MOE_TN_E8, MOE_GEMM_STAGES>;
   }
   return nullptr;
 }
 static size_t moe_gemm_smem_bytes(bool e8) {
-  if (!e8) return TG_SMEM_BYTES;
-  return (size_t)MOE_GEMM_STAGES * (GM_A_BYTES + (size_t)MOE_TN * 128) + (3 * MOE_GEMM_STAGES + 5) * 8 + 16 + 1024;
+  if (!e8) return TgShape<MOE_TN>::SMEM_BYTES;
+  return (size_t)MOE_GEMM_STAGES * (GM_A_BYTES + (size_t)MOE_TN_E8 * 128) + (3 * MOE_GEMM_STAGES + 5) * 8 + 16 + 1024;
 }
 // routed tokens per expert (average) from which the tensor-core form is used (measured, 128 experts, top 8, streaming /
 // tensor-core: 64 tokens 260 / 263 us, 128 tokens 283 / 264, 256 tokens 333 / 271, 512 tokens 518 / 325; at an average of 8:
@@ -1347,8 +1350,9 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
     MoeDev& G = P->devg;
     G = M;
     G.gemm = 1; G.kch13 = 1; G.kch2 = 1;
+    G.tile_tn = e8 ? MOE_TN_E8 : MOE_TN;
     G.k13a = k13a; G.k13b = k13b; G.k2a = k2a; G.k2b = k2b;
-    const size_t tiles = R / MOE_TN + M.E;
+    const size_t tiles = R / G.tile_tn + M.E;
     const size_t mt13 = (d->w13_out + GM_TILE_M - 1) / GM_TILE_M, mt2 = (d->hidden + GM_TILE_M - 1) / GM_TILE_M;
     G.max_items13 = (int)(tiles * mt13);
     G.max_items2 = (int)(tiles * mt2);

@@ -262,9 +262,10 @@ def test_moe_even_tiles():
     assert np.abs(y.float().cpu().numpy() - ref).max() <= 5e-3 * np.abs(ref).max()
 
 
-# routings around the share of a grouping CTA (256), of many CTAs (32 x 256), and past the one-launch form (65536): a token's
+# routings around the share of a grouping CTA (256), of many CTAs (32 x 256), and past the one-launch form (65536), experts
+# of about one and two token tiles (160 and 320): a token's
 # result does not depend on the tokens around it.  inter 736 = 512 + 128 + 64 + 32: blocks of fewer values than a warp's chunk.
-@pytest.mark.parametrize("T", [127, 128, 129, 4096, 4097, 32767, 32768])
+@pytest.mark.parametrize("T", [127, 128, 129, 640, 1281, 4096, 4097, 32767, 32768])
 def test_moe_grouping_sizes(T, monkeypatch):
     from glq_b200 import ops
     monkeypatch.setenv("GLQB_MOE_GEMM_MIN_AVG", "0")
