@@ -1013,12 +1013,12 @@ int glqb_plan_run_tokens(GlqbPlan* P, const void* x_base, void* y_base, int32_t 
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
   if (!P->items_in.empty()) {
-    rht_in_kernel<false><<<(unsigned)P->items_in.size(), RHT_THREADS, rht_smem(P->max_elems_in), stream>>>(
-        d_layers, P->d_items_in, reinterpret_cast<const uint8_t*>(x_base), ws, tokens);
+    launch_chained(true, rht_in_kernel<false>, (int)P->items_in.size(), RHT_THREADS, rht_smem(P->max_elems_in), stream, d_layers,
+                   P->d_items_in, reinterpret_cast<const uint8_t*>(x_base), ws, tokens);
   }
   if (!P->items_in_gemm.empty()) {
-    rht_in_gemm_kernel<<<(unsigned)P->items_in_gemm.size(), RHT_THREADS, rht_smem(P->max_elems_in), stream>>>(
-        d_layers, P->d_items_in_gemm, reinterpret_cast<const uint8_t*>(x_base), ws, tokens);
+    launch_chained(true, rht_in_gemm_kernel, (int)P->items_in_gemm.size(), RHT_THREADS, rht_smem(P->max_elems_in), stream, d_layers,
+                   P->d_items_in_gemm, reinterpret_cast<const uint8_t*>(x_base), ws, tokens);
   }
   if (P->timing) {
     while (P->ev.size() < P->ev_used + 2) {
@@ -1035,15 +1035,13 @@ int glqb_plan_run_tokens(GlqbPlan* P, const void* x_base, void* y_base, int32_t 
     } else if (s.tn) {
       gemm_launch(s, d_layers, d_gemm_items + s.item_first, ws, P->d_status, P->sm_count, tokens, stream);
     } else if (s.smem_table) {
-      pick_e8_smem_kernel(s)<<<s.grid, E8S_THREADS, E8S_SMEM_BYTES, stream>>>(
-          d_layers + s.first, s.count, s.total_groups, s.per_warp, ws, s.big_table, s.small_table, s.small_entries, tokens);
+      launch_chained(true, pick_e8_smem_kernel(s), s.grid, E8S_THREADS, E8S_SMEM_BYTES, stream, d_layers + s.first, s.count, s.total_groups,
+                     s.per_warp, ws, s.big_table, s.small_table, s.small_entries, tokens);
+    } else if (s.lut_table) {
+      trellis_lut_kernel(s.k1)<<<s.grid, MV_LUT_THREADS, MV_LUT_SMEM_BYTES, stream>>>(d_layers + s.first, s.count, s.total_groups,
+                                                                                     s.per_warp, ws, tokens);
     } else {
-      MvKernel kern = pick_kernel(s);
-      if (s.lut_table)
-        trellis_lut_kernel(s.k1)<<<s.grid, MV_LUT_THREADS, MV_LUT_SMEM_BYTES, stream>>>(d_layers + s.first, s.count, s.total_groups,
-                                                                                       s.per_warp, ws, tokens);
-      else
-        kern<<<s.grid, MV_THREADS, 0, stream>>>(d_layers + s.first, s.count, s.total_groups, s.per_warp, ws, tokens);
+      pick_kernel(s)<<<s.grid, MV_THREADS, 0, stream>>>(d_layers + s.first, s.count, s.total_groups, s.per_warp, ws, tokens);
     }
   }
   if (P->timing) {
@@ -1051,26 +1049,15 @@ int glqb_plan_run_tokens(GlqbPlan* P, const void* x_base, void* y_base, int32_t 
     P->ev_used += 2;
   }
   if (!P->items_out.empty()) {
-    // with programmatic stream serialization: behind the single-launch decode kernel its launch overlaps that
-    // kernel's tail (it waits for it before reading anything)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)P->items_out.size());
-    cfg.blockDim = dim3(RHT_THREADS);
-    cfg.dynamicSmemBytes = rht_smem(P->max_elems_out);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const DevLinear* dl = d_layers;
-    const RhtItem* di = P->d_items_out;
-    const uint8_t* cws = ws;
+    const int n_items = (int)P->items_out.size();
     uint8_t* yb = reinterpret_cast<uint8_t*>(y_base);
-    const float* none = nullptr;
-    if (out_plain(P, yb)) CUDA_TRY(cudaLaunchKernelEx(&cfg, rht_out_plain_kernel, dl, di, cws, yb, (int)tokens));
-    else CUDA_TRY(cudaLaunchKernelEx(&cfg, P->out_wide ? rht_out_kernel<true> : rht_out_kernel<false>, dl, di, cws, yb, none,
-                                     (int)tokens));
+    if (out_plain(P, yb)) {
+      CUDA_TRY(launch_chained(true, rht_out_plain_kernel, n_items, RHT_THREADS, rht_smem(P->max_elems_out), stream, d_layers, P->d_items_out, ws,
+                              yb, tokens));
+    } else {
+      CUDA_TRY(launch_chained(true, P->out_wide ? rht_out_kernel<true> : rht_out_kernel<false>, n_items, RHT_THREADS,
+                              rht_smem(P->max_elems_out), stream, d_layers, P->d_items_out, ws, yb, (const float*)nullptr, tokens));
+    }
   }
   CUDA_TRY(cudaGetLastError());
   return GLQB_OK;

@@ -55,7 +55,6 @@ void fused_launch(const Segment& s, const DevLinear* layers, const uint8_t* x_ba
   // Launched with programmatic stream serialization: when the previous kernel of the stream is another
   // single-launch decode kernel, this one's prologue (scheduling, table reads, the first weight loads) overlaps
   // its tail; the kernel itself waits (griddepcontrol.wait) before it reads activations or writes anything.
-  static const bool pdl = [] { const char* e = getenv("GLQB_PDL"); return !e || atoi(e) != 0; }();
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)s.grid);
   cfg.blockDim = dim3(MV_THREADS);
@@ -65,7 +64,7 @@ void fused_launch(const Segment& s, const DevLinear* layers, const uint8_t* x_ba
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
   FusedLayers T;
   memcpy(T.L, layers, sizeof(DevLinear) * (size_t)s.count);          // `layers`: the plan's HOST copy of the segment's entries
   CommDev C;

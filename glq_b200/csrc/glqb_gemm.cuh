@@ -162,6 +162,8 @@ static __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_gemm_kern
                                                                   const uint8_t* __restrict__ x_base,
                                                                   uint8_t* __restrict__ ws, int tokens) {
   extern __shared__ __align__(16) float fbuf[];
+  pdl_wait();
+  pdl_trigger();
   RhtItem it = items[blockIdx.x];
   if (!rht_item_trim(it, tokens)) return;
   const DevLinear& L = layers[it.layer];
@@ -314,8 +316,10 @@ template <int FORMAT, int K1, int K2, int TN, int STAGES>
 __global__ void __launch_bounds__(GM_THREADS, 1)
 glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict__ items, int n_items,
                 uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev, int tokens) {
-  // work lists built on the device (grouped expert matmul) pass their length through memory
-  if (n_items_dev) n_items = min(n_items, *n_items_dev);
+  pdl_trigger();
+  // work lists built on the device (grouped expert matmul) pass their length through memory; other lists and the weights are
+  // there before: then only the loader and the epilogue wait for the kernel before this one
+  if (n_items_dev) { pdl_wait(); n_items = min(n_items, *n_items_dev); }
   constexpr int B_BYTES = TN * 128;
   constexpr bool VAR = TN == 192;
   constexpr int TMEM_COLS = VAR ? 512 : 2 * TN;
@@ -541,6 +545,7 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
   } else if (warp == GM_LOAD_WARP) {
     // ------------------------------------------------------------------ activation loader
     if (lane == 0) {
+      pdl_wait();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -572,6 +577,7 @@ glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict
   }
   else {
     // ------------------------------------------------------------------ epilogue warps
+    pdl_wait();
     const int quarter = warp & 3;                          // TMEM lanes 32*quarter .. 32*quarter + 31
     uint32_t seq = 0;
     bool ok = true;
@@ -775,6 +781,7 @@ __global__ void __launch_bounds__(E8TS_THREADS, 1)
 e8_tiles_smem_kernel(const DevLinear* __restrict__ layers, int first, int count, uint8_t* __restrict__ ws,
                      const uint32_t* __restrict__ big_table, const uint32_t* __restrict__ small_table, int small_entries) {
   extern __shared__ __align__(16) uint32_t e8t_smem[];    // table, small table, 512 bytes of indices per warp
+  pdl_trigger();
   const uint4* src = reinterpret_cast<const uint4*>(big_table);
   uint4* dst = reinterpret_cast<uint4*>(e8t_smem);
   for (int i = threadIdx.x; i < E8T_RESIDENT / 4; i += blockDim.x) dst[i] = __ldg(src + i);
@@ -787,6 +794,7 @@ e8_tiles_smem_kernel(const DevLinear* __restrict__ layers, int first, int count,
   const int warp = threadIdx.x >> 5;
   e8_tiles_body<NS, 1>(layers, first, count, ws, T, blockIdx.x * (E8TS_THREADS / 32) + warp, gridDim.x * (E8TS_THREADS / 32),
                        reinterpret_cast<uint4*>(e8t_smem + E8T_RESIDENT + 256) + warp * 32);
+  pdl_wait();
 }
 
 // ---- decode once: trellis bit-streams -> swizzled fp16 weight tiles ------------------------------------------
@@ -800,6 +808,7 @@ template <int K1, int K2>
 __global__ void __launch_bounds__(TT_THREADS, 3)
 trellis_tiles_kernel(const DevLinear* __restrict__ layers, int first, int count, uint8_t* __restrict__ ws) {
   __shared__ __align__(1024) uint8_t slices[TT_THREADS / 32][4096];
+  pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int warp0 = blockIdx.x * (TT_THREADS / 32) + warp, warps = gridDim.x * (TT_THREADS / 32);
   const uint32_t slice = smem_u32(slices[warp]);
@@ -850,6 +859,7 @@ trellis_tiles_kernel(const DevLinear* __restrict__ layers, int first, int count,
       __syncwarp();
     }
   }
+  pdl_wait();                                    // (the decode itself needs nothing of the kernel before: the GEMM behind does)
 }
 
 }  // namespace glqb

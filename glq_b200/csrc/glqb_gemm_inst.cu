@@ -99,14 +99,14 @@ cudaError_t tiles_smem_prepare(int ns) {
 void gemm_launch(const Segment& s, const DevLinear* layers, const GemmItem* items, uint8_t* ws, int* status,
                  int sm_count, int tokens, cudaStream_t stream) {
   if (s.two_phase && s.format == GLQB_FMT_TRELLIS_3INST)
-    pick_trellis_tiles_kernel(s.k1, s.k2)<<<sm_count * 3, TT_THREADS, 0, stream>>>(layers, s.first, s.count, ws);
+    launch_chained(true, pick_trellis_tiles_kernel(s.k1, s.k2), sm_count * 3, TT_THREADS, 0, stream, layers, s.first, s.count, ws);
   else if (s.two_phase && s.smem_table)
-    pick_tiles_smem_kernel(s.ns)<<<sm_count, E8TS_THREADS, E8TS_SMEM_BYTES, stream>>>(
-        layers, s.first, s.count, ws, s.big_table, s.small_table, s.small_entries);
+    launch_chained(true, pick_tiles_smem_kernel(s.ns), sm_count, E8TS_THREADS, E8TS_SMEM_BYTES, stream, layers, s.first, s.count, ws,
+                   s.big_table, s.small_table, s.small_entries);
   else if (s.two_phase)
     pick_tiles_kernel(s.ns)<<<sm_count * 8, 256, 0, stream>>>(layers, s.first, s.count, ws);
-  pick_gemm_kernel(s)<<<s.grid, trellis_form(s) ? TG_THREADS : GM_THREADS, segment_smem(s), stream>>>(
-      layers, items, s.item_count, ws, status, nullptr, tokens);
+  launch_chained(true, pick_gemm_kernel(s), s.grid, trellis_form(s) ? TG_THREADS : GM_THREADS, segment_smem(s), stream, layers, items,
+                 s.item_count, ws, status, nullptr, tokens);
 }
 
 }  // namespace glqb

@@ -65,6 +65,15 @@ struct RhtItem {
                // the short factor applied while loading, so S CTAs share a long block without talking
 };
 
+#ifdef __CUDACC__
+// Programmatic dependent launch (launch_chained): `pdl_trigger` lets the next kernel of the stream start, `pdl_wait` waits
+// until the one before has completed and its writes are visible.  Every kernel launched that way has threads that wait before
+// the grid can end, so that "the one before has completed" holds for all kernels further back as well; the input transforms,
+// which lead a call, trigger after they have waited: what follows them may write to the workspace without waiting.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 // Stores the message glqb_last_error() returns for the calling thread (defined in glqb_api.cu).
 void set_error_message(const char* msg);
 

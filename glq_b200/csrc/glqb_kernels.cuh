@@ -626,6 +626,7 @@ e8_mv_smem_kernel(const DevLinear* __restrict__ layers, int n_layers, long long 
                   uint8_t* __restrict__ ws, const uint32_t* __restrict__ big_table,
                   const uint32_t* __restrict__ small_table, int small_entries, int tokens) {
   extern __shared__ __align__(16) uint32_t e8_smem[];
+  pdl_trigger();
   const uint4* src = reinterpret_cast<const uint4*>(big_table);
   uint4* dst = reinterpret_cast<uint4*>(e8_smem);
   for (int i = threadIdx.x; i < E8S_RESIDENT / 4; i += blockDim.x) dst[i] = __ldg(src + i);
@@ -635,6 +636,7 @@ e8_mv_smem_kernel(const DevLinear* __restrict__ layers, int n_layers, long long 
   T.table_base = local;
   T.small_base = local + E8S_RESIDENT * 4;
   __syncthreads();
+  pdl_wait();                                    // (the table fill overlaps the input transform)
   e8_mv_body<NS, NB, 1>(layers, n_layers, total_groups, per_warp, ws, T, E8S_THREADS / 32, tokens);
 }
 

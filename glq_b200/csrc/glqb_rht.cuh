@@ -310,9 +310,8 @@ __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_kernel(const Dev
                                                              const uint8_t* __restrict__ x_base,
                                                              uint8_t* __restrict__ ws, int tokens) {
   extern __shared__ __align__(16) float fbuf[];
-  // a successor launched with programmatic stream serialization (the single-launch decode kernel) may start
-  // its prologue now; it waits for this kernel's completion before it reads the activations
-  asm volatile("griddepcontrol.launch_dependents;");
+  pdl_wait();
+  pdl_trigger();
   RhtItem it = items[blockIdx.x];
   if (rht_item_trim(it, tokens)) rht_in_body<PLAIN_F32>(layers[it.layer], it, x_base, ws, fbuf);
 }
@@ -556,8 +555,8 @@ static __global__ void __launch_bounds__(RHT_THREADS, 4) rht_out_plain_kernel(co
                                                               const uint8_t* __restrict__ ws,
                                                               uint8_t* __restrict__ y_base, int tokens) {
   extern __shared__ __align__(16) float fbuf[];
-  asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
   RhtItem it = items[blockIdx.x];
   if (!rht_item_trim(it, tokens)) return;
   const DevLinear& L = layers[it.layer];
@@ -571,10 +570,8 @@ __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_out_kernel(const De
                                                               uint8_t* __restrict__ y_base,
                                                               const float* __restrict__ yrht_in, int tokens) {
   extern __shared__ __align__(16) float fbuf[];
-  // launched with programmatic stream serialization behind the decode kernels: wait for them here; the next
-  // kernel of the stream may start its prologue
-  asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
   RhtItem it = items[blockIdx.x];
   if (rht_item_trim(it, tokens)) rht_out_body<false, WIDE>(layers[it.layer], it, ws, y_base, yrht_in, fbuf);
 }

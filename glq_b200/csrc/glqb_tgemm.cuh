@@ -92,8 +92,9 @@ template <int K1, int K2, int TN>
 __global__ void __launch_bounds__(TG_THREADS, 1)
 trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict__ items, int n_items,
                     uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev, int tokens) {
-  // work lists built on the device (grouped expert matmul) pass their length through memory
-  if (n_items_dev) n_items = min(n_items, *n_items_dev);
+  pdl_trigger();
+  // (as in glq_gemm_kernel: of a plan's layers the producers decode before the kernel in front of this one has completed)
+  if (n_items_dev) { pdl_wait(); n_items = min(n_items, *n_items_dev); }
   // first token and tokens of an item's tile (none: every role skips the item), the activation rows in front of it, and the
   // tokens of its second tile, which lies right behind (whole tiles are multiples of 16)
   struct Tile { int tok0, ntok, row0, ntok2; };
@@ -199,6 +200,7 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
   } else if (warp == LOAD_WARP) {
     // ------------------------------------------------------------------ activation loader
     if (lane == 0) {
+      pdl_wait();
       uint32_t q = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
@@ -323,6 +325,7 @@ trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __rest
     if (!ok) { *abort_flag = 1; if (lane == 0) atomicCAS(status, 0, (int)ST_GAVE_UP_PRODUCER); }
   } else if (warp >= TG_EPI_WARP0) {
     // ------------------------------------------------------------------ epilogue warps
+    pdl_wait();
     const int quarter = warp & 3;                          // TMEM lanes 32*quarter .. 32*quarter + 31
     uint32_t seq = 0;
     bool ok = true;
