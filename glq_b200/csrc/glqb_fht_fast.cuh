@@ -132,35 +132,17 @@ __device__ __forceinline__ void fht_fast_e(float* smem, int logbs, Load& load, P
 }
 
 // dispatch on the array length (2^logbs, 32 .. 8192)
-template <int MAXLOG, int LATE, bool PACK, class Load1, class Load4, class Pre, class Store>
-__device__ __forceinline__ void fht_fast(float* smem, int logbs, Load1 load1, Load4 load4, Pre pre, Store store) {
-  // load1(i) -> value i;  load4(i0, float (&q)[4]) -> values i0 .. i0 + 3 (i0 a multiple of 4);
-  // pre(i) -> what store(i, value, x) gets as x (fp32; PACK: given as fp16)
-  auto ld1 = [&](int i0, float (&v)[1]) { v[0] = load1(i0); };
-  auto ld2 = [&](int i0, float (&v)[2]) { v[0] = load1(i0); v[1] = load1(i0 + 1); };
-  auto ld4 = [&](int i0, float (&v)[4]) { load4(i0, v); };
-  auto ld8 = [&](int i0, float (&v)[8]) {
-    float q[4];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) { load4(i0 + 4 * k, q); v[4 * k] = q[0]; v[4 * k + 1] = q[1]; v[4 * k + 2] = q[2]; v[4 * k + 3] = q[3]; }
-  };
-  auto ld16 = [&](int i0, float (&v)[16]) {
-    float q[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) { load4(i0 + 4 * k, q); v[4 * k] = q[0]; v[4 * k + 1] = q[1]; v[4 * k + 2] = q[2]; v[4 * k + 3] = q[3]; }
-  };
-  auto ld32 = [&](int i0, float (&v)[32]) {
-    float q[4];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { load4(i0 + 4 * k, q); v[4 * k] = q[0]; v[4 * k + 1] = q[1]; v[4 * k + 2] = q[2]; v[4 * k + 3] = q[3]; }
-  };
+// load(i0, float (&v)[E]) -> values i0 .. i0 + E - 1 (i0 a multiple of E): a thread's values in one call, so that their loads
+// can all be in flight;  pre(i) -> what store(i, value, x) gets as x (fp32; PACK: given as fp16)
+template <int MAXLOG, int LATE, bool PACK, class Load, class Pre, class Store>
+__device__ __forceinline__ void fht_fast(float* smem, int logbs, Load load, Pre pre, Store store) {
   // arrays longer than 2^MAXLOG never reach this instantiation (their cases are not compiled)
-  if (logbs == 9) { fht_fast_e<2, LATE, PACK>(smem, logbs, ld2, pre, store); return; }
-  if (logbs == 10) { fht_fast_e<4, LATE, PACK>(smem, logbs, ld4, pre, store); return; }
-  if constexpr (MAXLOG >= 11) if (logbs == 11) { fht_fast_e<8, LATE, PACK>(smem, logbs, ld8, pre, store); return; }
-  if constexpr (MAXLOG >= 12) if (logbs == 12) { fht_fast_e<16, LATE, PACK>(smem, logbs, ld16, pre, store); return; }
-  if constexpr (MAXLOG >= 13) if (logbs == 13) { fht_fast_e<32, LATE, PACK>(smem, logbs, ld32, pre, store); return; }
-  fht_fast_e<1, LATE, PACK>(smem, logbs, ld1, pre, store);                        // 32 .. 256 values
+  if (logbs == 9) { fht_fast_e<2, LATE, PACK>(smem, logbs, load, pre, store); return; }
+  if (logbs == 10) { fht_fast_e<4, LATE, PACK>(smem, logbs, load, pre, store); return; }
+  if constexpr (MAXLOG >= 11) if (logbs == 11) { fht_fast_e<8, LATE, PACK>(smem, logbs, load, pre, store); return; }
+  if constexpr (MAXLOG >= 12) if (logbs == 12) { fht_fast_e<16, LATE, PACK>(smem, logbs, load, pre, store); return; }
+  if constexpr (MAXLOG >= 13) if (logbs == 13) { fht_fast_e<32, LATE, PACK>(smem, logbs, load, pre, store); return; }
+  fht_fast_e<1, LATE, PACK>(smem, logbs, load, pre, store);                       // 32 .. 256 values
 }
 constexpr int FHT_FAST_MAX_LOG = 13;
 

@@ -585,11 +585,20 @@ __device__ __forceinline__ void rht_out_short(const DevLinear& L, const RhtItem 
   const __half* su = L.su + off;
   const long long o = L.y_off + (long long)it.tok0 * L.y_stride + off;
   const float rs = rsqrtf((float)(1 << logbs));
-  auto load4 = [&](int i, float (&q)[4]) {
-    const float4 t = __ldcg(reinterpret_cast<const float4*>(p + i));
-    q[0] = t.x; q[1] = t.y; q[2] = t.z; q[3] = t.w;
+  auto load = [&](int i, auto& v) {
+    constexpr int E = sizeof(v) / sizeof(float);
+    if constexpr (E >= 4) {
+#pragma unroll
+      for (int q = 0; q < E; q += 4) {
+        const float4 t = __ldcg(reinterpret_cast<const float4*>(p + i + q));
+        v[q] = t.x; v[q + 1] = t.y; v[q + 2] = t.z; v[q + 3] = t.w;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < E; ++q) v[q] = __ldcg(p + i + q);
+    }
   };
-  fht_fast<10, 64, false>(fbuf, logbs, [&](int i) { return __ldcg(p + i); }, load4, [&](int i) { return __half2float(su[i]); },
+  fht_fast<10, 64, false>(fbuf, logbs, load, [&](int i) { return __half2float(su[i]); },
                           [&](int i, float v, float sign) { store_act(y_base, o + i, L.y_dtype, v * rs * sign); });
 }
 
