@@ -73,6 +73,7 @@ struct GlqbPlan {
   size_t ws_bytes = 0;
   int max_batch = 1;
   bool out_plain_static = false; // every output item takes the plain transform when the output is aligned
+  bool in_few = false, out_few = false;          // few tiles: the transforms with 1024 threads per tile
   bool out_wide = false;         // some layer has 2^32 partial sums per slot or more
   int max_elems_in = 32, max_elems_out = 32;    // floats of shared memory the transform CTAs need
   int sm_count = 0;
@@ -886,6 +887,14 @@ static int build_plan(GlqbPlan* P) {
   add_rht_items(P->items_in, rht_in, P->sm_count, P->max_elems_in);
   add_rht_items(P->items_in_gemm, rht_in_gemm, P->sm_count, P->max_elems_in);
   add_rht_items(P->items_out, rht_out, P->sm_count, P->max_elems_out);
+  // Launches of at most a tile per SM, without GEMM layers: the time of one tile counts, not the SMs' throughput.
+  bool decode = true;
+  for (const DevLinear& L : P->dev) decode = decode && L.gemm_tn == 0;
+  // (inputs: only where norm or activation are computed on the way; plain loads of groups of four are the faster ones there)
+  bool steps = false;
+  for (const RhtItem& it : P->items_in) steps = steps || P->dev[it.layer].in_gated_act || P->dev[it.layer].in_norm_w;
+  P->in_few = steps && P->items_in.size() <= (size_t)P->sm_count;
+  P->out_few = decode && P->items_out.size() <= (size_t)P->sm_count;
   P->ws_bytes = ws;
   P->out_wide = false;
   for (const DevLinear& L : P->dev) P->out_wide = P->out_wide || (long long)L.batch * L.m > 0xFFFFFFFFll;
@@ -1013,8 +1022,8 @@ int glqb_plan_run_tokens(GlqbPlan* P, const void* x_base, void* y_base, int32_t 
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
   if (!P->items_in.empty()) {
-    launch_chained(true, rht_in_kernel<false>, (int)P->items_in.size(), RHT_THREADS, rht_smem(P->max_elems_in), stream, d_layers,
-                   P->d_items_in, reinterpret_cast<const uint8_t*>(x_base), ws, tokens);
+    launch_chained(true, P->in_few ? rht_in_wide_kernel : rht_in_kernel<false>, (int)P->items_in.size(), P->in_few ? FHT_WIDE_THREADS : RHT_THREADS,
+                   rht_smem(P->max_elems_in), stream, d_layers, P->d_items_in, reinterpret_cast<const uint8_t*>(x_base), ws, tokens);
   }
   if (!P->items_in_gemm.empty()) {
     launch_chained(true, rht_in_gemm_kernel, (int)P->items_in_gemm.size(), RHT_THREADS, rht_smem(P->max_elems_in), stream, d_layers,
@@ -1051,7 +1060,10 @@ int glqb_plan_run_tokens(GlqbPlan* P, const void* x_base, void* y_base, int32_t 
   if (!P->items_out.empty()) {
     const int n_items = (int)P->items_out.size();
     uint8_t* yb = reinterpret_cast<uint8_t*>(y_base);
-    if (out_plain(P, yb)) {
+    if (P->out_few) {
+      CUDA_TRY(launch_chained(true, rht_out_wide_kernel, n_items, FHT_WIDE_THREADS, rht_smem(P->max_elems_out), stream, d_layers,
+                              P->d_items_out, ws, yb, tokens));
+    } else if (out_plain(P, yb)) {
       CUDA_TRY(launch_chained(true, rht_out_plain_kernel, n_items, RHT_THREADS, rht_smem(P->max_elems_out), stream, d_layers, P->d_items_out, ws,
                               yb, tokens));
     } else {

@@ -220,6 +220,75 @@ __device__ __forceinline__ void fht_block(float* sm, int logbs, int total, Load 
   });
 }
 
+// The tile transform for launches of few tiles, where the latency of one tile is the launch's: 1024 threads with eight values
+// each instead of 256 with 32, single values instead of groups of four (no alignment to ask for).  Passes:
+//   1  e = k << 10 | warp << 5 | lane     bits 10 .. 12 in registers, 0 .. 4 across the lanes
+//   2  e = warp << 8 | k << 5 | lane      bits 5 .. 7
+//   3  e = (warp >> 3) << 11 | k << 8 | (warp & 7) << 5 | lane      bits 8 and 9
+// so every access, global or shared, is 32 consecutive values per warp.  `sm`: `total` floats.  load(e, k) is asked for values
+// below `total` only; all 1024 threads call.
+constexpr int FHT_WIDE_THREADS = 1024;
+template <class Load, class Store>
+__device__ __forceinline__ void fht_wide(float* sm, int logbs, int total, Load load, Store store) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float v[8];
+  const int e0 = (warp << 5) | lane;
+  auto stage = [&](int s) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (!(k & (1 << s))) {
+        const float a = v[k], b = v[k | (1 << s)];
+        v[k] = a + b;
+        v[k | (1 << s)] = a - b;
+      }
+  };
+  load(e0, v);
+#pragma unroll
+  for (int s = 0; s < 5; ++s)
+    if (logbs > s && (e0 & ~31) < total) {                 // (uniform per warp)
+      const float sg = (lane >> s) & 1 ? -1.f : 1.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = fmaf(v[k], sg, __shfl_xor_sync(0xffffffffu, v[k], 1 << s));
+    }
+#pragma unroll
+  for (int s = 0; s < 3; ++s)
+    if (logbs > 10 + s) stage(s);
+  if (logbs <= 5) {                                        // (no stage crosses a warp)
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (e0 + (k << 10) < total) store(e0 + (k << 10), v[k]);
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (e0 + (k << 10) < total) sm[e0 + (k << 10)] = v[k];
+  __syncthreads();
+  const int e1 = (warp << 8) | lane;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = e1 + (k << 5) < total ? sm[e1 + (k << 5)] : 0.f;
+#pragma unroll
+  for (int s = 0; s < 3; ++s)
+    if (logbs > 5 + s) stage(s);
+  if (logbs <= 8) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (e1 + (k << 5) < total) store(e1 + (k << 5), v[k]);
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (e1 + (k << 5) < total) sm[e1 + (k << 5)] = v[k];
+  __syncthreads();
+  const int e2 = ((warp >> 3) << 11) | ((warp & 7) << 5) | lane;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = e2 + (k << 8) < total ? sm[e2 + (k << 8)] : 0.f;
+  stage(0);
+  if (logbs > 9) stage(1);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (e2 + (k << 8) < total) store(e2 + (k << 8), v[k]);
+}
+
 // One warp, 1024 values, two register passes and no block barrier: v[k] holds values k << 7 | lane << 2 | j (bits 0, 1
 // and 7 .. 9), the second pass bits 2 .. 6; arrays of 2^logbs <= 1024 values side by side (logbs >= 5).  Blocks longer
 // than 1024 are 1024-value chunks whose remaining bits the consumer of the results combines.  Results: value e at

@@ -316,6 +316,67 @@ __global__ void __launch_bounds__(RHT_THREADS, RHT_MINB) rht_in_kernel(const Dev
   if (rht_item_trim(it, tokens)) rht_in_body<PLAIN_F32>(layers[it.layer], it, x_base, ws, fbuf);
 }
 
+// The same for launches of few tiles whose inputs come with fused steps (the [gate | up] rows of a down projection in a decode
+// step).  Four decoder layers, one token 333.5 / 328.6 us.
+static __global__ void __launch_bounds__(FHT_WIDE_THREADS, 1) rht_in_wide_kernel(const DevLinear* __restrict__ layers,
+                                                              const RhtItem* __restrict__ items,
+                                                              const uint8_t* __restrict__ x_base,
+                                                              uint8_t* __restrict__ ws, int tokens) {
+  extern __shared__ __align__(16) float fbuf[];
+  __shared__ float rstd_s[FUSED_MAX_TOKENS_C];
+  pdl_wait();
+  pdl_trigger();
+  RhtItem it = items[blockIdx.x];
+  if (!rht_item_trim(it, tokens)) return;
+  const DevLinear& L = layers[it.layer];
+  const int off = L.bn_off[it.block], logbs = L.bn_log[it.block], bs = 1 << logbs;
+  const bool trellis = L.format == GLQB_FMT_TRELLIS_3INST, fusions = L.in_gated_act != 0 || L.in_norm_w != nullptr;
+  const bool normed = L.in_norm_w != nullptr, rotated = L.x_is_rotated != 0;
+  const float rs = rotated ? 1.0f : rsqrtf((float)bs);
+  const int S = it.sub >= 0 ? bs >> FHT_LOG : 1, log_t = min(logbs, FHT_LOG), run0 = max(it.sub, 0) << FHT_LOG;
+  const int total = it.ntok << log_t;
+  if (normed)                                              // (at most 8 tokens)
+    for (int r = 0; r < it.ntok; ++r) {
+      const float v = token_rstd(L, x_base, L.x_off + (long long)(it.tok0 + r) * L.x_stride, fbuf);
+      if (threadIdx.x == 0) rstd_s[r] = v;
+      __syncthreads();
+    }
+  auto load = [&](int e0, float (&v)[8]) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = 0.f;
+    for (int kk = 0; kk < S; ++kk) {
+      if (rotated && kk != max(it.sub, 0)) continue;
+      const float sg = !rotated && (__popc(max(it.sub, 0) & kk) & 1) ? -1.f : 1.f;
+      float t[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int e = e0 + (k << 10), col = off + (kk << FHT_LOG) + (e & ((1 << log_t) - 1));
+        t[k] = 0.f;
+        if (e < total && col < L.in_f) {
+          const long long xt0 = L.x_off + (long long)(it.tok0 + (e >> log_t)) * L.x_stride;
+          t[k] = fusions ? input_value(L, x_base, xt0, col) : load_act(x_base, xt0 + col, L.x_dtype);
+          if (normed) t[k] *= load_act(L.in_norm_w, col, L.in_norm_dtype);
+          if (!rotated) t[k] *= __half2float(L.sv[col]);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = fmaf(t[k], sg, v[k]);
+    }
+  };
+  auto store = [&](int e, float v) {
+    const int row = e >> log_t, col = off + run0 + (e & ((1 << log_t) - 1));
+    const long long token = it.tok0 + row;
+    v *= normed ? rs * rstd_s[row] : rs;
+    if (trellis) {
+      const int pos = (col & ~31) * XR_TRELLIS_EXPAND + xr_pos_trellis(col & 31);   // half index, even
+      (reinterpret_cast<__half2*>(ws + L.xr_off) + token * L.n)[pos >> 1] = __halves2half2(__float2half_rn(v), __float2half_rn(0.f));
+    } else {
+      reinterpret_cast<__half*>(ws + L.xr_off)[xr_index_e8(token, col, L.n, L.batch)] = __float2half_rn(v);
+    }
+  };
+  fht_wide(fbuf, rotated ? 0 : log_t, total, load, store);
+}
+
 // One layer described entirely in kernel-parameter space (no device table, nothing to allocate or copy):
 // the unfused input_rht / output_rht ops.  CTA b of Hadamard block k handles the token tile
 // b - first_cta[k]; tile_tokens[k] tokens per tile (blocks longer than a tile: one token and one run per CTA).
@@ -491,6 +552,83 @@ __device__ __forceinline__ void rht_out_body(const DevLinear& L, const RhtItem i
     }
   };
   fht_block(fbuf, log_t, total, load, store);
+}
+
+// The same for launches of few tiles (decode steps).  Whole calls, 256 threads a tile / this: 16 tokens of 4096 x 14336 70.6 /
+// 67.3 us, 27 tokens of 11008 x 2048 (4 + 2 bits) 55.0 / 54.2, one token of 14336 x 4096 49.4 / 49.2.
+static __global__ void __launch_bounds__(FHT_WIDE_THREADS, 1) rht_out_wide_kernel(const DevLinear* __restrict__ layers,
+                                                              const RhtItem* __restrict__ items,
+                                                              const uint8_t* __restrict__ ws,
+                                                              uint8_t* __restrict__ y_base, int tokens) {
+  extern __shared__ __align__(16) float fbuf[];
+  pdl_trigger();
+  RhtItem it = items[blockIdx.x];
+  if (!rht_item_trim(it, tokens)) return;
+  const DevLinear& L = layers[it.layer];
+  const int off = L.bm_off[it.block], logbs = L.bm_log[it.block], bs = 1 << logbs;
+  const int strip_log = (L.format == GLQB_FMT_TRELLIS_3INST) ? 5 : 4;
+  const int m = L.m, gps = L.groups_per_strip, fixed_slots = L.fixed_slots;
+  const unsigned per_warp = (unsigned)L.per_warp;
+  const long long slot_stride = (long long)L.batch * m;
+  const float* src = reinterpret_cast<const float*>(ws + L.part_off);
+  const float* row_scale = L.row_scale;
+  const int S = it.sub >= 0 ? bs >> FHT_LOG : 1, log_t = min(logbs, FHT_LOG), run0 = max(it.sub, 0) << FHT_LOG;
+  const int total = it.ntok << log_t;
+  auto slots_of = [&](int row) -> int {                    // (rht_out_body)
+    if (fixed_slots > 0) return fixed_slots;
+    const long long g0 = L.group_base + (long long)(row >> strip_log) * gps;
+    if (g0 + gps <= 0xFFFFFFFFll) return (int)(((unsigned)g0 + gps - 1) / per_warp - (unsigned)g0 / per_warp) + 1;
+    return (int)((g0 + gps - 1) / per_warp - g0 / per_warp) + 1;
+  };
+  const float rs = rsqrtf((float)bs), wscale = L.wscale;
+  const float* rstd = (L.in_norm_w && !L.xr_global) ? reinterpret_cast<const float*>(ws + L.rstd_off) : nullptr;
+  const bool stop = L.stop_at_yrht != 0, accumulate = L.y_accumulate != 0;
+  auto load = [&](int e0, float (&v)[8]) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = 0.f;
+    for (int kk = 0; kk < S; ++kk) {
+      if (stop && kk != max(it.sub, 0)) continue;
+      const float sg = !stop && (__popc(max(it.sub, 0) & kk) & 1) ? -1.f : 1.f;
+      float t[8];
+      int cnt[8], most = 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int e = e0 + (k << 10), row = off + (kk << FHT_LOG) + (e & ((1 << log_t) - 1));
+        cnt[k] = e < total && row < m ? slots_of(row) : 0;
+        most = max(most, cnt[k]);
+        t[k] = 0.f;
+      }
+      for (int s = 0; s < most; ++s) {
+        float q[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int e = e0 + (k << 10), row = off + (kk << FHT_LOG) + (e & ((1 << log_t) - 1));
+          q[k] = s < cnt[k] ? __ldcg(src + s * slot_stride + (long long)(it.tok0 + (e >> log_t)) * m + row) : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t[k] += q[k];
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        float w = t[k] * wscale;
+        if (row_scale && cnt[k]) w *= row_scale[off + (kk << FHT_LOG) + ((e0 + (k << 10)) & ((1 << log_t) - 1))];
+        v[k] = fmaf(w, sg, v[k]);
+      }
+    }
+  };
+  auto store = [&](int e, float v) {
+    const int token = it.tok0 + (e >> log_t), row = off + run0 + (e & ((1 << log_t) - 1));
+    const long long o = L.y_off + (long long)token * L.y_stride + row;
+    if (stop) {
+      if (row < m) reinterpret_cast<float*>(y_base)[o] = v;
+    } else if (row < L.out_f) {
+      float r = v * (rstd ? rs * rstd[token] : rs) * __half2float(L.su[row]);
+      if (accumulate) r += load_act(y_base, o, L.y_dtype);            // residual add
+      store_act(y_base, o, L.y_dtype, r);
+    }
+  };
+  pdl_wait();
+  fht_wide(fbuf, stop ? 0 : log_t, total, load, store);
 }
 
 // The prefill case: partial sums in a fixed number of slots, whole blocks, aligned rows, no per-row scales or residual.
