@@ -38,7 +38,7 @@ _META_CACHE: dict = {}
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def _require_cuda(t: torch.Tensor, name: str) -> None:
@@ -59,7 +59,7 @@ def _blocks(t, fallback: int) -> list[int]:
 def e8_packed_table(codebook: torch.Tensor) -> torch.Tensor:
     """fp16 (entries, 8) codebook -> cached nibble-packed int32 (entries,) table on its device."""
     _require_cuda(codebook, "codebook")
-    key = (codebook.data_ptr(), codebook.shape[0], codebook.device.index, codebook.dtype)
+    key = (codebook.data_ptr(), codebook.shape[0], codebook.get_device(), codebook.dtype)
     tb = _TABLE_CACHE.get(key)
     if tb is None:
         cb = codebook.to(torch.float16).contiguous()
@@ -87,8 +87,8 @@ def token_bucket(b: int) -> int:
 def shared_workspace(device, nbytes: int) -> torch.Tensor:
     """The workspace every cached plan on (device, current stream) runs in; grows geometrically."""
     dev = torch.device(device)
-    key = (dev.index if dev.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(dev).cuda_stream)
+    index = dev.index if dev.index is not None else torch.cuda.current_device()
+    key = (index, torch._C._cuda_getCurrentRawStream(index))
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < nbytes:
         if ws is not None:
@@ -167,8 +167,9 @@ def _run_sliced(x2d: torch.Tensor, out: torch.Tensor, key_base, make_spec, max_t
             raise
         plan.run(xin, yout, workspace=shared_workspace(xin.device, plan.workspace_bytes), tokens=b)
 
-    if B > DECODE_MAX_TOKENS:
-        run(x2d, B, out)
+    if B > DECODE_MAX_TOKENS or B <= max_tokens:
+        if B:
+            run(x2d, B, out)
         return
     done = 0
     while done < B:
@@ -193,6 +194,12 @@ class _InKernel:
     def __init__(self, comm):
         self.comm = comm
         self.world = comm.world
+
+
+def _rows(x: torch.Tensor, cols: int) -> torch.Tensor:
+    """x as (tokens, cols) rows of consecutive values."""
+    x2d = x if x.dim() == 2 and x.shape[1] == cols else x.reshape(-1, cols)
+    return x2d if x2d.stride(1) == 1 else x2d.contiguous()
 
 
 def _apply_input_steps(x2d, in_features, in_norm_weight, in_norm_eps, gated_act):
@@ -246,10 +253,7 @@ def _fused_trellis(x, sv, su, packed, packed2, blocks_n, blocks_m, wscale, inv_r
             accumulate_into.add_(part.reshape(accumulate_into.shape).to(accumulate_into.dtype))
             return accumulate_into
         return part.to(out_dtype or x.dtype)
-    x_cols = in_features * (2 if gated_act is not None else 1)
-    x2d = x.reshape(-1, x_cols)
-    if x2d.stride(-1) != 1:
-        x2d = x2d.contiguous()
+    x2d = _rows(x, in_features * (2 if gated_act is not None else 1))
     extras = in_norm_weight is not None or gated_act is not None or accumulate_into is not None
     if extras:
         if y_rht_out is not None:
@@ -264,9 +268,6 @@ def _fused_trellis(x, sv, su, packed, packed2, blocks_n, blocks_m, wscale, inv_r
                 return accumulate_into
             return y
     has2 = packed2 is not None and packed2.numel() > 0
-    codes = [packed] + ([packed2] if has2 else [])
-    bits = [_trellis_bits(packed)] + ([_trellis_bits(packed2)] if has2 else [])
-    bn, bm = _blocks(blocks_n, n_pad), _blocks(blocks_m, m_pad)
     if accumulate_into is not None:
         tgt, yoff, stop = accumulate_into.reshape(-1, out_features), 0, False
         if tgt.data_ptr() != accumulate_into.data_ptr() or tgt.stride(-1) != 1:
@@ -279,9 +280,10 @@ def _fused_trellis(x, sv, su, packed, packed2, blocks_n, blocks_m, wscale, inv_r
 
     def make_spec(b, x_stride, y_stride, y_offset):
         return LinearSpec(format=_lib.FMT_TRELLIS_3INST, m_pad=m_pad, n_pad=n_pad, in_features=in_features,
-                          out_features=out_features if not stop else m_pad, codes=codes, bits=bits, su=su, sv=sv,
+                          out_features=out_features if not stop else m_pad, codes=[packed] + ([packed2] if has2 else []),
+                          bits=[_trellis_bits(packed)] + ([_trellis_bits(packed2)] if has2 else []), su=su, sv=sv,
                           wscale=float(wscale), stage_scale=[float(inv_rs2)] if has2 else [],
-                          blocks_n=bn, blocks_m=bm, batch=b, x_dtype=x2d.dtype, y_dtype=tgt.dtype,
+                          blocks_n=_blocks(blocks_n, n_pad), blocks_m=_blocks(blocks_m, m_pad), batch=b, x_dtype=x2d.dtype, y_dtype=tgt.dtype,
                           x_stride=x_stride, y_stride=y_stride, y_offset=y_offset, stop_at_yrht=stop,
                           in_norm_weight=in_norm_weight, in_norm_eps=in_norm_eps, in_gated_act=gated_act,
                           y_accumulate=accumulate_into is not None)
@@ -525,9 +527,7 @@ def _fused_e8(x, sv, su, codes, tables, scales, wscale, in_features, out_feature
             return accumulate_into
         return y if comm is None else y.to(out_dtype or x.dtype)
     feat_in = n_pad if x_is_rotated else in_features
-    x2d = x.reshape(-1, feat_in * (2 if gated_act is not None else 1))
-    if x2d.stride(-1) != 1:
-        x2d = x2d.contiguous()
+    x2d = _rows(x, feat_in * (2 if gated_act is not None else 1))
     odt = torch.float32 if stop else (out_dtype or x2d.dtype)
     if accumulate_into is not None:
         out = accumulate_into.reshape(-1, out_features)
@@ -540,7 +540,7 @@ def _fused_e8(x, sv, su, codes, tables, scales, wscale, in_features, out_feature
     def make_spec(b, x_stride, y_stride, y_offset):
         return LinearSpec(format=_lib.FMT_E8_SHELL, m_pad=m_pad, n_pad=n_pad, in_features=feat_in,
                           out_features=m_pad if stop else out_features, codes=codes, tables=tables,
-                          stage_scale=scales, su=su, sv=sv, wscale=float(wscale), blocks_n=bn, blocks_m=bm,
+                          stage_scale=scales, su=su, sv=sv, wscale=float(wscale), blocks_n=_blocks(bn, n_pad), blocks_m=_blocks(bm, m_pad),
                           batch=b, x_dtype=x2d.dtype, y_dtype=odt, x_stride=x_stride, y_stride=y_stride,
                           y_offset=y_offset, stop_at_yrht=stop, x_is_rotated=x_is_rotated,
                           in_norm_weight=in_norm_weight, in_norm_eps=in_norm_eps, in_gated_act=gated_act,
@@ -583,7 +583,7 @@ def fused_linear_block_diag(x, sv, su, qidxs, codebook, wscale, in_features, out
     codes, tables, scales = _e8_stages(qidxs, codebook, qidxs2, codebook2, inv_resid_scale, qidxs3, codebook3,
                                        inv_resid_scale2, qidxs4, codebook4, inv_resid_scale3)
     return _fused_e8(x, sv, su, codes, tables, scales, wscale, in_features, out_features, n_pad, m_pad,
-                     _blocks(blocks_n, n_pad), _blocks(blocks_m, m_pad), out_dtype=out_dtype,
+                     blocks_n, blocks_m, out_dtype=out_dtype,
                      in_norm_weight=in_norm_weight, in_norm_eps=in_norm_eps, gated_act=gated_act,
                      accumulate_into=accumulate_into, reduce_over=reduce_over)
 

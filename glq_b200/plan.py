@@ -122,7 +122,8 @@ class Plan:
         self.specs = list(specs)
         if not self.specs:
             raise RuntimeError("glq_b200: empty plan")
-        self.device = device or self.specs[0].su.device
+        self.device = torch.device(device or self.specs[0].su.device)
+        self.device_index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         arr = (_lib.LinearDesc * len(self.specs))(*[s.to_desc() for s in self.specs])
         handle = C.c_void_p()
         with torch.cuda.device(self.device):
@@ -140,12 +141,13 @@ class Plan:
             workspace: Optional[torch.Tensor] = None, tokens: int = 2 ** 31 - 1) -> None:
         """Enqueue on ``stream`` (default: the current torch stream); does not synchronise.  ``tokens``: rows of x and y
         to process when they are fewer than the plan was built for."""
-        st = stream if stream is not None else torch.cuda.current_stream(self.device)
+        st = stream.cuda_stream if stream is not None else torch._C._cuda_getCurrentRawStream(self.device_index)
         ws = workspace if workspace is not None else self.workspace
         if ws is None:
             raise RuntimeError("glq_b200: this plan owns no workspace; pass one to run()")
-        _lib.check(self.lib.glqb_plan_run_tokens(self.handle, x.data_ptr(), y.data_ptr(), tokens, ws.data_ptr(),
-                                                 ws.numel(), st.cuda_stream), "plan_run")
+        rc = self.lib.glqb_plan_run_tokens(self.handle, x.data_ptr(), y.data_ptr(), tokens, ws.data_ptr(), ws.numel(), st)
+        if rc:
+            _lib.check(rc, "plan_run")
 
     def set_timing(self, on: bool) -> None:
         _lib.check(self.lib.glqb_plan_set_timing(self.handle, 1 if on else 0), "plan_set_timing")
