@@ -112,16 +112,16 @@ class GLQLinear(nn.Module):
             raise RuntimeError("glq_b200.GLQLinear has no CPU path")
         s = self._resolve()
         shape = x.shape
-        x2d = x if x.dim() == 2 else x.reshape(-1, self.in_features)
+        rows = x.dim() == 2 and shape[1] == self.in_features
+        x2d = x if rows else x.reshape(-1, self.in_features)
         bn, bm = self.blocks_n, self.blocks_m
-        b = self._buffers
         if self._is_trellis:
             if s["has2"]:
-                y = ops.fused_linear_trellis_3inst_rvq2(x2d, b["SV"], b["SU"], b["trellis_packed"], b["trellis_packed2"],
+                y = ops.fused_linear_trellis_3inst_rvq2(x2d, self.SV, self.SU, self.trellis_packed, self.trellis_packed2,
                                                         bn, bm, None, None, s["wscale"], s["inv2"], self.in_features,
                                                         self.out_features, self.n_pad, self.m_pad)
             else:
-                y = ops.fused_linear_trellis_3inst(x2d, b["SV"], b["SU"], b["trellis_packed"], bn, bm, None, None,
+                y = ops.fused_linear_trellis_3inst(x2d, self.SV, self.SU, self.trellis_packed, bn, bm, None, None,
                                                    s["wscale"], self.in_features, self.out_features, self.n_pad,
                                                    self.m_pad)
         else:
@@ -131,19 +131,19 @@ class GLQLinear(nn.Module):
             cb = self._table(self.codebook, dev)
             ns, inv = s["n_stages"], s["inv"]
             cb2 = self._table(self.codebook2, dev) if ns >= 2 else None
-            tail = (b["Qidxs2"] if ns >= 2 else None, cb2, inv[0] if ns >= 2 else 0.0,
-                    b["Qidxs3"] if ns >= 3 else None, cb if ns >= 3 else None, inv[1] if ns >= 3 else 0.0,
-                    b["Qidxs4"] if ns >= 4 else None, cb if ns >= 4 else None, inv[2] if ns >= 4 else 0.0)
+            tail = (self.Qidxs2 if ns >= 2 else None, cb2, inv[0] if ns >= 2 else 0.0,
+                    self.Qidxs3 if ns >= 3 else None, cb if ns >= 3 else None, inv[1] if ns >= 3 else 0.0,
+                    self.Qidxs4 if ns >= 4 else None, cb if ns >= 4 else None, inv[2] if ns >= 4 else 0.0)
             if self.block_diagonal:
-                y = ops.fused_linear_block_diag(x2d, b["SV"], b["SU"], b["Qidxs"], cb, s["wscale"], self.in_features,
+                y = ops.fused_linear_block_diag(x2d, self.SV, self.SU, self.Qidxs, cb, s["wscale"], self.in_features,
                                                 self.out_features, self.n_pad, self.m_pad, bn, bm, None, None, *tail)
             else:
-                y = ops.fused_linear(x2d, b["SV"], b["SU"], b["Qidxs"], cb, s["wscale"], self.in_features,
+                y = ops.fused_linear(x2d, self.SV, self.SU, self.Qidxs, cb, s["wscale"], self.in_features,
                                      self.out_features, self.n_pad, self.m_pad, self.n_pad.bit_length() - 1,
                                      self.m_pad.bit_length() - 1, *tail)
         if self.bias is not None:
             y = y + self.bias.unsqueeze(0).to(y.dtype)
-        return y if len(shape) == 2 else y.reshape(*shape[:-1], self.out_features)
+        return y if rows else y.reshape(*shape[:-1], self.out_features)
 
     # -- debugging -------------------------------------------------------------------------------------
     def dequantize_rotated(self) -> torch.Tensor:

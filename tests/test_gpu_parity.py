@@ -655,6 +655,15 @@ def test_glq_linear_module_matches_oracle(e8_table, e8_cb):
     assert relerr(tl(xt).cpu().numpy(), O.linear_forward(xt.cpu().numpy(), Wt, tsu, tsv, 0.02)) <= TOL
 
 
+def test_glq_linear_module_refuses_other_widths(e8_cb):
+    """Rows of another width whose values would fill whole rows are refused, as from nn.Linear."""
+    from glq_b200.linear import GLQLinear
+    lin = GLQLinear(256, 128).cuda()
+    lin.set_codebook(e8_cb[0])
+    with pytest.raises(RuntimeError):
+        lin(torch.zeros(4, 512, dtype=torch.float16, device="cuda"))
+
+
 # ---------------------------------------------------------------------------------------------
 # edge cases: empty and ragged inputs, strided rows
 # ---------------------------------------------------------------------------------------------

@@ -136,6 +136,44 @@ def test_wide_inputs_of_decode_steps(tokens, shift):
     _check(x, W, E, yb, block_decompose(n), block_decompose(m))
 
 
+@pytest.mark.parametrize("tokens", [1, 8, 9, 64])
+@pytest.mark.parametrize("shape", [(16352, 64), (16416, 64), (64, 16352), (64, 16416)], ids=str)
+def test_decode_steps_every_block_length(shape, tokens):
+    """16352 has one block of every length from 32 to 8192, 16416 one that two tiles share: the transforms of decode calls,
+    plain, behind a norm and behind an activation, with rows that are not aligned and results added to a residual."""
+    from glq_b200 import synth
+    from glq_b200.plan import block_decompose
+    m, n = shape
+    g = torch.Generator(device="cuda").manual_seed(m + tokens)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w = randn(tokens, 2 * n + 1)[:, 1:], 1 + 0.2 * randn(n)
+    gate, up = x[:, :n].double(), x[:, n:].double()
+    # (fp32 inputs: nothing is rounded between the steps)
+    steps = [(x[:, :n], gate, {}),
+             (x[:, :n], gate * torch.rsqrt(gate.pow(2).mean(-1, keepdim=True) + 1e-5) * w.double(), dict(in_norm_weight=w, in_norm_eps=1e-5)),
+             (x, torch.nn.functional.silu(gate) * up, dict(gated_act=0))]
+    table = synth.load_e8_table("cuda")
+    nib = (table.cpu().numpy().view(np.uint32)[:, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15
+    cb = nib.astype(np.float64) * 0.5 - 3.0
+    T = synth.trellis_layer("t", m, n, [4], g, "cuda")
+    E = synth.e8_layer("e", m, n, 1, table, g, "cuda")
+    half = torch.from_numpy(cb).to("cuda", torch.float16)
+    none = (None, None, 0.0)
+    forms = [(T, ops.glq_decompress_trellis_3inst_cuda(T.codes[0], m, n).double().cpu().numpy(),
+              lambda a, **kw: ops.fused_linear_trellis_3inst(a, T.sv, T.su, T.codes[0], None, None, None, None, T.wscale,
+                                                             n, m, n, m, **kw)),
+             (E, cb[E.codes[0].cpu().numpy().view(np.uint16)].reshape(m, n),
+              lambda a, **kw: ops.fused_linear_block_diag(a, E.sv, E.su, E.codes[0], half, E.wscale, n, m, n, m, block_decompose(n),
+                                                          block_decompose(m), None, None, *none * 3, **kw))]
+    for L, W, call in forms:
+        for a, seen, kw in steps:
+            _check(seen, W, L, call(a, **kw), block_decompose(n), block_decompose(m))
+            h0 = randn(tokens, m)
+            h = h0.clone()
+            call(a, accumulate_into=h, **kw)
+            _check(seen, W, L, h.double() - h0.double(), block_decompose(n), block_decompose(m))
+
+
 def test_plan_output_beyond_32_bit_offsets():
     """32769 tokens of a layer of 131072 rows: the last token's partial sums start 2^32 elements in (rows of the result are
     not aligned, so the general body runs).  Against the same token alone."""
