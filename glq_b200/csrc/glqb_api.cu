@@ -899,6 +899,7 @@ static int build_plan(GlqbPlan* P) {
   for (const RhtItem& it : P->items_in) steps = steps || P->dev[it.layer].in_gated_act || P->dev[it.layer].in_norm_w;
   P->in_few = steps && P->items_in.size() <= (size_t)P->sm_count;
   P->out_few = decode && P->items_out.size() <= (size_t)P->sm_count;
+  for (const RhtItem& it : P->items_out) P->out_few = P->out_few && !P->dev[it.layer].row_scale;
   P->ws_bytes = ws;
   P->out_wide = false;
   for (const DevLinear& L : P->dev) P->out_wide = P->out_wide || (long long)L.batch * L.m > 0xFFFFFFFFll;

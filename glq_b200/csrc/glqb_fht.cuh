@@ -225,8 +225,9 @@ __device__ __forceinline__ void fht_block(float* sm, int logbs, int total, Load 
 //   1  e = k << 10 | warp << 5 | lane     bits 10 .. 12 in registers, 0 .. 4 across the lanes
 //   2  e = warp << 8 | k << 5 | lane      bits 5 .. 7
 //   3  e = (warp >> 3) << 11 | k << 8 | (warp & 7) << 5 | lane      bits 8 and 9
-// so every access, global or shared, is 32 consecutive values per warp.  `sm`: `total` floats.  load(e, k) is asked for values
-// below `total` only; all 1024 threads call.
+// so every access, global or shared, is 32 consecutive values per warp.  The stages come in fht_block's order (0, 1, 10 .. 12,
+// 2 .. 9), so that a value has the same bits whichever of the two computed it.  `sm`: `total` floats; load(e0, v) fills all
+// eight values, those past `total` with zeros; all 1024 threads call.
 constexpr int FHT_WIDE_THREADS = 1024;
 template <class Load, class Store>
 __device__ __forceinline__ void fht_wide(float* sm, int logbs, int total, Load load, Store store) {
@@ -242,17 +243,21 @@ __device__ __forceinline__ void fht_wide(float* sm, int logbs, int total, Load l
         v[k | (1 << s)] = a - b;
       }
   };
-  load(e0, v);
-#pragma unroll
-  for (int s = 0; s < 5; ++s)
-    if (logbs > s && (e0 & ~31) < total) {                 // (uniform per warp)
+  auto lanes = [&](int s) {                                // (uniform per warp)
+    if (logbs > s && (e0 & ~31) < total) {
       const float sg = (lane >> s) & 1 ? -1.f : 1.f;
 #pragma unroll
       for (int k = 0; k < 8; ++k) v[k] = fmaf(v[k], sg, __shfl_xor_sync(0xffffffffu, v[k], 1 << s));
     }
+  };
+  load(e0, v);
+  lanes(0);
+  lanes(1);
 #pragma unroll
   for (int s = 0; s < 3; ++s)
     if (logbs > 10 + s) stage(s);
+#pragma unroll
+  for (int s = 2; s < 5; ++s) lanes(s);
   if (logbs <= 5) {                                        // (no stage crosses a warp)
 #pragma unroll
     for (int k = 0; k < 8; ++k)

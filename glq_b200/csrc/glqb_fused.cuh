@@ -203,9 +203,11 @@ __device__ __forceinline__ void fused_phase1(const DevLinear& L0, int batch, con
 #pragma unroll
                   for (int j = 0; j < E / 4; ++j) load_act4(nw, off + i0 + 4 * j, decltype(dt)::value, w4[j]);
 #pragma unroll
-                  for (int j = 0; j < E / 4; ++j)
+                  for (int j = 0; j < E / 4; ++j) {
+                    ss += q[j][0] * q[j][0] + q[j][1] * q[j][1] + q[j][2] * q[j][2] + q[j][3] * q[j][3];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) { ss += q[j][c] * q[j][c]; q[j][c] *= w4[j][c]; }
+                    for (int c = 0; c < 4; ++c) q[j][c] *= w4[j][c];
+                  }
                 });
               }
 #pragma unroll

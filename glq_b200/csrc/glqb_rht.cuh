@@ -554,7 +554,7 @@ __device__ __forceinline__ void rht_out_body(const DevLinear& L, const RhtItem i
   fht_block(fbuf, log_t, total, load, store);
 }
 
-// The same for launches of few tiles (decode steps).  Whole calls, 256 threads a tile / this: 16 tokens of 4096 x 14336 70.6 /
+// The same for launches of few tiles (decode steps) without per-row scales.  Whole calls, 256 threads a tile / this: 16 tokens of 4096 x 14336 70.6 /
 // 67.3 us, 27 tokens of 11008 x 2048 (4 + 2 bits) 55.0 / 54.2, one token of 14336 x 4096 49.4 / 49.2.
 static __global__ void __launch_bounds__(FHT_WIDE_THREADS, 1) rht_out_wide_kernel(const DevLinear* __restrict__ layers,
                                                               const RhtItem* __restrict__ items,
@@ -571,7 +571,6 @@ static __global__ void __launch_bounds__(FHT_WIDE_THREADS, 1) rht_out_wide_kerne
   const unsigned per_warp = (unsigned)L.per_warp;
   const long long slot_stride = (long long)L.batch * m;
   const float* src = reinterpret_cast<const float*>(ws + L.part_off);
-  const float* row_scale = L.row_scale;
   const int S = it.sub >= 0 ? bs >> FHT_LOG : 1, log_t = min(logbs, FHT_LOG), run0 = max(it.sub, 0) << FHT_LOG;
   const int total = it.ntok << log_t;
   auto slots_of = [&](int row) -> int {                    // (rht_out_body)
@@ -583,7 +582,9 @@ static __global__ void __launch_bounds__(FHT_WIDE_THREADS, 1) rht_out_wide_kerne
   const float rs = rsqrtf((float)bs), wscale = L.wscale;
   const float* rstd = (L.in_norm_w && !L.xr_global) ? reinterpret_cast<const float*>(ws + L.rstd_off) : nullptr;
   const bool stop = L.stop_at_yrht != 0, accumulate = L.y_accumulate != 0;
-  auto load = [&](int e0, float (&v)[8]) {
+  // (the sums in rht_out_body's order, which is another one where it loads groups of four: the same bits)
+  auto load = [&](auto in_fours, int e0, float (&v)[8]) {
+    constexpr bool fours = decltype(in_fours)::value;
 #pragma unroll
     for (int k = 0; k < 8; ++k) v[k] = 0.f;
     for (int kk = 0; kk < S; ++kk) {
@@ -596,7 +597,7 @@ static __global__ void __launch_bounds__(FHT_WIDE_THREADS, 1) rht_out_wide_kerne
         const int e = e0 + (k << 10), row = off + (kk << FHT_LOG) + (e & ((1 << log_t) - 1));
         cnt[k] = e < total && row < m ? slots_of(row) : 0;
         most = max(most, cnt[k]);
-        t[k] = 0.f;
+        t[k] = fours ? v[k] : 0.f;
       }
       for (int s = 0; s < most; ++s) {
         float q[8];
@@ -606,15 +607,14 @@ static __global__ void __launch_bounds__(FHT_WIDE_THREADS, 1) rht_out_wide_kerne
           q[k] = s < cnt[k] ? __ldcg(src + s * slot_stride + (long long)(it.tok0 + (e >> log_t)) * m + row) : 0.f;
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) t[k] += q[k];
+        for (int k = 0; k < 8; ++k) t[k] = fours ? fmaf(q[k], sg, t[k]) : t[k] + q[k];
       }
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        float w = t[k] * wscale;
-        if (row_scale && cnt[k]) w *= row_scale[off + (kk << FHT_LOG) + ((e0 + (k << 10)) & ((1 << log_t) - 1))];
-        v[k] = fmaf(w, sg, v[k]);
-      }
+      for (int k = 0; k < 8; ++k) v[k] = fours ? t[k] : fmaf(t[k] * wscale, sg, v[k]);
     }
+    if (fours)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] *= wscale;
   };
   auto store = [&](int e, float v) {
     const int token = it.tok0 + (e >> log_t), row = off + run0 + (e & ((1 << log_t) - 1));
@@ -628,7 +628,10 @@ static __global__ void __launch_bounds__(FHT_WIDE_THREADS, 1) rht_out_wide_kerne
     }
   };
   pdl_wait();
-  fht_wide(fbuf, stop ? 0 : log_t, total, load, store);
+  if (!stop && ((m | off) & 3) == 0 && log_t >= 2)
+    fht_wide(fbuf, log_t, total, [&](int e0, float (&v)[8]) { load(IntC<1>(), e0, v); }, store);
+  else
+    fht_wide(fbuf, stop ? 0 : log_t, total, [&](int e0, float (&v)[8]) { load(IntC<0>(), e0, v); }, store);
 }
 
 // The prefill case: partial sums in a fixed number of slots, whole blocks, aligned rows, no per-row scales or residual.

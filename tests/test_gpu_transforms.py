@@ -174,6 +174,50 @@ def test_decode_steps_every_block_length(shape, tokens):
             _check(seen, W, L, h.double() - h0.double(), block_decompose(n), block_decompose(m))
 
 
+@pytest.mark.parametrize("kind", ["trellis", "e8"])
+@pytest.mark.parametrize("m", [64, 16352, 16416])
+def test_few_tiles_and_many_give_the_same_bits(m, kind):
+    """A layer alone takes the output transform with 1024 threads per tile (at most a tile per SM), four of it in one plan the
+    general one: every block length from 32 to 8192 (16352) and one that two tiles share (16416)."""
+    from glq_b200 import synth
+    from glq_b200.plan import Plan
+    n, tokens = 32 if kind == "trellis" else 64, 16          # one column group: one partial sum per row, whatever the plan
+    copies = 4 if m > 64 else 160
+    g = torch.Generator(device="cuda").manual_seed(m)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda") if kind == "trellis" else synth.e8_layer("e", m, n, 1, synth.load_e8_table("cuda"), g, "cuda")
+    x = torch.randn(tokens, n, generator=g, device="cuda").half()
+    got = []
+    for k in (1, copies):
+        plan = Plan([L.spec(batch=tokens, x_dtype=x.dtype, y_dtype=torch.float32, y_stride=k * m, y_offset=i * m) for i in range(k)])
+        y = torch.empty(tokens, k, m, device="cuda")
+        plan.run(x, y)
+        plan.close()
+        got.append(y)
+    assert torch.equal(got[1], got[0].expand(tokens, copies, m))
+
+
+@pytest.mark.parametrize("n,copies,step", [(224, 50, "norm"), (2016, 25, "gate")])
+def test_few_and_many_input_tiles_give_the_same_bits(n, copies, step):
+    """The same for the input transform behind a norm or an activation: two layers of different inputs, or many.  (A row of up to
+    256 values is a value per thread in both forms of the norm, so that its sum has one order.)"""
+    from glq_b200 import synth
+    from glq_b200.plan import Plan
+    m = 32
+    g = torch.Generator(device="cuda").manual_seed(n)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda")
+    x = torch.randn(2 * n, generator=g, device="cuda").half()
+    steps = dict(in_norm_weight=1 + 0.2 * torch.randn(n, generator=g, device="cuda"), in_norm_eps=1e-5) if step == "norm" else dict(in_gated_act=0)
+    got = []
+    for k in (2, copies):
+        plan = Plan([L.spec(batch=1, x_dtype=x.dtype, y_dtype=torch.float32, x_stride=2 * n, x_offset=2 * n * i, y_offset=i * m, **steps)
+                     for i in range(k)])
+        y = torch.empty(k, m, device="cuda")
+        plan.run(x.repeat(k), y)
+        plan.close()
+        got.append(y)
+    assert torch.equal(got[1], got[0][:1].expand(copies, m))
+
+
 def test_plan_output_beyond_32_bit_offsets():
     """32769 tokens of a layer of 131072 rows: the last token's partial sums start 2^32 elements in (rows of the result are
     not aligned, so the general body runs).  Against the same token alone."""
