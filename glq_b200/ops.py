@@ -38,6 +38,8 @@ _META_CACHE: dict = {}
 
 
 def _stream(t: torch.Tensor) -> int:
+    if not t.is_cuda:                # (device index -1 would be taken for the current device)
+        raise ValueError(f"glq_b200: expected a CUDA tensor, got one on {t.device}")
     return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 

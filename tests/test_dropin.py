@@ -261,3 +261,16 @@ def test_device_status_surfaces_as_an_error(monkeypatch):
     with pytest.raises(RuntimeError, match=r"code -4.*gave up"):
         ops.check_device_status()
     p.handle = None
+
+
+def test_tensors_of_the_host_are_refused_before_a_launch():
+    """Ops whose first tensor argument is not checked by name take their stream from it: one on the host has none."""
+    import torch
+    from glq_b200 import ops
+    packed, x = torch.zeros(4, 64, dtype=torch.int16), torch.zeros(1, 32)
+    with pytest.raises(ValueError, match="CUDA tensor"):
+        ops.decompress_trellis_3inst_rvq2(packed, packed, 0.1, 32, 32)
+    with pytest.raises(ValueError, match="CUDA tensor"):
+        ops.input_rht_blocks(x, torch.ones(32, dtype=torch.float16), torch.empty(1, 32), 32, 32, [32])
+    with pytest.raises(ValueError, match="CUDA tensor"):
+        ops._stream(x)
