@@ -278,7 +278,17 @@ def _fused_trellis(x, sv, su, packed, packed2, blocks_n, blocks_m, wscale, inv_r
         out = torch.empty(x2d.shape[0], out_features, dtype=out_dtype or x2d.dtype, device=x2d.device)
         tgt, yoff, stop = out, 0, False
     else:
-        tgt, yoff, stop = y_rht_out, int(col), True
+        _require_cuda(y_rht_out, "y_rht_out")
+        tgt, yoff, stop = y_rht_out.view(-1, y_rht_out.shape[-1]), int(col), True
+        if tgt.shape[0] < x2d.shape[0] or yoff < 0 or yoff + m_pad > tgt.shape[1]:
+            raise RuntimeError(f"glq_b200: y_rht_out of {tuple(tgt.shape)} values cannot take {x2d.shape[0]} rows of {m_pad} "
+                               f"from column {yoff} on")
+        if tgt.stride(1) != 1:                     # (the kernels write rows of consecutive values)
+            part = torch.empty(x2d.shape[0], m_pad, dtype=tgt.dtype, device=tgt.device)
+            _fused_trellis(x2d, sv, su, packed, packed2, blocks_n, blocks_m, wscale, inv_rs2, in_features, out_features, n_pad, m_pad,
+                           y_rht_out=part)
+            tgt[:x2d.shape[0], yoff:yoff + m_pad] = part
+            return None
 
     def make_spec(b, x_stride, y_stride, y_offset):
         return LinearSpec(format=_lib.FMT_TRELLIS_3INST, m_pad=m_pad, n_pad=n_pad, in_features=in_features,

@@ -745,3 +745,25 @@ def test_e8_two_phase_prefill_resident_table_equals_global_table(ops, e8_table, 
     ref = O.linear_forward(x.float().cpu().numpy(), W, su, sv, 0.02)
     assert relerr(y_glob.cpu().numpy(), ref) <= TOL
     assert torch.equal(y_smem, y_glob)
+
+
+@pytest.mark.parametrize("tokens", [1, 27, 57, 70])
+def test_rotated_results_go_where_they_fit(ops, tokens):
+    """y_rht_out may hold more rows and columns than a call fills, in any order of its dimensions; one that is too small is
+    refused (nothing is launched)."""
+    from glq_b200 import synth
+    m, n, col = 96, 160, 32
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda")
+    x = torch.randn(tokens, n, generator=g, device="cuda").half()
+    call = lambda out, c: ops.fused_linear_trellis_3inst_yrht(x, L.sv, L.codes[0], None, None, L.wscale, n, n, m, out, c)
+    dense = torch.full((tokens + 2, 160), -7.0, device="cuda")
+    call(dense, col)
+    assert (dense[tokens:] == -7).all() and (dense[:, :col] == -7).all() and (dense[:, col + m:] == -7).all()
+    assert (dense[:tokens, col:col + m] != -7).any()
+    turned = torch.full((160, tokens + 2), -7.0, device="cuda").t()
+    call(turned, col)
+    assert torch.equal(turned, dense)
+    for rows, cols, c in ((tokens - 1, 160, 0), (tokens, m - 1, 0), (tokens, m + col - 1, col), (tokens, 160, -1)):
+        with pytest.raises(RuntimeError, match="y_rht_out"):
+            call(torch.empty(rows, cols, device="cuda"), c)
