@@ -58,6 +58,11 @@ def _blocks(t, fallback: int) -> list[int]:
     return [int(v) for v in t]
 
 
+def _block_key(t):
+    """A Hadamard block list as part of a plan's key: what the caller's list or tensor holds now (None: the default)."""
+    return None if t is None else tuple(t.tolist() if isinstance(t, torch.Tensor) else t)
+
+
 def e8_packed_table(codebook: torch.Tensor) -> torch.Tensor:
     """fp16 (entries, 8) codebook -> cached nibble-packed int32 (entries,) table on its device."""
     _require_cuda(codebook, "codebook")
@@ -301,7 +306,7 @@ def _fused_trellis(x, sv, su, packed, packed2, blocks_n, blocks_m, wscale, inv_r
                           y_accumulate=accumulate_into is not None)
 
     key = ("trellis", packed.data_ptr(), packed2.data_ptr() if has2 else 0, su.data_ptr() if su is not None else 0,
-           sv.data_ptr(), float(wscale), float(inv_rs2), m_pad, n_pad, out_features, stop,
+           sv.data_ptr(), float(wscale), float(inv_rs2), m_pad, n_pad, out_features, stop, _block_key(blocks_n), _block_key(blocks_m),
            in_norm_weight.data_ptr() if in_norm_weight is not None else 0, float(in_norm_eps), gated_act,
            accumulate_into is not None)
     # two decoded stages keep two accumulator sets: 32 tokens per pass instead of 64
@@ -560,7 +565,7 @@ def _fused_e8(x, sv, su, codes, tables, scales, wscale, in_features, out_feature
 
     key = ("e8", tuple(c.data_ptr() for c in codes), tuple(t.data_ptr() for t in tables), tuple(scales),
            su.data_ptr(), sv.data_ptr(), float(wscale), m_pad, n_pad, in_features, out_features, stop, x_is_rotated,
-           in_norm_weight.data_ptr() if in_norm_weight is not None else 0, float(in_norm_eps), gated_act,
+           _block_key(bn), _block_key(bm), in_norm_weight.data_ptr() if in_norm_weight is not None else 0, float(in_norm_eps), gated_act,
            accumulate_into is not None)
     _run_sliced(x2d, out, key, make_spec, 32 if len(codes) > 2 else DECODE_MAX_TOKENS, comm=comm)
     return accumulate_into if accumulate_into is not None else out

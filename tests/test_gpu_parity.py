@@ -767,3 +767,34 @@ def test_rotated_results_go_where_they_fit(ops, tokens):
     for rows, cols, c in ((tokens - 1, 160, 0), (tokens, m - 1, 0), (tokens, m + col - 1, col), (tokens, 160, -1)):
         with pytest.raises(RuntimeError, match="y_rht_out"):
             call(torch.empty(rows, cols, device="cuda"), c)
+
+
+@pytest.mark.parametrize("tokens", [1, 27, 70])
+@pytest.mark.parametrize("kind", ["trellis", "e8"])
+def test_block_lists_are_read_on_every_call(ops, e8_cb, kind, tokens):
+    """The same weights with other Hadamard blocks are another layer, also behind a first call and in the same tensor; a list
+    that does not add up is refused."""
+    from glq_b200 import synth
+    m = n = 256
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda") if kind == "trellis" else synth.e8_layer("e", m, n, 1, synth.load_e8_table("cuda"), g, "cuda")
+    x = torch.randn(tokens, n, generator=g, device="cuda")
+    if kind == "trellis":
+        call = lambda bn, bm: ops.fused_linear_trellis_3inst(x, L.sv, L.su, L.codes[0], bn, bm, None, None, L.wscale, n, m, n, m)
+    else:
+        call = lambda bn, bm: ops.fused_linear_block_diag(x, L.sv, L.su, L.codes[0], e8_cb[0], L.wscale, n, m, n, m, bn, bm, None, None)
+    lists = [([256], [256]), ([128, 128], [256]), ([256], [128, 64, 64])]
+    ops.clear_caches()
+    first = [call(bn, bm) for bn, bm in lists]
+    held = torch.tensor([64, 128, 64])
+    held[:] = torch.tensor([128, 64, 64])
+    assert torch.equal(call([256], held), first[2])
+    held[:] = torch.tensor([64, 64, 128])
+    other = call([256], held)
+    for (bn, bm), y in zip(lists + [([256], [64, 64, 128])], first + [other]):
+        ops.clear_caches()
+        assert torch.equal(call(bn, bm), y)
+    assert not any(torch.equal(first[0], y) for y in first[1:] + [other])
+    for bn, bm in (([256, 32], [256]), ([256], [128])):
+        with pytest.raises(RuntimeError, match="blocks"):
+            call(bn, bm)
