@@ -391,8 +391,9 @@ def fused_linear_trellis_3inst_shards(x, sv, shards, blocks_n=None, out_dtype=No
     bb = token_bucket(B)
     xin = x2d
     out = torch.empty((B, total_m), dtype=odt, device=x2d.device)
-    key = ("trellis_shards", tuple(sh[1].data_ptr() for sh in shards), sv.data_ptr(), tuple(float(sh[3]) for sh in shards),
-           bb, xin.dtype, odt, xin.stride(0), in_norm_weight.data_ptr() if in_norm_weight is not None else 0, float(in_norm_eps))
+    parts = tuple((su.data_ptr(), p.data_ptr(), p2.data_ptr(), float(w), float(inv), int(m)) if p2 is not None and p2.numel() > 0 else
+                  (su.data_ptr(), p.data_ptr(), float(w), int(m)) for su, p, p2, w, inv, m in shards)
+    key = ("trellis_shards", parts, sv.data_ptr(), tuple(bn), bb, xin.dtype, odt, xin.stride(0), in_norm_weight.data_ptr() if in_norm_weight is not None else 0, float(in_norm_eps))
 
     def make_specs():
         specs, col = [], 0
@@ -435,8 +436,9 @@ def fused_linear_e8_shards(x, sv, shards, codebook, codebook2=None, blocks_n=Non
     out = torch.empty((B, total_m), dtype=odt, device=x2d.device)
     t1 = e8_packed_table(codebook)
     t2 = e8_packed_table(codebook2) if codebook2 is not None else t1
-    key = ("e8_shards", tuple(sh[1][0].data_ptr() for sh in shards), sv.data_ptr(), tuple(float(sh[3]) for sh in shards),
-           t1.data_ptr(), t2.data_ptr(), bb, xin.dtype, odt, xin.stride(0),
+    parts = tuple((su.data_ptr(), tuple(q.data_ptr() for q in qs), tuple(float(v) for v in inv), float(w), int(m))
+                  for su, qs, inv, w, m in shards)
+    key = ("e8_shards", parts, sv.data_ptr(), tuple(bn), t1.data_ptr(), t2.data_ptr(), bb, xin.dtype, odt, xin.stride(0),
            in_norm_weight.data_ptr() if in_norm_weight is not None else 0, float(in_norm_eps))
 
     def make_specs():

@@ -798,3 +798,31 @@ def test_block_lists_are_read_on_every_call(ops, e8_cb, kind, tokens):
     for bn, bm in (([256, 32], [256]), ([256], [128])):
         with pytest.raises(RuntimeError, match="blocks"):
             call(bn, bm)
+
+
+@pytest.mark.parametrize("tokens", [1, 27])
+@pytest.mark.parametrize("kind", ["trellis", "e8"])
+def test_shards_of_one_packed_tensor_differ_by_every_argument(ops, e8_cb, kind, tokens):
+    """Calls that share their first code tensors but differ in signs, second-stage codes, residual scale, input blocks or the
+    split of the columns give the results of fresh plans."""
+    from glq_b200 import synth
+    n = 256
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    if kind == "trellis":
+        A, B = (synth.trellis_layer("t", 128, n, [4, 2], g, "cuda") for _ in range(2))
+        part = lambda su, c2, inv, m: (su, A.codes[0], c2, A.wscale, inv, m)
+        call = lambda parts, bn: ops.fused_linear_trellis_3inst_shards(x, A.sv, parts, bn)
+    else:
+        A, B = (synth.e8_layer("e", 128, n, 2, synth.load_e8_table("cuda"), g, "cuda") for _ in range(2))
+        part = lambda su, c2, inv, m: (su, [A.codes[0], c2], [inv], A.wscale, m)
+        call = lambda parts, bn: ops.fused_linear_e8_shards(x, A.sv, parts, e8_cb[0], None, bn)
+    x = torch.randn(tokens, n, generator=g, device="cuda")
+    variants = [([part(A.su, A.codes[1], 0.2, 128)] * 2, [256]), ([part(A.su, A.codes[1], 0.2, 128)] * 2, [128, 128]),
+                ([part(B.su, A.codes[1], 0.2, 128)] * 2, [256]), ([part(A.su, B.codes[1], 0.2, 128)] * 2, [256]),
+                ([part(A.su, A.codes[1], 0.1, 128)] * 2, [256]), ([part(A.su, A.codes[1], 0.2, 96)] * 2, [256])]
+    ops.clear_caches()
+    got = [call(*v) for v in variants]
+    for v, y in zip(variants, got):
+        ops.clear_caches()
+        assert torch.equal(call(*v), y)
+    assert not any(y.shape == got[0].shape and torch.equal(got[0], y) for y in got[1:])
