@@ -59,8 +59,15 @@ def _blocks(t, fallback: int) -> list[int]:
 
 
 def _block_key(t):
-    """A Hadamard block list as part of a plan's key: what the caller's list or tensor holds now (None: the default)."""
-    return None if t is None else tuple(t.tolist() if isinstance(t, torch.Tensor) else t)
+    """A Hadamard block list as part of a plan's key: what the caller's list or tensor holds now (None: the default).  One on the
+    device goes by its address and version, since reading it would wait for the device and end a capture; the plan keeps it."""
+    if t is None:
+        return None
+    if not isinstance(t, torch.Tensor):
+        return tuple(t)
+    if t.is_cuda:
+        return (t.data_ptr(), t.numel(), t.stride(), t.dtype, 0 if t.is_inference() else t._version)
+    return tuple(t.tolist())
 
 
 def e8_packed_table(codebook: torch.Tensor) -> torch.Tensor:
@@ -303,7 +310,7 @@ def _fused_trellis(x, sv, su, packed, packed2, blocks_n, blocks_m, wscale, inv_r
                           blocks_n=_blocks(blocks_n, n_pad), blocks_m=_blocks(blocks_m, m_pad), batch=b, x_dtype=x2d.dtype, y_dtype=tgt.dtype,
                           x_stride=x_stride, y_stride=y_stride, y_offset=y_offset, stop_at_yrht=stop,
                           in_norm_weight=in_norm_weight, in_norm_eps=in_norm_eps, in_gated_act=gated_act,
-                          y_accumulate=accumulate_into is not None)
+                          y_accumulate=accumulate_into is not None, keep=[blocks_n, blocks_m])
 
     key = ("trellis", packed.data_ptr(), packed2.data_ptr() if has2 else 0, su.data_ptr() if su is not None else 0,
            sv.data_ptr(), float(wscale), float(inv_rs2), m_pad, n_pad, out_features, stop, _block_key(blocks_n), _block_key(blocks_m),
@@ -563,7 +570,7 @@ def _fused_e8(x, sv, su, codes, tables, scales, wscale, in_features, out_feature
                           batch=b, x_dtype=x2d.dtype, y_dtype=odt, x_stride=x_stride, y_stride=y_stride,
                           y_offset=y_offset, stop_at_yrht=stop, x_is_rotated=x_is_rotated,
                           in_norm_weight=in_norm_weight, in_norm_eps=in_norm_eps, in_gated_act=gated_act,
-                          y_accumulate=accumulate_into is not None)
+                          y_accumulate=accumulate_into is not None, keep=[bn, bm])
 
     key = ("e8", tuple(c.data_ptr() for c in codes), tuple(t.data_ptr() for t in tables), tuple(scales),
            su.data_ptr(), sv.data_ptr(), float(wscale), m_pad, n_pad, in_features, out_features, stop, x_is_rotated,

@@ -826,3 +826,25 @@ def test_shards_of_one_packed_tensor_differ_by_every_argument(ops, e8_cb, kind, 
         ops.clear_caches()
         assert torch.equal(call(*v), y)
     assert not any(y.shape == got[0].shape and torch.equal(got[0], y) for y in got[1:])
+
+
+def test_block_lists_on_the_device(ops):
+    """A list on the device is read for a new plan, not on every call (which could not be captured), and again when it was
+    written to."""
+    from glq_b200 import synth
+    m = n = 256
+    g = torch.Generator(device="cuda").manual_seed(3)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda")
+    x = torch.randn(2, n, generator=g, device="cuda")
+    call = lambda bn: ops.fused_linear_trellis_3inst(x, L.sv, L.su, L.codes[0], bn, None, None, None, L.wscale, n, m, n, m)
+    ref = [call([128, 64, 64]), call([64, 64, 128])]
+    held = torch.tensor([128, 64, 64], device="cuda")
+    assert torch.equal(call(held), ref[0])
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=side):
+        y = call(held)
+    graph.replay()
+    assert torch.equal(y, ref[0])
+    held.copy_(torch.tensor([64, 64, 128]))
+    assert torch.equal(call(held), ref[1])
