@@ -118,7 +118,10 @@ def _cached_plan(key, make_specs) -> Plan:
     if p is not None:
         _PLAN_CACHE.move_to_end(key)
         return p
-    p = Plan(make_specs(), own_workspace=False)
+    return _keep_plan(key, Plan(make_specs(), own_workspace=False))
+
+
+def _keep_plan(key, p):
     _PLAN_CACHE[key] = p
     if len(_PLAN_CACHE) > PLAN_CACHE_MAX and not torch.cuda.is_current_stream_capturing():
         # evict the least recently used plans; their device tables may still be read by queued work
@@ -759,6 +762,10 @@ class MoePlan:
             self.handle = None
 
 
+def _ptrs(*tensors) -> tuple:
+    return tuple(t.data_ptr() if t is not None else 0 for t in tensors)
+
+
 def _moe_capacity(tokens: int) -> int:
     cap = 16
     while cap < tokens:
@@ -792,8 +799,13 @@ def fused_moe_trellis_3inst(x, topk_ids, topk_weights,
     has2 = w2_trellis_packed2 is not None and w2_trellis_packed2.numel() > E
     cap = _moe_capacity(T)
     odt = out_dtype or x.dtype
-    key = ("moe3", w13_trellis_packed.data_ptr(), w2_trellis_packed.data_ptr(), cap, ids.shape[1], x.dtype, ids.dtype,
-           int(activation_type), has13, has2, odt)
+    # all that the plan is built from, by address (it keeps the tensors, so that an address stays theirs) or by value
+    weights = [w13_trellis_packed, w13_trellis_packed2 if has13 else None, w13_SU, w13_SV, w13_Wscale,
+               w13_inv_resid_scale2 if has13 else None, w2_trellis_packed, w2_trellis_packed2 if has2 else None, w2_SU, w2_SV, w2_Wscale,
+               w2_inv_resid_scale2 if has2 else None]
+    key = ("moe3", _ptrs(*weights), hidden_size, intermediate_size, w13_out_features, n_pad_w13, m_pad_w13, n_pad_w2, m_pad_w2,
+           _block_key(blocks_n_w13), _block_key(blocks_m_w13), _block_key(blocks_n_w2), _block_key(blocks_m_w2), cap, ids.shape[1], x.dtype,
+           ids.dtype, int(activation_type), odt)
     plan = _PLAN_CACHE.get(key)
     if plan is not None:
         _PLAN_CACHE.move_to_end(key)
@@ -817,9 +829,7 @@ def fused_moe_trellis_3inst(x, topk_ids, topk_weights,
         _fill_moe_blocks(d, blocks_n_w13, n_pad_w13, blocks_m_w13, m_pad_w13, blocks_n_w2, n_pad_w2, blocks_m_w2, m_pad_w2)
         d.ids_are_int64 = 1 if ids.dtype == torch.int64 else 0
         d.x_dtype, d.y_dtype = _dt(x.dtype), _dt(odt)
-        plan = MoePlan(d, x.device, [w13_trellis_packed, w13_trellis_packed2, w13_SU, w13_SV, ws13, i13,
-                                     w2_trellis_packed, w2_trellis_packed2, w2_SU, w2_SV, ws2, i2])
-        _PLAN_CACHE[key] = plan
+        plan = _keep_plan(key, MoePlan(d, x.device, [weights, ws13, i13, ws2, i2]))
     y = torch.empty(T, hidden_size, dtype=odt, device=x.device)
     plan.run(x, ids, tw, y)
     return y
@@ -869,12 +879,14 @@ def fused_moe_grouped_gemm(x, topk_ids, topk_weights,
               q13.numel() == full13 and q2.numel() == full2 and cb.numel() > 0 and i13.numel() == E and i2.numel() == E)
         if not ok:
             break
-        stages13.append((q13, i13.to(torch.float32).contiguous(), cb))
-        stages2.append((q2, i2.to(torch.float32).contiguous(), cb))
+        stages13.append((q13, i13, cb))
+        stages2.append((q2, i2, cb))
     ns = len(stages13)
     cap = _moe_capacity(T)
-    key = ("moe_e8", tuple(s[0].data_ptr() for s in stages13), tuple(s[0].data_ptr() for s in stages2), cap,
-           ids.shape[1], x.dtype, ids.dtype, int(activation_type))
+    weights = [w13_SU, w13_SV, w13_Wscale, w2_SU, w2_SV, w2_Wscale]
+    key = ("moe_e8", _ptrs(*weights), tuple(_ptrs(*s) for s in stages13), tuple(_ptrs(*s) for s in stages2), hidden_size,
+           intermediate_size, w13_out_features, _block_key(blocks_n_w13), _block_key(blocks_m_w13), _block_key(blocks_n_w2),
+           _block_key(blocks_m_w2), cap, ids.shape[1], x.dtype, ids.dtype, int(activation_type))
     plan = _PLAN_CACHE.get(key)
     if plan is None:
         d = _lib.MoeDesc()
@@ -884,21 +896,21 @@ def fused_moe_grouped_gemm(x, topk_ids, topk_weights,
         ws13 = w13_Wscale.to(torch.float32).contiguous()
         ws2 = w2_Wscale.to(torch.float32).contiguous()
         tables = [e8_packed_table(s[2]) for s in stages13]
+        inv13, inv2 = ([s[1].to(torch.float32).contiguous() for s in st[1:]] for st in (stages13, stages2))
         for s in range(ns):
             d.w13_qidxs[s] = stages13[s][0].data_ptr()
             d.w2_qidxs[s] = stages2[s][0].data_ptr()
             d.e8_table[s] = tables[s].data_ptr()
             d.e8_table_entries[s] = tables[s].numel()
             if s:
-                d.w13_inv_rs[s - 1] = stages13[s][1].data_ptr()
-                d.w2_inv_rs[s - 1] = stages2[s][1].data_ptr()
+                d.w13_inv_rs[s - 1] = inv13[s - 1].data_ptr()
+                d.w2_inv_rs[s - 1] = inv2[s - 1].data_ptr()
         d.w13_su, d.w13_sv, d.w13_wscale = w13_SU.data_ptr(), w13_SV.data_ptr(), ws13.data_ptr()
         d.w2_su, d.w2_sv, d.w2_wscale = w2_SU.data_ptr(), w2_SV.data_ptr(), ws2.data_ptr()
         _fill_moe_blocks(d, blocks_n_w13, n_pad_w13, blocks_m_w13, m_pad_w13, blocks_n_w2, n_pad_w2, blocks_m_w2, m_pad_w2)
         d.ids_are_int64 = 1 if ids.dtype == torch.int64 else 0
         d.x_dtype = d.y_dtype = _dt(x.dtype)
-        plan = MoePlan(d, x.device, [stages13, stages2, tables, w13_SU, w13_SV, ws13, w2_SU, w2_SV, ws2])
-        _PLAN_CACHE[key] = plan
+        plan = _keep_plan(key, MoePlan(d, x.device, [weights, stages13, stages2, tables, inv13, inv2, ws13, ws2]))
     else:
         _PLAN_CACHE.move_to_end(key)
     y = torch.empty(T, hidden_size, dtype=x.dtype, device=x.device)

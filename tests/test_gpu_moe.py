@@ -281,3 +281,33 @@ def test_moe_grouping_sizes(T, monkeypatch):
     cut = T // 2 + 3
     assert torch.equal(y, torch.cat([run(0, cut), run(cut, T)]))
     ops.clear_caches()
+
+
+@pytest.mark.parametrize("T", [5, 200])
+def test_moe_plans_differ_by_every_argument(T):
+    """Steps on the same packed weights with other signs, scales, second-stage scales or blocks give what fresh plans give."""
+    from glq_b200 import ops
+    E, hidden, inter, k = 8, 256, 128, 2
+    rng = np.random.default_rng(T)
+    d, w13_out = _make(rng, E, hidden, inter, 4, 2)
+    o, _ = _make(rng, E, hidden, inter, 4, 2)
+    d, o = ({key: cuda(v) for key, v in t.items()} for t in (d, o))
+    x = cuda(rng.standard_normal((T, hidden)).astype(np.float32), torch.float16)
+    ids = cuda(np.stack([rng.permutation(E)[:k] for _ in range(T)]).astype(np.int64))
+    w = cuda(rng.random((T, k)).astype(np.float32))
+    bl = [O.block_decompose(v) for v in (hidden, w13_out, inter, hidden)]
+
+    def call(t, b):
+        return ops.fused_moe_trellis_3inst(x, ids, w, t["w13"], t["w13_2"], t["su13"], t["sv13"], t["ws13"], t["inv13"], t["w2"], t["w2_2"],
+                                           t["su2"], t["sv2"], t["ws2"], t["inv2"], hidden, inter, w13_out, hidden, w13_out, inter, hidden,
+                                           b[0], b[1], None, None, b[2], b[3], None, None, 0)
+    o["ws13"], o["ws2"], o["inv13"], o["inv2"] = 2 * d["ws13"], 2 * d["ws2"], 2 * d["inv13"], 2 * d["inv2"]
+    variants = [(d, bl)] + [(dict(d, **{key: o[key]}), bl) for key in ("w13_2", "su13", "sv13", "ws13", "inv13", "w2_2", "su2", "sv2", "ws2", "inv2")]
+    variants += [(d, bl[:i] + [[bl[i][0] // 2] * 2] + bl[i + 1:]) for i in range(4)]
+    ops.clear_caches()
+    got = [call(*v) for v in variants]
+    for v, y in zip(variants, got):
+        ops.clear_caches()
+        assert torch.equal(call(*v), y)
+    assert not any(torch.equal(got[0], y) for y in got[1:])
+    ops.clear_caches()
