@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -66,7 +67,12 @@ struct GlqbPlan {
   DevLinear* d_few_layers = nullptr;
   GemmItem* d_few_items = nullptr;
   int* d_status = nullptr;
-  int* d_tickets = nullptr;      // completion tickets of the single-launch form, all zero between runs
+  // Completion tickets of the single-launch form, all zero between runs.  A set belongs to a workspace: runs on one workspace
+  // follow one another, runs that may overlap (other streams, a graph beside eager calls) have a workspace each.
+  struct TicketSet { const void* workspace; int* tickets; bool captured; };     // captured: a graph may replay on it at any time
+  std::mutex ticket_mutex;
+  std::vector<TicketSet> ticket_sets;
+  std::vector<int*> free_tickets, ticket_chunks;
   const GlqbComm* comm = nullptr;  // tensor-parallel ranks whose outputs the single-launch kernel sums (glqb_plan_set_comm)
   int n_tickets = 0;
   int max_batch_gemm = 1;
@@ -465,6 +471,58 @@ static void add_rht_items(std::vector<RhtItem>& items, const std::vector<RhtLaye
         max_elems = std::max(max_elems, nt * bs);
       }
     }
+}
+
+constexpr int TICKET_SETS = 64;                  // sets allocated at a time
+// Another TICKET_SETS sets.  `running`: for a run, which may be under capture (a stream of its own clears them; making one takes
+// 0.2 ms, which a new plan does not pay).
+static int add_ticket_sets(GlqbPlan* P, bool running) {
+  const size_t n = P->n_tickets, bytes = n * TICKET_SETS * sizeof(int);
+  int* p = nullptr;
+  cudaStream_t st = nullptr;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (running) CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+  cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaSuccess) P->ticket_chunks.push_back(p);
+  if (e == cudaSuccess && running) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = running ? cudaMemsetAsync(p, 0, bytes, st) : cudaMemset(p, 0, bytes);
+  if (e == cudaSuccess && running) e = cudaStreamSynchronize(st);
+  if (st) cudaStreamDestroy(st);
+  if (running) cudaThreadExchangeStreamCaptureMode(&mode);
+  CUDA_TRY(e);
+  for (int i = TICKET_SETS - 1; i >= 0; --i) P->free_tickets.push_back(p + i * n);
+  return GLQB_OK;
+}
+
+// The tickets of a run in `workspace`.  A caller with ever new workspaces gets the sets of its earlier ones again, behind a
+// device synchronisation; sets that a graph holds stay its own.
+static int tickets_for(GlqbPlan* P, const void* workspace, cudaStream_t stream, int** out) {
+  std::lock_guard<std::mutex> hold(P->ticket_mutex);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CUDA_TRY(cudaStreamIsCapturing(stream, &capture));
+  const bool captured = capture != cudaStreamCaptureStatusNone;
+  for (GlqbPlan::TicketSet& t : P->ticket_sets)
+    if (t.workspace == workspace) {
+      t.captured = t.captured || captured;
+      *out = t.tickets;
+      return GLQB_OK;
+    }
+  if (P->free_tickets.empty() && !captured) {
+    CUDA_TRY(cudaDeviceSynchronize());
+    size_t kept = 0;
+    for (const GlqbPlan::TicketSet& t : P->ticket_sets)
+      if (t.captured) P->ticket_sets[kept++] = t;
+      else P->free_tickets.push_back(t.tickets);
+    P->ticket_sets.resize(kept);
+  }
+  if (P->free_tickets.empty()) {
+    const int rc = add_ticket_sets(P, true);
+    if (rc) return rc;
+  }
+  P->ticket_sets.push_back({workspace, P->free_tickets.back(), captured});
+  P->free_tickets.pop_back();
+  *out = P->ticket_sets.back().tickets;
+  return GLQB_OK;
 }
 
 static int build_plan(GlqbPlan* P) {
@@ -935,8 +993,10 @@ static int build_plan(GlqbPlan* P) {
                       cudaMemcpyHostToDevice));
   CUDA_TRY(cudaMalloc(&P->d_status, sizeof(int)));
   CUDA_TRY(cudaMemset(P->d_status, 0, sizeof(int)));
-  CUDA_TRY(cudaMalloc(&P->d_tickets, sizeof(int) * std::max(1, P->n_tickets)));
-  CUDA_TRY(cudaMemset(P->d_tickets, 0, sizeof(int) * std::max(1, P->n_tickets)));
+  if (P->n_tickets) {
+    const int rc = add_ticket_sets(P, false);
+    if (rc) return rc;
+  }
   CUDA_TRY(cudaMalloc(&P->d_items_out, sizeof(RhtItem) * std::max<size_t>(1, P->items_out.size())));
   CUDA_TRY(cudaMemcpy(P->d_items_out, P->items_out.data(), sizeof(RhtItem) * P->items_out.size(), cudaMemcpyHostToDevice));
   return GLQB_OK;
@@ -1026,6 +1086,11 @@ int glqb_plan_run_tokens(GlqbPlan* P, const void* x_base, void* y_base, int32_t 
     return fail(GLQB_E_WORKSPACE, "workspace must be 256-byte aligned");
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
+  int* tickets = nullptr;
+  if (P->n_tickets) {
+    const int rc = tickets_for(P, workspace, stream, &tickets);
+    if (rc) return rc;
+  }
   if (!P->items_in.empty()) {
     launch_chained(true, P->in_few ? rht_in_wide_kernel : rht_in_kernel<false>, (int)P->items_in.size(), P->in_few ? FHT_WIDE_THREADS : RHT_THREADS,
                    rht_smem(P->max_elems_in), stream, d_layers, P->d_items_in, reinterpret_cast<const uint8_t*>(x_base), ws, tokens);
@@ -1045,7 +1110,7 @@ int glqb_plan_run_tokens(GlqbPlan* P, const void* x_base, void* y_base, int32_t 
   for (const Segment& s : segs) {
     if (s.fused) {
       fused_launch(s, P->dev.data() + s.first, reinterpret_cast<const uint8_t*>(x_base), reinterpret_cast<uint8_t*>(y_base),
-                   ws, P->d_tickets, P->comm ? comm_dev(P->comm) : nullptr, stream);
+                   ws, tickets, P->comm ? comm_dev(P->comm) : nullptr, stream);
     } else if (s.tn) {
       gemm_launch(s, d_layers, d_gemm_items + s.item_first, ws, P->d_status, P->sm_count, tokens, stream);
     } else if (s.smem_table) {
@@ -1136,7 +1201,7 @@ void glqb_plan_destroy(GlqbPlan* plan) {
   if (plan->d_items_in_gemm) cudaFree(plan->d_items_in_gemm);
   if (plan->d_gemm_items) cudaFree(plan->d_gemm_items);
   if (plan->d_status) cudaFree(plan->d_status);
-  if (plan->d_tickets) cudaFree(plan->d_tickets);
+  for (int* p : plan->ticket_chunks) cudaFree(p);
   for (cudaEvent_t e : plan->ev) cudaEventDestroy(e);
   delete plan;
 }

@@ -104,7 +104,8 @@ int64_t glqb_plan_flops(const GlqbPlan* plan);
 /* kernels launched by one glqb_plan_run */
 int32_t glqb_plan_launches(const GlqbPlan* plan);
 /* Enqueue on `stream`; returns without synchronising.  x_base / y_base are device pointers the
- * descriptors' offsets are applied to. */
+ * descriptors' offsets are applied to.  Runs of a plan may overlap (other streams, graph replays) when each has a workspace
+ * of its own. */
 int glqb_plan_run(GlqbPlan* plan, const void* x_base, void* y_base,
                   void* workspace, size_t workspace_bytes, void* stream);
 /* The same for the first `tokens` tokens (>= 1; layers of fewer take all of theirs): no other row of x is read, no other

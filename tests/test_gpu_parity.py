@@ -848,3 +848,64 @@ def test_block_lists_on_the_device(ops):
     assert torch.equal(y, ref[0])
     held.copy_(torch.tensor([64, 64, 128]))
     assert torch.equal(call(held), ref[1])
+
+
+@pytest.mark.parametrize("kind", ["trellis", "e8"])
+def test_one_layer_on_several_streams(ops, e8_cb, kind):
+    """Single-launch decode calls of one layer on two streams at a time, beside a graph replayed on a third, then alone: every
+    output block is completed by the run it belongs to."""
+    from glq_b200 import synth
+    m, n, calls = 544, 1024, 40
+    g = torch.Generator(device="cuda").manual_seed(11)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda") if kind == "trellis" else synth.e8_layer("e", m, n, 1, synth.load_e8_table("cuda"), g, "cuda")
+    xs = [torch.randn(1, n, generator=g, device="cuda") for _ in range(3)]
+    if kind == "trellis":
+        call = lambda x: ops.fused_linear_trellis_3inst(x, L.sv, L.su, L.codes[0], None, None, None, None, L.wscale, n, m, n, m)
+    else:
+        call = lambda x: ops.fused_linear_block_diag(x, L.sv, L.su, L.codes[0], e8_cb[0], L.wscale, n, m, n, m, None, None, None, None)
+    refs = [call(x) for x in xs]
+    torch.cuda.synchronize()
+    streams, graph, held = [torch.cuda.Stream() for _ in range(3)], torch.cuda.CUDAGraph(), []
+    with torch.cuda.graph(graph, stream=streams[2]):
+        for _ in range(calls):
+            held.append(call(xs[2]))
+    got = [[], []]
+    for _ in range(3):
+        with torch.cuda.stream(streams[2]):
+            graph.replay()
+        for _ in range(calls):
+            for i in range(2):
+                with torch.cuda.stream(streams[i]):
+                    got[i].append(call(xs[i]))
+    torch.cuda.synchronize()
+    for ys, ref in zip(got + [held], refs):
+        assert all(torch.equal(y, ref) for y in ys)
+    assert all(torch.equal(call(x), ref) for x, ref in zip(xs, refs))
+
+
+def test_a_plan_in_many_workspaces():
+    """More workspaces than a plan has tickets for at first, outside and inside a capture."""
+    from glq_b200 import synth
+    from glq_b200.plan import Plan
+    m, n = 96, 256
+    g = torch.Generator(device="cuda").manual_seed(12)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda")
+    x = torch.randn(1, n, generator=g, device="cuda")
+    plan = Plan([L.spec(batch=1, x_dtype=x.dtype, y_dtype=torch.float32)], own_workspace=False)
+    size = -(-plan.workspace_bytes // 256) * 256
+    area = torch.empty(200 * size, dtype=torch.uint8, device="cuda")
+    y = torch.empty(200, m, device="cuda")
+    run = lambda a, b: [plan.run(x, y[i], workspace=area[i * size:(i + 1) * size]) for i in range(a, b)]
+    run(0, 150)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        run(100, 200)
+    run(0, 100)
+    y[100:] = 0
+    graph.replay()
+    run(0, 150)
+    graph.replay()
+    torch.cuda.synchronize()
+    plan.close()
+    assert (y[0] != 0).any() and torch.equal(y, y[:1].expand(200, m))
