@@ -640,15 +640,13 @@ static int build_plan(GlqbPlan* P) {
       }
       for (int i = 1; i < s.count && ok; ++i) ok = same_input(d0, P->descs[P->order[s.first + i]]);
       if (!e8) ok = ok && d0.in_features == d0.n_pad;   // (trellis layers are never padded; the kernel's loads rely on it)
-      if (e8) {
-        // E8 strips are 16 rows: every output block must hold whole strips; the in-kernel input transform takes
-        // blocks of 32 values or more
-        for (int i = 0; i < s.count && ok; ++i) {
-          const GlqbLinearDesc& d = P->descs[P->order[s.first + i]];
-          for (int b = 0; b < d.n_blocks_m; ++b) ok = ok && d.blocks_m[b] >= 16;
-        }
-        for (int b = 0; b < d0.n_blocks_n; ++b) ok = ok && d0.blocks_n[b] >= 32;
+      // The transforms inside the kernel hold a warp's values at least (fht_fast: with fewer its shuffles would wait for lanes
+      // that never come), and an output block holds whole strips: lists with blocks of less than 32 values take the other form.
+      for (int i = 0; i < s.count && ok; ++i) {
+        const GlqbLinearDesc& d = P->descs[P->order[s.first + i]];
+        for (int b = 0; b < d.n_blocks_m; ++b) ok = ok && d.blocks_m[b] >= 32;
       }
+      for (int b = 0; b < d0.n_blocks_n; ++b) ok = ok && d0.blocks_n[b] >= 32;
       // wide inputs are transformed once by rht_in_kernel (every CTA recomputing them would cost more than
       // the extra launch); so is a fused RMSNorm whose output block is too long for the in-kernel transform
       static const int in_max_n = [] { const char* e = getenv("GLQB_FUSED_IN_MAX_N"); return e ? atoi(e) : 4096; }();

@@ -218,6 +218,26 @@ def test_few_and_many_input_tiles_give_the_same_bits(n, copies, step):
     assert torch.equal(got[1], got[0][:1].expand(copies, m))
 
 
+@pytest.mark.parametrize("tokens", [1, 8, 9])
+@pytest.mark.parametrize("bn,bm", [([64], [32, 16]), ([64], [16, 16]), ([64, 8], [64, 16, 8, 2]), ([16, 32, 16], [16, 32, 8, 8])], ids=str)
+def test_blocks_shorter_than_a_warp(bn, bm, tokens):
+    """Output and input blocks of less than 32 values, which the transforms inside the single-launch kernel cannot take."""
+    from glq_b200 import synth
+    m, n = sum(bm), sum(bn)
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    x = torch.randn(tokens, n, generator=g, device="cuda")
+    table = synth.load_e8_table("cuda")
+    nib = (table.cpu().numpy().view(np.uint32)[:, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15
+    cb = nib.astype(np.float64) * 0.5 - 3.0
+    E = synth.e8_layer("e", m, n, 1, table, g, "cuda")
+    y = ops.fused_linear_block_diag(x, E.sv, E.su, E.codes[0], torch.from_numpy(cb).to("cuda", torch.float16), E.wscale, n, m, n, m, bn, bm, None, None)
+    _check(x, cb[E.codes[0].cpu().numpy().view(np.uint16)].reshape(m, n), E, y, bn, bm)
+    if m % 32 == 0 and n % 32 == 0:
+        L = synth.trellis_layer("t", m, n, [4], g, "cuda")
+        y = ops.fused_linear_trellis_3inst(x, L.sv, L.su, L.codes[0], bn, bm, None, None, L.wscale, n, m, n, m)
+        _check(x, ops.glq_decompress_trellis_3inst_cuda(L.codes[0], m, n).double().cpu().numpy(), L, y, bn, bm)
+
+
 def test_plan_output_beyond_32_bit_offsets():
     """32769 tokens of a layer of 131072 rows: the last token's partial sums start 2^32 elements in (rows of the result are
     not aligned, so the general body runs).  Against the same token alone."""
