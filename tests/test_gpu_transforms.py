@@ -238,6 +238,39 @@ def test_blocks_shorter_than_a_warp(bn, bm, tokens):
         _check(x, ops.glq_decompress_trellis_3inst_cuda(L.codes[0], m, n).double().cpu().numpy(), L, y, bn, bm)
 
 
+@pytest.mark.parametrize("kind", ["trellis", "e8"])
+def test_one_cta_completes_many_output_blocks(kind):
+    """Seven layers of sixteen output blocks of 32 rows (one strip, E8: two) beside one of 12288 strips (E8: 22528): a CTA takes
+    some 41 (76 or more) strips in a row, and with them more than 32 blocks."""
+    from glq_b200 import synth
+    from glq_b200.plan import Plan
+    n, m, big = 64, 512, (12 if kind == "trellis" else 11) * 32768
+    g = torch.Generator(device="cuda").manual_seed(big)
+    table = synth.load_e8_table("cuda")
+    layer = lambda k: synth.trellis_layer("t", k, n, [4], g, "cuda") if kind == "trellis" else synth.e8_layer("e", k, n, 1, table, g, "cuda")
+    layers = [layer(m) for _ in range(7)]
+    for L in layers[1:]:
+        L.sv = layers[0].sv
+    L = layer(big)
+    L.sv = layers[0].sv
+    x = torch.randn(1, n, generator=g, device="cuda")
+
+    def spec(L, off):
+        s = L.spec(batch=1, x_dtype=x.dtype, y_dtype=torch.float32, y_offset=off)
+        s.blocks_m = [32] * 16 if L.m == m else [32768] * (big // 32768)
+        return s
+    plan = Plan([spec(a, i * m) for i, a in enumerate(layers)] + [spec(L, 7 * m)])
+    y = torch.full((7 * m + big,), -7.0, device="cuda")
+    plan.run(x, y)
+    plan.close()
+    for i, a in enumerate(layers):
+        alone = torch.empty(m, device="cuda")
+        plan = Plan([spec(a, 0)])
+        plan.run(x, alone)
+        plan.close()
+        assert torch.equal(y[i * m:(i + 1) * m], alone)
+
+
 def test_plan_output_beyond_32_bit_offsets():
     """32769 tokens of a layer of 131072 rows: the last token's partial sums start 2^32 elements in (rows of the result are
     not aligned, so the general body runs).  Against the same token alone."""
