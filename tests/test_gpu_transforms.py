@@ -271,6 +271,28 @@ def test_one_cta_completes_many_output_blocks(kind):
         assert torch.equal(y[i * m:(i + 1) * m], alone)
 
 
+@pytest.mark.parametrize("normed", [False, True])
+@pytest.mark.parametrize("tokens", [1, 3, 8])
+@pytest.mark.parametrize("feat", [303, 700, 1361, 2050, 3640, 3643])
+def test_padded_inputs_of_decode_steps(feat, tokens, normed):
+    """Layers padded to 512, 1024, 2048 and 4096 columns, whose inputs end inside a thread's values and inside a group of four."""
+    from glq_b200 import synth
+    n, m = 1 << (feat - 1).bit_length(), 64
+    g = torch.Generator(device="cuda").manual_seed(feat + tokens)
+    E = synth.e8_layer("e", m, n, 1, synth.load_e8_table("cuda"), g, "cuda")
+    nib = (synth.load_e8_table("cuda").cpu().numpy().view(np.uint32)[:, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15
+    cb = nib.astype(np.float64) * 0.5 - 3.0
+    W = cb[E.codes[0].cpu().numpy().view(np.uint16)].reshape(m, n)
+    x = torch.randn(tokens, 3648, generator=g, device="cuda")[:, :feat]
+    w = 1 + 0.2 * torch.randn(feat, generator=g, device="cuda")
+    steps = dict(in_norm_weight=w, in_norm_eps=1e-5) if normed else {}
+    y = ops.fused_linear(x, E.sv, E.su, E.codes[0], torch.from_numpy(cb).to("cuda", torch.float16), E.wscale, feat, m, n, m, 0, 0, **steps)
+    seen = x.double()
+    if normed:
+        seen = seen * torch.rsqrt(seen.pow(2).mean(-1, keepdim=True) + 1e-5) * w.double()
+    _check(torch.nn.functional.pad(seen, (0, n - feat)), W, E, y, [n], [m])
+
+
 def test_plan_output_beyond_32_bit_offsets():
     """32769 tokens of a layer of 131072 rows: the last token's partial sums start 2^32 elements in (rows of the result are
     not aligned, so the general body runs).  Against the same token alone."""
