@@ -125,8 +125,6 @@ __device__ __forceinline__ int moe_expert_of(const MoeDev& M, const void* ids, i
 __global__ void __launch_bounds__(1024) moe_count_kernel(const __grid_constant__ MoeDev M, const void* __restrict__ ids,
                                                          int T, uint8_t* __restrict__ ws) {
   extern __shared__ int sh[];            // counts[E] of this CTA's chunk
-  pdl_trigger();
-  pdl_wait();
   const int R = T * M.top_k;
   for (int e = threadIdx.x; e < M.E; e += blockDim.x) sh[e] = 0;
   __syncthreads();
@@ -146,8 +144,6 @@ __global__ void __launch_bounds__(1024) moe_count_kernel(const __grid_constant__
 __global__ void __launch_bounds__(1024) moe_place_kernel(const __grid_constant__ MoeDev M, const void* __restrict__ ids,
                                                          int T, uint8_t* __restrict__ ws) {
   extern __shared__ int sh[];            // counts[E], then cursor[E]
-  pdl_trigger();
-  pdl_wait();
   int* cnt = sh;
   int* cur = sh + M.E;
   const int R = T * M.top_k;
@@ -189,8 +185,6 @@ __global__ void __launch_bounds__(1024) moe_place_kernel(const __grid_constant__
 __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__ MoeDev M, const void* __restrict__ ids,
                                                          int T, uint8_t* __restrict__ ws, int phase) {
   extern __shared__ int sh[];            // counts[E], cursor[E], first slot[E], first token tile[E + 1], first row[E], in front[E]
-  pdl_trigger();
-  pdl_wait();
   int* cnt = sh;
   int* cur = sh + M.E;
   int* base_s = sh + 2 * M.E;
@@ -412,7 +406,6 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_rht_in_kernel(const __g
   extern __shared__ __align__(16) float fb[];
   const int hidden = M.hidden;
   pdl_trigger();
-  pdl_wait();
   __half2* xr = reinterpret_cast<__half2*>(ws + M.o_xr1);
   moe_rht_in_body(M, T, tt, x, fb, [&](int t, int c, int logbs, int n, const f2 (&v)[8][2]) {
 #pragma unroll
@@ -438,7 +431,6 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_rht_in_gemm_kernel(cons
                                                                             const uint8_t* __restrict__ x, uint8_t* __restrict__ ws) {
   extern __shared__ __align__(16) float fb[];
   pdl_trigger();
-  pdl_wait();
   const int* slot_of = reinterpret_cast<const int*>(ws + M.o_slot_of);
   const int2* trow = reinterpret_cast<const int2*>(ws + M.o_trow);
   const int kchunks = M.hidden / GM_TILE_K;
@@ -695,7 +687,6 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_mid_kernel(const __grid
                                                                     uint8_t* __restrict__ ws) {
   extern __shared__ __align__(16) float fb[];   // chunks of sg w13 rows, then of sg w2 rows
   pdl_trigger();
-  pdl_wait();
   const int R = T * M.top_k;
   const int* g_count = reinterpret_cast<const int*>(ws + M.o_count);
   const int* g_base = reinterpret_cast<const int*>(ws + M.o_base);
@@ -838,7 +829,6 @@ __global__ void __launch_bounds__(MIDW_WARPS * 32, 4) moe_mid_warp_kernel(const 
                                                                           uint8_t* __restrict__ ws) {
   extern __shared__ __align__(16) uint8_t fb8[];
   pdl_trigger();
-  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int R = T * M.top_k;
   const int used = reinterpret_cast<const int*>(ws + M.o_base)[M.E - 1] + reinterpret_cast<const int*>(ws + M.o_count)[M.E - 1];
@@ -1025,8 +1015,6 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_out_kernel(const __grid
                                                                     const float* __restrict__ topk_w,
                                                                     const uint8_t* __restrict__ ws, uint8_t* __restrict__ y) {
   extern __shared__ __align__(16) float fb[];   // chunks of rg rows of hidden (+ hidden floats when several passes are needed)
-  pdl_trigger();
-  pdl_wait();
   const int t = blockIdx.x, lane = threadIdx.x & 31;
   const int R = T * M.top_k;
   const int* slot_of = reinterpret_cast<const int*>(ws + M.o_slot_of);
@@ -1212,32 +1200,35 @@ static int fill_blocks(const int32_t* blocks, int nb, int total, int* off, int* 
   return GLQB_OK;
 }
 
-// Steps of fewer routings launch their kernels chained (launch_chained).  128 experts, top 8, in the ordinary way / chained:
-// 256 tokens 253.5 / 246.6 us, 4096 tokens 791 / 804 us.
+// The two matmuls of trellis experts are chained to the transforms in front of them (launch_chained) in steps of fewer routings.
+// The other launches are not: what starts early holds the registers, and above all the shared memory that is the L1 of the
+// kernels that gather.  In a graph, none / the matmuls / every launch chained: 128 experts, top 8, of 2048 x 768: 16 tokens 179.4 /
+// 178.6 / 184.4 us, 256 tokens 239.7 / 238.2 / 240.9; 32 experts, top 2, of 1024 x 512, 32 tokens 58.2 / 57.6 / 67.6; E8, 32 experts, top 4,
+// of 2048 x 768, 256 tokens 236.5 / 306.9 / 396.1.
 constexpr long long MOE_CHAIN_MAX = 8192;
 
 // grouping: one launch; count / tables / place kernels (many CTAs) for steps in which counting all routings in every CTA
 // would take longer than three launches.  128 experts, top 8, one CTA or three launches / one launch of many: 256 tokens
 // 24 / 19 us, 4096 tokens 56 / 25 us (cold, by ncu).
-static void moe_launch_group(const MoeDev& M, const void* ids, int tokens, uint8_t* ws, bool chain, cudaStream_t st) {
+static void moe_launch_group(const MoeDev& M, const void* ids, int tokens, uint8_t* ws, cudaStream_t st) {
   const int R = tokens * M.top_k;
   const size_t sh = (6 * (size_t)M.E + 1) * sizeof(int);
   if (R < MOE_GROUP_SPLIT_MIN) {
     const int ctas = std::max(1, std::min(MOE_GROUP_CTAS, (R + MOE_GROUP_SHARE - 1) / MOE_GROUP_SHARE));
-    launch_chained(chain, moe_group_kernel, ctas, 1024, sh, st, M, ids, tokens, ws, 0);
+    moe_group_kernel<<<ctas, 1024, sh, st>>>(M, ids, tokens, ws, 0);
     return;
   }
   const int nb = (R + MOE_GROUP_CHUNK - 1) / MOE_GROUP_CHUNK;
   cudaMemsetAsync(ws + M.o_count, 0, sizeof(int) * M.E, st);
-  launch_chained(chain, moe_count_kernel, nb, 1024, M.E * sizeof(int), st, M, ids, tokens, ws);
-  launch_chained(chain, moe_group_kernel, 1, 1024, sh, st, M, ids, tokens, ws, 1);
-  launch_chained(chain, moe_place_kernel, nb, 1024, 2 * M.E * sizeof(int), st, M, ids, tokens, ws);
+  moe_count_kernel<<<nb, 1024, M.E * sizeof(int), st>>>(M, ids, tokens, ws);
+  moe_group_kernel<<<1, 1024, sh, st>>>(M, ids, tokens, ws, 1);
+  moe_place_kernel<<<nb, 1024, 2 * M.E * sizeof(int), st>>>(M, ids, tokens, ws);
 }
 
-static void moe_launch_mid(const GlqbMoePlan* P, const MoeDev& M, int tokens, uint8_t* ws, bool chain, cudaStream_t st) {
+static void moe_launch_mid(const GlqbMoePlan* P, const MoeDev& M, int tokens, uint8_t* ws, cudaStream_t st) {
   const int R = tokens * M.top_k, per = P->mid_warp ? MIDW_ROWS * MIDW_WARPS : P->mid_sg;
-  if (P->mid_warp) launch_chained(chain, moe_mid_warp_kernel, (R + per - 1) / per, MIDW_WARPS * 32, P->mid_smem, st, M, tokens, ws);
-  else launch_chained(chain, moe_mid_kernel, (R + per - 1) / per, MOE_XF_THREADS, P->mid_smem, st, M, tokens, per, ws);
+  if (P->mid_warp) moe_mid_warp_kernel<<<(R + per - 1) / per, MIDW_WARPS * 32, P->mid_smem, st>>>(M, tokens, ws);
+  else moe_mid_kernel<<<(R + per - 1) / per, MOE_XF_THREADS, P->mid_smem, st>>>(M, tokens, per, ws);
 }
 
 // tokens per CTA of the input transform: one tile of 8192 values, fewer when that would leave SMs without work
@@ -1467,15 +1458,15 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return moe_fail(GLQB_E_WORKSPACE, "workspace must be 256-byte aligned");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_);
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
-  const bool chain = (long long)tokens * P->dev.top_k < MOE_CHAIN_MAX;
+  const bool chain = P->dev.format != GLQB_FMT_E8_SHELL && (long long)tokens * P->dev.top_k < MOE_CHAIN_MAX;
   if (P->gemm_ok && (P->dev.format == GLQB_FMT_E8_SHELL ||
                      (long long)tokens * P->dev.top_k >= (long long)P->dev.E * moe_gemm_min_avg(P->two_stages))) {
     const MoeDev& G = P->devg;
     const int R = tokens * G.top_k;
-    moe_launch_group(G, topk_ids, tokens, ws, chain, st);
+    moe_launch_group(G, topk_ids, tokens, ws, st);
     const int tt = moe_in_tokens(G, tokens);
-    launch_chained(chain, moe_rht_in_gemm_kernel, (tokens + tt - 1) / tt, MOE_XF_THREADS, (fht_words(8192) + 2 * tt * G.top_k) * 4, st, G, tokens,
-                   tt, reinterpret_cast<const uint8_t*>(x), ws);
+    moe_rht_in_gemm_kernel<<<(tokens + tt - 1) / tt, MOE_XF_THREADS, (fht_words(8192) + 2 * tt * G.top_k) * 4, st>>>(
+        G, tokens, tt, reinterpret_cast<const uint8_t*>(x), ws);
     const bool g_e8 = G.format == GLQB_FMT_E8_SHELL;
     const int g_threads = g_e8 ? GM_THREADS : TG_THREADS;
     int* status = reinterpret_cast<int*>(ws + G.o_status);
@@ -1486,25 +1477,23 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
                      reinterpret_cast<const DevLinear*>(ws + G.o_layers13), reinterpret_cast<const GemmItem*>(ws + G.o_items13),
                      G.max_items13, ws, status, nitems, tokens);
     }
-    moe_launch_mid(P, G, tokens, ws, chain, st);
+    moe_launch_mid(P, G, tokens, ws, st);
     {
       MoeTimer t(P, st);
       launch_chained(chain, P->g2, std::min(P->sm_count, G.max_items2), g_threads, moe_gemm_smem_bytes(g_e8), st,
                      reinterpret_cast<const DevLinear*>(ws + G.o_layers2), reinterpret_cast<const GemmItem*>(ws + G.o_items2),
                      G.max_items2, ws, status, nitems + 1, tokens);
     }
-    launch_chained(chain, moe_out_kernel, tokens, MOE_XF_THREADS, P->out_smem, st, G, tokens, P->out_rg, topk_weights, ws,
-                   reinterpret_cast<uint8_t*>(y));
+    moe_out_kernel<<<tokens, MOE_XF_THREADS, P->out_smem, st>>>(G, tokens, P->out_rg, topk_weights, ws, reinterpret_cast<uint8_t*>(y));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return moe_fail(GLQB_E_CUDA, "moe_plan_run: %s", cudaGetErrorString(e));
     return GLQB_OK;
   }
   const MoeDev& M = P->dev;
   const int R = tokens * M.top_k;
-  moe_launch_group(M, topk_ids, tokens, ws, chain, st);
+  moe_launch_group(M, topk_ids, tokens, ws, st);
   const int tt = moe_in_tokens(M, tokens);
-  launch_chained(chain, moe_rht_in_kernel, (tokens + tt - 1) / tt, MOE_XF_THREADS, fht_words(8192) * 4, st, M, tokens, tt,
-                 reinterpret_cast<const uint8_t*>(x), ws);
+  moe_rht_in_kernel<<<(tokens + tt - 1) / tt, MOE_XF_THREADS, fht_words(8192) * 4, st>>>(M, tokens, tt, reinterpret_cast<const uint8_t*>(x), ws);
   MoeMvArgs A;
   memset(&A, 0, sizeof A);
   A.codes[0] = M.w13[0]; A.codes[1] = M.w13[1]; A.stride[0] = M.w13_stride[0]; A.stride[1] = M.w13_stride[1];
@@ -1521,7 +1510,7 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
     MoeTimer t(P, st);
     launch_chained(chain, P->k13, P->grid13, MV_THREADS, 0, st, A);
   }
-  moe_launch_mid(P, M, tokens, ws, chain, st);
+  moe_launch_mid(P, M, tokens, ws, st);
   A.codes[0] = M.w2[0]; A.codes[1] = M.w2[1]; A.stride[0] = M.w2_stride[0]; A.stride[1] = M.w2_stride[1];
   A.inv2 = M.w2_inv2;
   A.row_map = nullptr;
@@ -1534,8 +1523,7 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
     MoeTimer t(P, st);
     launch_chained(chain, P->k2, P->grid2, MV_THREADS, 0, st, A);
   }
-  launch_chained(chain, moe_out_kernel, tokens, MOE_XF_THREADS, P->out_smem, st, M, tokens, P->out_rg, topk_weights, ws,
-                 reinterpret_cast<uint8_t*>(y));
+  moe_out_kernel<<<tokens, MOE_XF_THREADS, P->out_smem, st>>>(M, tokens, P->out_rg, topk_weights, ws, reinterpret_cast<uint8_t*>(y));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return moe_fail(GLQB_E_CUDA, "moe_plan_run: %s", cudaGetErrorString(e));
   return GLQB_OK;
