@@ -27,6 +27,7 @@
 // padded to a multiple of 16.  The transforms write the activations straight into the swizzled tile images the GEMM's
 // bulk copies fetch.
 #include <algorithm>
+#include <climits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -1141,7 +1142,7 @@ struct GlqbMoePlan {
   MoeMvKernel k13 = nullptr, k2 = nullptr;
   int grid13 = 0, grid2 = 0;
   int mid_sg = 1, out_rg = 1;          // slots per CTA of the mid kernel, routings per pass of the combine
-  bool mid_warp = false;               // moe_mid_warp_kernel instead of moe_mid_kernel
+  int mid_warp_min = INT_MAX;          // routings from which moe_mid_warp_kernel is used (moe_mid_warp_min; INT_MAX: not for these blocks)
   size_t mid_smem = 0, out_smem = 0;
   // tensor-core form
   bool gemm_ok = false, two_stages = false;
@@ -1225,9 +1226,19 @@ static void moe_launch_group(const MoeDev& M, const void* ids, int tokens, uint8
   moe_place_kernel<<<nb, 1024, 2 * M.E * sizeof(int), st>>>(M, ids, tokens, ws);
 }
 
+// moe_mid_warp_kernel spreads a pair of slots over one warp, moe_mid_kernel some slots' chunks over eight: fewer routings leave
+// the warps too few.  128 experts, top 8, of 2048 x 768, in a graph, by CTAs / by warps: 1 token 88.7 / 102.8 us, 64 tokens
+// 243.1 / 254.9, 256 tokens 239.7 / 243.1, 512 tokens 286.6 / 281.7, 2048 tokens 432 / 418; 32 experts, top 4, 512 tokens 107.7 /
+// 110.7, 1024 tokens 147.7 / 144.5.
+static int moe_mid_warp_min() {
+  const char* e = getenv("GLQB_MOE_MID_WARP_MIN");
+  return e ? atoi(e) : 4096;
+}
 static void moe_launch_mid(const GlqbMoePlan* P, const MoeDev& M, int tokens, uint8_t* ws, cudaStream_t st) {
-  const int R = tokens * M.top_k, per = P->mid_warp ? MIDW_ROWS * MIDW_WARPS : P->mid_sg;
-  if (P->mid_warp) moe_mid_warp_kernel<<<(R + per - 1) / per, MIDW_WARPS * 32, P->mid_smem, st>>>(M, tokens, ws);
+  const int R = tokens * M.top_k;
+  const bool by_warps = R >= P->mid_warp_min;
+  const int per = by_warps ? MIDW_ROWS * MIDW_WARPS : P->mid_sg;
+  if (by_warps) moe_mid_warp_kernel<<<(R + per - 1) / per, MIDW_WARPS * 32, MIDW_WARPS * moe_midw_warp_bytes(M.w13_out), st>>>(M, tokens, ws);
   else moe_mid_kernel<<<(R + per - 1) / per, MOE_XF_THREADS, P->mid_smem, st>>>(M, tokens, per, ws);
 }
 
@@ -1404,9 +1415,9 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
     // (running sums between passes are only needed when one pass cannot hold all routings of a token)
     while (P->out_rg > 1 && out_bytes(P->out_rg) > budget) --P->out_rg;
     P->mid_smem = mid_bytes(P->mid_sg);
-    P->mid_warp = !M.wide_m13 && MIDW_WARPS * moe_midw_warp_bytes(d->w13_out) <= limit;
-    for (int b = 0; b < M.nb_n2; ++b) P->mid_warp = P->mid_warp && M.log_n2[b] <= 10;
-    if (P->mid_warp) P->mid_smem = MIDW_WARPS * moe_midw_warp_bytes(d->w13_out);
+    bool by_warps = !M.wide_m13 && MIDW_WARPS * moe_midw_warp_bytes(d->w13_out) <= budget;
+    for (int b = 0; b < M.nb_n2; ++b) by_warps = by_warps && M.log_n2[b] <= 10;
+    if (by_warps) P->mid_warp_min = moe_mid_warp_min();
     P->out_smem = out_bytes(P->out_rg);
     if (P->mid_smem > limit || P->out_smem > limit) {
       delete P;

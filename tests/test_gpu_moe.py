@@ -311,3 +311,27 @@ def test_moe_plans_differ_by_every_argument(T):
         assert torch.equal(call(*v), y)
     assert not any(torch.equal(got[0], y) for y in got[1:])
     ops.clear_caches()
+
+
+@pytest.mark.parametrize("E,hidden,inter,k,T,act", [(8, 256, 736, 2, 37, 1), (8, 256, 192, 3, 200, 0), (4, 128, 96, 2, 9, 4)])
+def test_moe_between_the_matmuls_by_warps_and_by_ctas(E, hidden, inter, k, T, act, monkeypatch):
+    """The two kernels between the matmuls give the oracle's result and each other's bits, over blocks of 32 to 1024 values, an odd
+    number of slots, gated and plain activations, in the streaming and in the tensor-core form."""
+    from glq_b200 import ops
+    rng = np.random.default_rng(E + hidden + inter + T)
+    d, w13_out = _make(rng, E, hidden, inter, 4, 0)
+    if act > 2:
+        w13_out = inter
+        d["w13"], d["su13"] = d["w13"][:, :(w13_out // 16) * (hidden // 16)].copy(), d["su13"][:, :w13_out].copy()
+    x_t = cuda(rng.standard_normal((T, hidden)).astype(np.float32), torch.float16)
+    ids = np.stack([rng.permutation(E)[:k] for _ in range(T)]).astype(np.int64)
+    w = rng.random((T, k)).astype(np.float32)
+    ref = _oracle(d, x_t.float().cpu().numpy(), ids, w, E, hidden, inter, w13_out, 4, 0, O.ACT_CODES[act])
+    got = []
+    for least in ("1", "1000000"):
+        monkeypatch.setenv("GLQB_MOE_MID_WARP_MIN", least)
+        ops.clear_caches()
+        got.append(_run(ops, d, x_t, cuda(ids), cuda(w), E, hidden, inter, w13_out, 0, act))
+        assert np.abs(got[-1].float().cpu().numpy() - ref).max() <= 5e-3 * np.abs(ref).max()
+    assert torch.equal(*got)
+    ops.clear_caches()
