@@ -335,3 +335,30 @@ def test_moe_between_the_matmuls_by_warps_and_by_ctas(E, hidden, inter, k, T, ac
         assert np.abs(got[-1].float().cpu().numpy() - ref).max() <= 5e-3 * np.abs(ref).max()
     assert torch.equal(*got)
     ops.clear_caches()
+
+
+@pytest.mark.parametrize("K2", [0, 2])
+def test_moe_pairs_of_token_tiles(K2, monkeypatch):
+    """Routed tokens per expert at the edges of tiles of 160 and of the pairs of tiles that an item takes.  inter 704 is eleven
+    chunks of 64 columns (an odd number: the last pair of chunks is half) and blocks of 512, 128 and 64.  With two stages the
+    GEMM multiplies fp16 sums of weights and the streaming form does not: other bits show which one ran."""
+    from glq_b200 import ops
+    counts = [0, 1, 16, 17, 159, 160, 161, 319, 320, 321, 480, 481, 640, 641]
+    E, hidden, inter, T = len(counts), 128, 704, sum(counts)
+    assert hidden % 64 == 0 and inter % 64 == 0              # else there is no tensor-core form
+    rng = np.random.default_rng(78)
+    d, w13_out = _make(rng, E, hidden, inter, 4, K2)
+    x_t = cuda(rng.standard_normal((T, hidden)).astype(np.float32), torch.float16)
+    ids = rng.permutation(np.repeat(np.arange(E), counts)).astype(np.int64)[:, None]
+    w = rng.random((T, 1)).astype(np.float32)
+    got = []
+    for least in ("0", "1000000"):
+        monkeypatch.setenv("GLQB_MOE_GEMM_MIN_AVG", least)
+        ops.clear_caches()
+        got.append(_run(ops, d, x_t, cuda(ids), cuda(w), E, hidden, inter, w13_out, K2, 1))
+    ops.clear_caches()
+    ref = _oracle(d, x_t.float().cpu().numpy(), ids, w, E, hidden, inter, w13_out, 4, K2, O.ACT_CODES[1])
+    for y in got:
+        assert np.abs(y.float().cpu().numpy() - ref).max() <= 5e-3 * np.abs(ref).max()
+    if K2:
+        assert not torch.equal(*got)
