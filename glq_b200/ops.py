@@ -722,7 +722,7 @@ def dequant_e8(qidxs_list: Sequence[torch.Tensor], codebooks: Sequence[torch.Ten
 # MoE grouped expert matmul (glq_vllm/custom_ops.py:22-36)
 # ------------------------------------------------------------------------------------------------
 class MoePlan:
-    """Owns a GlqbMoePlan handle and its workspace."""
+    """Owns a GlqbMoePlan handle and a workspace per stream it ran on (steps on different streams may overlap)."""
 
     def __init__(self, desc: "_lib.MoeDesc", device, keep):
         self.lib = _lib.load()
@@ -732,20 +732,24 @@ class MoePlan:
             _lib.check(self.lib.glqb_moe_plan_create(C.byref(desc), C.byref(handle)), "moe_plan_create")
         self.handle = handle
         self.max_tokens = desc.max_tokens
-        self.workspace = torch.empty(max(256, int(self.lib.glqb_moe_plan_workspace_bytes(handle))), dtype=torch.uint8,
-                                     device=device)
+        self.workspace_bytes = max(256, int(self.lib.glqb_moe_plan_workspace_bytes(handle)))
+        self.workspaces: dict = {}
         self.code_bytes = int(self.lib.glqb_moe_plan_code_bytes(handle))
 
     def run(self, x, topk_ids, topk_weights, y):
+        stream = _stream(x)
+        ws = self.workspaces.get(stream)
+        if ws is None:
+            ws = self.workspaces[stream] = torch.empty(self.workspace_bytes, dtype=torch.uint8, device=x.device)
         _lib.check(self.lib.glqb_moe_plan_run(self.handle, x.data_ptr(), topk_ids.data_ptr(), topk_weights.data_ptr(),
-                                              y.data_ptr(), x.shape[0], self.workspace.data_ptr(),
-                                              self.workspace.numel(), _stream(x)), "moe_plan_run")
+                                              y.data_ptr(), x.shape[0], ws.data_ptr(), ws.numel(), stream), "moe_plan_run")
 
     def check_status(self, x=None):
-        """Synchronises the stream of ``x`` (default: the current stream of the plan's device) and raises if a
-        bounded wait inside the GEMM kernels gave up."""
-        _lib.check(self.lib.glqb_moe_plan_status(self.handle, self.workspace.data_ptr(),
-                                                 _stream(x if x is not None else self.workspace)), "moe_plan_status")
+        """Synchronises the current stream of ``x``'s device (default: every stream that the plan ran on) and raises if a
+        bounded wait inside the GEMM kernels gave up there."""
+        for stream, ws in list(self.workspaces.items()):
+            if x is None or stream == _stream(x):
+                _lib.check(self.lib.glqb_moe_plan_status(self.handle, ws.data_ptr(), stream), "moe_plan_status")
 
     def set_timing(self, on: bool) -> None:
         _lib.check(self.lib.glqb_moe_plan_set_timing(self.handle, 1 if on else 0), "moe_plan_set_timing")

@@ -362,3 +362,34 @@ def test_moe_pairs_of_token_tiles(K2, monkeypatch):
         assert np.abs(y.float().cpu().numpy() - ref).max() <= 5e-3 * np.abs(ref).max()
     if K2:
         assert not torch.equal(*got)
+
+
+@pytest.mark.parametrize("T", [6, 150])
+def test_moe_steps_on_two_streams(T):
+    """Steps of one layer that may overlap, in the streaming and the tensor-core form, then alone again."""
+    from glq_b200 import ops
+    E, hidden, inter, k = 8, 256, 128, 2
+    rng = np.random.default_rng(T)
+    d, w13_out = _make(rng, E, hidden, inter, 4)
+    d = {key: cuda(v) if v is not None else None for key, v in d.items()}
+    none, bl = torch.zeros(E, 1, 1, dtype=torch.int16, device="cuda"), [O.block_decompose(v) for v in (hidden, w13_out, inter, hidden)]
+    steps = []
+    for _ in range(2):
+        steps.append((cuda(rng.standard_normal((T, hidden)).astype(np.float32), torch.float16),
+                      cuda(np.stack([rng.permutation(E)[:k] for _ in range(T)]).astype(np.int64)), cuda(rng.random((T, k)).astype(np.float32))))
+    call = lambda x, ids, w: ops.fused_moe_trellis_3inst(
+        x, ids, w, d["w13"], none, d["su13"], d["sv13"], d["ws13"], d["inv13"], d["w2"], none, d["su2"], d["sv2"], d["ws2"], d["inv2"],
+        hidden, inter, w13_out, hidden, w13_out, inter, hidden, bl[0], bl[1], None, None, bl[2], bl[3], None, None, 0)
+    ops.clear_caches()
+    refs = [call(*s) for s in steps]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in steps], [[], []]
+    for _ in range(20):
+        for i, s in enumerate(steps):
+            with torch.cuda.stream(streams[i]):
+                got[i].append(call(*s))
+    torch.cuda.synchronize()
+    ops.check_device_status()
+    assert all(torch.equal(y, ref) for ys, ref in zip(got, refs) for y in ys)
+    assert all(torch.equal(call(*s), ref) for s, ref in zip(steps, refs))
+    ops.clear_caches()
