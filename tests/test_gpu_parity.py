@@ -909,3 +909,27 @@ def test_a_plan_in_many_workspaces():
     torch.cuda.synchronize()
     plan.close()
     assert (y[0] != 0).any() and torch.equal(y, y[:1].expand(200, m))
+
+
+@pytest.mark.parametrize("tokens", [9, 27, 70, 333])
+@pytest.mark.parametrize("kind", ["trellis", "e8"])
+def test_ragged_rows_anywhere(ops, e8_cb, kind, tokens):
+    """Rows of a ragged count give the same bits dense, with a stride, one value past an aligned address and with an odd stride."""
+    from glq_b200 import synth
+    m, n = 96, 320
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda") if kind == "trellis" else synth.e8_layer("e", m, n, 1, synth.load_e8_table("cuda"), g, "cuda")
+    if kind == "trellis":
+        calls = [lambda x: ops.fused_linear_trellis_3inst(x, L.sv, L.su, L.codes[0], None, None, None, None, L.wscale, n, m, n, m),
+                 lambda x: ops.fused_linear_trellis_3inst_shards(x, L.sv, [(L.su, L.codes[0], None, L.wscale, 0.0, m)])]
+    else:
+        calls = [lambda x: ops.fused_linear_block_diag(x, L.sv, L.su, L.codes[0], e8_cb[0], L.wscale, n, m, n, m, None, None, None, None),
+                 lambda x: ops.fused_linear_e8_shards(x, L.sv, [(L.su, L.codes, [], L.wscale, m)], e8_cb[0])]
+    for dtype in (torch.bfloat16, torch.float32):
+        x = torch.randn(tokens, n, generator=g, device="cuda").to(dtype)
+        forms = [x.new_zeros(tokens, n + 8)[:, :n], x.new_zeros(tokens * n + 1)[1:].view(tokens, n), x.new_zeros(tokens, n + 3)[:, 2:2 + n]]
+        for call in calls:
+            ref = call(x)
+            for rows in forms:
+                rows.copy_(x)
+                assert torch.equal(call(rows), ref)
