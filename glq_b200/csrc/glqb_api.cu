@@ -1021,7 +1021,11 @@ int glqb_plan_create(const GlqbLinearDesc* descs, int32_t count, GlqbPlan** out_
   }
   GlqbPlan* P = new GlqbPlan();
   P->descs.assign(descs, descs + count);
+  // (a stream that is being captured must not keep another layout of the same call from getting its plan)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
   int rc = build_plan(P);
+  cudaThreadExchangeStreamCaptureMode(&mode);
   if (rc) {
     glqb_plan_destroy(P);
     return rc;

@@ -933,3 +933,22 @@ def test_ragged_rows_anywhere(ops, e8_cb, kind, tokens):
             for rows in forms:
                 rows.copy_(x)
                 assert torch.equal(call(rows), ref)
+
+
+@pytest.mark.parametrize("tokens", [5, 27, 70])
+def test_other_strides_under_capture(ops, tokens):
+    """Rows in another layout than those of the calls before a capture."""
+    from glq_b200 import synth
+    m, n = 96, 256
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda")
+    x = torch.randn(tokens, n, generator=g, device="cuda")
+    call = lambda x: ops.fused_linear_trellis_3inst(x, L.sv, L.su, L.codes[0], None, None, None, None, L.wscale, n, m, n, m)
+    ref, rows, graph = call(x), torch.randn(tokens, 2 * n, generator=g, device="cuda")[:, n:], torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        y = call(rows)
+    rows.copy_(x)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, ref)
