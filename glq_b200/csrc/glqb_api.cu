@@ -285,11 +285,14 @@ static void gemm_schedule(Segment& s, int limit, int sm_count, std::vector<DevLi
   auto tokens_of = [&](const DevLinear& L) { return std::min(L.batch, limit); };
   auto tile_of = [&](const DevLinear& L) { return trellis_form(s) ? tile_tokens(tokens_of(L)) : s.tn; };
   auto splits = [](int kchunks, int ks, int& per) { per = (kchunks + ks - 1) / ks; return (kchunks + per - 1) / per; };
+  const char* e = getenv("GLQB_GEMM_PAIRS");     // 0: single tiles, 1: pairs, whatever they cost
+  const int forced = e ? atoi(e) : -1;
   int best = 1;
   bool pairs = false;                            // an item takes two token tiles
   double best_cost = 0;
   for (int ks = 1; ks <= 16; ++ks)
     for (int two = 0; two <= (trellis_form(s) ? 1 : 0); ++two) {
+      if (forced >= 0 && trellis_form(s) && two != (forced != 0)) continue;
       long long n = 0;
       int longest = 0, per = 0;
       double sums = 0;
@@ -305,7 +308,7 @@ static void gemm_schedule(Segment& s, int limit, int sm_count, std::vector<DevLi
         paired = paired || (two && n_tiles > 1);
       }
       const double cost = (double)((n + sm_count - 1) / sm_count) * longest * (paired ? 1.6 : 1.0) + sums * 8 / 5e12 / 0.3e-6;
-      if ((ks == 1 && !two) || (ok && cost < best_cost)) { best = ks; pairs = two; best_cost = cost; }
+      if (best_cost == 0 || (ok && cost < best_cost)) { best = ks; pairs = two; best_cost = cost; }
     }
   s.item_first = (int)items.size();
   for (int i = 0; i < s.count; ++i) {

@@ -104,3 +104,55 @@ def test_run_of_fewer_tokens(kind, bucket, tokens, monkeypatch):
     plan.close()
     assert (y[tokens:] == -7.0).all()
     assert (y[:tokens] - full[:tokens]).abs().max() <= 2e-5 * full.abs().max()
+
+
+# two token tiles per item: two whole tiles, an odd last tile, a second tile that the tokens of the run cut short or away, the
+# schedule for one tile fewer, columns that end inside a pair of chunks.  352 columns are one K range in both forms and so the same
+# bits; 1056 may be split, see above.
+@pytest.mark.parametrize("bits", [[4], [2], [4, 2]], ids=str)
+@pytest.mark.parametrize("n", [352, 1056])
+@pytest.mark.parametrize("bucket,tokens", [(256, 193), (256, 256), (512, 512), (512, 500), (512, 385), (512, 300), (768, 768), (768, 600),
+                                           (768, 577), (768, 390), (1024, 1000), (1024, 20)])
+def test_pairs_of_token_tiles(bits, n, bucket, tokens, monkeypatch):
+    m = 160
+    monkeypatch.setenv("GLQB_TRELLIS_TWO_PHASE_MIN_FLOPS", "1e30")
+    g = torch.Generator(device="cuda").manual_seed(n + tokens)
+    L = synth.trellis_layer("t", m, n, bits, g, "cuda")
+    x = torch.randn(bucket, n, generator=g, device="cuda").half()
+    x[tokens:] = float("nan")
+    got = []
+    for pairs in ("0", "1"):
+        monkeypatch.setenv("GLQB_GEMM_PAIRS", pairs)
+        plan = Plan([L.spec(batch=bucket, x_dtype=x.dtype, y_dtype=torch.float32)])
+        y = torch.full((bucket, m), -7.0, device="cuda")
+        plan.run(x, y, tokens=tokens)
+        plan.check_status()
+        plan.close()
+        assert (y[tokens:] == -7.0).all()
+        got.append(y[:tokens])
+    if n == 352:
+        assert torch.equal(*got)
+    assert (got[0] - got[1]).abs().max() <= 2e-5 * got[0].abs().max()
+
+
+# a shape for which the costs choose pairs: all tokens, and a ragged number of them
+@pytest.mark.parametrize("tokens", [1024, 1000])
+def test_pairs_of_token_tiles_by_cost(tokens, monkeypatch):
+    from glq_b200 import ops
+    m, n = 11008, 2048
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    L = synth.trellis_layer("t", m, n, [4], g, "cuda")
+    x = torch.randn(tokens, n, generator=g, device="cuda").half()
+    H = torch.ones(1, 1, dtype=torch.float64, device="cuda")
+    had = {}
+    for k in range(14):
+        had[1 << k] = H
+        H = torch.cat([torch.cat([H, H], 1), torch.cat([H, -H], 1)])
+    turn = lambda v, blocks: torch.cat([p @ had[b] / b ** 0.5 for p, b in zip(v.split(blocks, 1), blocks)], 1)
+    W = ops.glq_decompress_trellis_3inst_cuda(L.codes[0], m, n).double()
+    ref = turn(turn(x.double() * L.sv.double(), [2048]) @ W.T * L.wscale, [8192, 2048, 512, 256]) * L.su.double()
+    ops.clear_caches()
+    y = ops.fused_linear_trellis_3inst(x, L.sv, L.su, L.codes[0], None, None, None, None, L.wscale, n, m, n, m, out_dtype=torch.float32)
+    # the rotated activations are fp16: 2e-3 of the largest output, as for every linear
+    assert (y.double() - ref).abs().max() <= 2e-3 * ref.abs().max()
+    ops.clear_caches()
