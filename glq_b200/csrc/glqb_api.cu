@@ -528,12 +528,6 @@ static int tickets_for(GlqbPlan* P, const void* workspace, cudaStream_t stream, 
   return GLQB_OK;
 }
 
-// The output transform is chained to the kernel in front of it (launch_chained) in plans of up to this many tokens.  Its CTAs wait on
-// the SMs of a GEMM of many rounds, which is longer than their launch.  Chained / not, in a graph: E8, 128 tokens of 11008 x
-// 2048 54 / 62 us, trellis, 256 tokens of 2048 x 11008 35.8 / 36.2, 1024 tokens of 512 x 2048 21.6 / 20.8, of 1088 x 544 23.3 / 22.5,
-// 2048 tokens of 11008 x 2048 131.4 / 129.0, of 1088 x 544 25.7 / 23.9.
-constexpr int OUT_CHAIN_MAX_TOKENS = 512;
-
 static int build_plan(GlqbPlan* P) {
   const int n = (int)P->descs.size();
   int dev_id = 0;
@@ -1140,16 +1134,15 @@ int glqb_plan_run_tokens(GlqbPlan* P, const void* x_base, void* y_base, int32_t 
   }
   if (!P->items_out.empty()) {
     const int n_items = (int)P->items_out.size();
-    const bool chain = P->max_batch <= OUT_CHAIN_MAX_TOKENS;
     uint8_t* yb = reinterpret_cast<uint8_t*>(y_base);
     if (P->out_few) {
-      CUDA_TRY(launch_chained(chain, rht_out_wide_kernel, n_items, FHT_WIDE_THREADS, rht_smem(P->max_elems_out), stream, d_layers,
+      CUDA_TRY(launch_chained(true, rht_out_wide_kernel, n_items, FHT_WIDE_THREADS, rht_smem(P->max_elems_out), stream, d_layers,
                               P->d_items_out, ws, yb, tokens));
     } else if (out_plain(P, yb)) {
-      CUDA_TRY(launch_chained(chain, rht_out_plain_kernel, n_items, RHT_THREADS, rht_smem(P->max_elems_out), stream, d_layers, P->d_items_out, ws,
+      CUDA_TRY(launch_chained(true, rht_out_plain_kernel, n_items, RHT_THREADS, rht_smem(P->max_elems_out), stream, d_layers, P->d_items_out, ws,
                               yb, tokens));
     } else {
-      CUDA_TRY(launch_chained(chain, P->out_wide ? rht_out_kernel<true> : rht_out_kernel<false>, n_items, RHT_THREADS,
+      CUDA_TRY(launch_chained(true, P->out_wide ? rht_out_kernel<true> : rht_out_kernel<false>, n_items, RHT_THREADS,
                               rht_smem(P->max_elems_out), stream, d_layers, P->d_items_out, ws, yb, (const float*)nullptr, tokens));
     }
   }
