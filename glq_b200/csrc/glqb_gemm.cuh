@@ -316,7 +316,11 @@ template <int FORMAT, int K1, int K2, int TN, int STAGES>
 __global__ void __launch_bounds__(GM_THREADS, 1)
 glq_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict__ items, int n_items,
                 uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev, int tokens) {
-  pdl_trigger();
+  // No trigger, except in the form that gathers: CTAs of the output transform that start early go where the GEMM leaves room, which
+  // is a few SMs, and these then do all of it.  In a graph, trigger / none: trellis, 256 tokens of 1024 x 4096 22.5 / 20.1 us, of 5376 x
+  // 4096 31.5 / 30.3, 2048 tokens of 11008 x 2048 131.4 / 129.0.  E8, 128 tokens of 11008 x 2048 54.3 / 61.3, of 5376 x 4096 45.8 / 50.1,
+  // of 2048 x 11008 49.9 / 47.9.
+  if constexpr (FORMAT == 1) pdl_trigger();
   // work lists built on the device (grouped expert matmul) pass their length through memory; other lists and the weights are
   // there before: then only the loader and the epilogue wait for the kernel before this one
   if (n_items_dev) { pdl_wait(); n_items = min(n_items, *n_items_dev); }

@@ -92,8 +92,7 @@ template <int K1, int K2, int TN>
 __global__ void __launch_bounds__(TG_THREADS, 1)
 trellis_gemm_kernel(const DevLinear* __restrict__ layers, const GemmItem* __restrict__ items, int n_items,
                     uint8_t* __restrict__ ws, int* __restrict__ status, const int* __restrict__ n_items_dev, int tokens) {
-  pdl_trigger();
-  // (as in glq_gemm_kernel: of a plan's layers the producers decode before the kernel in front of this one has completed)
+  // (as in glq_gemm_kernel: no trigger; of a plan's layers the producers decode before the kernel in front of this one has completed)
   if (n_items_dev) { pdl_wait(); n_items = min(n_items, *n_items_dev); }
   // first token and tokens of an item's tile (none: every role skips the item), the activation rows in front of it, and the
   // tokens of its second tile, which lies right behind (whole tiles are multiples of 16)
