@@ -16,7 +16,9 @@ struct GemmItem;
 // Whole calls back to back, ordinary / chained: one token of 14336 x 4096 (E8: the 224 KiB table is copied during the input
 // transform) 52.2 / 47.3 us, 333 tokens of 2048 x 11008 44.2 / 40.9, 2048 tokens of 11008 x 2048 155 / 151, 700 tokens of
 // 5376 x 21504 309 / 304.  Not chained: e8_tiles_kernel, whose gathers need the L1 that the input transform's shared memory
-// would still hold (2048 tokens of 14336 x 4096 346 / 368 us), and the streaming trellis kernel, which has nothing to do early.
+// would still hold (2048 tokens of 14336 x 4096 346 / 368 us), the streaming trellis kernel, which has nothing to do early, and the
+// launches of experts but their trellis matmuls (MOE_CHAIN_MAX).  A kernel whose successor would take the room it needs, or find
+// room on a few SMs only, does not trigger (glq_gemm_kernel).
 inline bool pdl_enabled() {
   static const bool on = [] { const char* e = getenv("GLQB_PDL"); return !e || atoi(e) != 0; }();
   return on;

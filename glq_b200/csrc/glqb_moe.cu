@@ -11,6 +11,7 @@
 //   3 trellis_moe_mv_kernel  w13: experts' weights decoded once per 8*NB routed tokens, partial sums per slot
 //   4 moe_mid_kernel       a few slots per CTA: sum partials, Wscale, output transform, SU, gated activation,
 //                          then the w2 input transform (SV, Hadamard) — three reference launches in one
+//                          (moe_mid_warp_kernel from 4096 routings on, where no block is longer than 1024 values)
 //   5 trellis_moe_mv_kernel  w2
 //   6 moe_out_kernel       per token: its routings are the rows of one tile transform; then, for j in fixed
 //                          order, acc += w * SU * H(Wscale * partials)

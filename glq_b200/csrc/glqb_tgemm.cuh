@@ -15,7 +15,8 @@
 // (group p % 2 decodes pair p; warp w of a group rows 32 (w % 4) and chunk w / 4 of the pair: two 32 x 32 trellis groups).
 // Experts of 4096 tokens, top 8 of 128 (256 tokens each on average), a tile of up to 192 tokens / two of up to 160 per item:
 // 788 / 717 us.
-// Bound by the instructions of the state decode (issue slots 74 % busy at 256 routed tokens per expert): with a loop
+// Bound by the instructions of the state decode (issue slots 76 and 73 % busy in the two matmuls with 16 routed tokens per expert, 55
+// and 51 % with 256, where the tensor pipe is 56 and 43 % busy): with a loop
 // turn per pair instead of per chunk a trellis group takes 229 instructions instead of 263, and 80 registers hold both
 // decoded groups until the stage is free.  24 producer warps, a chunk per turn / this: experts of 256 tokens 273 / 257 us,
 // 333 tokens of 2048 x 11008 80 / 76 us.
