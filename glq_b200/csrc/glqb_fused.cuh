@@ -282,19 +282,19 @@ __device__ __forceinline__ int fused_first_unit(int b, int total_units) {
 // `done` more units of an output block are finished: whoever completes it (`need` units) transforms it.  Release (the CTA's
 // stores, ordered before this by a barrier) and acquire (the other CTAs' stores, released before their increments) in one
 // device-scope atomic; nobody ever waits on a ticket.
-__device__ __forceinline__ void fused_ticket(int* __restrict__ tickets, int ticket, int done, int need, int code, uint16_t* todo, int* n_todo) {
+__device__ __forceinline__ void fused_ticket(int* __restrict__ tickets, int ticket, int done, int need, int code, int* todo, int* n_todo) {
   int old;
   asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(tickets + ticket), "r"(done) : "memory");
   if (old + done == need) {
     tickets[ticket] = 0;                                      // ready for the next run
-    todo[(*n_todo)++] = (uint16_t)code;
+    todo[(*n_todo)++] = code;
   }
 }
 
 // Phase 3 of the single-launch decode kernels: output transforms of the blocks this CTA completed (`todo` entries
 // are (layer << 8) | block), with the sum over tensor-parallel ranks when the layer asks for it.
 template <bool E8FMT, int LATE>
-__device__ __forceinline__ void fused_phase3(const DevLinear* layers, const uint16_t* todo, int nt, int batch, const float* rstd_s,
+__device__ __forceinline__ void fused_phase3(const DevLinear* layers, const int* todo, int nt, int batch, const float* rstd_s,
                                              const uint8_t* __restrict__ ws, uint8_t* __restrict__ y_base, float* fbuf,
                                              int scratch_elems, const CommDev& C, int comm_e) {
   for (int k = 0; k < nt; ++k) {
@@ -362,7 +362,7 @@ trellis_fused_kernel(const __grid_constant__ FusedLayers T, int n_layers, int to
   __half2* xs = reinterpret_cast<__half2*>(fsm);                              // [batch][n] (x, 0) pairs, fragment order
   float* fbuf = reinterpret_cast<float*>(fsm + (size_t)batch * n * 4);
   float* red = fbuf + scratch_elems + scratch_elems / 32;                       // [8 warps][8 values][32 lanes]
-  __shared__ uint16_t todo[FUSED_MAX_TODO];
+  __shared__ int todo[FUSED_MAX_TODO];
   __shared__ int n_todo;
   if (threadIdx.x == 0) n_todo = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -538,7 +538,7 @@ e8_fused_kernel(const __grid_constant__ FusedLayers T, int n_layers, int total_u
   __half2* xs = reinterpret_cast<__half2*>(fsm);
   float* fbuf = reinterpret_cast<float*>(fsm + ((fused_xs_bytes<true>(n, batch) + 15) & ~(size_t)15));
   float* red = fbuf + scratch_elems + scratch_elems / 32;                       // [8 warps][4 values][32 lanes]
-  __shared__ uint16_t todo[FUSED_MAX_TODO];
+  __shared__ int todo[FUSED_MAX_TODO];
   __shared__ int n_todo;
   if (threadIdx.x == 0) n_todo = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
