@@ -11,7 +11,7 @@
 //   3 trellis_moe_mv_kernel  w13: experts' weights decoded once per 8*NB routed tokens, partial sums per slot
 //   4 moe_mid_kernel       a few slots per CTA: sum partials, Wscale, output transform, SU, gated activation,
 //                          then the w2 input transform (SV, Hadamard) — three reference launches in one
-//                          (moe_mid_warp_kernel from 4096 routings on, where no block is longer than 1024 values)
+//                          (moe_mid_warp_kernel with enough routings, where no block is longer than 1024 values)
 //   5 trellis_moe_mv_kernel  w2
 //   6 moe_out_kernel       per token: its routings are the rows of one tile transform; then, for j in fixed
 //                          order, acc += w * SU * H(Wscale * partials)
@@ -1143,7 +1143,8 @@ struct GlqbMoePlan {
   MoeMvKernel k13 = nullptr, k2 = nullptr;
   int grid13 = 0, grid2 = 0;
   int mid_sg = 1, out_rg = 1;          // slots per CTA of the mid kernel, routings per pass of the combine
-  int mid_warp_min = INT_MAX;          // routings from which moe_mid_warp_kernel is used (moe_mid_warp_min; INT_MAX: not for these blocks)
+  // routings from which moe_mid_warp_kernel is used, streaming and tensor-core form (moe_mid_warp_min; INT_MAX: not for these blocks)
+  int mid_warp_min = INT_MAX, mid_warp_min_gemm = INT_MAX;
   size_t mid_smem = 0, out_smem = 0;
   // tensor-core form
   bool gemm_ok = false, two_stages = false;
@@ -1227,17 +1228,19 @@ static void moe_launch_group(const MoeDev& M, const void* ids, int tokens, uint8
   moe_place_kernel<<<nb, 1024, 2 * M.E * sizeof(int), st>>>(M, ids, tokens, ws);
 }
 
-// moe_mid_warp_kernel spreads a pair of slots over one warp, moe_mid_kernel some slots' chunks over eight: fewer routings leave
-// the warps too few.  128 experts, top 8, of 2048 x 768, in a graph, by CTAs / by warps: 1 token 88.7 / 102.8 us, 64 tokens
-// 243.1 / 254.9, 256 tokens 239.7 / 243.1, 512 tokens 286.6 / 281.7, 2048 tokens 432 / 418; 32 experts, top 4, 512 tokens 107.7 /
-// 110.7, 1024 tokens 147.7 / 144.5.
-static int moe_mid_warp_min() {
+// moe_mid_warp_kernel works through the chunks of a pair of slots in one warp, moe_mid_kernel spreads those of some slots over
+// eight: the longer that chain, the more routings it takes to fill the SMs in spite of it.  `steps`: chunks that a pair loads.
+// By CTAs / by warps, in a graph.  128 experts, top 8, of 2048 x 768: eight steps (streaming form), 1 token 88.7 / 102.8 us, 64 tokens
+// 243 / 255; five, 256 tokens 239.7 / 243.1, 512 tokens 286.6 / 281.7, 2048 tokens 432 / 418.  Three (32 experts, top 2, of 1024 x 512): 1 token 51.2 /
+// 53.8, 4 tokens 56.1 / 55.2, 64 tokens 59.0 / 57.8; 64 experts, 1024 tokens 94.0 / 92.7.  Five, of which four are partial sums (8
+// experts, top 2, of 2048 x 512): 8 tokens 60.3 / 63.6.
+static int moe_mid_warp_min(int steps) {
   const char* e = getenv("GLQB_MOE_MID_WARP_MIN");
-  return e ? atoi(e) : 4096;
+  return e ? atoi(e) : steps <= 3 ? 8 : 4096;
 }
 static void moe_launch_mid(const GlqbMoePlan* P, const MoeDev& M, int tokens, uint8_t* ws, cudaStream_t st) {
   const int R = tokens * M.top_k;
-  const bool by_warps = R >= P->mid_warp_min;
+  const bool by_warps = R >= (M.gemm ? P->mid_warp_min_gemm : P->mid_warp_min);
   const int per = by_warps ? MIDW_ROWS * MIDW_WARPS : P->mid_sg;
   if (by_warps) moe_mid_warp_kernel<<<(R + per - 1) / per, MIDW_WARPS * 32, MIDW_WARPS * moe_midw_warp_bytes(M.w13_out), st>>>(M, tokens, ws);
   else moe_mid_kernel<<<(R + per - 1) / per, MOE_XF_THREADS, P->mid_smem, st>>>(M, tokens, per, ws);
@@ -1418,7 +1421,11 @@ int glqb_moe_plan_create(const GlqbMoeDesc* d, GlqbMoePlan** out) {
     P->mid_smem = mid_bytes(P->mid_sg);
     bool by_warps = !M.wide_m13 && MIDW_WARPS * moe_midw_warp_bytes(d->w13_out) <= budget;
     for (int b = 0; b < M.nb_n2; ++b) by_warps = by_warps && M.log_n2[b] <= 10;
-    if (by_warps) P->mid_warp_min = moe_mid_warp_min();
+    if (by_warps) {
+      const int c13 = moe_chunks_all(MIDW_ROWS, M.nb_m13, M.log_m13), c2 = moe_chunks_all(MIDW_ROWS, M.nb_n2, M.log_n2);
+      P->mid_warp_min = moe_mid_warp_min(c13 * M.kch13 + c2);
+      P->mid_warp_min_gemm = moe_mid_warp_min(c13 + c2);
+    }
     P->out_smem = out_bytes(P->out_rg);
     if (P->mid_smem > limit || P->out_smem > limit) {
       delete P;
