@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(1024) moe_place_kernel(const __grid_constant__
 __global__ void __launch_bounds__(1024) moe_group_kernel(const __grid_constant__ MoeDev M, const void* __restrict__ ids,
                                                          int T, uint8_t* __restrict__ ws, int phase) {
   extern __shared__ int sh[];            // counts[E], cursor[E], first slot[E], first token tile[E + 1], first row[E], in front[E]
+  pdl_trigger();
   int* cnt = sh;
   int* cur = sh + M.E;
   int* base_s = sh + 2 * M.E;
@@ -433,6 +434,7 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_rht_in_gemm_kernel(cons
                                                                             const uint8_t* __restrict__ x, uint8_t* __restrict__ ws) {
   extern __shared__ __align__(16) float fb[];
   pdl_trigger();
+  pdl_wait();
   const int* slot_of = reinterpret_cast<const int*>(ws + M.o_slot_of);
   const int2* trow = reinterpret_cast<const int2*>(ws + M.o_trow);
   const int kchunks = M.hidden / GM_TILE_K;
@@ -689,6 +691,7 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_mid_kernel(const __grid
                                                                     uint8_t* __restrict__ ws) {
   extern __shared__ __align__(16) float fb[];   // chunks of sg w13 rows, then of sg w2 rows
   pdl_trigger();
+  pdl_wait();
   const int R = T * M.top_k;
   const int* g_count = reinterpret_cast<const int*>(ws + M.o_count);
   const int* g_base = reinterpret_cast<const int*>(ws + M.o_base);
@@ -831,6 +834,7 @@ __global__ void __launch_bounds__(MIDW_WARPS * 32, 4) moe_mid_warp_kernel(const 
                                                                           uint8_t* __restrict__ ws) {
   extern __shared__ __align__(16) uint8_t fb8[];
   pdl_trigger();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int R = T * M.top_k;
   const int used = reinterpret_cast<const int*>(ws + M.o_base)[M.E - 1] + reinterpret_cast<const int*>(ws + M.o_count)[M.E - 1];
@@ -1017,6 +1021,7 @@ __global__ void __launch_bounds__(MOE_XF_THREADS, 3) moe_out_kernel(const __grid
                                                                     const float* __restrict__ topk_w,
                                                                     const uint8_t* __restrict__ ws, uint8_t* __restrict__ y) {
   extern __shared__ __align__(16) float fb[];   // chunks of rg rows of hidden (+ hidden floats when several passes are needed)
+  pdl_wait();
   const int t = blockIdx.x, lane = threadIdx.x & 31;
   const int R = T * M.top_k;
   const int* slot_of = reinterpret_cast<const int*>(ws + M.o_slot_of);
@@ -1203,11 +1208,12 @@ static int fill_blocks(const int32_t* blocks, int nb, int total, int* off, int* 
   return GLQB_OK;
 }
 
-// The two matmuls of trellis experts are chained to the transforms in front of them (launch_chained) in steps of fewer routings.
-// The other launches are not: what starts early holds the registers, and above all the shared memory that is the L1 of the
-// kernels that gather.  In a graph, none / the matmuls / every launch chained: 128 experts, top 8, of 2048 x 768: 16 tokens 179.4 /
-// 178.6 / 184.4 us, 256 tokens 239.7 / 238.2 / 240.9; 32 experts, top 2, of 1024 x 512, 32 tokens 58.2 / 57.6 / 67.6; E8, 32 experts, top 4,
-// of 2048 x 768, 256 tokens 236.5 / 306.9 / 396.1.
+// Steps of fewer routings through trellis experts are chained (launch_chained): every launch of the tensor-core form, whose GEMMs let
+// what follows them start when they end, the two matmuls of the streaming form.  Its other launches, started early, take
+// registers and shared memory from the matmul that they wait for; E8 experts, whose shared memory is the L1 that their gathers
+// live in, are not chained at all.  Eager calls of 128 experts, top 8, of 2048 x 768, 512 tokens, matmuls / every launch 290.8 / 286.0 us, of
+// 64 experts, top 2, of 1024 x 512, 97.4 / 91.5.  In a graph, none / the matmuls / every launch with triggers in all of them: 32 experts,
+// top 2, of 1024 x 512, 32 tokens (streaming) 58.2 / 57.6 / 67.6; E8, 32 experts, top 4, of 2048 x 768, 256 tokens 236.5 / 306.9 / 396.1.
 constexpr long long MOE_CHAIN_MAX = 8192;
 
 // grouping: one launch; count / tables / place kernels (many CTAs) for steps in which counting all routings in every CTA
@@ -1238,12 +1244,12 @@ static int moe_mid_warp_min(int steps) {
   const char* e = getenv("GLQB_MOE_MID_WARP_MIN");
   return e ? atoi(e) : steps <= 3 ? 8 : 4096;
 }
-static void moe_launch_mid(const GlqbMoePlan* P, const MoeDev& M, int tokens, uint8_t* ws, cudaStream_t st) {
+static void moe_launch_mid(const GlqbMoePlan* P, const MoeDev& M, int tokens, uint8_t* ws, bool chain, cudaStream_t st) {
   const int R = tokens * M.top_k;
   const bool by_warps = R >= (M.gemm ? P->mid_warp_min_gemm : P->mid_warp_min);
   const int per = by_warps ? MIDW_ROWS * MIDW_WARPS : P->mid_sg;
-  if (by_warps) moe_mid_warp_kernel<<<(R + per - 1) / per, MIDW_WARPS * 32, MIDW_WARPS * moe_midw_warp_bytes(M.w13_out), st>>>(M, tokens, ws);
-  else moe_mid_kernel<<<(R + per - 1) / per, MOE_XF_THREADS, P->mid_smem, st>>>(M, tokens, per, ws);
+  if (by_warps) launch_chained(chain, moe_mid_warp_kernel, (R + per - 1) / per, MIDW_WARPS * 32, MIDW_WARPS * moe_midw_warp_bytes(M.w13_out), st, M, tokens, ws);
+  else launch_chained(chain, moe_mid_kernel, (R + per - 1) / per, MOE_XF_THREADS, P->mid_smem, st, M, tokens, per, ws);
 }
 
 // tokens per CTA of the input transform: one tile of 8192 values, fewer when that would leave SMs without work
@@ -1484,8 +1490,8 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
     const int R = tokens * G.top_k;
     moe_launch_group(G, topk_ids, tokens, ws, st);
     const int tt = moe_in_tokens(G, tokens);
-    moe_rht_in_gemm_kernel<<<(tokens + tt - 1) / tt, MOE_XF_THREADS, (fht_words(8192) + 2 * tt * G.top_k) * 4, st>>>(
-        G, tokens, tt, reinterpret_cast<const uint8_t*>(x), ws);
+    launch_chained(chain, moe_rht_in_gemm_kernel, (tokens + tt - 1) / tt, MOE_XF_THREADS, (fht_words(8192) + 2 * tt * G.top_k) * 4, st, G, tokens,
+                   tt, reinterpret_cast<const uint8_t*>(x), ws);
     const bool g_e8 = G.format == GLQB_FMT_E8_SHELL;
     const int g_threads = g_e8 ? GM_THREADS : TG_THREADS;
     int* status = reinterpret_cast<int*>(ws + G.o_status);
@@ -1496,14 +1502,15 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
                      reinterpret_cast<const DevLinear*>(ws + G.o_layers13), reinterpret_cast<const GemmItem*>(ws + G.o_items13),
                      G.max_items13, ws, status, nitems, tokens);
     }
-    moe_launch_mid(P, G, tokens, ws, st);
+    moe_launch_mid(P, G, tokens, ws, chain, st);
     {
       MoeTimer t(P, st);
       launch_chained(chain, P->g2, std::min(P->sm_count, G.max_items2), g_threads, moe_gemm_smem_bytes(g_e8), st,
                      reinterpret_cast<const DevLinear*>(ws + G.o_layers2), reinterpret_cast<const GemmItem*>(ws + G.o_items2),
                      G.max_items2, ws, status, nitems + 1, tokens);
     }
-    moe_out_kernel<<<tokens, MOE_XF_THREADS, P->out_smem, st>>>(G, tokens, P->out_rg, topk_weights, ws, reinterpret_cast<uint8_t*>(y));
+    launch_chained(chain, moe_out_kernel, tokens, MOE_XF_THREADS, P->out_smem, st, G, tokens, P->out_rg, topk_weights, ws,
+                   reinterpret_cast<uint8_t*>(y));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return moe_fail(GLQB_E_CUDA, "moe_plan_run: %s", cudaGetErrorString(e));
     return GLQB_OK;
@@ -1529,7 +1536,7 @@ int glqb_moe_plan_run(GlqbMoePlan* P, const void* x, const void* topk_ids, const
     MoeTimer t(P, st);
     launch_chained(chain, P->k13, P->grid13, MV_THREADS, 0, st, A);
   }
-  moe_launch_mid(P, M, tokens, ws, st);
+  moe_launch_mid(P, M, tokens, ws, false, st);
   A.codes[0] = M.w2[0]; A.codes[1] = M.w2[1]; A.stride[0] = M.w2_stride[0]; A.stride[1] = M.w2_stride[1];
   A.inv2 = M.w2_inv2;
   A.row_map = nullptr;
