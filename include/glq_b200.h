@@ -105,7 +105,7 @@ int64_t glqb_plan_flops(const GlqbPlan* plan);
 int32_t glqb_plan_launches(const GlqbPlan* plan);
 /* Enqueue on `stream`; returns without synchronising.  x_base / y_base are device pointers the
  * descriptors' offsets are applied to.  Runs of a plan may overlap (other streams, graph replays) when each has a workspace
- * of its own. */
+ * of its own; a plan keeps a few words per workspace, and every 64th new one may allocate or wait for the device. */
 int glqb_plan_run(GlqbPlan* plan, const void* x_base, void* y_base,
                   void* workspace, size_t workspace_bytes, void* stream);
 /* The same for the first `tokens` tokens (>= 1; layers of fewer take all of theirs): no other row of x is read, no other
